@@ -61,7 +61,7 @@ struct Model {
         bool failed = false;  // capture refused once (an allocation or a synchronisation inside): stay eager
         uint64_t last_use = 0;
     };
-    // on-device sampling: per-row uniform draws (pinned + device) and the [rows, vocab] work area of sample_kernel
+    // on-device sampling: per-row uniform draws (pinned + device) and the [rows, vocab] work area of the sampler (sample.cu)
     float *h_u = nullptr, *d_u = nullptr, *d_samp = nullptr;
     int samp_rows = 0;
     std::vector<DecodeGraph> decode_graphs;
@@ -704,103 +704,12 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
     }
 }
 
-// sampleNextToken on the device (src/main/java/com/veles/llm/jgpt/model/GptAutoregressiveGenerator.java:208-286), one
-// CTA per row, every step of the reference in its own order so that the token is the one the host routine picks:
-// logits / temperature; keep the top_k by (logit descending, index ascending), the rest -inf; maximum;
-// e = (float)exp((double)(z - max)); sum and the running CDF accumulated in fp32 in INDEX order by one thread
-// (a float sum is not associative: a parallel reduction would move CDF boundaries); first index with u <= cdf,
-// else the last one.  The uniform draw u is supplied per row (the reference draws from an unseeded
-// ThreadLocalRandom).
-__global__ void __launch_bounds__(256) sample_kernel(const float *__restrict__ logits, float *__restrict__ work, int V, float temperature,
-                                                     int top_k, const float *__restrict__ u01, int *__restrict__ out) {
-    __shared__ float bv[8];
-    __shared__ int bi[8];
-    __shared__ float s_thr_v, s_mx;
-    __shared__ int s_thr_i;
-    const float *row = logits + (size_t)blockIdx.x * V;
-    float *z = work + (size_t)blockIdx.x * V;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < V; i += 256) z[i] = temperature != 1.0f ? row[i] / temperature : row[i];
-    __syncthreads();
-    // block-wide "best" by (value descending, index ascending) among elements strictly after (pv, pi) in that order
-    auto next_best = [&](float pv, int pi, bool first) {
-        float best = -INFINITY;
-        int idx = 0x7fffffff;
-        for (int i = tid; i < V; i += 256) {
-            const float v = z[i];
-            const bool eligible = first || v < pv || (v == pv && i > pi);
-            if (eligible && (v > best || (v == best && i < idx) || idx == 0x7fffffff)) best = v, idx = i;
-        }
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-            if (oi != 0x7fffffff && (idx == 0x7fffffff || ov > best || (ov == best && oi < idx))) best = ov, idx = oi;
-        }
-        if (lane == 0) bv[warp] = best, bi[warp] = idx;
-        __syncthreads();
-        if (tid == 0) {
-            for (int w = 1; w < 8; w++)
-                if (bi[w] != 0x7fffffff && (idx == 0x7fffffff || bv[w] > best || (bv[w] == best && bi[w] < idx))) best = bv[w], idx = bi[w];
-            s_thr_v = best, s_thr_i = idx;
-        }
-        __syncthreads();
-    };
-    if (top_k > 0 && top_k < V) {
-        next_best(0.f, 0, true);
-        for (int r = 1; r < top_k; r++) next_best(s_thr_v, s_thr_i, false);
-        const float tv = s_thr_v;
-        const int ti = s_thr_i;  // the top_k-th element: everything after it in the order is dropped
-        for (int i = tid; i < V; i += 256) {
-            const float v = z[i];
-            if (v < tv || (v == tv && i > ti)) z[i] = -INFINITY;
-        }
-        __syncthreads();
-    }
-    float mx = -INFINITY;
-    for (int i = tid; i < V; i += 256) mx = fmaxf(mx, z[i]);
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if (lane == 0) bv[warp] = mx;
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < 8; w++) mx = fmaxf(mx, bv[w]);
-        s_mx = mx;
-    }
-    __syncthreads();
-    mx = s_mx;
-    for (int i = tid; i < V; i += 256) z[i] = (float)exp((double)(z[i] - mx));
-    __syncthreads();
-    if (tid == 0) {
-        float sum = 0.f;
-        for (int i = 0; i < V; i++) sum += z[i];
-        const float u = u01[blockIdx.x];
-        float cum = 0.f;
-        int tok = V - 1;
-        for (int i = 0; i < V; i++) {
-            cum += z[i] / sum;
-            if (u <= cum) {
-                tok = i;
-                break;
-            }
-        }
-        out[blockIdx.x] = tok;
-    }
-}
-
 // The token choice for models that run their own forward step (decoder.cu).
 int32_t launch_argmax(const float *logits, int rows, int vocab, int *next_dev, cudaStream_t st) {
     argmax_kernel<<<rows, 256, 0, st>>>(logits, vocab, next_dev);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t launch_sample(const float *logits, float *work, int rows, int vocab, const SampleSpec &spec, const float *u01_dev, int *next_dev,
-                      cudaStream_t st) {
-    sample_kernel<<<rows, 256, 0, st>>>(logits, work, vocab, spec.temperature, spec.top_k, u01_dev, next_dev);
-    JGPT_CUDA_TRY(cudaGetLastError());
-    return JGPT_OK;
-}
-
 // ------------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------------
@@ -1276,7 +1185,7 @@ static int32_t lm_head(Model *m, int rows, int n_sel, const SampleSpec &spec = S
     if (spec.temperature > 0.f) {  // the draws are in m->d_u (uploaded by the caller)
         rc = ensure_sample_work(m, out_rows);
         if (rc) return rc;
-        sample_kernel<<<out_rows, 256, 0, st>>>(m->logits, m->d_samp, m->vocab, spec.temperature, spec.top_k, m->d_u, m->d_next);
+        if ((rc = launch_sample(m->logits, m->d_samp, out_rows, m->vocab, spec, m->d_u, m->d_next, st))) return rc;
     } else {
         if (to_host && early && small_mode(m, rows)) {  // moves in under the LM head's last CTAs
             cudaLaunchConfig_t cfg = {};
@@ -1986,10 +1895,7 @@ static int32_t forward_decode_impl(jgpt_model h, jgpt_kvpool poolh, const int32_
         } else if (rc) {
             return rc;
         } else {
-            if (sampled) {
-                sample_kernel<<<n, 256, 0, st>>>(m->logits, m->d_samp, m->vocab, spec.temperature, spec.top_k, m->d_u, m->d_next);
-                JGPT_CUDA_TRY(cudaGetLastError());
-            }
+            if (sampled && (rc = launch_sample(m->logits, m->d_samp, n, m->vocab, spec, m->d_u, m->d_next, st))) return rc;
             if (form == 2 || sampled) JGPT_CUDA_TRY(cudaMemcpyAsync(m->h_next, m->d_next, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, st));
             JGPT_CUDA_TRY(status_enqueue_read(m->ctx));
             one_launch = true;

@@ -381,6 +381,35 @@ def test_device_sampler_picks_the_oracles_token(ctx):
         pool_s.close(), pool_l.close(), gm.close(), om.close()
 
 
+@pytest.mark.parametrize("vocab", [5, 33, 1000, 8000, 50004])
+def test_device_sampler_over_vocabularies_and_ties(ctx, vocab):
+    """Rows shorter than a warp, ragged over the sampler's warps, with more kept elements than its list holds, and too long for
+    shared memory; columns of the output matrix repeat, so that equal logits lie on both sides of the top-k boundary."""
+    MS, D = 64, 64
+    rng = np.random.default_rng(vocab)
+    gm = GPTModel(ctx, vocab, MS, D, 4, 1, 128, rmsNormEps=1e-5, maxRows=64)
+    om = O.Model(vocab, MS, D, 4, 1, 128, eps=1e-5).init_random(seed=3, std=0.3)
+    tensors = om.tensors()
+    tensors[-1] = np.ascontiguousarray(tensors[-1][:, np.arange(vocab) % max(2, vocab // 3)])
+    gm.setParameters(tensors)
+    pool_s, pool_l = gm.newPool(8, 2), gm.newPool(8, 2)
+    try:
+        seqs = [[pool.seq_alloc() for _ in range(2)] for pool in (pool_s, pool_l)]
+        lens = np.zeros(2, np.int32)
+        ids = np.array([1, 3], np.int32)
+        for k in (0, 1, 2, 7, 40, 1023, 1024, 1025, 2000, vocab - 1, vocab, vocab + 1):
+            u = rng.random(2).astype(np.float32) if k != 7 else np.array([0.0, 1.0], np.float32)
+            temp = float(rng.choice([0.3, 1.0, 1.7]))
+            logits, _ = gm.forwardDecodeBatch(pool_l, seqs[1], ids, lens, lens)
+            got = gm.forwardDecodeSampleBatch(pool_s, seqs[0], ids, lens, lens, temp, k, u)
+            assert list(got) == [gm.sampleNextToken(logits[i], temp, k, float(u[i])) for i in range(2)], (k, temp, u)
+            assert len(np.unique(logits[0])) < vocab
+            lens += 1
+            ids = rng.integers(0, vocab, 2).astype(np.int32)
+    finally:
+        pool_s.close(), pool_l.close(), gm.close(), om.close()
+
+
 def test_forward_step_reports_a_failed_device_self_check_itself(ctx, small16):
     """A corrupted block-table entry (-1 where the step reads or appends) must come back as an error from the
     forward call itself -- no jgpt_sync needed, no tokens, no length change -- and the pool must stay usable:
