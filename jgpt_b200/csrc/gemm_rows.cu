@@ -1,0 +1,320 @@
+// Products of few rows with fp32-level accuracy: the projections of a decode step and of a short prompt.
+//
+// At these sizes a product is not bound by bytes or by the tensor cores but by its longest chain: wait for the previous kernel, fetch
+// the rows, multiply, add the k slices, store.  So everything that does not depend on the previous kernel is done before the wait and
+// nothing in the loop meets at a barrier.  A CTA owns 16 or 32 columns; its eight warps split k, and a warp holds the weights of
+// its k slice in registers, in the order the tensor core reads them (one 16-byte load per 8 columns, 16 k and lane, out of an image
+// built once per weight set): requested before the wait, used for every row tile the CTA walks.  A warp fetches its own k slice of
+// 16 rows with cp.async, the next tile's while this one is multiplied; the only barrier of a row tile is the one in front of the sum
+// over the eight slices.
+//
+// Accuracy: an fp32 operand is an fp16 high and an fp16 low part, 11 + 11 bits as the TF32 pair has, at half the tensor time (m16n8k16
+// instead of two m16n8k8) and, for the weights, in the four bytes of the original.  fp16's narrow exponent is dealt with by powers of
+// two, which change no bit: weights are scaled per column (image), rows per warp and row tile from the largest element of the slice,
+// and the partial sums are scaled back before they are added.  An element 2^18 below the largest of its slice keeps all 22 bits,
+// below that an absolute error of 2^-40 of the largest remains.  Products high x high in one accumulator, the two mixed ones in another.
+//
+// Against the form with shared-memory k tiles, TF32 pairs split in the loop and a barrier per 64 k (12 layers of 384, per launch inside
+// a decode step of 64 rows, from the previous kernel's end to its own): Q,K,V 5.2 -> 3.6, Wo 4.1 -> 2.3, W1/W3 7.0 -> 4.0, W2 6.6 -> 3.0 us;
+// per step: 8 rows 0.32 -> 0.27, 64 rows 0.45 -> 0.38, 250 rows 1.37 -> 1.24 ms; a prompt of 201 tokens 0.72 -> 0.59 ms.  Error against
+// float64 of the LM head's 384 x 8000 product: 1.5e-7 of the result (2-norm), 1.8e-7 with TF32 pairs.
+#include "gemm_rows.cuh"
+
+#include <algorithm>
+
+#include "ptx.cuh"
+
+namespace jgpt {
+namespace rows {
+
+constexpr int kWarps = 8, kThreads = 256, kRows = 16;
+
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h), lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+// One CTA per 8 columns: a warp per column finds its largest element, then every lane writes its 16 bytes per 16 k.  Inside 16 k the
+// tensor core's positions 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of lane t hold k = 4 t .. 4 t + 3, so that a row's four elements are one load.
+__global__ void __launch_bounds__(256) pack_kernel(const float *W, const float *W3, const float *gamma, int K, int N, uint4 *image, float *unscale) {
+    __shared__ float s_scale[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto element = [&](int k, int n) {
+        if (k >= K || n >= N) return 0.f;
+        float w;
+        if (W3) {
+            const int col = (n >> 5) * 16 + (n & 15);
+            w = (n & 16 ? W3 : W)[(size_t)k * (N / 2) + col];
+        } else {
+            w = W[(size_t)k * N + n];
+        }
+        return gamma ? gamma[k] * w : w;
+    };
+    const int n0 = blockIdx.x * 8;
+    float mx = 0.f;
+    for (int k = lane; k < K; k += 32) mx = fmaxf(mx, fabsf(element(k, n0 + warp)));
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    if (lane == 0) {
+        float s, inv;
+        pow2_scale(mx, s, inv);
+        s_scale[warp] = s;
+        unscale[n0 + warp] = inv;
+    }
+    __syncthreads();
+    const int steps = (K + 15) / 16, g = lane >> 2, t = lane & 3;
+    const float s = s_scale[g];
+    for (int step = warp; step < steps; step += kWarps) {
+        const int k = step * 16 + 4 * t;
+        uint4 o;
+        split_pair(element(k, n0 + g) * s, element(k + 1, n0 + g) * s, o.x, o.z);
+        split_pair(element(k + 2, n0 + g) * s, element(k + 3, n0 + g) * s, o.y, o.w);
+        image[((size_t)blockIdx.x * steps + step) * 32 + lane] = o;
+    }
+}
+
+int32_t pack(const float *W, const float *W3, const float *gamma, int K, int N, void *image, cudaStream_t st) {
+    const unsigned tiles = (unsigned)((N + 7) / 8);
+    uint4 *im = static_cast<uint4 *>(image);
+    pack_kernel<<<tiles, 256, 0, st>>>(W, W3, gamma, K, N, im, reinterpret_cast<float *>(im + (size_t)tiles * k_steps(K) * 32));
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+
+// S: steps of 16 k per warp.  NT: column groups of 8 per CTA.
+template <int S>
+__host__ __device__ constexpr int slice_stride() { return S * 16 + 16; }  // floats: eight rows' chunks fall into different banks
+template <int S>
+constexpr size_t slice_bytes() { return sizeof(float) * kWarps * kRows * (size_t)slice_stride<S>(); }
+
+// CTAs of a kernel on an SM: two while 128 registers hold the weights, the rows and the sums.
+template <int S, int NT>
+constexpr int per_sm() { return S * NT <= 12 && S <= 4 ? 2 : 1; }
+
+template <int S, int NT, int KIND>
+__global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(const float *A, const Batch B, int M, int K, int N, const int *rowsel,
+                                                                                  const Fuse F, int two_tiles) {
+    constexpr int BN = NT * 8, AS = slice_stride<S>(), RS = BN + 8;
+    constexpr int OUT = KIND == NORM_SWIGLU ? BN / 2 : BN;  // columns of the result per CTA
+    constexpr int PER = kRows * OUT / kThreads;             // of them per thread: columns fixed, rows row0 + i * kThreads / OUT
+    static_assert(PER >= 1 && (KIND != NORM_SWIGLU || NT == 4), "tile");
+    extern __shared__ __align__(16) float rows_smem[];
+    __shared__ __align__(16) float red[2][kWarps][kRows][RS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int z = blockIdx.z;
+#ifdef JGPT_B200_DECODE_TRACE
+    timeline_in(F.timeline);
+#endif
+    const int steps = (K + 15) / 16, tiles = (N + 7) / 8;
+    const uint4 *image = static_cast<const uint4 *>(z == 0 ? B.image[0] : (z == 1 ? B.image[1] : B.image[2]));
+    float *C = z == 0 ? B.C[0] : (z == 1 ? B.C[1] : B.C[2]);
+    const float *unscale = reinterpret_cast<const float *>(image + (size_t)tiles * steps * 32);
+    const int step0 = warp * S, k0 = step0 * 16;
+    uint4 w[S][NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            const int tile = blockIdx.x * NT + j;
+            w[s][j] = (tile < tiles && step0 + s < steps) ? __ldg(image + ((size_t)tile * steps + step0 + s) * 32 + lane) : make_uint4(0, 0, 0, 0);
+        }
+    const int oc = tid % OUT, row0 = tid / OUT, col = blockIdx.x * OUT + oc, Nout = KIND == NORM_SWIGLU ? N / 2 : N;
+    const bool col_ok = col < Nout;
+    const int wcol = KIND == NORM_SWIGLU ? blockIdx.x * BN + oc : col;
+    const float un0 = col_ok ? __ldg(unscale + wcol) : 0.f, un1 = (KIND == NORM_SWIGLU && col_ok) ? __ldg(unscale + wcol + 16) : 0.f;
+
+    if (F.pdl & 1) griddep_wait();
+#ifdef JGPT_B200_DECODE_TRACE
+    timeline_at(F.timeline, 1);
+#endif
+    if (F.pdl & 2) griddep_launch_dependents();
+
+    // this warp's k slice of 16 rows; rows and k past the end become zeros
+    float *ring = rows_smem + (size_t)warp * kRows * AS;
+    constexpr size_t kBuf = (size_t)kWarps * kRows * AS;
+    auto fetch = [&](int rt, int buf) {
+#pragma unroll
+        for (int i = 0; i < 2 * S; i++) {
+            const int c = lane + 32 * i, r = c / (4 * S), q = (c % (4 * S)) * 4, m = rt * kRows + r;
+            const bool ok = m < M && k0 + q < K;
+            const int src = ok ? (rowsel ? rowsel[m] : m) : 0;
+            cp_async16(ring + buf * kBuf + r * AS + q, A + (size_t)src * K + (ok ? k0 + q : 0), ok);
+        }
+    };
+    const int row_tiles = (M + kRows - 1) / kRows;
+    int rt = blockIdx.y, buf = 0, rb = 0;
+    fetch(rt, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (; rt < row_tiles; rt += gridDim.y) {
+        if (two_tiles && rt + (int)gridDim.y < row_tiles) fetch(rt + gridDim.y, buf ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        // what the epilogue adds or multiplies, requested now
+        float extra[PER];
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int m = rt * kRows + row0 + i * (kThreads / OUT);
+            extra[i] = 0.f;
+            if (KIND == RESIDUAL) {
+                if (m < M && col_ok) extra[i] = C[(size_t)m * N + col];
+            } else if (m < M) {  // the lanes that share a row add its partial sums of squares, always in the same order
+                const float *pp = F.ss_in + (size_t)(rowsel ? rowsel[m] : m) * F.parts_in;
+                for (int p = oc; p < F.parts_in; p += OUT) extra[i] += pp[p];
+            }
+        }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        float4 lo_row[S], hi_row[S];
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            lo_row[s] = *reinterpret_cast<const float4 *>(ring + buf * kBuf + g * AS + s * 16 + 4 * t);
+            hi_row[s] = *reinterpret_cast<const float4 *>(ring + buf * kBuf + (g + 8) * AS + s * 16 + 4 * t);
+        }
+        float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            m0 = fmaxf(m0, fmaxf(fmaxf(fabsf(lo_row[s].x), fabsf(lo_row[s].y)), fmaxf(fabsf(lo_row[s].z), fabsf(lo_row[s].w))));
+            m1 = fmaxf(m1, fmaxf(fmaxf(fabsf(hi_row[s].x), fabsf(hi_row[s].y)), fmaxf(fabsf(hi_row[s].z), fabsf(hi_row[s].w))));
+        }
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1)), m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 1));
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 2)), m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 2));
+        float s0, s1, u0, u1;
+        pow2_scale(m0, s0, u0), pow2_scale(m1, s1, u1);
+        float acc[NT][4], cor[NT][4];
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[j][e] = 0.f, cor[j][e] = 0.f;
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            uint32_t ah[4], al[4];
+            split_pair(lo_row[s].x * s0, lo_row[s].y * s0, ah[0], al[0]);
+            split_pair(hi_row[s].x * s1, hi_row[s].y * s1, ah[1], al[1]);
+            split_pair(lo_row[s].z * s0, lo_row[s].w * s0, ah[2], al[2]);
+            split_pair(hi_row[s].z * s1, hi_row[s].w * s1, ah[3], al[3]);
+#pragma unroll
+            for (int j = 0; j < NT; j++) mma_16816(acc[j], ah, w[s][j].x, w[s][j].y);
+#pragma unroll
+            for (int j = 0; j < NT; j++) mma_16816(cor[j], al, w[s][j].x, w[s][j].y);
+#pragma unroll
+            for (int j = 0; j < NT; j++) mma_16816(cor[j], ah, w[s][j].z, w[s][j].w);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            *reinterpret_cast<float2 *>(&red[rb][warp][g][j * 8 + 2 * t]) = make_float2((acc[j][0] + cor[j][0]) * u0, (acc[j][1] + cor[j][1]) * u0);
+            *reinterpret_cast<float2 *>(&red[rb][warp][g + 8][j * 8 + 2 * t]) = make_float2((acc[j][2] + cor[j][2]) * u1, (acc[j][3] + cor[j][3]) * u1);
+        }
+        // the buffer of slices written here is rewritten two tiles later, behind the next tile's barrier
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int r = row0 + i * (kThreads / OUT), m = rt * kRows + r;
+            float v = 0.f, v2 = 0.f;
+#pragma unroll
+            for (int q = kWarps - 1; q >= 0; q--) {
+                v += red[rb][q][r][oc];
+                if (KIND == NORM_SWIGLU) v2 += red[rb][q][r][oc + 16];
+            }
+            v *= un0;
+            if (KIND == RESIDUAL) {
+                v = extra[i] + v;
+                const bool ok = m < M && col_ok;
+                if (ok) C[(size_t)m * N + col] = v;
+                float sq = ok ? v * v : 0.f;
+#pragma unroll
+                for (int off = OUT / 2; off >= 1; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+                if (oc == 0 && m < M) F.ss_out[(size_t)m * gridDim.x + blockIdx.x] = sq;
+            } else {
+                float tot = extra[i];
+#pragma unroll
+                for (int off = OUT / 2; off >= 1; off >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, off);
+                const float rms = sqrtf(tot / (float)K + F.eps);
+                const float inv = (rms > 0.f && isfinite(rms)) ? (1.f / rms) : 0.f;
+                v *= inv;
+                if (KIND == NORM_SWIGLU) {
+                    v2 *= un1;
+                    v2 *= inv;
+                    float sg;
+                    if (v2 >= 20.f) sg = 1.f;
+                    else if (v2 <= -20.f) sg = 0.f;
+                    else sg = 1.f / (1.f + expf(-v2));
+                    v = v * (v2 * sg);
+                }
+                if (m < M && col_ok) C[(size_t)m * Nout + col] = v;
+            }
+        }
+        buf ^= two_tiles, rb ^= 1;
+    }
+#ifdef JGPT_B200_DECODE_TRACE
+    timeline_at(F.timeline, 2);
+#endif
+}
+
+constexpr int kMaxSteps32 = 4, kMaxSteps16 = 8;  // steps of 16 k per warp whose weights fit: 64 registers either way
+constexpr size_t kSoloBytes = 115 * 1024;        // static and dynamic: more than half an SM, no two CTAs of the launch share one
+
+bool shape_ok(Kind kind, int K) {
+    const int s = (k_steps(K) + kWarps - 1) / kWarps;
+    return K % 4 == 0 && k_steps(K) >= kWarps && s <= (kind == RESIDUAL ? kMaxSteps16 : kMaxSteps32);
+}
+
+template <int S, int NT, int KIND>
+static int32_t launch_t(Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse) {
+    auto *kernel = gemm_rows_kernel<S, NT, KIND>;
+    constexpr size_t fixed = sizeof(float) * 2 * kWarps * kRows * (NT * 8 + 8);
+    constexpr size_t most = std::max(2 * slice_bytes<S>(), kSoloBytes - fixed);
+    static bool opted[64] = {};
+    if (!opted[ctx->device & 63]) {
+        JGPT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        opted[ctx->device & 63] = true;
+    }
+    // As many row groups as stay resident at once, every one with the same number of row tiles where that goes: a CTA keeps its weights
+    // over its row tiles, and a second round of CTAs would fetch theirs behind the wait.
+    const int cols = (N + NT * 8 - 1) / (NT * 8) * nb, row_tiles = (M + kRows - 1) / kRows;
+    static_assert(per_sm<S, NT>() * (2 * slice_bytes<S>() + fixed + 1024) <= 228 * 1024, "shared memory");
+    int groups = std::min(row_tiles, std::max(1, per_sm<S, NT>() * ctx->sm_count / cols));
+    const int per_group = (row_tiles + groups - 1) / groups;
+    groups = (row_tiles + per_group - 1) / per_group;
+    size_t smem = (per_group > 1 ? 2 : 1) * slice_bytes<S>();
+    // A launch of at most one CTA per SM that moves in early, while the previous kernel holds most SMs, would be packed onto the few
+    // with room.  More than this and the attention's CTAs could not move in beside it in turn.
+    if ((fuse.pdl & 1) && cols * groups <= ctx->sm_count) smem = std::max(smem, kSoloBytes - fixed);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)(cols / nb), (unsigned)groups, (unsigned)nb), cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem, cfg.stream = ctx->stream, cfg.attrs = attr, cfg.numAttrs = fuse.pdl & 1;
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, b, M, K, N, rowsel, fuse, per_group > 1 ? 1 : 0));
+    return JGPT_OK;
+}
+
+template <int NT, int KIND, int MAX>
+static int32_t launch_s(int s, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse) {
+    if (s <= 1) return launch_t<1, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if (s <= 2) return launch_t<2, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if (s <= 3) return launch_t<3, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if (s <= 4) return launch_t<4, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if constexpr (MAX > 4) {
+        if (s <= 6) return launch_t<6, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+        return launch_t<8, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+    }
+    return fail(JGPT_ERR_UNSUPPORTED, "gemm_rows: K=%d", K);
+}
+
+int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse_in) {
+    JGPT_REQUIRE(shape_ok(kind, K) && M > 0 && nb >= 1 && nb <= 3 && (kind != NORM_SWIGLU || N % 32 == 0), JGPT_ERR_UNSUPPORTED,
+                 "gemm_rows: unsupported shape M=%d K=%d N=%d", M, K, N);
+    Fuse fuse = fuse_in;
+#ifdef JGPT_B200_DECODE_TRACE
+    fuse.timeline = timeline_next();
+#endif
+    const int s = (k_steps(K) + kWarps - 1) / kWarps;
+    if (kind == NORM) return launch_s<4, NORM, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if (kind == NORM_SWIGLU) return launch_s<4, NORM_SWIGLU, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
+    return launch_s<2, RESIDUAL, kMaxSteps16>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
+}
+
+}  // namespace rows
+}  // namespace jgpt

@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "ptx.cuh"
 #include "decoder.cuh"
+#include "gemm_rows.cuh"
 #include "gemm_umma.cuh"
 
 #include <algorithm>
@@ -46,7 +47,9 @@ struct Model {
     float *aimg = nullptr, *aimg2 = nullptr;  // activation images (grow-only): [rows, d_model]-sized and [rows, d_ff]-sized
     uint64_t aimg_floats = 0, aimg2_floats = 0;
     // Decode-sized steps (rows <= 512): RMSNorm and SwiGLU live inside the projections.
-    float *ss_a = nullptr, *ss_b = nullptr;           // [max_rows][ceil(d_model / 32)] partial row sums of squares of x
+    float *ss_a = nullptr, *ss_b = nullptr;           // [max_rows][ceil(d_model / 16)] partial row sums of squares of x
+    int x_parts = 1;                                  // partials per row that the last layer of the step being enqueued leaves in ss_a
+    std::unordered_map<const float *, void *> wrows;  // images of gemm_rows.cu by the weights' pointer (W1's for a pair); dropped when weights change
     std::unordered_map<const float *, float *> w13i;  // interleaved W1/W3 pairs by W1's pointer; dropped when weights change
     std::unordered_map<const float *, float *> wscaled;  // weights with row k scaled by the preceding norm's gamma[k] (decode-sized steps), by the weights' pointer
     // Decode steps replayed as CUDA graphs (JGPT_B200_DECODE_GRAPH=0 turns it off).  A step's launches depend on
@@ -104,7 +107,8 @@ static void drop_weight_images(Model *m) {
     for (auto &kv : m->wpair) cudaFree(kv.second);
     for (auto &kv : m->w13i) cudaFree(kv.second);
     for (auto &kv : m->wscaled) cudaFree(kv.second);
-    m->wimg.clear(), m->wpair.clear(), m->w13i.clear(), m->wscaled.clear();
+    for (auto &kv : m->wrows) cudaFree(kv.second);
+    m->wimg.clear(), m->wpair.clear(), m->w13i.clear(), m->wscaled.clear(), m->wrows.clear();
 }
 
 Registry<Model> &model_registry() {
@@ -1125,9 +1129,81 @@ static int32_t run_layers_small(Model *m, int rows, AttnFn &&attn) {
     return JGPT_OK;
 }
 
+// Decode-sized steps of models whose weights fit the registers of gemm_rows.cu (d_model 116 to 512, d_ff up to 1024).
+static bool rows_mode(const Model *m, int n) {
+    return small_mode(m, n) && rows::shape_ok(rows::NORM, m->d_model) && rows::shape_ok(rows::RESIDUAL, m->d_ff);
+}
+// The image of W [K, N] (with W3: of the alternating pair, N columns together), built once per weight set.  *fresh: just written by a
+// kernel on this stream, so the launch that reads it must not run ahead of its wait.
+static int32_t rows_image(Model *m, const float *W, const float *W3, const float *gamma, int K, int N, const void **out, bool *fresh) {
+    auto it = m->wrows.find(W);
+    if (it == m->wrows.end()) {
+        void *buf = nullptr;
+        JGPT_CUDA_TRY(cudaMalloc(&buf, rows::image_bytes(K, N)));
+        it = m->wrows.emplace(W, buf).first;
+        int32_t rc = rows::pack(W, W3, gamma, K, N, buf, m->ctx->stream);
+        if (rc) return rc;
+        *fresh = true;
+    }
+    *out = it->second;
+    return JGPT_OK;
+}
+template <class AttnFn>
+static int32_t run_layers_rows(Model *m, int n, AttnFn &&attn) {
+#ifdef JGPT_B200_DECODE_TRACE
+    g_timeline_slot = 0;
+#endif
+    const int D = m->d_model, F = m->d_ff, ov = step_overlap_level(m, n);
+    int32_t rc;
+    // wait: this launch may move in early; next: it lets its successor do so (levels as in run_layers_small)
+    auto fuse = [&](const float *ss_in, float *ss_out, int parts, bool wait, bool next) {
+        rows::Fuse f;
+        f.ss_in = ss_in, f.ss_out = ss_out, f.parts_in = parts, f.eps = m->eps, f.pdl = (wait ? 1 : 0) | (next ? 2 : 0);
+        return f;
+    };
+    // x += A W, with the row sums of squares; returns how many partials a row has.  JGPT_B200_K_SPLIT=0 keeps the shared-memory form,
+    // one CTA per output tile, where that form would otherwise split k over pairs of CTAs.
+    const bool tiles = !m->k_split && 2 * ((D + 31) / 32) * ((n + 15) / 16) <= m->ctx->sm_count;
+    int parts = 1;  // x's sums of squares: one partial per row from the embedding
+    auto residual = [&](const float *A, const float *W, int K, float *ss, bool wait) -> int32_t {
+        int32_t r2;
+        if (tiles) {
+            const float *Wt[1] = {W}, *Rx[1] = {m->x};
+            float *Cx[1] = {m->x};
+            parts = (D + 31) / 32;
+            return small_launch<false, 1>(m, A, n, K, D, 1, Wt, Cx, Rx, nullptr, SmallFuse{nullptr, nullptr, ss, 0, 0.f, (wait ? 1 : 0) | (ov >= 3 ? 2 : 0)});
+        }
+        rows::Batch b{{nullptr}, {m->x}};
+        bool fresh = false;
+        parts = rows::ss_parts(D);
+        if ((r2 = rows_image(m, W, nullptr, nullptr, K, D, &b.image[0], &fresh))) return r2;
+        return rows::launch(rows::RESIDUAL, m->ctx, A, b, 1, n, K, D, nullptr, fuse(nullptr, ss, 0, wait && !fresh, ov >= 3));
+    };
+    for (int l = 0; l < m->layers; l++) {
+        const LayerW &y = m->L[(size_t)l];
+        bool fresh = false;
+        rows::Batch qkv{{nullptr, nullptr, nullptr}, {m->q, m->k, m->v}};
+        const float *w[3] = {y.wq, y.wk, y.wv};
+        for (int z = 0; z < 3; z++)
+            if ((rc = rows_image(m, w[z], nullptr, y.norm1, D, D, &qkv.image[z], &fresh))) return rc;
+        if ((rc = rows::launch(rows::NORM, m->ctx, m->x, qkv, 3, n, D, D, nullptr,
+                               fuse(m->ss_a, nullptr, parts, ov >= 3 && (l > 0 || m->first_launch_early) && !fresh, ov >= 1)))) return rc;
+        if ((rc = attn(l, nullptr, false))) return rc;
+        if ((rc = residual(m->att, y.wo, D, m->ss_b, ov >= 2))) return rc;
+        rows::Batch w13{{nullptr}, {m->h1}};
+        fresh = false;
+        if ((rc = rows_image(m, y.w1, y.w3, y.norm2, D, 2 * F, &w13.image[0], &fresh))) return rc;
+        if ((rc = rows::launch(rows::NORM_SWIGLU, m->ctx, m->x, w13, 1, n, D, 2 * F, nullptr, fuse(m->ss_b, nullptr, parts, ov >= 3 && !fresh, ov >= 3)))) return rc;
+        if ((rc = residual(m->h1, y.w2, F, m->ss_a, ov >= 3))) return rc;
+    }
+    m->x_parts = parts;
+    return JGPT_OK;
+}
+
 template <class AttnFn>
 static int32_t run_layers(Model *m, int rows, const PagedAppendArgs *paged, AttnFn &&attn) {
     const int D = m->d_model, F = m->d_ff;
+    if (rows_mode(m, rows)) return run_layers_rows(m, rows, attn);
     if (small_mode(m, rows)) return run_layers_small(m, rows, attn);
     if (!m->strict && m->umma_min_rows > 0 && rows >= m->umma_min_rows && umma::shape_ok(D, D) && umma::shape_ok(D, F) &&
         umma::shape_ok(F, D) && sizeof(float) * 8 * (size_t)(D + 4) <= 48 * 1024)
@@ -1172,7 +1248,14 @@ static int32_t lm_head(Model *m, int rows, int n_sel, const SampleSpec &spec = S
     const float *W[1] = {m->lm_head};
     float *C[1] = {m->logits};
     const int *rowsel = n_sel > 0 ? m->d_rowsel : nullptr;
-    if (small_mode(m, rows)) {  // the last W2 projection left the row sums of squares in ss_a
+    if (rows_mode(m, rows)) {  // the last W2 product left the row sums of squares in ss_a
+        bool fresh = false;
+        rows::Batch b{{nullptr}, {m->logits}};
+        if ((rc = rows_image(m, m->lm_head, nullptr, m->norm_final, D, m->vocab, &b.image[0], &fresh))) return rc;
+        rows::Fuse f;
+        f.ss_in = m->ss_a, f.parts_in = m->x_parts, f.eps = m->eps, f.pdl = early ? (fresh ? 2 : 3) : 0;
+        rc = rows::launch(rows::NORM, m->ctx, m->x, b, 1, out_rows, D, m->vocab, rowsel, f);
+    } else if (small_mode(m, rows)) {
         bool fresh = false;
         if ((rc = scaled_weight(m, m->lm_head, m->norm_final, D, m->vocab, &W[0], &fresh))) return rc;
         rc = small_launch<true, 0>(m, m->x, out_rows, D, m->vocab, 1, W, C, nullptr, rowsel,
@@ -1517,8 +1600,8 @@ int32_t jgpt_model_create(jgpt_ctx ctxh, int32_t vocab, int32_t max_seq_len, int
     JGPT_CUDA_TRY(cudaMalloc(&m->d_rowsel, sizeof(int) * R));
     JGPT_CUDA_TRY(cudaHostAlloc(&m->h_u, sizeof(float) * R, cudaHostAllocDefault));
     JGPT_CUDA_TRY(A(&m->d_u, R));
-    JGPT_CUDA_TRY(A(&m->ss_a, R * ((D + 31) / 32)));
-    JGPT_CUDA_TRY(A(&m->ss_b, R * ((D + 31) / 32)));
+    JGPT_CUDA_TRY(A(&m->ss_a, R * rows::ss_parts((int)D)));
+    JGPT_CUDA_TRY(A(&m->ss_b, R * rows::ss_parts((int)D)));
     *out = model_registry().add(m);
     return JGPT_OK;
 }

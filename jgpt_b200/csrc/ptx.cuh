@@ -114,6 +114,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// The power of two that brings values whose largest magnitude is mx to [2^14, 2^15) and its inverse, both normal numbers: 0 and
+// subnormal ones get the largest factor, an infinite or NaN one a small one (the parts become inf and NaN, and so do the sums).
+__device__ __forceinline__ void pow2_scale(float mx, float &s, float &inv) {
+    const int e = (int)(__float_as_uint(mx) >> 23);  // mx >= 0
+    const int f = min(268 - e, 253);
+    s = __uint_as_float((uint32_t)f << 23), inv = __uint_as_float((uint32_t)(254 - f) << 23);
+}
+
 // Four 8x8 b16 matrices from shared memory; lane l supplies the address of row (l % 8) of matrix (l / 8).
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void *smem_row) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"

@@ -410,6 +410,57 @@ def test_device_sampler_over_vocabularies_and_ties(ctx, vocab):
         pool_s.close(), pool_l.close(), gm.close(), om.close()
 
 
+@pytest.mark.parametrize("dm,dff,rows", [(128, 112, 5), (144, 1024, 17), (384, 768, 16), (384, 768, 33), (512, 272, 300), (320, 896, 130)])
+@pytest.mark.parametrize("spread", [0.0, 5.0])
+def test_products_of_few_rows_against_float64(ctx, dm, dff, rows, spread):
+    """One block whose attention adds nothing (Wo = 0), so that logits are norm -> W1/W3 -> SwiGLU -> W2 -> norm -> LM head of the
+    embeddings: k slices with and without a remainder, row tiles that are full, ragged and walked by one CTA in turn.  spread: rows and
+    columns scaled by up to 10^spread either way, which fp16 parts survive only with their powers of two.
+
+    Tolerance: an operand has 22 bits, a sum fewer than 64 fp32 additions of parts that are no larger than sum |x w|, so a product is
+    within 2 * 2^-22 + 64 * 2^-24 < 5e-6 of sum |x w|; each of three products in a row hands on an error of that size, which the
+    norms keep relative to its row."""
+    V = 260
+    rng = np.random.default_rng(dm + rows)
+
+    def scales(n):
+        return 10.0 ** rng.uniform(-spread, spread, n)
+
+    tok = rng.standard_normal((V, dm)) * scales(V)[:, None]
+    mats = [rng.standard_normal((dm, dm)) for _ in range(3)] + [np.zeros((dm, dm))]
+    w1, w3 = rng.standard_normal((dm, dff)) / np.sqrt(dm) * scales(dff), rng.standard_normal((dm, dff)) / np.sqrt(dm)
+    w2 = rng.standard_normal((dff, dm)) / np.sqrt(dff) * 10.0 ** -spread
+    n1, n2, nf = (1 + 0.2 * rng.standard_normal(dm) for _ in range(3))
+    head = rng.standard_normal((dm, V)) * scales(V)
+    T = [np.ascontiguousarray(t, np.float32) for t in (tok, np.zeros((64, dm)), *mats, w1, w2, w3, n1, n2, nf, head)]
+    gm = GPTModel(ctx, V, 64, dm, dm // 16, 1, dff, rmsNormEps=1e-6, maxRows=512)
+    gm.setParameters(T)
+    pool = gm.newPool(rows, rows)
+    try:
+        seqs = [pool.seq_alloc() for _ in range(rows)]
+        ids, zero = rng.integers(0, V, rows).astype(np.int32), np.zeros(rows, np.int32)
+        got, _ = gm.forwardDecodeBatch(pool, seqs, ids, zero, zero)
+        tok, w1, w2, w3, n2, nf, head = (t.astype(np.float64) for t in (T[0], T[6], T[7], T[8], T[10], T[11], T[12]))
+
+        def norm(x, w):
+            return x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6) * w
+
+        h = norm(tok[ids], n2)
+        g = h @ w3
+        act = h @ w1 * g / (1 + np.exp(-g))
+        x = tok[ids] + act @ w2
+        y = norm(x, nf)
+        # errors of the row in front of the last norm, relative to its size
+        off_act = 5e-6 * (np.abs(h) @ np.abs(w1) * np.abs(g) + np.abs(h @ w1) * (np.abs(h) @ np.abs(w3)) * 1.2)
+        off_x = off_act @ np.abs(w2) + 5e-6 * (np.abs(act) @ np.abs(w2)) + 1e-6 * np.abs(x)
+        rel = np.sqrt((off_x ** 2).mean(-1, keepdims=True) / ((x * x).mean(-1, keepdims=True) + 1e-6))
+        off_y = norm(off_x, np.abs(nf)) * np.sqrt((off_x ** 2).mean(-1, keepdims=True) + 1e-6) / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6) + rel * np.abs(y)
+        bound = off_y @ np.abs(head) + 5e-6 * (np.abs(y) @ np.abs(head))
+        assert np.all(np.abs(got - y @ head) <= bound), float((np.abs(got - y @ head) / bound).max())
+    finally:
+        pool.close(), gm.close()
+
+
 def test_forward_step_reports_a_failed_device_self_check_itself(ctx, small16):
     """A corrupted block-table entry (-1 where the step reads or appends) must come back as an error from the
     forward call itself -- no jgpt_sync needed, no tokens, no length change -- and the pool must stay usable:
