@@ -4,10 +4,11 @@
 // Work item = (layer, sequence, head group, chunk of `chunk_blocks` KV blocks).  A CTA owns a
 // ring of shared-memory stages; one producer warp walks the block table and fetches, per KV
 // block, the contiguous [head group][K tile | V tile] slab with ONE bulk async copy (TMA engine,
-// cp.async.bulk + mbarrier complete_tx).  Consumer threads are (head, token-in-block) pairs: a
-// thread scores its token against q (fp32 FMA), keeps a private online-softmax state
-// (m, l, o[DH]) and, at the end of the chunk, the 16 lanes of a head merge their states with warp
-// shuffles.  Chunks of one sequence are merged by the last CTA to arrive (atomic ticket, no
+// cp.async.bulk + mbarrier complete_tx).  At dhead 16 a consumer warp owns four heads and runs their
+// products on the tensor cores with high + low operands; at the other head sizes consumer threads are
+// (head, token-in-block) pairs: a thread scores its token against q (fp32 FMA), keeps a private
+// online-softmax state (m, l, o[DH]) and, at the end of the chunk, the 16 lanes of a head merge their
+// states with warp shuffles.  Chunks of one sequence are merged by the last CTA to arrive (atomic ticket, no
 // waiting), through a small fp32 scratch buffer.
 //
 // The kernel is HBM-bound (about 1 FLOP per byte at dhead 16): what matters is bytes in flight
@@ -160,8 +161,15 @@ __device__ __forceinline__ void halfwarp_reduce_scatter(float (&v)[DH], int t) {
 template <int DH>
 constexpr int max_head_group() { return (384 / DH) < 30 ? (384 / DH) : 30; }
 
-template <int DH, bool FUSED, bool MMA>
-__global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) attn_decode_kernel(const DecodeParams P) {
+// Consumer threads of a CTA: (head, token) pairs, or a warp per four heads with the products of dhead 16 on the tensor cores.
+template <int DH>
+__host__ __device__ constexpr int consumer_threads(int HG) {
+    return DH == 16 ? (HG + 3) / 4 * 32 : (kBlockTokens * HG + 31) / 32 * 32;
+}
+
+template <int DH, bool FUSED>
+__global__ void __launch_bounds__(consumer_threads<DH>(max_head_group<DH>()) + 32, DH == 16 ? 3 : 2) attn_decode_kernel(const DecodeParams P) {
+    constexpr bool MMA = DH == 16;
     constexpr int BT = kBlockTokens;
     constexpr int TILE = BT * DH * 2;    // bytes of one K (or V) tile
     constexpr int HEAD_BYTES = 2 * TILE; // K tile | V tile
@@ -185,7 +193,7 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
     timeline_in(P.timeline);
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(tr_gt0));
 #endif
-    const int n_cons = ((BT * P.HG + 31) / 32) * 32;  // consumer threads (padded to whole warps)
+    const int n_cons = consumer_threads<DH>(P.HG);  // padded to whole warps
     const int n_cons_warps = n_cons / 32;
     const int stage_bytes = P.HG * HEAD_BYTES;
     const int NS = P.stages;
@@ -211,8 +219,8 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
     // q / k_new / v_new come from the previous kernel on the stream, and the split-K scratch and counters are shared
     // with it: the consumers always wait for it.  The producer touches neither; it waits unless the caller has
     // promised that what it reads (lengths, tables, cached K/V) is not written by that kernel.
-    // With overlap 2 the scalar consumers wait later still: right before they read q (see below).
-    const bool late_wait = P.overlap == 2 && !MMA;
+    // With overlap 2 the consumers wait later still: right before they read q (see below).
+    const bool late_wait = P.overlap == 2;
     if (P.overlap && !(P.overlap == 2 && is_producer) && !(late_wait && !is_producer)) griddep_wait();
 #ifdef JGPT_B200_DECODE_TRACE
     if (!late_wait) timeline_at(P.timeline, 1);
@@ -385,12 +393,18 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
 
         if constexpr (MMA) {
             // ---------------- consumers, tensor-core form (dhead 16) ----------------
-            // A warp owns two heads.  Per KV block and head: scores^T[16 tok x 8] = K[16 x 16] . Q^T[16 x 8] and
-            // O^T[16 dh x 8] += V^T[16 x 16] . P^T[16 x 8] with mma.sync m16n8k16, K and V^T fragments straight
-            // from the staged fp16 tile (ldmatrix: no fp16->fp32 conversion instructions at all).  Column 0 of
-            // Q^T / P^T holds the fp16 high part of q / p, column 1 the low part, so sums over the two columns
-            // keep fp32-level accuracy.  Scores and outputs live in the 8 lanes with (lane & 3) == 0.
-            static_assert(!MMA || DH == 16, "the tensor-core consumer is written for dhead 16");
+            // A warp owns four heads.  Per KV block and head one m16n8k16 product K [16 tok x 16] . Q^T [16 x 8] and one
+            // V^T [16 dh x 16 tok] . P^T [16 x 8], K and V^T straight from the staged fp16 tile (ldmatrix: no conversions).  Columns
+            // 2 c and 2 c + 1 of Q^T and P^T hold the fp16 high and low part of head c's q and p, so the four products share their B
+            // operand and the sum over a column pair keeps fp32-level accuracy; of head i's product only the pair i is used, which
+            // sits in the lanes with lane % 4 == i.  Lane (g, t) thus carries the scores of tokens g and g + 8 and the sums of
+            // dims g and g + 8 of head t: every lane has work, and maximum, exponentials and rescaling serve four heads at once.
+            // A product's unused columns stay unused, so an infinity in one head does not reach another.
+            // q is scaled by a power of two per head and p by 2^14, both to keep the low parts clear of fp16's subnormals: the
+            // running reference m lies 14 below the maximum, p = 2^(s - m) <= 2^14, and the factor cancels in o / l.
+            // About 95 instructions per 4 heads x 16 tokens where fp32 FMAs on converted rows took 380: one CTA alone was
+            // issue-bound at 43 GB/s.
+            constexpr float kLift = 14.f;
             const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
             int rp = rp_raw;
             if (rp < 0 || rp >= P.max_positions) {
@@ -398,44 +412,72 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
                 rp = 0;
             }
             const float2 *cs = P.rope + (size_t)rp * (DH / 2);
-            bool act[2];
-            int hh_head[2];
-            uint32_t qb[2][2];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const int hl = 2 * warp + hh;
-                act[hh] = hl < P.HG;
-                hh_head[hh] = head0 + (act[hh] ? hl : 0);
-                const float *qp = P.q + row + (size_t)hh_head[hh] * DH;
-                const float2 x0 = *reinterpret_cast<const float2 *>(qp + 2 * t4);      // dims 2t, 2t+1
-                const float2 x1 = *reinterpret_cast<const float2 *>(qp + 2 * t4 + 8);  // dims 2t+8, 2t+9
-                const float2 w0 = cs[t4], w1 = cs[t4 + 4];
-                float v[4];
-                v[0] = __fsub_rn(__fmul_rn(x0.x, w0.x), __fmul_rn(x0.y, w0.y)) * P.scale_log2e;
-                v[1] = __fadd_rn(__fmul_rn(x0.x, w0.y), __fmul_rn(x0.y, w0.x)) * P.scale_log2e;
-                v[2] = __fsub_rn(__fmul_rn(x1.x, w1.x), __fmul_rn(x1.y, w1.y)) * P.scale_log2e;
-                v[3] = __fadd_rn(__fmul_rn(x1.x, w1.y), __fmul_rn(x1.y, w1.x)) * P.scale_log2e;
-                __half part[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const __half hi = __float2half_rn(v[e]);
-                    const __half lo = __float2half_rn(v[e] - __half2float(hi));
-                    part[e] = g == 0 ? hi : (g == 1 ? lo : __float2half_rn(0.f));
-                }
-                const __half2 p01 = __halves2half2(part[0], part[1]), p23 = __halves2half2(part[2], part[3]);
-                qb[hh][0] = *reinterpret_cast<const uint32_t *>(&p01);
-                qb[hh][1] = *reinterpret_cast<const uint32_t *>(&p23);
+            const int hl = 4 * warp + t4, hl_q = min(4 * warp + (g >> 1), P.HG - 1);
+            const bool act = hl < P.HG;
+            const int h = head0 + (act ? hl : 0);
+            auto turned = [](float2 x, float2 w) {  // RoPE with separate roundings
+                return make_float2(__fsub_rn(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y)), __fadd_rn(__fmul_rn(x.x, w.y), __fmul_rn(x.y, w.x)));
+            };
+            // column g of the B operand: dims 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of head g / 2, high parts for even g, low parts for odd g
+            auto column = [&](float x, float y) {
+                const __half2 hi = __floats2half2_rn(x, y);
+                const float2 f = __half22float2(hi);
+                const __half2 v = g & 1 ? __floats2half2_rn(x - f.x, y - f.y) : hi;
+                return *reinterpret_cast<const uint32_t *>(&v);
+            };
+            uint32_t qb0, qb1;
+            float q_un;  // undoes head t's power of two
+            {
+                const float *qp = P.q + row + (size_t)(head0 + hl_q) * DH;
+                const float2 x0 = turned(*reinterpret_cast<const float2 *>(qp + 2 * t4), cs[t4]);
+                const float2 x1 = turned(*reinterpret_cast<const float2 *>(qp + 2 * t4 + 8), cs[t4 + 4]);
+                float mx = fmaxf(fmaxf(fabsf(x0.x), fabsf(x0.y)), fmaxf(fabsf(x1.x), fabsf(x1.y)));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                float up, down;
+                pow2_scale(mx * P.scale_log2e, up, down);
+                const float f = P.scale_log2e;
+                qb0 = column(x0.x * f * up, x0.y * f * up), qb1 = column(x1.x * f * up, x1.y * f * up);
+                q_un = __shfl_sync(0xffffffffu, down, 8 * t4);
             }
-            float m2[2] = {-INFINITY, -INFINITY}, ls[2] = {0.f, 0.f}, acc[2][4];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) acc[hh][e] = 0.f;
-            const int new_tok = len - 1;  // fused mode: the token being appended
-            const bool has_new = FUSED && (new_tok / BT >= b0) && (new_tok / BT < b1);
+            float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};  // o: dim g (high, low column), dim g + 8; l: this lane's tokens
+            const int len_cached = FUSED ? len - 1 : len;
+            if (FUSED && len_cached / BT >= b0 && len_cached / BT < b1) {
+                // Fused append: the eight lanes of a head compute the stored payload (RoPE'd K, raw V, both rounded to fp16), write
+                // it to the cache and start the softmax state from it; the loop below covers the tokens already cached.
+                const size_t at = row + (size_t)h * DH + 2 * g;
+                const float2 w = cs[g];
+                const float2 qr = turned(*reinterpret_cast<const float2 *>(P.q + at), w);
+                const float2 kr = turned(*reinterpret_cast<const float2 *>(P.k_new + at), w);
+                const float2 vr = *reinterpret_cast<const float2 *>(P.v_new + at);
+                const float va = P.v_new[row + (size_t)h * DH + g], vb = P.v_new[row + (size_t)h * DH + g + 8];
+                const __half2 kh = __floats2half2_rn(kr.x, kr.y), vh = __floats2half2_rn(vr.x, vr.y);
+                const float2 kf = __half22float2(kh);
+                float sc = (qr.x * P.scale_log2e) * kf.x + (qr.y * P.scale_log2e) * kf.y;
+                sc += __shfl_xor_sync(0xffffffffu, sc, 4);
+                sc += __shfl_xor_sync(0xffffffffu, sc, 8);
+                sc += __shfl_xor_sync(0xffffffffu, sc, 16);
+                m = sc - kLift;
+                const float p = fast_exp2(sc - m);
+                l = g == 0 ? p : 0.f;
+                o[0] = p * __half2float(__float2half_rn(va)), o[2] = p * __half2float(__float2half_rn(vb));
+                const int phys = P.table[(size_t)seq * P.mbs + len_cached / BT];
+                if (phys < 0 || phys >= P.n_blocks) {
+                    if (lane == 0) atomicOr(P.status, DEV_STATUS_BAD_BLOCK);
+                } else if (act) {
+                    __half *dst = P.kv + ((layer_base + phys) * P.H + h) * (size_t)(2 * BT * DH) + (size_t)(len_cached % BT) * DH + 2 * g;
+                    *reinterpret_cast<__half2 *>(dst) = kh;
+                    *reinterpret_cast<__half2 *>(dst + BT * DH) = vh;
+                }
+            }
             const int mi = lane >> 3, rr = lane & 7;
             const int k_off = ((mi & 1) * 8 + rr) * 32 + (mi >> 1) * 16;          // K tile as the A operand (rows = tokens)
             const int v_off = TILE + ((mi >> 1) * 8 + rr) * 32 + (mi & 1) * 16;   // V tile, transposed load (rows = dims)
+            auto of_head_t = [&](float a0, float a1, float a2, float a3) {
+                const float e = t4 & 1 ? a1 : a0, f = t4 & 1 ? a3 : a2;
+                return t4 & 2 ? f : e;
+            };
+            const int src0 = 8 * t4 + (g >> 1), src1 = src0 + 4;  // the lanes with p of tokens 2 t and 2 t + 1 of head g / 2
 
             bool aborted = false;
             for (int j = 0; j < nb; j++, it++) {
@@ -443,139 +485,125 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
                 const uint32_t ph = phase;
                 if (++stage == NS) stage = 0, phase ^= 1u;
                 if (!aborted && !mbar_wait_bounded(&full_bar[s], ph, P.status, s_abort)) aborted = true;
-                if (aborted) continue;
-                unsigned char *base = smem + (size_t)s * stage_bytes;
-                if (FUSED && has_new && (b0 + j) == new_tok / BT) {
-                    // Lanes 0 and 1 append the new token of the warp's two heads: RoPE'd K and raw V rounded to fp16,
-                    // stored to the paged cache and into the staged tile (the bulk copy brought the slot's old content).
-                    const bool my_act = lane == 0 ? act[0] : act[1];
-                    if (lane < 2 && my_act) {
-                        const int h = lane == 0 ? hh_head[0] : hh_head[1];
-                        const float *kp = P.k_new + row + (size_t)h * DH, *vp = P.v_new + row + (size_t)h * DH;
-                        __align__(16) __half kh[DH], vh[DH];
+                if (aborted) continue;  // keep counting blocks, touch nothing
+#ifdef JGPT_B200_DECODE_TRACE
+                if (j == 0 && tr_c2 == 0) tr_c2 = clock64();
+#endif
+                const int left = len_cached - (b0 + j) * BT;  // tokens of this block that are cached
+                if (left > 0) {  // else the block holds the appended token alone
+                    const unsigned char *base = smem + (size_t)s * stage_bytes;
+                    float d[4][4];
+                    uint32_t va[4][4];
 #pragma unroll
-                        for (int jj = 0; jj < DH / 2; jj++) {
-                            const float2 x = *reinterpret_cast<const float2 *>(kp + 2 * jj);
-                            const float2 y = *reinterpret_cast<const float2 *>(vp + 2 * jj);
-                            const float2 w = cs[jj];
-                            kh[2 * jj] = __float2half_rn(__fsub_rn(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y)));
-                            kh[2 * jj + 1] = __float2half_rn(__fadd_rn(__fmul_rn(x.x, w.y), __fmul_rn(x.y, w.x)));
-                            vh[2 * jj] = __float2half_rn(y.x);
-                            vh[2 * jj + 1] = __float2half_rn(y.y);
-                        }
-                        const int slot = new_tok % BT;
-                        unsigned char *tile = base + (size_t)(2 * warp + lane) * HEAD_BYTES;
-                        reinterpret_cast<uint4 *>(tile + slot * 32)[0] = reinterpret_cast<const uint4 *>(kh)[0];
-                        reinterpret_cast<uint4 *>(tile + slot * 32)[1] = reinterpret_cast<const uint4 *>(kh)[1];
-                        reinterpret_cast<uint4 *>(tile + TILE + slot * 32)[0] = reinterpret_cast<const uint4 *>(vh)[0];
-                        reinterpret_cast<uint4 *>(tile + TILE + slot * 32)[1] = reinterpret_cast<const uint4 *>(vh)[1];
-                        const int phys = P.table[(size_t)seq * P.mbs + new_tok / BT];
-                        if (phys < 0 || phys >= P.n_blocks) {
-                            atomicOr(P.status, DEV_STATUS_BAD_BLOCK);
-                        } else {
-                            __half *dst = P.kv + ((layer_base + phys) * P.H + h) * (size_t)(2 * BT * DH) + (size_t)slot * DH;
-                            reinterpret_cast<uint4 *>(dst)[0] = reinterpret_cast<const uint4 *>(kh)[0];
-                            reinterpret_cast<uint4 *>(dst)[1] = reinterpret_cast<const uint4 *>(kh)[1];
-                            reinterpret_cast<uint4 *>(dst + BT * DH)[0] = reinterpret_cast<const uint4 *>(vh)[0];
-                            reinterpret_cast<uint4 *>(dst + BT * DH)[1] = reinterpret_cast<const uint4 *>(vh)[1];
-                        }
-                        // these generic-proxy stores must be ordered before the next bulk copy into this stage
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    }
-                    __syncwarp();
-                }
-                if ((b0 + j) == nblk - 1 && (len % BT) != 0) {
-                    // Last block of the sequence: the V rows beyond the last token hold whatever the slot held before.
-                    // Their probabilities are exactly 0, but 0 x Inf/NaN is NaN inside the MMA: clear them in the tile.
-                    const int first_dead = len % BT;
-                    for (int e = lane; e < 2 * (BT - first_dead) * 2; e += 32) {
-                        const int hh = e & 1, half16 = (e >> 1) & 1, r = first_dead + (e >> 2);
-                        if (hh == 0 ? act[0] : act[1])
-                            *reinterpret_cast<uint4 *>(base + (size_t)(2 * warp + hh) * HEAD_BYTES + TILE + r * 32 + half16 * 16) =
-                                make_uint4(0, 0, 0, 0);
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                }
-                const int tok0 = (b0 + j) * BT + g;
+                    for (int i = 0; i < 4; i++) {
+                        const unsigned char *tile = base + (size_t)min(4 * warp + i, P.HG - 1) * HEAD_BYTES;
+                        uint32_t ka[4];
+                        ldmatrix_x4(ka, tile + k_off);
+                        ldmatrix_x4_trans(va[i], tile + v_off);
 #pragma unroll
-                for (int hh = 0; hh < 2; hh++) {
-                    if (!act[hh]) continue;  // warp-uniform
-                    const unsigned char *tile = base + (size_t)(2 * warp + hh) * HEAD_BYTES;
-                    uint32_t ka[4];
-                    ldmatrix_x4(ka, tile + k_off);
-                    float sc[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_16816(sc, ka, qb[hh][0], qb[hh][1]);
-                    float s0 = sc[0] + sc[1], s1 = sc[2] + sc[3];  // tokens g and g+8 (lanes with t4 == 0)
-                    if (tok0 >= len) s0 = -INFINITY;
-                    if (tok0 + 8 >= len) s1 = -INFINITY;
+                        for (int e = 0; e < 4; e++) d[i][e] = 0.f;
+                        mma_16816(d[i], ka, qb0, qb1);
+                    }
+                    float s0 = of_head_t(d[0][0] + d[0][1], d[1][0] + d[1][1], d[2][0] + d[2][1], d[3][0] + d[3][1]) * q_un;
+                    float s1 = of_head_t(d[0][2] + d[0][3], d[1][2] + d[1][3], d[2][2] + d[2][3], d[3][2] + d[3][3]) * q_un;
+                    if (left < BT) {
+                        // The slots beyond the last cached token hold whatever they held before: no score, and zeros in place of V
+                        // (their probabilities are 0, but 0 x Inf or NaN is NaN inside the product).
+                        if (g >= left) s0 = -INFINITY;
+                        if (g + 8 >= left) s1 = -INFINITY;
+                        const uint32_t lo = (2 * t4 < left ? 0xffffu : 0u) | (2 * t4 + 1 < left ? 0xffff0000u : 0u);
+                        const uint32_t hi = (2 * t4 + 8 < left ? 0xffffu : 0u) | (2 * t4 + 9 < left ? 0xffff0000u : 0u);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) va[i][0] &= lo, va[i][1] &= lo, va[i][2] &= hi, va[i][3] &= hi;
+                    }
                     float bm = fmaxf(s0, s1);
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 4));
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 8));
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 16));
-                    bm = __shfl_sync(0xffffffffu, bm, 0);  // the value of the t4 == 0 lanes, for every lane
-                    const float mn = fmaxf(m2[hh], bm);    // finite: the block holds at least one attended token
-                    const float corr = fast_exp2(m2[hh] - mn);
+                    const float mn = fmaxf(m, bm - kLift);
+                    const float corr = fast_exp2(m - mn);
                     const float p0 = fast_exp2(s0 - mn), p1 = fast_exp2(s1 - mn);
-                    ls[hh] = ls[hh] * corr + (p0 + p1);
-                    m2[hh] = mn;
+                    m = mn;
+                    l = l * corr + (p0 + p1);
+                    const uint32_t pb0 = column(__shfl_sync(0xffffffffu, p0, src0), __shfl_sync(0xffffffffu, p0, src1));
+                    const uint32_t pb1 = column(__shfl_sync(0xffffffffu, p1, src0), __shfl_sync(0xffffffffu, p1, src1));
 #pragma unroll
-                    for (int e = 0; e < 4; e++) acc[hh][e] *= corr;
-                    // P^T as the B operand: lanes with g == 0 carry the high parts of p[2t], p[2t+1], p[2t+8], p[2t+9],
-                    // lanes with g == 1 the low parts, the other columns are zero.
-                    const float x0 = __shfl_sync(0xffffffffu, p0, 8 * t4), x1 = __shfl_sync(0xffffffffu, p0, 8 * t4 + 4);
-                    const float y0 = __shfl_sync(0xffffffffu, p1, 8 * t4), y1 = __shfl_sync(0xffffffffu, p1, 8 * t4 + 4);
-                    const float pv[4] = {x0, x1, y0, y1};
-                    __half part[4];
+                    for (int i = 0; i < 4; i++) {
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const __half hi = __float2half_rn(pv[e]);
-                        const __half lo = __float2half_rn(pv[e] - __half2float(hi));
-                        part[e] = g == 0 ? hi : (g == 1 ? lo : __float2half_rn(0.f));
+                        for (int e = 0; e < 4; e++) d[i][e] = 0.f;
+                        mma_16816(d[i], va[i], pb0, pb1);
                     }
-                    const __half2 b01 = __halves2half2(part[0], part[1]), b23 = __halves2half2(part[2], part[3]);
-                    uint32_t va[4];
-                    ldmatrix_x4_trans(va, tile + v_off);
-                    mma_16816(acc[hh], va, *reinterpret_cast<const uint32_t *>(&b01), *reinterpret_cast<const uint32_t *>(&b23));
+#pragma unroll
+                    for (int e = 0; e < 4; e++) o[e] = fmaf(o[e], corr, of_head_t(d[0][e], d[1][e], d[2][e], d[3][e]));
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty_bar[s]);
             }
-
-            // ---- per head: totals over the 8 score lanes, then write / publish ----
-            constexpr int PSTRIDE = DH + 2;
-            const size_t prow = (((size_t)z * P.n + i) * P.max_chunks) * (size_t)P.H;
-            float og[2][2], lt[2];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                float l = ls[hh];
-                l += __shfl_xor_sync(0xffffffffu, l, 4);
-                l += __shfl_xor_sync(0xffffffffu, l, 8);
-                l += __shfl_xor_sync(0xffffffffu, l, 16);
-                lt[hh] = l;
-                og[hh][0] = acc[hh][0] + acc[hh][1];  // dim g
-                og[hh][1] = acc[hh][2] + acc[hh][3];  // dim g + 8
-            }
-            const bool lane_writes = t4 == 0 && !aborted;
+#ifdef JGPT_B200_DECODE_TRACE
+            tr_c3 = clock64();
+#endif
+            // After a timed-out wait the thread keeps walking the barriers below (so nobody is left waiting for it) but stores
+            // nothing; the item loop ends at its next iteration.
+            l += __shfl_xor_sync(0xffffffffu, l, 4);
+            l += __shfl_xor_sync(0xffffffffu, l, 8);
+            l += __shfl_xor_sync(0xffffffffu, l, 16);
+            const float o0 = o[0] + o[1], o1 = o[2] + o[3];  // dims g, g + 8 of head h
+            const bool writer = act && !aborted;
+            float *op = P.out + row + (size_t)h * DH + g;
             if (nsplit == 1) {
-#pragma unroll
-                for (int hh = 0; hh < 2; hh++)
-                    if (lane_writes && act[hh]) {
-                        const float inv = 1.f / fmaxf(lt[hh], 1e-12f);
-                        float *op = P.out + row + (size_t)hh_head[hh] * DH;
-                        op[g] = og[hh][0] * inv;
-                        op[g + 8] = og[hh][1] * inv;
-                    }
+                if (writer) {
+                    const float inv = 1.f / fmaxf(l, 1e-12f);
+                    op[0] = o0 * inv, op[8] = o1 * inv;
+                }
+                if (P.cluster) cluster_sync(), cluster_sync();
                 continue;
             }
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++)
-                if (lane_writes && act[hh]) {
-                    float *pp = P.partials + (prow + (size_t)c * P.H + hh_head[hh]) * PSTRIDE;
-                    pp[2 + g] = og[hh][0];
-                    pp[2 + g + 8] = og[hh][1];
-                    if (g == 0) pp[0] = m2[hh], pp[1] = lt[hh];
+            constexpr int PS = DH + 2;
+            if (P.cluster) {
+                // ---- split-K inside a cluster: partials stay in shared memory, the CTA of chunk 0 merges them ----
+                float *pp = cl_part + (act ? hl : 0) * PS;
+                if (writer) {
+                    pp[2 + g] = o0, pp[10 + g] = o1;
+                    if (g == 0) pp[0] = m, pp[1] = l;
+                } else if (act && g == 0) {
+                    pp[0] = -INFINITY, pp[1] = 0.f;  // a chunk that gave up contributes nothing
                 }
+                cluster_sync();
+                if (c == 0 && writer) {
+                    float mc[8], lc[8], a0[8], a1[8];  // at most eight chunks: all of them requested before the first is used
+#pragma unroll
+                    for (int cc = 0; cc < 8; cc++) {
+                        const bool in = cc < nsplit;
+                        mc[cc] = in ? ld_cluster_f32(pp, (uint32_t)cc) : -INFINITY;
+                        lc[cc] = in ? ld_cluster_f32(pp + 1, (uint32_t)cc) : 0.f;
+                        a0[cc] = in ? ld_cluster_f32(pp + 2 + g, (uint32_t)cc) : 0.f;
+                        a1[cc] = in ? ld_cluster_f32(pp + 10 + g, (uint32_t)cc) : 0.f;
+                    }
+                    float Mx = -INFINITY, L = 0.f, r0 = 0.f, r1 = 0.f;
+#pragma unroll
+                    for (int cc = 0; cc < 8; cc++) Mx = fmaxf(Mx, mc[cc]);
+#pragma unroll
+                    for (int cc = 0; cc < 8; cc++)
+                        if (cc < nsplit) {
+                            const float w = mc[cc] == -INFINITY ? 0.f : exp2f(mc[cc] - Mx);
+                            L = fmaf(lc[cc], w, L), r0 = fmaf(a0[cc], w, r0), r1 = fmaf(a1[cc], w, r1);
+                        }
+                    const float inv = 1.f / fmaxf(L, 1e-12f);
+                    op[0] = r0 * inv, op[8] = r1 * inv;
+                }
+                cluster_sync();  // nobody leaves (and frees its shared memory) before chunk 0 has read it
+                continue;
+            }
+            // ---- split-K: publish the partial, last CTA of the sequence row merges ----
+            const size_t prow = (((size_t)z * P.n + i) * P.max_chunks) * (size_t)P.H;  // + c*H + head
+            if (writer) {
+                float *pp = P.partials + (prow + (size_t)c * P.H + h) * PS;
+                pp[2 + g] = o0, pp[10 + g] = o1;
+                if (g == 0) pp[0] = m, pp[1] = l;
+            }
+#ifdef JGPT_B200_TRACE_NOMERGE
+            if (P.n > 0) continue;  // timing experiment only: partials written, nobody merges
+#endif
             __threadfence();
             named_bar_sync(1, n_cons);
             int *ticket = P.tickets + ((size_t)z * P.n + i) * P.n_hg + hg;
@@ -587,25 +615,18 @@ __global__ void __launch_bounds__(max_head_group<DH>() * kBlockTokens + 32, 2) a
             named_bar_sync(1, n_cons);
             if (s_last) {
                 __threadfence();
-#pragma unroll
-                for (int hh = 0; hh < 2; hh++)
-                    if (lane_writes && act[hh]) {
-                        const int h = hh_head[hh];
-                        float Mx = -INFINITY;
-                        for (int cc = 0; cc < nsplit; cc++) Mx = fmaxf(Mx, __ldcg(P.partials + (prow + (size_t)cc * P.H + h) * PSTRIDE));
-                        float L = 0.f, a0 = 0.f, a1 = 0.f;
-                        for (int cc = 0; cc < nsplit; cc++) {
-                            const float *pp = P.partials + (prow + (size_t)cc * P.H + h) * PSTRIDE;
-                            const float w = exp2f(__ldcg(pp) - Mx);
-                            L = fmaf(__ldcg(pp + 1), w, L);
-                            a0 = fmaf(__ldcg(pp + 2 + g), w, a0);
-                            a1 = fmaf(__ldcg(pp + 2 + g + 8), w, a1);
-                        }
-                        const float inv = 1.f / fmaxf(L, 1e-12f);
-                        float *op = P.out + row + (size_t)h * DH;
-                        op[g] = a0 * inv;
-                        op[g + 8] = a1 * inv;
+                if (writer) {
+                    float Mx = -INFINITY, L = 0.f, r0 = 0.f, r1 = 0.f;
+                    for (int cc = 0; cc < nsplit; cc++) Mx = fmaxf(Mx, __ldcg(P.partials + (prow + (size_t)cc * P.H + h) * PS));
+                    for (int cc = 0; cc < nsplit; cc++) {
+                        const float *pp = P.partials + (prow + (size_t)cc * P.H + h) * PS;
+                        const float w = exp2f(__ldcg(pp) - Mx);
+                        L = fmaf(__ldcg(pp + 1), w, L);
+                        r0 = fmaf(__ldcg(pp + 2 + g), w, r0), r1 = fmaf(__ldcg(pp + 10 + g), w, r1);
                     }
+                    const float inv = 1.f / fmaxf(L, 1e-12f);
+                    op[0] = r0 * inv, op[8] = r1 * inv;
+                }
             }
             continue;
         }
@@ -891,21 +912,10 @@ static int pick_head_group(int H, int DH, int forced, long long pairs = 0, long 
 
 template <int DH>
 static int32_t launch_decode_t(Pool *p, const DecodeParams &P, bool fused, int threads, size_t smem, int grid) {
-    // JGPT_B200_DECODE_MMA=1 selects the tensor-core consumer for dhead 16.  It is exact to the same tolerance but
-    // measured 40 % slower on B200 (285 us against 203 us on the 12-layer batch-64 context-1024 step): per KV block
-    // a warp runs two short dependent chains (ldmatrix, MMA, quad-strided shuffle reductions, exp2, hi/lo split of
-    // p, MMA) on only 8 useful lanes, and the decode step is HBM-bound anyway.  The scalar consumer is the default.
-    const bool want_mma = p->decode_mma != 0;  // read from the environment when the pool was created
-    constexpr bool kCanMma = DH == 16;
-    const bool mma = kCanMma && want_mma;
-    void (*kern)(const DecodeParams) = fused ? attn_decode_kernel<DH, true, false> : attn_decode_kernel<DH, false, false>;
-    if constexpr (kCanMma) {
-        if (mma) kern = fused ? attn_decode_kernel<DH, true, true> : attn_decode_kernel<DH, false, true>;
-    }
+    void (*kern)(const DecodeParams) = fused ? attn_decode_kernel<DH, true> : attn_decode_kernel<DH, false>;
     // Opt in to > 48 KiB of dynamic shared memory once per kernel and device: the most a launch can ask for
     // (kMaxStages stages of a 24 KiB slab), so that no later, smaller request ever lowers the limit again.
-    JGPT_CUDA_TRY(decode_opt_in_smem(kern, (fused ? 1 : 0) + (mma ? 2 : 0) + 4 * (DH == 4 ? 0 : DH == 8 ? 1 : DH == 16 ? 2 : 3),
-                                     p->ctx->device));
+    JGPT_CUDA_TRY(decode_opt_in_smem(kern, (fused ? 1 : 0) + 4 * (DH == 4 ? 0 : DH == 8 ? 1 : DH == 16 ? 2 : 3), p->ctx->device));
     if (P.overlap || P.cluster) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3((unsigned)threads), cfg.dynamicSmemBytes = smem, cfg.stream = p->ctx->stream;
@@ -957,10 +967,10 @@ static int cluster_capacity(Pool *p, bool fused, int threads, size_t smem, int c
     void (*kern)(const DecodeParams) = nullptr;
     int variant = -1;
     switch (p->dhead) {
-        case 4: kern = fused ? attn_decode_kernel<4, true, false> : attn_decode_kernel<4, false, false>, variant = 0; break;
-        case 8: kern = fused ? attn_decode_kernel<8, true, false> : attn_decode_kernel<8, false, false>, variant = 4; break;
-        case 16: kern = fused ? attn_decode_kernel<16, true, false> : attn_decode_kernel<16, false, false>, variant = 8; break;
-        case 32: kern = fused ? attn_decode_kernel<32, true, false> : attn_decode_kernel<32, false, false>, variant = 12; break;
+        case 4: kern = fused ? attn_decode_kernel<4, true> : attn_decode_kernel<4, false>, variant = 0; break;
+        case 8: kern = fused ? attn_decode_kernel<8, true> : attn_decode_kernel<8, false>, variant = 4; break;
+        case 16: kern = fused ? attn_decode_kernel<16, true> : attn_decode_kernel<16, false>, variant = 8; break;
+        case 32: kern = fused ? attn_decode_kernel<32, true> : attn_decode_kernel<32, false>, variant = 12; break;
         default: return 0;
     }
     int n = 0;
@@ -1021,11 +1031,11 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     const long long slots = (long long)per_sm * p->ctx->sm_count;
     const bool dynamic = p->persistent > 0;
     P.stages = p->stages > 0 ? p->stages : (overlapped_single ? 3 : 4);
-    const int n_cons = ((kBlockTokens * P.HG + 31) / 32) * 32;
+    const int n_cons = DH == 16 ? consumer_threads<16>(P.HG) : consumer_threads<4>(P.HG);
     const int threads = n_cons + 32;
     const size_t stage_bytes = (size_t)P.HG * 2 * kBlockTokens * DH * 2;
     const size_t smem = stage_bytes * P.stages;
-    const bool may_cluster = p->cluster_merge && !dynamic && !p->decode_mma;
+    const bool may_cluster = p->cluster_merge && !dynamic;
     if (p->chunk_blocks > 0) {
         P.chunk_blocks = p->chunk_blocks;
     } else if (overlapped_single && may_cluster) {
@@ -1072,7 +1082,7 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     JGPT_REQUIRE(items < (1ll << 31), JGPT_ERR_INVALID_ARGUMENT, "too many work items (%lld)", items);
     P.n_items = (int)items;
     // The chunks of one sequence as one thread-block cluster (up to the portable size of 8): merge in shared memory.
-    // Not for the work queue (its CTAs take several items) nor for the tensor-core consumer (its own epilogue).
+    // Not for the work queue (its CTAs take several items).
     // Only for launches of a wave or two: there the merge's global round trips are a visible part of the launch (per-layer
     // launch at batch 64 / context 1024: 24.1 -> 22.7 us).  A launch of many waves hides them behind other CTAs' copies,
     // and co-scheduling pairs of CTAs costs it more than it saves (12-layer launch: 198 us without, 202 us with).
@@ -1400,10 +1410,10 @@ static int32_t static_scratch_setup(const Pool *p, float **partials, int **ticke
                         "cudaGetSymbolAddress(static decode scratch) on device %d: %s", c->device, cudaGetErrorString(e));
         cudaError_t a = cudaSuccess;
         switch (p->dhead) {
-            case 4: a = decode_opt_in_smem(attn_decode_kernel<4, false, false>, 0, c->device); break;
-            case 8: a = decode_opt_in_smem(attn_decode_kernel<8, false, false>, 4, c->device); break;
-            case 16: a = decode_opt_in_smem(attn_decode_kernel<16, false, false>, 8, c->device); break;
-            case 32: a = decode_opt_in_smem(attn_decode_kernel<32, false, false>, 12, c->device); break;
+            case 4: a = decode_opt_in_smem(attn_decode_kernel<4, false>, 0, c->device); break;
+            case 8: a = decode_opt_in_smem(attn_decode_kernel<8, false>, 4, c->device); break;
+            case 16: a = decode_opt_in_smem(attn_decode_kernel<16, false>, 8, c->device); break;
+            case 32: a = decode_opt_in_smem(attn_decode_kernel<32, false>, 12, c->device); break;
             default: break;
         }
         if (a != cudaSuccess) return fail(JGPT_ERR_CUDA, "static decode scratch set-up on device %d: %s", c->device, cudaGetErrorString(a));
@@ -1453,15 +1463,15 @@ static int32_t launch_attn_decode_static(Pool *p, int layer, const float *q, con
         // the counters must start at zero (they reset themselves, but not if an earlier launch gave up half way).
         JGPT_CUDA_TRY(cudaMemsetAsync(P.tickets, 0, sizeof(int) * need_tickets, p->ctx->stream));
     }
-    const int n_cons = ((kBlockTokens * P.HG + 31) / 32) * 32;
+    const int n_cons = DH == 16 ? consumer_threads<16>(P.HG) : consumer_threads<4>(P.HG);
     const int threads = n_cons + 32;
     const size_t smem = (size_t)P.HG * 2 * kBlockTokens * DH * 2 * P.stages;
     void (*kern)(const DecodeParams) = nullptr;
     switch (DH) {
-        case 4: kern = attn_decode_kernel<4, false, false>; break;
-        case 8: kern = attn_decode_kernel<8, false, false>; break;
-        case 16: kern = attn_decode_kernel<16, false, false>; break;
-        case 32: kern = attn_decode_kernel<32, false, false>; break;
+        case 4: kern = attn_decode_kernel<4, false>; break;
+        case 8: kern = attn_decode_kernel<8, false>; break;
+        case 16: kern = attn_decode_kernel<16, false>; break;
+        case 32: kern = attn_decode_kernel<32, false>; break;
         default: return fail(JGPT_ERR_UNSUPPORTED, "dhead %d not supported", DH);
     }
     kern<<<P.n_items, threads, smem, p->ctx->stream>>>(P);

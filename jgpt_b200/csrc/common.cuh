@@ -125,7 +125,6 @@ struct Pool {
     int stages = 0;  // copy-ring stages, 0 = automatic
     int persistent = -1;  // < 0: automatic
     int head_group = 0;  // 0 = automatic
-    int decode_mma = 0;  // 1: tensor-core consumer in the decode kernel (dhead 16)
     int prefill_fast = 0;  // d_head-16 prefill attention with single fp16 q / p operands (JGPT_B200_PREFILL_FAST)
     int cluster_merge = 1;  // split-K chunks of a sequence as a thread-block cluster, merged in shared memory (JGPT_B200_CLUSTER_MERGE=0: off)
     int stream_hint = 1;  // decode attention fetches K/V with an evict-first L2 policy (JGPT_B200_STREAM_HINT=0: off)

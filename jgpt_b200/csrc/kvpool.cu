@@ -417,7 +417,6 @@ int32_t jgpt_kvpool_create(jgpt_ctx ctxh, int32_t layers, int32_t heads, int32_t
     if (p->stages != 0) p->stages = std::min(8, std::max(2, p->stages));
     p->persistent = env_int("JGPT_B200_PERSISTENT", -1);
     p->head_group = env_int("JGPT_B200_HEAD_GROUP", 0);
-    p->decode_mma = env_int("JGPT_B200_DECODE_MMA", 0);
     p->prefill_fast = env_int("JGPT_B200_PREFILL_FAST", 0);
     p->stream_hint = env_int("JGPT_B200_STREAM_HINT", 1);
     p->cluster_merge = env_int("JGPT_B200_CLUSTER_MERGE", 1);

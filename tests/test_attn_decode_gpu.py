@@ -69,6 +69,51 @@ def test_split_and_pipeline_settings_agree(ctx, chunk_blocks, stages, persistent
         case.close()
 
 
+@pytest.mark.parametrize("H,chunk", [(1, 0), (4, 1), (6, 2), (7, 0), (24, 3)])
+def test_tensor_core_consumer_head_groups_scales_and_infinities(ctx, H, chunk):
+    """d_head 16: warps with one to four heads, queries of very different sizes side by side (each head has its own power of two), and
+    a head whose cached value is infinite, which must not reach the others though they share product operands.
+
+    Tolerance: a score is the sum of 16 products whose query has 22 bits, so it is within 2^-21 sum |q k| of the exact one (the
+    fp32 oracle is no closer); that moves an output by at most that much times the spread of V (about 8)."""
+    lens = [1, 16, 31, 200]
+    os.environ["JGPT_B200_CHUNK_BLOCKS"] = str(chunk)
+    try:
+        case = PagedCase(ctx, lens, H=H, Dh=16, layers=1, seed=31 + H)
+    finally:
+        os.environ.pop("JGPT_B200_CHUNK_BLOCKS")
+    try:
+        from jgpt_b200 import binding as B
+        rng = np.random.default_rng(H)
+        n, Dh = case.n, 16
+        size = 10.0 ** rng.uniform(-30, 1, H)
+        size[-1] = 10.0
+        q = (rng.standard_normal((n, H, Dh)) * size[None, :, None]).reshape(n, H * Dh).astype(np.float32)
+        rope = np.array([l - 1 for l in lens], np.int32)
+        want = _oracle_decode(case, 0, q, lens, rope)
+        ptr, nbytes = case.pool.storage()
+        raw = np.empty(nbytes // 2, np.uint16)
+        B.check(ctx._lib.jgpt_d2h(ctx.handle, raw.ctypes.data, ptr, nbytes))
+        tiles = raw.reshape(1, case.n_blocks, H, 2, 16, Dh)
+        bad = H // 2
+        for i, l in enumerate(lens):
+            tiles[0, case.tables[i][0], bad, 1, 0, 3] = 0x7C00  # +inf in the value of the first token
+        B.check(ctx._lib.jgpt_h2d(ctx.handle, ptr, raw.ctypes.data, nbytes))
+        out = ctx.alloc((n, H * Dh))
+        case.pool.attn_decode(0, 1, ctx.from_host(q), case.seq_ids_dev(), ctx.from_host(rope), ctx.from_host(case.lens), n, max(lens), out)
+        ctx.synchronize()
+        got, want = out.to_host().reshape(n, H, Dh), want.reshape(n, H, Dh)
+        reach = np.abs(q.reshape(n, H, Dh)).sum(-1) * 4.0 * 2.0 ** -21 / 4.0  # |k| < 4, score scale 1 / 4
+        for h in range(H):
+            for d in range(Dh):
+                if h == bad and d == 3:
+                    assert not np.isfinite(got[:, h, d]).any()
+                else:
+                    assert np.all(np.abs(got[:, h, d] - want[:, h, d]) <= TOL + 8 * reach[:, h]), (h, d)
+    finally:
+        case.close()
+
+
 @pytest.mark.parametrize("fused", [False, True])
 def test_tensor_core_consumer_matches_oracle(ctx, fused):
     """JGPT_B200_DECODE_MMA=1: scores and P.V on mma.sync with fp16 hi/lo split operands (d_head 16).  Same tolerance
