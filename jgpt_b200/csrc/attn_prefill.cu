@@ -24,7 +24,8 @@ struct PrefillParams {
     const float2 *rope;
     const float *q, *k, *v;
     float *out;
-    float *out_image;  // != nullptr (d_head 16): write the output as the tcgen05 projection's operand image instead
+    float *out_image;        // != nullptr (d_head 16, an even number of heads): write the output as the tcgen05 projection's fp16 operand image instead
+    const float *out_scale;  // of that image: one power of two per column
     const PrefillSeq *seqs;
     int *status;
     int n_seqs, n_rows, H, layer, n_blocks, mbs, max_positions;
@@ -344,21 +345,19 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     const float iA = 1.f / fmaxf(lA, 1e-12f), iB = 1.f / fmaxf(lB, 1e-12f);
     const size_t D = (size_t)P.H * DH;
     if (P.out_image) {
-        // Operand image of the next projection (see gemm_umma.cu): 128-row tiles x 16-wide k tiles, TF32 high parts
-        // then low parts; head h is k tile h.  Lane (g, t) holds columns 8j + 2t, 8j + 2t + 1: half of the 16-byte
-        // chunk 2j + t / 2, so a warp store covers eight rows x two chunks = two full 128-byte lines.
+        // fp16 operand image of the next projection (see gemm_umma.cu): 128-row tiles x 32-wide k tiles, high parts then low
+        // parts; head h is half of k tile h / 2.  Lane (g, t) holds columns 8 j + 2 t, 8 j + 2 t + 1 of the head, times the powers of two
+        // that the image's columns carry: a warp store covers eight rows x one 16-byte chunk = one full 128-byte line.
         auto put = [&](int row, int j, float a, float b) {
             const size_t grow = (size_t)sd.row0 + row;
-            float *tile = P.out_image + ((grow >> 7) * (size_t)P.H + h) * (size_t)(128 * 16 * 2);
-            const int rr = (int)(grow & 127), k4 = 2 * j + (t >> 1);
-            float *dst = tile + (rr >> 3) * 128 + k4 * 32 + (rr & 7) * 4 + (t & 1) * 2;
-            uint32_t ha, hb, la, lb;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ha) : "f"(a));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(b));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(la) : "f"(a - __uint_as_float(ha)));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(b - __uint_as_float(hb)));
-            *reinterpret_cast<float2 *>(dst) = make_float2(__uint_as_float(ha), __uint_as_float(hb));
-            *reinterpret_cast<float2 *>(dst + 128 * 16) = make_float2(__uint_as_float(la), __uint_as_float(lb));
+            const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
+            unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
+            const int rr = (int)(grow & 127);
+            unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
+            uint32_t hi, lo;
+            split_half2(a * up.x, b * up.y, hi, lo);
+            *reinterpret_cast<uint32_t *>(dst) = hi;
+            *reinterpret_cast<uint32_t *>(dst + 128 * 32 * 2) = lo;
         };
 #pragma unroll
         for (int j = 0; j < 2; j++) {
@@ -467,14 +466,14 @@ int32_t prefill_upload_descriptors(Pool *p, const int *seq_ids_host, const int *
 
 int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, const int *seq_ids_host,
                             const int *seq_starts_host, const int *rope_offsets_host, int n_seqs, float *out, float *out_image,
-                            bool skip_append, int fast_mode) {
-    JGPT_REQUIRE(!out_image || p->dhead == 16, JGPT_ERR_INVALID_ARGUMENT, "image output needs d_head 16");
+                            const float *out_scale, bool skip_append, int fast_mode) {
+    JGPT_REQUIRE(!out_image || (p->dhead == 16 && p->heads % 2 == 0 && out_scale), JGPT_ERR_INVALID_ARGUMENT, "image output needs d_head 16 and pairs of heads");
     int max_S = 0, n_rows = 0;
     int32_t rc0 = prefill_upload_descriptors(p, seq_ids_host, seq_starts_host, rope_offsets_host, n_seqs, &max_S, &n_rows);
     if (rc0) return rc0;
     PrefillParams P;
     memset(&P, 0, sizeof(P));
-    P.kv = p->kv, P.table = p->d_table, P.rope = p->d_rope, P.q = q, P.k = k, P.v = v, P.out = out, P.out_image = out_image;
+    P.kv = p->kv, P.table = p->d_table, P.rope = p->d_rope, P.q = q, P.k = k, P.v = v, P.out = out, P.out_image = out_image, P.out_scale = out_scale;
     P.seqs = reinterpret_cast<const PrefillSeq *>(p->d_prefill_desc), P.status = p->ctx->d_status;
     P.n_seqs = n_seqs, P.n_rows = n_rows, P.H = p->heads, P.layer = layer, P.n_blocks = p->n_blocks;
     P.mbs = p->max_blocks_per_seq, P.max_positions = p->max_positions;

@@ -29,13 +29,6 @@ namespace rows {
 
 constexpr int kWarps = 8, kThreads = 256, kRows = 16;
 
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(x, y);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
-    hi = *reinterpret_cast<const uint32_t *>(&h), lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-
 // One CTA per 8 columns: a warp per column finds its largest element, then every lane writes its 16 bytes per 16 k.  Inside 16 k the
 // tensor core's positions 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of lane t hold k = 4 t .. 4 t + 3, so that a row's four elements are one load.
 __global__ void __launch_bounds__(256) pack_kernel(const float *W, const float *W3, const float *gamma, int K, int N, uint4 *image, float *unscale) {

@@ -20,6 +20,20 @@
 // Activation images are written by whatever produces the activation: the RMSNorm packer, the SwiGLU epilogue
 // of the W1/W3 product, or the plain packer (attention output).
 //
+// fp16 images (kind::f16, the forward step of models with d_head 16).  The same 22 bits of an operand as an fp16 high and an fp16
+// low part: two bytes each instead of four, and the tensor cores take 16 k per step instead of 8 at the same rate, so a
+// product costs half the time and half the operand traffic.  A 16-byte chunk holds eight k, a k tile 32, everything else lies
+// where the TF32 layout has it.  What fp16's exponent lacks is made up by powers of two, which change no bit:
+//   weights: per column of W, from its largest element; undone in the epilogue (the factors stand behind the image);
+//   RMSNorm rows: per row, from the row's largest element; undone in the epilogue;
+//   attention and SwiGLU results, whose rows no single CTA sees: per column, from what the column can reach at all.  A normalised row
+//   is at most sqrt(D) long, so |v_n| <= sqrt(D) |gamma o Wv_n|, an attention output is a weighted mean of such values, and
+//   |h g sigmoid(g)| <= D |gamma o W1_n| |gamma o W3_n|.  The next weight's rows are divided by the same powers.
+// An element 2^18 below the largest its scale allows for keeps its 22 bits; below that an absolute error 2^-40 of it remains.
+// The attention output of a prefill is such a mean because every key it sees was produced by the same call's Q,K,V product.
+// Measured for 32 x 1024 tokens, 24 heads of 16 (ncu, us per launch, TF32 -> fp16 images): Q,K,V 139 -> 91, W1/W3 + SwiGLU 164 -> 116,
+// Wo / W2 87 -> 73, RMSNorm 26.8 -> 21.5; the prefill of 12 layers 9.9 -> 7.8 ms.
+//
 // Roles in the 320-thread CTA: warp 0 lane 0 issues the bulk copies, warp 1 allocates tensor memory and its
 // lane 0 issues the MMAs, warps 2-9 are the epilogue (TMEM lane quarter = warp % 4, two warps per quarter).  Stages are handed over
 // with mbarriers: full[s] by the copies' complete_tx, empty[s] and "accumulator buffer ready" by
@@ -153,6 +167,179 @@ __global__ void __launch_bounds__(256) rmsnorm_pack_kernel(const float *__restri
     }
 }
 
+// ---- fp16 images ----
+// Byte offset of the 16-byte chunk (row rr, eight k) inside one half (high or low) of a tile.
+__device__ __forceinline__ int half_chunk(int rr, int k8) { return (rr >> 3) * 512 + k8 * 128 + (rr & 7) * 16; }
+__device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo) {
+    split_pair(v[0], v[1], hi.x, lo.x), split_pair(v[2], v[3], hi.y, lo.y);
+    split_pair(v[4], v[5], hi.z, lo.z), split_pair(v[6], v[7], hi.w, lo.w);
+}
+// One thread per column: up[n] brings the column's largest element (row k divided by k_scale[k]) to [2^14, 2^15), un[n] undoes it.
+// Image row r is column r of W, or, for a pair, column (r / 256) * 128 + r % 128 of W1 (first 128 rows of a 256-row tile) or W3; the
+// factors of W1's rows also carry out_scale, so that the gated product leaves the epilogue scaled for the next image.
+__device__ __forceinline__ const float *half_source(const float *W, const float *W3, int r, int &col) {
+    if (!W3) return col = r, W;
+    col = (r >> 8) * 128 + (r & 127);
+    return r & 128 ? W3 : W;
+}
+__global__ void __launch_bounds__(256) half_scale_kernel(const float *W, const float *W3, const float *k_scale, const float *out_scale, int K, int N,
+                                                         int rows, float *un, float *up) {
+    const int r = blockIdx.x * 256 + threadIdx.x;
+    if (r >= rows) return;
+    int col;
+    const float *src = half_source(W, W3, r, col);
+    float mx = 0.f;
+    if (col < N)
+        for (int k = 0; k < K; k++) mx = fmaxf(mx, fabsf(src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f)));
+    float a, b;
+    pow2_scale(mx, a, b);
+    up[r] = a;
+    un[r] = (W3 && !(r & 128)) ? b * out_scale[col] : b;
+}
+template <int TR>
+__global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const float *W3, const float *k_scale, const float *up, int K, int N,
+                                                        uint8_t *image) {
+    const int kt = blockIdx.x, rt = blockIdx.y, nkt = K / HBK;
+    uint8_t *tile = image + ((size_t)rt * nkt + kt) * (size_t)(TR * HBK * 4);
+    for (int e = threadIdx.x; e < TR * 4; e += 256) {
+        const int rr = e % TR, k8 = e / TR, r = rt * TR + rr;
+        int col;
+        const float *src = half_source(W, W3, r, col);
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int k = kt * HBK + k8 * 8 + q;
+            v[q] = col < N ? src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f) * up[r] : 0.f;
+        }
+        uint4 hi, lo;
+        split8(v, hi, lo);
+        *reinterpret_cast<uint4 *>(tile + half_chunk(rr, k8)) = hi;
+        *reinterpret_cast<uint4 *>(tile + TR * HBK * 2 + half_chunk(rr, k8)) = lo;
+    }
+}
+__global__ void __launch_bounds__(256) column_scale_kernel(const float *W, const float *W3, const float *gamma, int K, int N, float *scale) {
+    const int n = blockIdx.x * 256 + threadIdx.x;
+    if (n >= N) return;
+    float a = 0.f, b = 0.f;
+    for (int k = 0; k < K; k++) {
+        const float g = gamma[k], x = g * W[(size_t)k * N + n], y = W3 ? g * W3[(size_t)k * N + n] : 0.f;
+        a += x * x, b += y * y;
+    }
+    const float reach = W3 ? (float)K * sqrtf(a) * sqrtf(b) : sqrtf((float)K) * sqrtf(a);
+    float up, un;
+    pow2_scale(reach, up, un);
+    scale[n] = up;
+}
+// RMSNorm of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers between the
+// sum of squares and the product.
+constexpr int kKept = 16;
+__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, const float *__restrict__ gamma, int M, int D, float eps,
+                                                                uint8_t *__restrict__ image, float *__restrict__ a_un) {
+    extern __shared__ __align__(16) float rp_rows[];  // [8][D + 4]
+    const int tid = threadIdx.x, rr = tid >> 5, lane = tid & 31;
+    const int row = blockIdx.x * 8 + rr;
+    const int stride = D + 4;
+    const float *xr = x + (size_t)(row < M ? row : 0) * D;
+    float *mine = rp_rows + rr * stride;
+    const bool kept = D <= 32 * kKept;
+    float v[kKept], ss[4] = {0.f, 0.f, 0.f, 0.f};
+    if (kept) {
+#pragma unroll
+        for (int i = 0; i < kKept; i++) v[i] = (32 * i + lane < D && row < M) ? xr[32 * i + lane] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kKept; i++) ss[i & 3] += v[i] * v[i];
+    } else if (row < M) {
+        for (int j0 = 0; j0 < D; j0 += 128) {
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                const int j = j0 + 32 * w + lane;
+                if (j < D) ss[w] += xr[j] * xr[j];
+            }
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < 4; w++)
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) ss[w] += __shfl_xor_sync(0xffffffffu, ss[w], off);
+    const float tot = ss[0] + ss[1] + ss[2] + ss[3];
+    const float rms = sqrtf(tot / (float)D + eps);
+    const float inv = (rms > 0.f && isfinite(rms)) ? (1.f / rms) : 0.f;
+    float mx = 0.f;
+    if (kept) {
+#pragma unroll
+        for (int i = 0; i < kKept; i++)
+            if (32 * i + lane < D) {
+                v[i] = v[i] * inv * gamma[32 * i + lane];
+                mx = fmaxf(mx, fabsf(v[i]));
+            }
+    } else {
+        for (int j = lane; j < D; j += 32) {
+            const float y = row < M ? xr[j] * inv * gamma[j] : 0.f;
+            mine[j] = y;
+            mx = fmaxf(mx, fabsf(y));
+        }
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    float up, un;
+    pow2_scale(mx, up, un);
+    if (lane == 0 && row < M) a_un[row] = un;
+    if (kept) {
+#pragma unroll
+        for (int i = 0; i < kKept; i++)
+            if (32 * i + lane < D) mine[32 * i + lane] = v[i] * up;
+    } else {
+        for (int j = lane; j < D; j += 32) mine[j] *= up;
+    }
+    __syncthreads();
+    const int nkt = D / HBK, mt = (blockIdx.x * 8) / BM, rg = ((blockIdx.x * 8) % BM) >> 3;
+    uint8_t *base = image + (size_t)mt * nkt * A_TILE_BYTES + rg * 512;
+    for (int e = tid; e < nkt * 32; e += 256) {
+        const int kt = e >> 5, k8 = (e >> 3) & 3, r8 = e & 7;
+        const float4 a = *reinterpret_cast<const float4 *>(&rp_rows[r8 * stride + kt * HBK + k8 * 8]);
+        const float4 b = *reinterpret_cast<const float4 *>(&rp_rows[r8 * stride + kt * HBK + k8 * 8 + 4]);
+        const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint4 hi, lo;
+        split8(w, hi, lo);
+        uint8_t *dst = base + (size_t)kt * A_TILE_BYTES + k8 * 128 + r8 * 16;
+        *reinterpret_cast<uint4 *>(dst) = hi;
+        *reinterpret_cast<uint4 *>(dst + BM * HBK * 2) = lo;
+    }
+}
+
+int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st) {
+    const int bn = tile_cols(N), tiles = (N + bn - 1) / bn, rows = tiles * bn;
+    float *un = image + (size_t)rows * K, *up = un + rows;
+    half_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(W, nullptr, k_scale, nullptr, K, N, rows, un, up);
+    dim3 grid(K / HBK, tiles);
+    uint8_t *im = reinterpret_cast<uint8_t *>(image);
+    if (bn == 256) half_pack_kernel<256><<<grid, 256, 0, st>>>(W, nullptr, k_scale, up, K, N, im);
+    else half_pack_kernel<192><<<grid, 256, 0, st>>>(W, nullptr, k_scale, up, K, N, im);
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *out_scale, int K, int F, float *image, cudaStream_t st) {
+    JGPT_REQUIRE(half_ok(K, F), JGPT_ERR_UNSUPPORTED, "pack_weight_pair_half: K=%d F=%d", K, F);
+    float *un = image + (size_t)2 * F * K, *up = un + 2 * F;
+    half_scale_kernel<<<(2 * F + 255) / 256, 256, 0, st>>>(W1, W3, nullptr, out_scale, K, F, 2 * F, un, up);
+    half_pack_kernel<256><<<dim3(K / HBK, F / 128), 256, 0, st>>>(W1, W3, nullptr, up, K, F, reinterpret_cast<uint8_t *>(image));
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st) {
+    column_scale_kernel<<<(N + 255) / 256, 256, 0, st>>>(W, W3, gamma, K, N, scale);
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+int32_t rmsnorm_pack_half(const float *x, const float *gamma, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
+    const size_t smem = sizeof(float) * 8 * (size_t)(D + 4);
+    JGPT_REQUIRE(D % HBK == 0 && smem <= 48 * 1024, JGPT_ERR_UNSUPPORTED, "rmsnorm_pack_half: d_model %d", D);
+    const int padded_rows = (M + BM - 1) / BM * BM;  // rows past M are written as zeros
+    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, gamma, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+
 int32_t pack_activations(const float *A, const int *rowsel, int M, int K, float *image, cudaStream_t st) {
     dim3 grid(K / BK, (M + BM - 1) / BM);
     pack_kernel<BM, false><<<grid, 256, 0, st>>>(A, rowsel, M, K, image);
@@ -191,11 +378,11 @@ int32_t pack_weight_pair(const float *W1, const float *W3, int K, int F, float *
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(LBO >> 4) << 16) | ((uint64_t)(SBO >> 4) << 32) | (1ull << 46);
 }
-// Instruction descriptor: D fp32 (bits 4-5 = 1), A and B TF32 (bits 7-9, 10-12 = 2), both K-major, N / 8 at
+// Instruction descriptor: D fp32 (bits 4-5 = 1), A and B TF32 or both f16 (bits 7-9, 10-12 = 2 or 0), both K-major, N / 8 at
 // bit 17, M / 16 at bit 24.
-template <int BN>
+template <int BN, bool HALF>
 __host__ __device__ constexpr uint32_t instr_desc() {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    return (1u << 4) | ((HALF ? 0u : 2u) << 7) | ((HALF ? 0u : 2u) << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_tf32_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -203,6 +390,14 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t tmem_d, uint64_t adesc, uin
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -224,12 +419,13 @@ struct TileWalk {
     int n_tiles_n, nb, total;  // tiles along N, products in the batch, total tiles
 };
 
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool HALF>
 __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__restrict__ Aimg, const Batch B, const TileWalk walk,
                                                                int M, int K, int N, int *__restrict__ status, const PagedAppendArgs pa) {
     constexpr int W_TILE_FLOATS = BN * BK * 2;
     constexpr uint32_t W_TILE_BYTES = W_TILE_FLOATS * 4, STAGE_BYTES = A_TILE_BYTES + W_TILE_BYTES;
-    constexpr uint32_t IDESC = instr_desc<BN>();
+    constexpr uint32_t IDESC = instr_desc<BN, HALF>();
+    constexpr int KT = HALF ? HBK : BK;  // k of a stage; the tile's bytes are the same
     static_assert(BN % 64 == 0 && BN <= 256 && (MODE != 1 || BN == 256), "bad tile width");
     static_assert(MODE >= 0 && MODE <= 3, "MODE 3: products 1 and 2 of the batch are K and V rows for the paged store");
     extern __shared__ uint8_t umma_smem_raw[];
@@ -239,7 +435,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
     volatile int *s_abort = &s_abort_mem;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nkt = K / BK;
+    const int nkt = K / KT;
     uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(umma_smem_raw) + 127) & ~(uintptr_t)127);
 
     if (tid == 0) {
@@ -299,13 +495,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                     const uint32_t a_hi = smem_u32(tiles + (size_t)s * STAGE_BYTES), a_lo = a_hi + A_TILE_BYTES / 2;
                     const uint32_t w_hi = a_hi + A_TILE_BYTES, w_lo = w_hi + W_TILE_BYTES / 2;
 #pragma unroll
-                    for (int ks = 0; ks < BK / 8; ks++) {
-                        const uint32_t adv = ks * 2 * LBO;  // two 16-byte core-matrix columns per K = 8 step
+                    for (int ks = 0; ks < 2; ks++) {
+                        const uint32_t adv = ks * 2 * LBO;  // two 16-byte core-matrix columns per K = 8 (f16: 16) step
                         const uint64_t ah = smem_desc(a_hi + adv), al = smem_desc(a_lo + adv);
                         const uint64_t wh = smem_desc(w_hi + adv), wl = smem_desc(w_lo + adv);
-                        mma_tf32_ss(acc, ah, wh, IDESC, (kt | ks) != 0);
-                        mma_tf32_ss(acc, al, wh, IDESC, 1);
-                        mma_tf32_ss(acc, ah, wl, IDESC, 1);
+                        if constexpr (HALF) {
+                            mma_f16_ss(acc, ah, wh, IDESC, (kt | ks) != 0);
+                            mma_f16_ss(acc, al, wh, IDESC, 1);
+                            mma_f16_ss(acc, ah, wl, IDESC, 1);
+                        } else {
+                            mma_tf32_ss(acc, ah, wh, IDESC, (kt | ks) != 0);
+                            mma_tf32_ss(acc, al, wh, IDESC, 1);
+                            mma_tf32_ss(acc, ah, wl, IDESC, 1);
+                        }
                     }
                     mma_commit(&empty_bar[s]);  // the stage is free once these MMAs have read it
                 }
@@ -337,6 +539,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
             }
+            // fp16 images: the factors that undo the operands' powers of two
+            const float a_un = (HALF && B.a_un && m < M) ? B.a_un[m] : 1.f;
+            const float *w_un = HALF ? (z == 0 ? B.Wimg[0] : (z == 1 ? B.Wimg[1] : B.Wimg[2])) +
+                                           (size_t)walk.n_tiles_n * nkt * W_TILE_FLOATS + (size_t)n_idx * BN
+                                     : nullptr;
+            auto unscale = [&](float (&v)[32], int c) {  // 32 columns of the tile from c on
+                if constexpr (HALF) {
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4) {
+                        const float4 u = __ldg(reinterpret_cast<const float4 *>(w_un + c + q));
+                        v[q] = v[q] * a_un * u.x, v[q + 1] = v[q + 1] * a_un * u.y, v[q + 2] = v[q + 2] * a_un * u.z, v[q + 3] = v[q + 3] * a_un * u.w;
+                    }
+                }
+            };
             int ok = 0;
             if (lane == 0) ok = mbar_wait_bounded(&acc_full[buf], round & 1u, status, s_abort) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -383,6 +599,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                     if (n0 + c0 >= N) break;  // uniform across the warp
                     float v[32];
                     load_acc32(acc, quarter, c0, v);
+                    unscale(v, c0);
                     if (row_ok) {
 #pragma unroll
                         for (int hh = 0; hh < 2; hh++) {
@@ -419,6 +636,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                     if (n0 + c0 >= N) break;  // uniform across the warp
                     float v[32];
                     load_acc32(acc, quarter, c0, v);
+                    unscale(v, c0);
                     if (m < M) {
 #pragma unroll
                         for (int q = 0; q < 8; q++) {
@@ -435,15 +653,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                     }
                 }
             } else {
-                // N is F here; the activation image has F / 16 k tiles per row tile.  Rows past M are zero in A,
+                // N is F here; the activation image has F / 16 (fp16: F / 32) k tiles per row tile.  Rows past M are zero in A,
                 // so h1 = g = 0 and zeros are written: the image stays fully defined.
-                const int out_nkt = N / BK;
+                const int out_nkt = N / KT;
                 float *__restrict__ out = B.C[0] + (size_t)m_idx * out_nkt * A_TILE_FLOATS + chunk_offset(rloc, 0);
 #pragma unroll 1
                 for (int c0 = half * 64; c0 < half * 64 + 64; c0 += 32) {
                     float h[32], g[32];
                     load_acc32(acc, quarter, c0, h);
                     load_acc32(acc, quarter, 128 + c0, g);
+                    unscale(h, c0), unscale(g, 128 + c0);
 #pragma unroll
                     for (int q = 0; q < 32; q++) {
                         const float gv = g[q];
@@ -453,6 +672,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                         else s = 1.f / (1.f + expf(-gv));
                         h[q] = h[q] * (gv * s);
                     }
+                    if constexpr (HALF) {  // these 32 columns are one k tile of the next product
+                        uint8_t *tile = reinterpret_cast<uint8_t *>(B.C[0] + ((size_t)m_idx * out_nkt + (n_idx * 128 + c0) / HBK) * A_TILE_FLOATS);
+#pragma unroll
+                        for (int k8 = 0; k8 < 4; k8++) {
+                            const float w[8] = {h[k8 * 8], h[k8 * 8 + 1], h[k8 * 8 + 2], h[k8 * 8 + 3], h[k8 * 8 + 4], h[k8 * 8 + 5], h[k8 * 8 + 6], h[k8 * 8 + 7]};
+                            uint4 hi, lo;
+                            split8(w, hi, lo);
+                            *reinterpret_cast<uint4 *>(tile + half_chunk(rloc, k8)) = hi;
+                            *reinterpret_cast<uint4 *>(tile + BM * HBK * 2 + half_chunk(rloc, k8)) = lo;
+                        }
+                    } else {
 #pragma unroll
                     for (int q = 0; q < 32; q += 4) {
                         const int k = n_idx * 128 + c0 + q;  // column of the activation = k of the next product
@@ -461,6 +691,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                         float *dst = out + (size_t)(k / BK) * A_TILE_FLOATS + ((k % BK) >> 2) * 32;
                         *reinterpret_cast<float4 *>(dst) = hi;
                         *reinterpret_cast<float4 *>(dst + BM * BK) = lo;
+                    }
                     }
                 }
             }
@@ -488,48 +719,72 @@ static int sm_count_of_current_device() {
     return c > 0 ? c : 1;
 }
 
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool HALF = false>
 static int32_t launch_t(const TileWalk &walk, const float *Aimg, const Batch &b, int M, int K, int N, int *d_status, cudaStream_t st,
                         const PagedAppendArgs &pa = PagedAppendArgs()) {
     constexpr uint32_t smem = smem_bytes<BN, STAGES>();
-    JGPT_CUDA_TRY(cudaFuncSetAttribute(gemm_umma_kernel<BN, STAGES, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JGPT_CUDA_TRY(cudaFuncSetAttribute(gemm_umma_kernel<BN, STAGES, MODE, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int grid = walk.total < sm_count_of_current_device() ? walk.total : sm_count_of_current_device();
-    gemm_umma_kernel<BN, STAGES, MODE><<<grid, THREADS, smem, st>>>(Aimg, b, walk, M, K, N, d_status, pa);
+    gemm_umma_kernel<BN, STAGES, MODE, HALF><<<grid, THREADS, smem, st>>>(Aimg, b, walk, M, K, N, d_status, pa);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
 
-int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
-    JGPT_REQUIRE(shape_ok(K, N) && M > 0 && nb >= 1 && nb <= 3, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma: unsupported shape M=%d K=%d N=%d", M, K, N);
+template <bool HALF>
+static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
+    JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && nb >= 1 && nb <= 3, JGPT_ERR_INVALID_ARGUMENT,
+                 "gemm_umma: unsupported shape M=%d K=%d N=%d", M, K, N);
     const int bn = tile_cols(N);
     TileWalk walk{(N + bn - 1) / bn, nb, 0};
     walk.total = walk.n_tiles_n * nb * ((M + BM - 1) / BM);
     bool residual = b.R[0] != nullptr;
     for (int z = 0; z < nb; z++)
         JGPT_REQUIRE((b.R[z] != nullptr) == residual, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma: residuals for all products of a batch or for none");
-    if (bn == 256) return residual ? launch_t<256, 4, 2>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<256, 4, 0>(walk, Aimg, b, M, K, N, d_status, st);
-    return residual ? launch_t<192, 5, 2>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<192, 5, 0>(walk, Aimg, b, M, K, N, d_status, st);
+    if (bn == 256)
+        return residual ? launch_t<256, 4, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<256, 4, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st);
+    return residual ? launch_t<192, 5, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<192, 5, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st);
+}
+int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
+    return launch_rows<false>(Aimg, b, nb, M, K, N, d_status, st);
+}
+int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
+    return launch_rows<true>(Aimg, b, nb, M, K, N, d_status, st);
 }
 
-int32_t launch_qkv_paged(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status,
-                         cudaStream_t st) {
-    JGPT_REQUIRE(shape_ok(K, N) && M > 0 && N == pa.H * 16, JGPT_ERR_INVALID_ARGUMENT,
+template <bool HALF>
+static int32_t launch_qkv(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
+    JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && N == pa.H * 16, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma qkv: unsupported shape M=%d K=%d N=%d (heads %d, d_head 16)", M, K, N, pa.H);
     const int bn = tile_cols(N);
     TileWalk walk{(N + bn - 1) / bn, 3, 0};
     walk.total = walk.n_tiles_n * 3 * ((M + BM - 1) / BM);
-    if (bn == 256) return launch_t<256, 4, 3>(walk, Aimg, b, M, K, N, d_status, st, pa);
-    return launch_t<192, 5, 3>(walk, Aimg, b, M, K, N, d_status, st, pa);
+    if (bn == 256) return launch_t<256, 4, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa);
+    return launch_t<192, 5, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa);
+}
+int32_t launch_qkv_paged(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
+    return launch_qkv<false>(Aimg, b, M, K, N, pa, d_status, st);
+}
+int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
+    return launch_qkv<true>(Aimg, b, M, K, N, pa, d_status, st);
 }
 
-int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, int F, float *act_image, int *d_status,
-                      cudaStream_t st) {
-    JGPT_REQUIRE(swiglu_shape_ok(K, F) && M > 0, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
+template <bool HALF>
+static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
+                           cudaStream_t st) {
+    JGPT_REQUIRE(swiglu_shape_ok(K, F) && (!HALF || K % HBK == 0) && M > 0, JGPT_ERR_INVALID_ARGUMENT,
+                 "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
     Batch b{};
-    b.Wimg[0] = Wpair_img, b.C[0] = act_image;
+    b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un;
     TileWalk walk{F / 128, 1, 0};
     walk.total = walk.n_tiles_n * ((M + BM - 1) / BM);
-    return launch_t<256, 4, 1>(walk, Aimg, b, M, K, F, d_status, st);
+    return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st);
+}
+int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, int F, float *act_image, int *d_status, cudaStream_t st) {
+    return launch_pair<false>(Aimg, Wpair_img, nullptr, M, K, F, act_image, d_status, st);
+}
+int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
+                           cudaStream_t st) {
+    return launch_pair<true>(Aimg, Wpair_img, a_un, M, K, F, act_image, d_status, st);
 }
 
 }  // namespace umma

@@ -36,6 +36,7 @@ struct Batch {
     const float *Wimg[3];
     float *C[3];
     const float *R[3];  // optional residual, may alias C
+    const float *a_un = nullptr;  // fp16 images: one factor per row of A that undoes its power of two (nullptr: none)
 };
 // C_z[M, N] = A . W_z (+ R_z) for z < nb; needs K % 16 == 0 and N % 4 == 0.
 int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
@@ -48,6 +49,35 @@ int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, i
 // append kernel, without the fp32 round trip through memory.
 int32_t launch_qkv_paged(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status,
                          cudaStream_t st);
+
+// The same products on fp16 images (kind::f16): a k tile holds 32 k in the bytes of 16 TF32 ones, so an image has half the bytes
+// and a product half the tensor time.  See gemm_umma.cu for the scaling.
+constexpr int HBK = 32;
+inline bool half_ok(int D, int F) { return D % HBK == 0 && F % 128 == 0; }
+inline uint64_t half_activation_floats(int M, int K) { return image_floats(M, K, BM) / 2; }
+// W [K, N], row k divided by k_scale[k] if given -> image, then one float per image row that undoes that row's (column of W's) power
+// of two, then work space of the same size.
+inline uint64_t half_weight_floats(int K, int N) {
+    const uint64_t rows = (uint64_t)((N + tile_cols(N) - 1) / tile_cols(N)) * (uint64_t)tile_cols(N);
+    return rows * (uint64_t)K + 2 * rows;
+}
+inline uint64_t half_pair_floats(int K, int F) { return (uint64_t)2 * F * (uint64_t)K + 4 * (uint64_t)F; }
+// Where the attention leaves its output for the next product: the image and its columns' powers of two (no image: row major).
+struct ImageOut {
+    float *image = nullptr;
+    const float *scale = nullptr;
+};
+int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st);
+// out_scale[F]: the powers of two that launch_swiglu_half gives its result's columns.
+int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *out_scale, int K, int F, float *image, cudaStream_t st);
+// scale[n] = the power of two that keeps column n below 2^15 in fp16: of rmsnorm(x) W (gamma applied), or of h g sigmoid(g) with W3.
+int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st);
+// RMSNorm into an fp16 image; a_un[M] receives the rows' factors.
+int32_t rmsnorm_pack_half(const float *x, const float *gamma, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
+int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
+int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
+                           cudaStream_t st);
+int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st);
 
 inline bool shape_ok(int K, int N) { return K >= BK && K % BK == 0 && N % 4 == 0; }
 inline bool swiglu_shape_ok(int K, int F) { return K >= BK && K % BK == 0 && F % 128 == 0; }

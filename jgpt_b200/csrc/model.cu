@@ -44,6 +44,7 @@ struct Model {
     int umma_min_rows = 513;  // JGPT_B200_UMMA_MIN_ROWS; 0: never
     std::unordered_map<const float *, float *> wimg;   // weight images by source pointer; dropped when weights change
     std::unordered_map<const float *, float *> wpair;  // W1/W3 pair images by W1's pointer
+    std::unordered_map<const float *, float *> whalf;  // fp16 images, and the column scales of what they are fed (by the scaled weight's pointer + 1)
     float *aimg = nullptr, *aimg2 = nullptr;  // activation images (grow-only): [rows, d_model]-sized and [rows, d_ff]-sized
     uint64_t aimg_floats = 0, aimg2_floats = 0;
     // Decode-sized steps (rows <= 512): RMSNorm and SwiGLU live inside the projections.
@@ -108,6 +109,8 @@ static void drop_weight_images(Model *m) {
     for (auto &kv : m->w13i) cudaFree(kv.second);
     for (auto &kv : m->wscaled) cudaFree(kv.second);
     for (auto &kv : m->wrows) cudaFree(kv.second);
+    for (auto &kv : m->whalf) cudaFree(kv.second);
+    m->whalf.clear();
     m->wimg.clear(), m->wpair.clear(), m->w13i.clear(), m->wscaled.clear(), m->wrows.clear();
 }
 
@@ -894,17 +897,79 @@ static int32_t ensure_sample_work(Model *m, int rows) {
     return JGPT_OK;
 }
 
+// fp16 images of the prefill's weights and the powers of two their inputs carry, made once per weight set.
+static int32_t half_buffer(Model *m, const float *key, uint64_t floats, float **out, bool *fresh) {
+    auto it = m->whalf.find(key);
+    *fresh = it == m->whalf.end();
+    if (*fresh) {
+        float *buf = nullptr;
+        JGPT_CUDA_TRY(cudaMalloc(&buf, sizeof(float) * floats));
+        it = m->whalf.emplace(key, buf).first;
+    }
+    *out = it->second;
+    return JGPT_OK;
+}
+struct HalfLayer {
+    float *wq, *wk, *wv, *wo, *pair, *w2, *att_scale, *h_scale;
+};
+static int32_t half_layer(Model *m, const LayerW &y, HalfLayer *o) {
+    const int D = m->d_model, F = m->d_ff;
+    cudaStream_t st = m->ctx->stream;
+    int32_t rc;
+    bool fresh;
+    if ((rc = half_buffer(m, y.wv + 1, D, &o->att_scale, &fresh)) || (fresh && (rc = umma::column_scales(y.wv, nullptr, y.norm1, D, D, o->att_scale, st)))) return rc;
+    if ((rc = half_buffer(m, y.w1 + 1, F, &o->h_scale, &fresh)) || (fresh && (rc = umma::column_scales(y.w1, y.w3, y.norm2, D, F, o->h_scale, st)))) return rc;
+    struct { const float *W, *k_scale; int K; float **out; } one[5] = {
+        {y.wq, nullptr, D, &o->wq}, {y.wk, nullptr, D, &o->wk}, {y.wv, nullptr, D, &o->wv}, {y.wo, o->att_scale, D, &o->wo}, {y.w2, o->h_scale, F, &o->w2}};
+    for (auto &w : one)
+        if ((rc = half_buffer(m, w.W, umma::half_weight_floats(w.K, D), w.out, &fresh)) || (fresh && (rc = umma::pack_weight_half(w.W, w.k_scale, w.K, D, *w.out, st)))) return rc;
+    if ((rc = half_buffer(m, y.w1, umma::half_pair_floats(D, F), &o->pair, &fresh)) ||
+        (fresh && (rc = umma::pack_weight_pair_half(y.w1, y.w3, o->h_scale, D, F, o->pair, st)))) return rc;
+    return JGPT_OK;
+}
+
+// The decoder blocks for prefill-sized `rows` of a d_head-16 model on fp16 operand images: every activation is handed from producer to
+// consumer as an image (RMSNorm, attention, the W1/W3 product's SwiGLU epilogue), and the Q,K,V product writes K / V straight into
+// the paged store (paged->layer is set per layer here).
+template <class AttnFn>
+static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged, AttnFn &&attn) {
+    const int D = m->d_model, F = m->d_ff;
+    cudaStream_t st = m->ctx->stream;
+    int *status = m->ctx->d_status;
+    const uint64_t image = umma::half_activation_floats(rows, D);
+    int32_t rc = ensure_image(m, &m->aimg, &m->aimg_floats, image + (uint64_t)rows);  // the rows' factors behind it
+    if (rc) return rc;
+    if ((rc = ensure_image(m, &m->aimg2, &m->aimg2_floats, umma::half_activation_floats(rows, F)))) return rc;
+    float *a_un = m->aimg + image;
+    for (int l = 0; l < m->layers; l++) {
+        const LayerW &y = m->L[(size_t)l];
+        HalfLayer w;
+        if ((rc = half_layer(m, y, &w))) return rc;
+        umma::Batch qkv{}, wo{}, w2{};
+        qkv.Wimg[0] = w.wq, qkv.Wimg[1] = w.wk, qkv.Wimg[2] = w.wv;
+        qkv.C[0] = m->q, qkv.C[1] = m->k, qkv.C[2] = m->v, qkv.a_un = a_un;
+        wo.Wimg[0] = w.wo, wo.C[0] = m->x, wo.R[0] = m->x;  // x1 = x + attn.Wo (each element read then written by the same thread)
+        w2.Wimg[0] = w.w2, w2.C[0] = m->x, w2.R[0] = m->x;
+        if ((rc = umma::rmsnorm_pack_half(m->x, y.norm1, rows, D, m->eps, m->aimg, a_un, st))) return rc;
+        PagedAppendArgs pa = paged;
+        pa.layer = l;
+        if ((rc = umma::launch_qkv_paged_half(m->aimg, qkv, rows, D, D, pa, status, st))) return rc;
+        if ((rc = attn(l, umma::ImageOut{m->aimg, w.att_scale}, true))) return rc;
+        if ((rc = umma::launch_half(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
+        if ((rc = umma::rmsnorm_pack_half(m->x, y.norm2, rows, D, m->eps, m->aimg, a_un, st))) return rc;
+        if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, rows, D, F, m->aimg2, status, st))) return rc;
+        if ((rc = umma::launch_half(m->aimg2, w2, 1, rows, F, D, status, st))) return rc;
+    }
+    return JGPT_OK;
+}
+
 // One decoder block over `rows` rows already in m->x.  Attention is supplied by the caller.
-// The same decoder blocks for prefill-sized `rows`: every projection on the tcgen05 kernel, activations handed
-// from producer to consumer as operand images (RMSNorm writes one, the W1/W3 product's SwiGLU epilogue writes
-// one; only the attention output is packed by a kernel of its own).
-// attn(l, image, kv_in_cache): attention of layer l; writes the Wo operand image itself when image != nullptr, the
-// row-major m->att otherwise; kv_in_cache: the K / V rows of the layer are already in the paged store.
-// `paged` != nullptr (a prefill at d_head 16): the attention can write that image, and the Q,K,V product writes
-// K / V straight into the paged store (paged->layer is set per layer here).
+// The same decoder blocks for other head and feed-forward sizes, on TF32 images; the attention output is packed by a kernel of its own.
+// attn(l, image, kv_in_cache): attention of layer l; writes the Wo operand image itself when there is one, the row-major m->att
+// otherwise; kv_in_cache: the K / V rows of the layer are already in the paged store.
+// `paged` != nullptr (a prefill at d_head 16): the Q,K,V product writes K / V straight into the paged store.
 template <class AttnFn>
 static int32_t run_layers_umma(Model *m, int rows, const PagedAppendArgs *paged, AttnFn &&attn) {
-    const bool attn_writes_image = paged != nullptr;
     const int D = m->d_model, F = m->d_ff;
     cudaStream_t st = m->ctx->stream;
     int *status = m->ctx->d_status;
@@ -932,8 +997,8 @@ static int32_t run_layers_umma(Model *m, int rows, const PagedAppendArgs *paged,
         } else {
             if ((rc = umma::launch(m->aimg, qkv, 3, rows, D, D, status, st))) return rc;
         }
-        if ((rc = attn(l, attn_writes_image ? m->aimg : nullptr, paged != nullptr))) return rc;
-        if (!attn_writes_image && (rc = umma::pack_activations(m->att, nullptr, rows, D, m->aimg, st))) return rc;
+        if ((rc = attn(l, umma::ImageOut{}, paged != nullptr))) return rc;
+        if ((rc = umma::pack_activations(m->att, nullptr, rows, D, m->aimg, st))) return rc;
         if ((rc = umma::launch(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
         if ((rc = umma::rmsnorm_pack(m->x, y.norm2, rows, D, m->eps, m->aimg, st))) return rc;
         if (fused_ffn) {
@@ -1108,7 +1173,7 @@ static int32_t run_layers_small(Model *m, int rows, AttnFn &&attn) {
         if (fresh_qkv) n1.pdl &= ~1;
         float *Cqkv[3] = {m->q, m->k, m->v};
         if ((rc = small_launch<true, 0>(m, m->x, rows, D, D, 3, Wqkv, Cqkv, nullptr, nullptr, n1))) return rc;
-        if ((rc = attn(l, nullptr, false))) return rc;
+        if ((rc = attn(l, umma::ImageOut{}, false))) return rc;
         const float *Wo[1] = {y.wo};
         float *Cx[1] = {m->x};
         const float *Rx[1] = {m->x};  // x1 = x + attn.Wo (each element read then written by the same thread)
@@ -1188,7 +1253,7 @@ static int32_t run_layers_rows(Model *m, int n, AttnFn &&attn) {
             if ((rc = rows_image(m, w[z], nullptr, y.norm1, D, D, &qkv.image[z], &fresh))) return rc;
         if ((rc = rows::launch(rows::NORM, m->ctx, m->x, qkv, 3, n, D, D, nullptr,
                                fuse(m->ss_a, nullptr, parts, ov >= 3 && (l > 0 || m->first_launch_early) && !fresh, ov >= 1)))) return rc;
-        if ((rc = attn(l, nullptr, false))) return rc;
+        if ((rc = attn(l, umma::ImageOut{}, false))) return rc;
         if ((rc = residual(m->att, y.wo, D, m->ss_b, ov >= 2))) return rc;
         rows::Batch w13{{nullptr}, {m->h1}};
         fresh = false;
@@ -1206,8 +1271,10 @@ static int32_t run_layers(Model *m, int rows, const PagedAppendArgs *paged, Attn
     if (rows_mode(m, rows)) return run_layers_rows(m, rows, attn);
     if (small_mode(m, rows)) return run_layers_small(m, rows, attn);
     if (!m->strict && m->umma_min_rows > 0 && rows >= m->umma_min_rows && umma::shape_ok(D, D) && umma::shape_ok(D, F) &&
-        umma::shape_ok(F, D) && sizeof(float) * 8 * (size_t)(D + 4) <= 48 * 1024)
+        umma::shape_ok(F, D) && sizeof(float) * 8 * (size_t)(D + 4) <= 48 * 1024) {
+        if (paged && umma::half_ok(D, F)) return run_layers_half(m, rows, *paged, attn);
         return run_layers_umma(m, rows, paged, attn);
+    }
     cudaStream_t st = m->ctx->stream;
     for (int l = 0; l < m->layers; l++) {
         const LayerW &y = m->L[(size_t)l];
@@ -1216,7 +1283,7 @@ static int32_t run_layers(Model *m, int rows, const PagedAppendArgs *paged, Attn
         float *Cqkv[3] = {m->q, m->k, m->v};
         int32_t rc = gemm(m, m->xn, rows, D, D, 3, Wqkv, Cqkv, nullptr);
         if (rc) return rc;
-        rc = attn(l, nullptr, false);
+        rc = attn(l, umma::ImageOut{}, false);
         if (rc) return rc;
         const float *Wo[1] = {y.wo};
         float *Co[1] = {m->x};
@@ -1835,8 +1902,8 @@ int32_t jgpt_forward_prefill_batch(jgpt_model h, jgpt_kvpool poolh, const int32_
         pa.max_positions = p->max_positions;
         paged = &pa;
     }
-    rc = run_layers(m, rows, paged, [&](int l, float *image, bool kv_in_cache) {
-        return launch_attn_prefill(p, l, m->q, m->k, m->v, seq_ids_host, seq_starts_host, rope_offsets_host, n, m->att, image,
+    rc = run_layers(m, rows, paged, [&](int l, umma::ImageOut out, bool kv_in_cache) {
+        return launch_attn_prefill(p, l, m->q, m->k, m->v, seq_ids_host, seq_starts_host, rope_offsets_host, n, m->att, out.image, out.scale,
                                    kv_in_cache, m->prefill_fast);
     });
     if (rc) return rc;
@@ -1945,7 +2012,7 @@ static int32_t forward_decode_impl(jgpt_model h, jgpt_kvpool poolh, const int32_
         m->first_launch_early = chain_early;
         if (no_copies) embed_pos_kernel<<<n, 128, 0, st>>>(m->tok, m->pos, nullptr, nullptr, m->x, m->d_model, m->ss_a, m->hd_idx, m->d_idx, R);
         else embed_pos_kernel<<<n, 128, 0, st>>>(m->tok, m->pos, m->d_idx, m->d_idx + R, m->x, m->d_model, m->ss_a);
-        int32_t r2 = run_layers(m, n, nullptr, [&](int l, float *, bool) {
+        int32_t r2 = run_layers(m, n, nullptr, [&](int l, umma::ImageOut, bool) {
             return launch_attn_decode(p, l, 1, m->q, m->k, m->v, m->d_idx + 2 * R, m->d_idx + 3 * R, m->d_idx + 4 * R, n, len_bucket, m->att,
                                       (small_mode(m, n) && step_overlap_level(m, n) >= 1) ? 2 : -1);
         });

@@ -121,6 +121,13 @@ __device__ __forceinline__ void pow2_scale(float mx, float &s, float &inv) {
     const int f = min(268 - e, 253);
     s = __uint_as_float((uint32_t)f << 23), inv = __uint_as_float((uint32_t)(254 - f) << 23);
 }
+// An fp32 pair as fp16 high and low parts, 11 + 11 bits.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h), lo = *reinterpret_cast<const uint32_t *>(&l);
+}
 
 // Four 8x8 b16 matrices from shared memory; lane l supplies the address of row (l % 8) of matrix (l / 8).
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void *smem_row) {

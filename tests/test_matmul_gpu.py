@@ -222,3 +222,64 @@ def test_ragged_batched_prefill_on_the_tcgen05_path(ctx):
             assert not k[:, len(pr):].any() and not v[:, len(pr):].any()
     finally:
         pool.close(), gm.close(), om.close()
+
+
+@pytest.mark.parametrize("dm,dff", [(64, 128), (96, 256), (384, 768), (256, 384)])
+@pytest.mark.parametrize("part", ["attention", "feed forward"])
+@pytest.mark.parametrize("spread", [0.0, 3.0])
+def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, part, spread):
+    """600 prompts of one token (a ragged last row tile) through one block with one of its parts switched off, on the fp16 operand images:
+    a token that sees itself alone has its own value as attention output.  spread: rows, and columns of the weights in front of a
+    part with the inverse behind it, scaled by up to 10^spread either way, which fp16 parts survive only with their powers of two.
+
+    Tolerance: operands of 22 bits and fewer than 128 fp32 additions of parts no larger than sum |x w| keep a product within
+    2 * 2^-22 + 128 * 2^-24 < 1e-5 of sum |x w|; a value is rounded to fp16 (2^-11); what reaches the last norm is relative to its row."""
+    V, n = 132, 600
+    rng = np.random.default_rng(dm + dff)
+
+    def scales(k):
+        return 10.0 ** rng.uniform(-spread, spread, k)
+
+    def mat(a, b):
+        return rng.standard_normal((a, b)) / np.sqrt(a)
+
+    sv, sf = scales(dm), scales(dff)
+    tok = rng.standard_normal((V, dm)) * scales(V)[:, None]
+    wq, wk, wv, wo = mat(dm, dm), mat(dm, dm), mat(dm, dm) * sv, mat(dm, dm) / sv[:, None]
+    w1, w2, w3 = mat(dm, dff) * sf, mat(dff, dm) / sf[:, None], mat(dm, dff)
+    if part == "attention":
+        w2 = 0 * w2
+    else:
+        wo = 0 * wo
+    n1, n2, nf = (1 + 0.2 * rng.standard_normal(dm) for _ in range(3))
+    T = [np.ascontiguousarray(t, np.float32) for t in (tok, np.zeros((64, dm)), wq, wk, wv, wo, w1, w2, w3, n1, n2, nf, mat(dm, V))]
+    gm = GPTModel(ctx, V, 64, dm, dm // 16, 1, dff, rmsNormEps=1e-6, maxRows=n)
+    gm.setParameters(T)
+    pool = gm.newPool(n, n)
+    try:
+        ids = rng.integers(0, V, n).astype(np.int32)
+        got, _ = gm.forwardPrefillBatch(pool, [pool.seq_alloc() for _ in range(n)], [[i] for i in ids])
+        tok, _, _, _, wv, wo, w1, w2, w3, n1, n2, nf, head = (t.astype(np.float64) for t in T)
+
+        def rms(x):
+            return np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+
+        x, E = tok[ids], 1e-5
+        if part == "attention":
+            h = x / rms(x) * n1
+            v = h @ wv
+            off = (2.0 ** -11 * np.abs(v) + E * (np.abs(h) @ np.abs(wv))) @ np.abs(wo) + E * (np.abs(v) @ np.abs(wo))
+            y = x + v @ wo
+        else:
+            h = x / rms(x) * n2
+            a, g = h @ w1, h @ w3
+            act = a * g / (1 + np.exp(-g))
+            off = E * ((np.abs(h) @ np.abs(w1)) * np.abs(g) + 1.2 * np.abs(a) * (np.abs(h) @ np.abs(w3)) + np.abs(act)) @ np.abs(w2)
+            y = x + act @ w2
+        off = off + 1e-6 * np.abs(y)
+        z = y / rms(y) * nf
+        off_z = off / rms(y) * np.abs(nf) + np.sqrt((off ** 2).mean(-1, keepdims=True)) / rms(y) * np.abs(z)
+        bound = off_z @ np.abs(head) + E * (np.abs(z) @ np.abs(head))
+        assert np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
+    finally:
+        pool.close(), gm.close()
