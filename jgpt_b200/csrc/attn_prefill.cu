@@ -29,6 +29,7 @@ struct PrefillParams {
     const PrefillSeq *seqs;
     int *status;
     int n_seqs, n_rows, H, layer, n_blocks, mbs, max_positions;
+    int pdl;  // 1: launched as a programmatic dependent; the kernel in front writes q, K and V, not descriptors, tables or angles
     float scale_log2e;
 };
 
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     const PrefillSeq sd = P.seqs[blockIdx.z];
     const int h = blockIdx.y;
     const int r0 = blockIdx.x * kQTile;
-    if (r0 >= sd.S) return;
+    if (r0 >= sd.S) return;  // (a CTA that leaves stands in nobody's way)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int nblk = min((sd.S + BT - 1) / BT, (r0 + kQTile - 1) / BT + 1);  // causal: nothing beyond the tile's last row
     for (int b = tid; b < nblk; b += blockDim.x) {
@@ -170,6 +171,10 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
         for (int b = 0; b < nb; b++)
             bulk_g2s(&tiles[c & 1][b][0], kv_head + (size_t)s_table[b0 + b] * block_stride, TILE_BYTES, &full_bar[c & 1]);
     };
+    if (P.pdl) {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
     if (tid == 0) issue(0);
 
     // ---- this warp's 16 query rows: RoPE, scale, split into fp16 hi/lo A fragments ----
@@ -464,13 +469,9 @@ int32_t prefill_upload_descriptors(Pool *p, const int *seq_ids_host, const int *
     return JGPT_OK;
 }
 
-int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, const int *seq_ids_host,
-                            const int *seq_starts_host, const int *rope_offsets_host, int n_seqs, float *out, float *out_image,
-                            const float *out_scale, bool skip_append, int fast_mode) {
+int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, int n_seqs, int max_S, int n_rows, float *out,
+                            float *out_image, const float *out_scale, bool skip_append, int fast_mode, int pdl) {
     JGPT_REQUIRE(!out_image || (p->dhead == 16 && p->heads % 2 == 0 && out_scale), JGPT_ERR_INVALID_ARGUMENT, "image output needs d_head 16 and pairs of heads");
-    int max_S = 0, n_rows = 0;
-    int32_t rc0 = prefill_upload_descriptors(p, seq_ids_host, seq_starts_host, rope_offsets_host, n_seqs, &max_S, &n_rows);
-    if (rc0) return rc0;
     PrefillParams P;
     memset(&P, 0, sizeof(P));
     P.kv = p->kv, P.table = p->d_table, P.rope = p->d_rope, P.q = q, P.k = k, P.v = v, P.out = out, P.out_image = out_image, P.out_scale = out_scale;
@@ -497,8 +498,13 @@ int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, 
         dim3 grid((unsigned)((max_S + kQTile - 1) / kQTile), (unsigned)p->heads, (unsigned)n_seqs);
         const size_t smem = sizeof(int) * (size_t)((max_S + kBlockTokens - 1) / kBlockTokens);
         const bool fast = fast_mode < 0 ? p->prefill_fast != 0 : fast_mode != 0;
-        if (fast) attn_prefill_mma_kernel<true><<<grid, 128, smem, st>>>(P);
-        else attn_prefill_mma_kernel<false><<<grid, 128, smem, st>>>(P);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        P.pdl = pdl && skip_append;  // behind the append kernel: an ordinary launch
+        cfg.gridDim = grid, cfg.blockDim = dim3(128), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = P.pdl ? 1 : 0;
+        JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, fast ? attn_prefill_mma_kernel<true> : attn_prefill_mma_kernel<false>, P));
     } else {
         dim3 grid((unsigned)((max_S + 127) / 128), (unsigned)p->heads, (unsigned)n_seqs);
         switch (DH) {
@@ -526,5 +532,8 @@ extern "C" int32_t jgpt_attn_prefill(jgpt_kvpool pool, int32_t layer, const floa
     if (n_seqs == 0) return JGPT_OK;
     JGPT_REQUIRE(n_seqs > 0 && q_dev && k_dev && v_dev && seq_ids_host && seq_starts_host && rope_offsets_host && out_dev,
                  JGPT_ERR_INVALID_ARGUMENT, "null pointer or negative count");
-    return launch_attn_prefill(p, layer, q_dev, k_dev, v_dev, seq_ids_host, seq_starts_host, rope_offsets_host, n_seqs, out_dev);
+    int max_S = 0, n_rows = 0;
+    int32_t rc = prefill_upload_descriptors(p, seq_ids_host, seq_starts_host, rope_offsets_host, n_seqs, &max_S, &n_rows);
+    if (rc) return rc;
+    return launch_attn_prefill(p, layer, q_dev, k_dev, v_dev, n_seqs, max_S, n_rows, out_dev);
 }

@@ -284,10 +284,9 @@ int32_t launch_kv_scrub(Pool *p, const std::vector<int> &blocks);
 int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, const float *k_new,
                            const float *v_new, const int *seq_ids, const int *rope_pos, const int *lens, int n,
                            int max_len, float *out, int overlap = -1);  // overlap < 0: the pool's setting
-int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v,
-                            const int *seq_ids_host, const int *seq_starts_host, const int *rope_offsets_host,
-                            int n_seqs, float *out, float *out_image = nullptr, const float *out_scale = nullptr, bool skip_append = false,
-                            int fast_mode = -1);
+int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, int n_seqs, int max_S, int n_rows, float *out,
+                            float *out_image = nullptr, const float *out_scale = nullptr, bool skip_append = false, int fast_mode = -1,
+                            int pdl = 0);
 
 #ifdef JGPT_B200_DECODE_TRACE
 // Step timeline (trace builds only, never in the shipped library): per launch of the multi-launch decode step, the

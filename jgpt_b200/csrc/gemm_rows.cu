@@ -88,7 +88,7 @@ constexpr int per_sm() { return S * NT <= 12 && S <= 4 ? 2 : 1; }
 
 template <int S, int NT, int KIND>
 __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(const float *A, const Batch B, int M, int K, int N, const int *rowsel,
-                                                                                  const Fuse F, int two_tiles) {
+                                                                                  const Fuse F, int two_tiles, const PagedAppendArgs pa) {
     constexpr int BN = NT * 8, AS = slice_stride<S>(), RS = BN + 8;
     constexpr int OUT = KIND == NORM_SWIGLU ? BN / 2 : BN;  // columns of the result per CTA
     constexpr int PER = kRows * OUT / kThreads;             // of them per thread: columns fixed, rows row0 + i * kThreads / OUT
@@ -143,7 +143,38 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
     for (; rt < row_tiles; rt += gridDim.y) {
         if (two_tiles && rt + (int)gridDim.y < row_tiles) fetch(rt + gridDim.y, buf ^ 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        // what the epilogue adds or multiplies, requested now
+        // what the epilogue adds or multiplies, and where its rows go, requested now
+        __half *kv_at[KIND == NORM_PAGED ? PER : 1];
+        float2 turn[KIND == NORM_PAGED ? PER : 1];
+        int dead[KIND == NORM_PAGED ? PER : 1];  // slots of the block behind the prompt's last row
+        if (KIND == NORM_PAGED) {
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int m = rt * kRows + row0 + i * (kThreads / OUT);
+                kv_at[i] = nullptr, turn[i] = make_float2(1.f, 0.f), dead[i] = 0;
+                if (z > 0 && m < M && col_ok) {
+                    int lo = 0, hi = pa.n_seqs - 1;
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (pa.seqs[mid].row0 <= m) lo = mid; else hi = mid - 1;
+                    }
+                    const PrefillSeq sd = pa.seqs[lo];
+                    const int slot = m - sd.row0, rp = sd.rope_off + slot;
+                    const bool pos_ok = slot >= 0 && slot < sd.S && rp >= 0 && rp < pa.max_positions;
+                    const int phys = pos_ok ? pa.table[(size_t)sd.seq_id * pa.mbs + slot / kBlockTokens] : 0;
+                    if (!pos_ok) {
+                        atomicOr(pa.status, DEV_STATUS_BAD_POSITION);
+                    } else if (phys < 0 || phys >= pa.n_blocks) {
+                        atomicOr(pa.status, DEV_STATUS_BAD_BLOCK);
+                    } else {
+                        kv_at[i] = pa.kv + (((size_t)pa.layer * pa.n_blocks + phys) * pa.H + col / 16) * (size_t)(2 * kBlockTokens * 16) +
+                                   (z == 2 ? kBlockTokens * 16 : 0) + (slot % kBlockTokens) * 16 + (col & 15);
+                        dead[i] = slot == sd.S - 1 ? kBlockTokens - 1 - slot % kBlockTokens : 0;
+                        if (z == 1) turn[i] = pa.rope[(size_t)rp * 8 + (col & 15) / 2];
+                    }
+                }
+            }
+        }
         float extra[PER];
 #pragma unroll
         for (int i = 0; i < PER; i++) {
@@ -234,7 +265,19 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
                     else sg = 1.f / (1.f + expf(-v2));
                     v = v * (v2 * sg);
                 }
-                if (m < M && col_ok) C[(size_t)m * Nout + col] = v;
+                if (KIND == NORM_PAGED && z > 0) {  // the even lane of a pair of columns stores both
+                    const float v_odd = __shfl_xor_sync(0xffffffffu, v, 1);
+                    if (kv_at[i] && !(lane & 1)) {
+                        const float2 w = turn[i];
+                        const __half2 p = z == 1 ? __floats2half2_rn(__fsub_rn(__fmul_rn(v, w.x), __fmul_rn(v_odd, w.y)),
+                                                                     __fadd_rn(__fmul_rn(v, w.y), __fmul_rn(v_odd, w.x)))
+                                                 : __floats2half2_rn(v, v_odd);
+                        *reinterpret_cast<__half2 *>(kv_at[i]) = p;
+                        for (int s = 1; s <= dead[i]; s++) *reinterpret_cast<__half2 *>(kv_at[i] + s * 16) = __floats2half2_rn(0.f, 0.f);
+                    }
+                } else if (m < M && col_ok) {
+                    C[(size_t)m * Nout + col] = v;
+                }
             }
         }
         buf ^= two_tiles, rb ^= 1;
@@ -253,7 +296,7 @@ bool shape_ok(Kind kind, int K) {
 }
 
 template <int S, int NT, int KIND>
-static int32_t launch_t(Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse) {
+static int32_t launch_t(Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse, const PagedAppendArgs &pa) {
     auto *kernel = gemm_rows_kernel<S, NT, KIND>;
     constexpr size_t fixed = sizeof(float) * 2 * kWarps * kRows * (NT * 8 + 8);
     constexpr size_t most = std::max(2 * slice_bytes<S>(), kSoloBytes - fixed);
@@ -279,24 +322,25 @@ static int32_t launch_t(Ctx *ctx, const float *A, const Batch &b, int nb, int M,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)(cols / nb), (unsigned)groups, (unsigned)nb), cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem, cfg.stream = ctx->stream, cfg.attrs = attr, cfg.numAttrs = fuse.pdl & 1;
-    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, b, M, K, N, rowsel, fuse, per_group > 1 ? 1 : 0));
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, b, M, K, N, rowsel, fuse, per_group > 1 ? 1 : 0, pa));
     return JGPT_OK;
 }
 
 template <int NT, int KIND, int MAX>
-static int32_t launch_s(int s, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse) {
-    if (s <= 1) return launch_t<1, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
-    if (s <= 2) return launch_t<2, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
-    if (s <= 3) return launch_t<3, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
-    if (s <= 4) return launch_t<4, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+static int32_t launch_s(int s, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse, const PagedAppendArgs &pa) {
+    if (s <= 1) return launch_t<1, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    if (s <= 2) return launch_t<2, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    if (s <= 3) return launch_t<3, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    if (s <= 4) return launch_t<4, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
     if constexpr (MAX > 4) {
-        if (s <= 6) return launch_t<6, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
-        return launch_t<8, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse);
+        if (s <= 6) return launch_t<6, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+        return launch_t<8, NT, KIND>(ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
     }
     return fail(JGPT_ERR_UNSUPPORTED, "gemm_rows: K=%d", K);
 }
 
-int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse_in) {
+int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse_in,
+               const PagedAppendArgs &pa) {
     JGPT_REQUIRE(shape_ok(kind, K) && M > 0 && nb >= 1 && nb <= 3 && (kind != NORM_SWIGLU || N % 32 == 0), JGPT_ERR_UNSUPPORTED,
                  "gemm_rows: unsupported shape M=%d K=%d N=%d", M, K, N);
     Fuse fuse = fuse_in;
@@ -304,9 +348,13 @@ int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int 
     fuse.timeline = timeline_next();
 #endif
     const int s = (k_steps(K) + kWarps - 1) / kWarps;
-    if (kind == NORM) return launch_s<4, NORM, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
-    if (kind == NORM_SWIGLU) return launch_s<4, NORM_SWIGLU, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
-    return launch_s<2, RESIDUAL, kMaxSteps16>(s, ctx, A, b, nb, M, K, N, rowsel, fuse);
+    if (kind == NORM) return launch_s<4, NORM, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    if (kind == NORM_SWIGLU) return launch_s<4, NORM_SWIGLU, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    if (kind == NORM_PAGED) {
+        JGPT_REQUIRE(nb == 3 && N == pa.H * 16, JGPT_ERR_UNSUPPORTED, "gemm_rows: paged products of %d columns, %d heads", N, pa.H);
+        return launch_s<4, NORM_PAGED, kMaxSteps32>(s, ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
+    }
+    return launch_s<2, RESIDUAL, kMaxSteps16>(s, ctx, A, b, nb, M, K, N, rowsel, fuse, pa);
 }
 
 }  // namespace rows

@@ -33,15 +33,18 @@ struct Fuse {
     Timeline timeline;
 #endif
 };
-enum Kind { NORM, NORM_SWIGLU, RESIDUAL };
+enum Kind { NORM, NORM_SWIGLU, RESIDUAL, NORM_PAGED };
 
 // Whether the kernel is built for a product of this kind: every warp has a k slice, and its weights fit its registers.
 bool shape_ok(Kind kind, int K);
 inline int ss_parts(int D) { return (D + 15) / 16; }
 
 // NORM: C_z[M, N] = rmsnorm(A) W_z (gamma is in the image), z < nb.  NORM_SWIGLU: C_0[M, N / 2] = h g sigmoid(g) over an
-// alternating pair.  RESIDUAL: C_0 += A W_0, with the row sums of squares for the next norm.  Row r of A is rowsel[r] if given.
-int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse);
+// alternating pair.  RESIDUAL: C_0 += A W_0, with the row sums of squares for the next norm.  NORM_PAGED: NORM for the Q, K, V products
+// of a prefill at d_head 16 (N = heads * 16); products 1 and 2 go to the paged store as fp16, K with its RoPE, as the append kernel
+// writes them.  Row r of A is rowsel[r] if given.
+int32_t launch(Kind kind, Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse,
+               const PagedAppendArgs &paged = PagedAppendArgs());
 
 }  // namespace rows
 }  // namespace jgpt

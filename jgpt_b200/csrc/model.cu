@@ -169,9 +169,9 @@ __global__ void __launch_bounds__(128) embed_pos_kernel(const float *__restrict_
 // RMSNorm, one block per row (rms_norm_fwd_block_kernel, same file :694-713):
 // rms = sqrtf(sum(x^2)/D + eps); inv = (rms > 0 && finite) ? 1/rms : 0; y = x * inv * gamma.
 __global__ void __launch_bounds__(128) rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ gamma,
-                                                      float *__restrict__ y, int D, float eps) {
+                                                      float *__restrict__ y, int D, float eps, const int *__restrict__ rowsel = nullptr) {
     __shared__ float red[4];
-    const float *xr = x + (size_t)blockIdx.x * D;
+    const float *xr = x + (size_t)(rowsel ? rowsel[blockIdx.x] : blockIdx.x) * D;
     float ss = 0.f;
     for (int j = threadIdx.x; j < D; j += blockDim.x) ss += xr[j] * xr[j];
 #pragma unroll
@@ -1213,8 +1213,9 @@ static int32_t rows_image(Model *m, const float *W, const float *W3, const float
     *out = it->second;
     return JGPT_OK;
 }
+// paged != nullptr (a prefill at d_head 16): the Q,K,V product appends K / V to the paged store itself.
 template <class AttnFn>
-static int32_t run_layers_rows(Model *m, int n, AttnFn &&attn) {
+static int32_t run_layers_rows(Model *m, int n, const PagedAppendArgs *paged, AttnFn &&attn) {
 #ifdef JGPT_B200_DECODE_TRACE
     g_timeline_slot = 0;
 #endif
@@ -1251,9 +1252,11 @@ static int32_t run_layers_rows(Model *m, int n, AttnFn &&attn) {
         const float *w[3] = {y.wq, y.wk, y.wv};
         for (int z = 0; z < 3; z++)
             if ((rc = rows_image(m, w[z], nullptr, y.norm1, D, D, &qkv.image[z], &fresh))) return rc;
-        if ((rc = rows::launch(rows::NORM, m->ctx, m->x, qkv, 3, n, D, D, nullptr,
-                               fuse(m->ss_a, nullptr, parts, ov >= 3 && (l > 0 || m->first_launch_early) && !fresh, ov >= 1)))) return rc;
-        if ((rc = attn(l, umma::ImageOut{}, false))) return rc;
+        PagedAppendArgs pa = paged ? *paged : PagedAppendArgs();
+        pa.layer = l;
+        if ((rc = rows::launch(paged ? rows::NORM_PAGED : rows::NORM, m->ctx, m->x, qkv, 3, n, D, D, nullptr,
+                               fuse(m->ss_a, nullptr, parts, ov >= 3 && (l > 0 || m->first_launch_early) && !fresh, ov >= 1), pa))) return rc;
+        if ((rc = attn(l, umma::ImageOut{}, paged != nullptr))) return rc;
         if ((rc = residual(m->att, y.wo, D, m->ss_b, ov >= 2))) return rc;
         rows::Batch w13{{nullptr}, {m->h1}};
         fresh = false;
@@ -1268,7 +1271,7 @@ static int32_t run_layers_rows(Model *m, int n, AttnFn &&attn) {
 template <class AttnFn>
 static int32_t run_layers(Model *m, int rows, const PagedAppendArgs *paged, AttnFn &&attn) {
     const int D = m->d_model, F = m->d_ff;
-    if (rows_mode(m, rows)) return run_layers_rows(m, rows, attn);
+    if (rows_mode(m, rows)) return run_layers_rows(m, rows, paged, attn);
     if (small_mode(m, rows)) return run_layers_small(m, rows, attn);
     if (!m->strict && m->umma_min_rows > 0 && rows >= m->umma_min_rows && umma::shape_ok(D, D) && umma::shape_ok(D, F) &&
         umma::shape_ok(F, D) && sizeof(float) * 8 * (size_t)(D + 4) <= 48 * 1024) {
@@ -1328,8 +1331,8 @@ static int32_t lm_head(Model *m, int rows, int n_sel, const SampleSpec &spec = S
         rc = small_launch<true, 0>(m, m->x, out_rows, D, m->vocab, 1, W, C, nullptr, rowsel,
                                    SmallFuse{m->norm_final, m->ss_a, nullptr, (D + 31) / 32, m->eps, (early && !fresh) ? 3 : (early ? 2 : 0)});
     } else {
-        rmsnorm_kernel<<<rows, 128, 0, st>>>(m->x, m->norm_final, m->xn, D, m->eps);
-        rc = gemm(m, m->xn, out_rows, D, m->vocab, 1, W, C, nullptr, rowsel);
+        rmsnorm_kernel<<<out_rows, 128, 0, st>>>(m->x, m->norm_final, m->xn, D, m->eps, rowsel);
+        rc = gemm(m, m->xn, out_rows, D, m->vocab, 1, W, C, nullptr);
     }
     if (rc) return rc;
     if (spec.temperature > 0.f) {  // the draws are in m->d_u (uploaded by the caller)
@@ -1887,26 +1890,6 @@ int32_t jgpt_forward_prefill_batch(jgpt_model h, jgpt_kvpool poolh, const int32_
     }
     cudaStream_t st = m->ctx->stream;
     JGPT_CUDA_TRY(cudaMemcpyAsync(m->d_idx, m->h_idx, sizeof(int) * 2 * (size_t)rows, cudaMemcpyHostToDevice, st));
-    embed_pos_kernel<<<rows, 128, 0, st>>>(m->tok, m->pos, m->d_idx, m->d_idx + rows, m->x, m->d_model, m->ss_a);
-    // d_head 16: one head is exactly one 16-wide k tile of the Wo operand image, which the attention kernel can
-    // then write itself, and the Q,K,V product can append K / V to the paged store from its epilogue
-    PagedAppendArgs pa{};
-    const PagedAppendArgs *paged = nullptr;
-    if (p->dhead == 16 && m->d_model == p->heads * 16) {
-        int max_S = 0, n_rows = 0;
-        rc = prefill_upload_descriptors(p, seq_ids_host, seq_starts_host, rope_offsets_host, n, &max_S, &n_rows);
-        if (rc) return rc;
-        pa.kv = p->kv, pa.table = p->d_table, pa.rope = p->d_rope;
-        pa.seqs = reinterpret_cast<const PrefillSeq *>(p->d_prefill_desc), pa.status = p->ctx->d_status;
-        pa.n_seqs = n, pa.H = p->heads, pa.layer = 0, pa.n_blocks = p->n_blocks, pa.mbs = p->max_blocks_per_seq;
-        pa.max_positions = p->max_positions;
-        paged = &pa;
-    }
-    rc = run_layers(m, rows, paged, [&](int l, umma::ImageOut out, bool kv_in_cache) {
-        return launch_attn_prefill(p, l, m->q, m->k, m->v, seq_ids_host, seq_starts_host, rope_offsets_host, n, m->att, out.image, out.scale,
-                                   kv_in_cache, m->prefill_fast);
-    });
-    if (rc) return rc;
     int n_sel = 0;
     if (!all_logits_host) {
         std::vector<int> sel((size_t)n);
@@ -1914,7 +1897,29 @@ int32_t jgpt_forward_prefill_batch(jgpt_model h, jgpt_kvpool poolh, const int32_
         JGPT_CUDA_TRY(cudaMemcpyAsync(m->d_rowsel, sel.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
         n_sel = n;
     }
-    rc = lm_head(m, rows, n_sel);
+    int max_S = 0, n_rows = 0;  // descriptors go up once, in front of the first kernel; every layer reads them
+    if ((rc = prefill_upload_descriptors(p, seq_ids_host, seq_starts_host, rope_offsets_host, n, &max_S, &n_rows))) return rc;
+    embed_pos_kernel<<<rows, 128, 0, st>>>(m->tok, m->pos, m->d_idx, m->d_idx + rows, m->x, m->d_model, m->ss_a);
+    // d_head 16: the attention can write the next product's operand image itself, and the Q,K,V product can append K / V to the paged
+    // store from its epilogue
+    PagedAppendArgs pa{};
+    const PagedAppendArgs *paged = nullptr;
+    if (p->dhead == 16 && m->d_model == p->heads * 16) {
+        pa.kv = p->kv, pa.table = p->d_table, pa.rope = p->d_rope;
+        pa.seqs = reinterpret_cast<const PrefillSeq *>(p->d_prefill_desc), pa.status = p->ctx->d_status;
+        pa.n_seqs = n, pa.H = p->heads, pa.layer = 0, pa.n_blocks = p->n_blocks, pa.mbs = p->max_blocks_per_seq;
+        pa.max_positions = p->max_positions;
+        paged = &pa;
+    }
+    // a short prompt is a chain of small launches like a decode step: every one moves in early
+    const bool early = rows_mode(m, rows) && step_overlap_level(m, rows) >= 3;
+    m->first_launch_early = early;
+    rc = run_layers(m, rows, paged, [&](int l, umma::ImageOut out, bool kv_in_cache) {
+        return launch_attn_prefill(p, l, m->q, m->k, m->v, n, max_S, n_rows, m->att, out.image, out.scale, kv_in_cache, m->prefill_fast, early);
+    });
+    m->first_launch_early = false;
+    if (rc) return rc;
+    rc = lm_head(m, rows, n_sel, SampleSpec(), false, early);
     if (rc) return rc;
     const int out_rows = n_sel ? n_sel : rows;
     if (all_logits_host)

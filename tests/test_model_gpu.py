@@ -461,6 +461,49 @@ def test_products_of_few_rows_against_float64(ctx, dm, dff, rows, spread):
         pool.close(), gm.close()
 
 
+@pytest.mark.parametrize("dm,lens,offset", [(128, [1, 15, 16, 17, 33], 0), (384, [40, 1, 64, 3], 5), (512, [31], 0)])
+def test_short_prompts_append_from_the_projection(ctx, dm, lens, offset):
+    """Prompts of few rows: the Q,K,V product writes K (rotated) and V of the first layer to the paged store itself - over block edges, row
+    tiles that hold several prompts, positions with an offset - and zeroes the rest of a prompt's last block.
+
+    Tolerance: the fp16 neighbour of the float64 value (2^-10 of it), and 1e-5 of sum |x w| for the product in front of the rounding."""
+    V, H = 100, dm // 16
+    rng = np.random.default_rng(dm)
+    T = [rng.standard_normal((V, dm)), rng.standard_normal((64 + offset, dm))] + [rng.standard_normal((dm, dm)) / np.sqrt(dm) for _ in range(4)]
+    T += [rng.standard_normal((dm, 128)), rng.standard_normal((128, dm)), rng.standard_normal((dm, 128)), 1 + 0.1 * rng.standard_normal(dm), np.ones(dm),
+          np.ones(dm), rng.standard_normal((dm, V))]
+    T = [np.ascontiguousarray(t, np.float32) for t in T]
+    gm = GPTModel(ctx, V, 64 + offset, dm, H, 1, 128, rmsNormEps=1e-5, maxRows=256)
+    gm.setParameters(T)
+    pool = gm.newPool(4 * len(lens) + 4, len(lens))
+    try:
+        seqs = [pool.seq_alloc() for _ in lens]
+        ptr, nbytes = pool.storage()
+        raw = np.full(nbytes // 2, 0x7E00, np.uint16)  # NaN everywhere
+        from jgpt_b200 import binding as B
+        B.check(ctx._lib.jgpt_h2d(ctx.handle, ptr, raw.ctypes.data, nbytes))
+        prompts = [rng.integers(0, V, n).astype(np.int32) for n in lens]
+        gm.forwardPrefillBatch(pool, seqs, prompts, np.full(len(lens), offset, np.int32))
+        B.check(ctx._lib.jgpt_d2h(ctx.handle, raw.ctypes.data, ptr, nbytes))
+        blocks = raw.view(np.float16).reshape(pool.n_blocks, H, 2, 16, 16).astype(np.float64)
+        T = [t.astype(np.float64) for t in T]
+        for s, ids in zip(seqs, prompts):
+            n = ids.size
+            x = T[0][ids] + T[1][offset:offset + n]
+            h = x / np.sqrt((x * x).mean(-1, keepdims=True) + 1e-5) * T[9]
+            size = np.abs(h) @ np.abs(T[3]) + np.abs(h) @ np.abs(T[4])
+            k, v = (h @ T[3]).reshape(n, H, 16), (h @ T[4]).reshape(n, H, 16)
+            th = (offset + np.arange(n))[:, None, None] / 10000.0 ** (2 * np.arange(8) / 16)
+            kr = np.stack([k[..., 0::2] * np.cos(th) - k[..., 1::2] * np.sin(th), k[..., 0::2] * np.sin(th) + k[..., 1::2] * np.cos(th)], -1).reshape(n, H, 16)
+            got = blocks[pool.block_table(s)]  # [blocks, H, 2, 16, 16]
+            for which, want in ((0, kr), (1, v)):
+                rows = got[:, :, which].transpose(0, 2, 1, 3).reshape(-1, H, 16)
+                assert np.all(np.abs(rows[:n] - want) <= 2.0 ** -10 * np.abs(want) + 1e-5 * (1 + size.reshape(n, H, 16)))
+                assert not rows[n:].any()
+    finally:
+        pool.close(), gm.close()
+
+
 def test_forward_step_reports_a_failed_device_self_check_itself(ctx, small16):
     """A corrupted block-table entry (-1 where the step reads or appends) must come back as an error from the
     forward call itself -- no jgpt_sync needed, no tokens, no length change -- and the pool must stay usable:
