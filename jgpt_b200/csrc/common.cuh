@@ -53,7 +53,9 @@ struct Ctx {
     int *d_status = nullptr;  // device status word
     int *h_status = nullptr;  // pinned mirror
     int sm_count = 0;
+    cudaMemPool_t scratch_pool = nullptr;  // scratch of calls that own no workspace; made on first use, given back with the context
 };
+constexpr uint64_t kScratchKept = 256ull << 20;  // of it, bytes that stay mapped while nothing uses them
 
 struct SeqState {
     bool used = false;

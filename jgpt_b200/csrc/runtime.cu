@@ -120,6 +120,7 @@ int32_t jgpt_ctx_destroy(jgpt_ctx h) {
     ctx_registry().remove(c);
     cudaFree(c->d_status);
     cudaFreeHost(c->h_status);
+    if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
     cudaStreamDestroy(c->stream);
     delete c;
     return JGPT_OK;

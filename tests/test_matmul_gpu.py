@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from jgpt_b200 import GPTModel, KvCacheGpu
+from jgpt_b200 import Context, GPTModel, KvCacheGpu
 
 pytestmark = pytest.mark.gpu
 
@@ -91,6 +91,32 @@ def test_operand_layout_is_exact_on_integers(ctx):
     want = a.astype(np.float64) @ b.astype(np.float64)
     got = _matmul(ctx, a, b, min_rows=1)
     assert (got == want).all()
+
+
+def test_scratch_stays_with_the_context_and_goes_with_it(ctx):
+    """Products of prefill size keep their scratch mapped between calls: nothing is left of it once the context is closed, and a call
+    inside a capture, which takes its memory from the graph, gives the same bits."""
+    rng = np.random.default_rng(8)
+    M, K, N = 700, 320, 256
+    a, b = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
+    free = []
+    for _ in range(3):
+        with Context(0) as c:
+            da, db, dc = c.from_host(a), c.from_host(b), c.alloc((M, N))
+            c.matmul(da, db, dc, M, K, N)
+            c.synchronize()
+            want = dc.to_host()
+            dc.fill_bytes(0x7F)
+            g = c.capture(lambda: c.matmul(da, db, dc, M, K, N))
+            g.launch()
+            c.synchronize()
+            assert np.array_equal(dc.to_host(), want)
+            g.close()
+            for x in (da, db, dc):
+                x.close()
+        ctx.synchronize()
+        free.append(ctx.mem_info()[0])
+    assert free[2] >= free[1], free
 
 
 def test_unaligned_k_falls_back_to_the_small_kernel(ctx):
