@@ -4,9 +4,9 @@
 // the rows, multiply, add the k slices, store.  So everything that does not depend on the previous kernel is done before the wait and
 // nothing in the loop meets at a barrier.  A CTA owns 16 or 32 columns; its eight warps split k, and a warp holds the weights of
 // its k slice in registers, in the order the tensor core reads them (one 16-byte load per 8 columns, 16 k and lane, out of an image
-// built once per weight set): requested before the wait, used for every row tile the CTA walks.  A warp fetches its own k slice of
-// 16 rows with cp.async, the next tile's while this one is multiplied; the only barrier of a row tile is the one in front of the sum
-// over the eight slices.
+// built once per weight set): requested before the wait, used for every row tile the CTA walks.  A lane loads the rows it multiplies
+// itself, the next tile's while this one is summed and stored; the only barrier of a row tile is the one in front of the sum over the
+// eight slices.  (Rows through a cp.async ring in shared memory: a prompt of 201 tokens 0.52 ms, against 0.45.)
 //
 // Accuracy: an fp32 operand is an fp16 high and an fp16 low part, 11 + 11 bits as the TF32 pair has, at half the tensor time (m16n8k16
 // instead of two m16n8k8) and, for the weights, in the four bytes of the original.  fp16's narrow exponent is dealt with by powers of
@@ -15,9 +15,10 @@
 // below that an absolute error of 2^-40 of the largest remains.  Products high x high in one accumulator, the two mixed ones in another.
 //
 // Against the form with shared-memory k tiles, TF32 pairs split in the loop and a barrier per 64 k (12 layers of 384, per launch inside
-// a decode step of 64 rows, from the previous kernel's end to its own): Q,K,V 5.2 -> 3.6, Wo 4.1 -> 2.3, W1/W3 7.0 -> 4.0, W2 6.6 -> 3.0 us;
-// per step: 8 rows 0.32 -> 0.27, 64 rows 0.45 -> 0.38, 250 rows 1.37 -> 1.24 ms; a prompt of 201 tokens 0.72 -> 0.59 ms.  Error against
-// float64 of the LM head's 384 x 8000 product: 1.5e-7 of the result (2-norm), 1.8e-7 with TF32 pairs.
+// a decode step of 64 rows, from the previous kernel's end to its own): Q,K,V 5.2 -> 3.2, Wo 4.1 -> 3.1, W1/W3 7.0 -> 3.7, W2 6.6 -> 2.8 us;
+// per step: 8 rows 0.32 -> 0.23, 64 rows 0.45 -> 0.37, 250 rows 1.37 -> 1.18 ms with the attention of the same time; a prompt of 201
+// tokens 0.72 -> 0.45 ms.  Error against float64 of the LM head's 384 x 8000 product: 1.5e-7 of the result (2-norm), 1.8e-7 with TF32
+// pairs.
 #include "gemm_rows.cuh"
 
 #include <algorithm>
@@ -38,8 +39,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float *W, const float *
         if (k >= K || n >= N) return 0.f;
         float w;
         if (W3) {
-            const int col = (n >> 5) * 16 + (n & 15);
-            w = (n & 16 ? W3 : W)[(size_t)k * (N / 2) + col];
+            w = (n & 1 ? W3 : W)[(size_t)k * (N / 2) + (n >> 1)];
         } else {
             w = W[(size_t)k * N + n];
         }
@@ -77,23 +77,17 @@ int32_t pack(const float *W, const float *W3, const float *gamma, int K, int N, 
 }
 
 // S: steps of 16 k per warp.  NT: column groups of 8 per CTA.
-template <int S>
-__host__ __device__ constexpr int slice_stride() { return S * 16 + 16; }  // floats: eight rows' chunks fall into different banks
-template <int S>
-constexpr size_t slice_bytes() { return sizeof(float) * kWarps * kRows * (size_t)slice_stride<S>(); }
-
 // CTAs of a kernel on an SM: two while 128 registers hold the weights, the rows and the sums.
 template <int S, int NT>
 constexpr int per_sm() { return S * NT <= 12 && S <= 4 ? 2 : 1; }
 
 template <int S, int NT, int KIND>
 __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(const float *A, const Batch B, int M, int K, int N, const int *rowsel,
-                                                                                  const Fuse F, int two_tiles, const PagedAppendArgs pa) {
-    constexpr int BN = NT * 8, AS = slice_stride<S>(), RS = BN + 8;
+                                                                             const Fuse F, const PagedAppendArgs pa) {
+    constexpr int BN = NT * 8, RS = BN + 8;
+    constexpr bool PAIR = KIND != RESIDUAL;  // a thread sums two neighbouring columns: two results, h and g, or a pair to be turned
     constexpr int OUT = KIND == NORM_SWIGLU ? BN / 2 : BN;  // columns of the result per CTA
-    constexpr int PER = kRows * OUT / kThreads;             // of them per thread: columns fixed, rows row0 + i * kThreads / OUT
-    static_assert(PER >= 1 && (KIND != NORM_SWIGLU || NT == 4), "tile");
-    extern __shared__ __align__(16) float rows_smem[];
+    static_assert(BN == (PAIR ? 32 : 16), "sixteen threads per row of the tile");
     __shared__ __align__(16) float red[2][kWarps][kRows][RS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int z = blockIdx.z;
@@ -113,10 +107,12 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
             const int tile = blockIdx.x * NT + j;
             w[s][j] = (tile < tiles && step0 + s < steps) ? __ldg(image + ((size_t)tile * steps + step0 + s) * 32 + lane) : make_uint4(0, 0, 0, 0);
         }
-    const int oc = tid % OUT, row0 = tid / OUT, col = blockIdx.x * OUT + oc, Nout = KIND == NORM_SWIGLU ? N / 2 : N;
-    const bool col_ok = col < Nout;
-    const int wcol = KIND == NORM_SWIGLU ? blockIdx.x * BN + oc : col;
-    const float un0 = col_ok ? __ldg(unscale + wcol) : 0.f, un1 = (KIND == NORM_SWIGLU && col_ok) ? __ldg(unscale + wcol + 16) : 0.f;
+    // the epilogue's share: row tid / 16 of the tile, column(s) c of it
+    const int orow = tid >> 4, oj = tid & 15, c = PAIR ? 2 * oj : oj;
+    const int Nout = KIND == NORM_SWIGLU ? N / 2 : N, col = blockIdx.x * OUT + (KIND == NORM_SWIGLU ? oj : c);
+    const bool col_ok = col < Nout;  // N % 4 == 0: a pair is inside or outside as a whole
+    float2 un = make_float2(0.f, 0.f);
+    if (col_ok) un = PAIR ? __ldg(reinterpret_cast<const float2 *>(unscale + blockIdx.x * BN + c)) : make_float2(__ldg(unscale + col), 0.f);
 
     if (F.pdl & 1) griddep_wait();
 #ifdef JGPT_B200_DECODE_TRACE
@@ -124,76 +120,58 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
 #endif
     if (F.pdl & 2) griddep_launch_dependents();
 
-    // this warp's k slice of 16 rows; rows and k past the end become zeros
-    float *ring = rows_smem + (size_t)warp * kRows * AS;
-    constexpr size_t kBuf = (size_t)kWarps * kRows * AS;
-    auto fetch = [&](int rt, int buf) {
+    // This warp's k slice of 16 rows, straight into the registers of the lanes that multiply it: rows g and g + 8, four k per step of
+    // 16.  Rows and k past the end become zeros.  Read through L2: an SM's L1 may hold the row of an earlier layer.
+    float4 lo_row[S], hi_row[S];
+    auto fetch = [&](int rt) {
+        const int ma = rt * kRows + g, mb = ma + 8;
+        const float *pa_ = A + (size_t)(ma < M ? (rowsel ? rowsel[ma] : ma) : 0) * K + k0 + 4 * t;
+        const float *pb_ = A + (size_t)(mb < M ? (rowsel ? rowsel[mb] : mb) : 0) * K + k0 + 4 * t;
 #pragma unroll
-        for (int i = 0; i < 2 * S; i++) {
-            const int c = lane + 32 * i, r = c / (4 * S), q = (c % (4 * S)) * 4, m = rt * kRows + r;
-            const bool ok = m < M && k0 + q < K;
-            const int src = ok ? (rowsel ? rowsel[m] : m) : 0;
-            cp_async16(ring + buf * kBuf + r * AS + q, A + (size_t)src * K + (ok ? k0 + q : 0), ok);
+        for (int s = 0; s < S; s++) {
+            const bool in = k0 + s * 16 + 4 * t < K;
+            lo_row[s] = in && ma < M ? __ldcg(reinterpret_cast<const float4 *>(pa_ + s * 16)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            hi_row[s] = in && mb < M ? __ldcg(reinterpret_cast<const float4 *>(pb_ + s * 16)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     const int row_tiles = (M + kRows - 1) / kRows;
-    int rt = blockIdx.y, buf = 0, rb = 0;
-    fetch(rt, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (; rt < row_tiles; rt += gridDim.y) {
-        if (two_tiles && rt + (int)gridDim.y < row_tiles) fetch(rt + gridDim.y, buf ^ 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        // what the epilogue adds or multiplies, and where its rows go, requested now
-        __half *kv_at[KIND == NORM_PAGED ? PER : 1];
-        float2 turn[KIND == NORM_PAGED ? PER : 1];
-        int dead[KIND == NORM_PAGED ? PER : 1];  // slots of the block behind the prompt's last row
-        if (KIND == NORM_PAGED) {
-#pragma unroll
-            for (int i = 0; i < PER; i++) {
-                const int m = rt * kRows + row0 + i * (kThreads / OUT);
-                kv_at[i] = nullptr, turn[i] = make_float2(1.f, 0.f), dead[i] = 0;
-                if (z > 0 && m < M && col_ok) {
-                    int lo = 0, hi = pa.n_seqs - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (pa.seqs[mid].row0 <= m) lo = mid; else hi = mid - 1;
-                    }
-                    const PrefillSeq sd = pa.seqs[lo];
-                    const int slot = m - sd.row0, rp = sd.rope_off + slot;
-                    const bool pos_ok = slot >= 0 && slot < sd.S && rp >= 0 && rp < pa.max_positions;
-                    const int phys = pos_ok ? pa.table[(size_t)sd.seq_id * pa.mbs + slot / kBlockTokens] : 0;
-                    if (!pos_ok) {
-                        atomicOr(pa.status, DEV_STATUS_BAD_POSITION);
-                    } else if (phys < 0 || phys >= pa.n_blocks) {
-                        atomicOr(pa.status, DEV_STATUS_BAD_BLOCK);
-                    } else {
-                        kv_at[i] = pa.kv + (((size_t)pa.layer * pa.n_blocks + phys) * pa.H + col / 16) * (size_t)(2 * kBlockTokens * 16) +
-                                   (z == 2 ? kBlockTokens * 16 : 0) + (slot % kBlockTokens) * 16 + (col & 15);
-                        dead[i] = slot == sd.S - 1 ? kBlockTokens - 1 - slot % kBlockTokens : 0;
-                        if (z == 1) turn[i] = pa.rope[(size_t)rp * 8 + (col & 15) / 2];
-                    }
-                }
-            }
+    int rb = 0;
+    fetch(blockIdx.y);
+    for (int rt = blockIdx.y; rt < row_tiles; rt += gridDim.y) {
+        // what the epilogue adds or multiplies, and where its row goes, requested now
+        const int m = rt * kRows + orow;
+        const bool ok = m < M && col_ok;
+        float *out = C + (size_t)m * Nout + col;
+        float extra = 0.f;
+        if (KIND == RESIDUAL) {
+            if (ok) extra = __ldcg(out);
+        } else if (m < M) {  // the sixteen lanes that share a row add its partial sums of squares, always in the same order
+            const float *pp = F.ss_in + (size_t)(rowsel ? rowsel[m] : m) * F.parts_in;
+            for (int p = oj; p < F.parts_in; p += 16) extra += __ldcg(pp + p);
         }
-        float extra[PER];
-#pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int m = rt * kRows + row0 + i * (kThreads / OUT);
-            extra[i] = 0.f;
-            if (KIND == RESIDUAL) {
-                if (m < M && col_ok) extra[i] = C[(size_t)m * N + col];
-            } else if (m < M) {  // the lanes that share a row add its partial sums of squares, always in the same order
-                const float *pp = F.ss_in + (size_t)(rowsel ? rowsel[m] : m) * F.parts_in;
-                for (int p = oc; p < F.parts_in; p += OUT) extra[i] += pp[p];
+        __half *kv_at = nullptr;
+        float2 turn = make_float2(1.f, 0.f);
+        int dead = 0;  // slots of the block behind the prompt's last row
+        if (KIND == NORM_PAGED && z > 0 && ok) {
+            int lo = 0, hi = pa.n_seqs - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (pa.seqs[mid].row0 <= m) lo = mid; else hi = mid - 1;
             }
-        }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncwarp();
-        float4 lo_row[S], hi_row[S];
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-            lo_row[s] = *reinterpret_cast<const float4 *>(ring + buf * kBuf + g * AS + s * 16 + 4 * t);
-            hi_row[s] = *reinterpret_cast<const float4 *>(ring + buf * kBuf + (g + 8) * AS + s * 16 + 4 * t);
+            const PrefillSeq sd = pa.seqs[lo];
+            const int slot = m - sd.row0, rp = sd.rope_off + slot;
+            const bool pos_ok = slot >= 0 && slot < sd.S && rp >= 0 && rp < pa.max_positions;
+            const int phys = pos_ok ? pa.table[(size_t)sd.seq_id * pa.mbs + slot / kBlockTokens] : 0;
+            if (!pos_ok) {
+                atomicOr(pa.status, DEV_STATUS_BAD_POSITION);
+            } else if (phys < 0 || phys >= pa.n_blocks) {
+                atomicOr(pa.status, DEV_STATUS_BAD_BLOCK);
+            } else {
+                kv_at = pa.kv + (((size_t)pa.layer * pa.n_blocks + phys) * pa.H + col / 16) * (size_t)(2 * kBlockTokens * 16) +
+                        (z == 2 ? kBlockTokens * 16 : 0) + (slot % kBlockTokens) * 16 + (col & 15);
+                dead = slot == sd.S - 1 ? kBlockTokens - 1 - slot % kBlockTokens : 0;
+                if (z == 1) turn = pa.rope[(size_t)rp * 8 + (col & 15) / 2];
+            }
         }
         float m0 = 0.f, m1 = 0.f;
 #pragma unroll
@@ -217,6 +195,8 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
             split_pair(hi_row[s].x * s1, hi_row[s].y * s1, ah[1], al[1]);
             split_pair(lo_row[s].z * s0, lo_row[s].w * s0, ah[2], al[2]);
             split_pair(hi_row[s].z * s1, hi_row[s].w * s1, ah[3], al[3]);
+            // the rows are in the parts: the next tile's are on their way during the last products, the sums and the stores
+            if (s == S - 1 && rt + (int)gridDim.y < row_tiles) fetch(rt + gridDim.y);
 #pragma unroll
             for (int j = 0; j < NT; j++) mma_16816(acc[j], ah, w[s][j].x, w[s][j].y);
 #pragma unroll
@@ -229,58 +209,54 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
             *reinterpret_cast<float2 *>(&red[rb][warp][g][j * 8 + 2 * t]) = make_float2((acc[j][0] + cor[j][0]) * u0, (acc[j][1] + cor[j][1]) * u0);
             *reinterpret_cast<float2 *>(&red[rb][warp][g + 8][j * 8 + 2 * t]) = make_float2((acc[j][2] + cor[j][2]) * u1, (acc[j][3] + cor[j][3]) * u1);
         }
+        float inv = 0.f;
+        if (KIND != RESIDUAL) {
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) extra += __shfl_xor_sync(0xffffffffu, extra, off);
+            const float rms = sqrtf(extra / (float)K + F.eps);
+            inv = (rms > 0.f && isfinite(rms)) ? (1.f / rms) : 0.f;
+        }
         // the buffer of slices written here is rewritten two tiles later, behind the next tile's barrier
         __syncthreads();
+        float2 v = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int r = row0 + i * (kThreads / OUT), m = rt * kRows + r;
-            float v = 0.f, v2 = 0.f;
-#pragma unroll
-            for (int q = kWarps - 1; q >= 0; q--) {
-                v += red[rb][q][r][oc];
-                if (KIND == NORM_SWIGLU) v2 += red[rb][q][r][oc + 16];
-            }
-            v *= un0;
-            if (KIND == RESIDUAL) {
-                v = extra[i] + v;
-                const bool ok = m < M && col_ok;
-                if (ok) C[(size_t)m * N + col] = v;
-                float sq = ok ? v * v : 0.f;
-#pragma unroll
-                for (int off = OUT / 2; off >= 1; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-                if (oc == 0 && m < M) F.ss_out[(size_t)m * gridDim.x + blockIdx.x] = sq;
+        for (int q = kWarps - 1; q >= 0; q--) {
+            if (PAIR) {
+                const float2 p = *reinterpret_cast<const float2 *>(&red[rb][q][orow][c]);
+                v.x += p.x, v.y += p.y;
             } else {
-                float tot = extra[i];
-#pragma unroll
-                for (int off = OUT / 2; off >= 1; off >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, off);
-                const float rms = sqrtf(tot / (float)K + F.eps);
-                const float inv = (rms > 0.f && isfinite(rms)) ? (1.f / rms) : 0.f;
-                v *= inv;
-                if (KIND == NORM_SWIGLU) {
-                    v2 *= un1;
-                    v2 *= inv;
-                    float sg;
-                    if (v2 >= 20.f) sg = 1.f;
-                    else if (v2 <= -20.f) sg = 0.f;
-                    else sg = 1.f / (1.f + expf(-v2));
-                    v = v * (v2 * sg);
-                }
-                if (KIND == NORM_PAGED && z > 0) {  // the even lane of a pair of columns stores both
-                    const float v_odd = __shfl_xor_sync(0xffffffffu, v, 1);
-                    if (kv_at[i] && !(lane & 1)) {
-                        const float2 w = turn[i];
-                        const __half2 p = z == 1 ? __floats2half2_rn(__fsub_rn(__fmul_rn(v, w.x), __fmul_rn(v_odd, w.y)),
-                                                                     __fadd_rn(__fmul_rn(v, w.y), __fmul_rn(v_odd, w.x)))
-                                                 : __floats2half2_rn(v, v_odd);
-                        *reinterpret_cast<__half2 *>(kv_at[i]) = p;
-                        for (int s = 1; s <= dead[i]; s++) *reinterpret_cast<__half2 *>(kv_at[i] + s * 16) = __floats2half2_rn(0.f, 0.f);
-                    }
-                } else if (m < M && col_ok) {
-                    C[(size_t)m * Nout + col] = v;
-                }
+                v.x += red[rb][q][orow][c];
             }
         }
-        buf ^= two_tiles, rb ^= 1;
+        v.x *= un.x, v.y *= un.y;
+        if (KIND == RESIDUAL) {
+            const float x = extra + v.x;
+            if (ok) *out = x;
+            float sq = ok ? x * x : 0.f;
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+            if (oj == 0 && m < M) F.ss_out[(size_t)m * gridDim.x + blockIdx.x] = sq;
+        } else {
+            v.x *= inv, v.y *= inv;
+            if (KIND == NORM_SWIGLU) {
+                float sg;
+                if (v.y >= 20.f) sg = 1.f;
+                else if (v.y <= -20.f) sg = 0.f;
+                else sg = 1.f / (1.f + expf(-v.y));
+                if (ok) *out = v.x * (v.y * sg);
+            } else if (KIND == NORM_PAGED && z > 0) {
+                if (kv_at) {
+                    const __half2 p = z == 1 ? __floats2half2_rn(__fsub_rn(__fmul_rn(v.x, turn.x), __fmul_rn(v.y, turn.y)),
+                                                                 __fadd_rn(__fmul_rn(v.x, turn.y), __fmul_rn(v.y, turn.x)))
+                                             : __floats2half2_rn(v.x, v.y);
+                    *reinterpret_cast<__half2 *>(kv_at) = p;
+                    for (int s = 1; s <= dead; s++) *reinterpret_cast<__half2 *>(kv_at + s * 16) = __floats2half2_rn(0.f, 0.f);
+                }
+            } else if (ok) {
+                *reinterpret_cast<float2 *>(out) = v;
+            }
+        }
+        rb ^= 1;
     }
 #ifdef JGPT_B200_DECODE_TRACE
     timeline_at(F.timeline, 2);
@@ -298,31 +274,28 @@ bool shape_ok(Kind kind, int K) {
 template <int S, int NT, int KIND>
 static int32_t launch_t(Ctx *ctx, const float *A, const Batch &b, int nb, int M, int K, int N, const int *rowsel, const Fuse &fuse, const PagedAppendArgs &pa) {
     auto *kernel = gemm_rows_kernel<S, NT, KIND>;
-    constexpr size_t fixed = sizeof(float) * 2 * kWarps * kRows * (NT * 8 + 8);
-    constexpr size_t most = std::max(2 * slice_bytes<S>(), kSoloBytes - fixed);
+    constexpr size_t fixed = sizeof(float) * 2 * kWarps * kRows * (NT * 8 + 8), solo = kSoloBytes - fixed;
     static bool opted[64] = {};
     if (!opted[ctx->device & 63]) {
-        JGPT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        JGPT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solo));
         opted[ctx->device & 63] = true;
     }
     // As many row groups as stay resident at once, every one with the same number of row tiles where that goes: a CTA keeps its weights
     // over its row tiles, and a second round of CTAs would fetch theirs behind the wait.
     const int cols = (N + NT * 8 - 1) / (NT * 8) * nb, row_tiles = (M + kRows - 1) / kRows;
-    static_assert(per_sm<S, NT>() * (2 * slice_bytes<S>() + fixed + 1024) <= 228 * 1024, "shared memory");
     int groups = std::min(row_tiles, std::max(1, per_sm<S, NT>() * ctx->sm_count / cols));
     const int per_group = (row_tiles + groups - 1) / groups;
     groups = (row_tiles + per_group - 1) / per_group;
-    size_t smem = (per_group > 1 ? 2 : 1) * slice_bytes<S>();
     // A launch of at most one CTA per SM that moves in early, while the previous kernel holds most SMs, would be packed onto the few
     // with room.  More than this and the attention's CTAs could not move in beside it in turn.
-    if ((fuse.pdl & 1) && cols * groups <= ctx->sm_count) smem = std::max(smem, kSoloBytes - fixed);
+    const size_t smem = (fuse.pdl & 1) && cols * groups <= ctx->sm_count ? solo : 0;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)(cols / nb), (unsigned)groups, (unsigned)nb), cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem, cfg.stream = ctx->stream, cfg.attrs = attr, cfg.numAttrs = fuse.pdl & 1;
-    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, b, M, K, N, rowsel, fuse, per_group > 1 ? 1 : 0, pa));
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, b, M, K, N, rowsel, fuse, pa));
     return JGPT_OK;
 }
 

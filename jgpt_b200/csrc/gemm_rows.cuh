@@ -15,7 +15,7 @@ inline uint64_t image_bytes(int K, int N) {
     const uint64_t tiles = (uint64_t)(N + 7) / 8;
     return tiles * (uint64_t)k_steps(K) * 512u + tiles * 8u * sizeof(float);
 }
-// W [K, N] (row k times gamma[k] when given) -> image.  With W3 the columns alternate in groups of 16: W's, then W3's (N = both).
+// W [K, N] (row k times gamma[k] when given) -> image.  With W3 the columns alternate, W's and W3's (N = both).
 int32_t pack(const float *W, const float *W3, const float *gamma, int K, int N, void *image, cudaStream_t st);
 
 struct Batch {
