@@ -1022,6 +1022,13 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     const bool overlapped_single = ov >= 1 && n_layers == 1 && p->persistent <= 0;
     P.HG = overlapped_single ? pick_head_group(p->heads, DH, p->head_group)
                              : pick_head_group(p->heads, DH, p->head_group, (long long)n_layers * n, 2ll * p->ctx->sm_count);
+    // With up to a row per SM and sequences of up to 1024 tokens the heads go to two CTAs (d_head 16, whose consumer warps take four heads
+    // each): smaller CTAs spread more evenly, and the last one is done sooner.  JGPT-35M step of context 512 at 8 / 32 / 64 / 128 / 160 / 200
+    // rows, us: one CTA 208 / 278 / 351 / 524 / 582 / 697, two 203 / 270 / 344 / 508 / 550 / 742, three 201 / 286 / 358 / 524 / 568 / 755.
+    // Long sequences stream, and whole slabs do that better (48 of 1024 to 8192 tokens, 12 layers: 567 us, 596 in halves).
+    if (overlapped_single && DH == 16 && p->head_group <= 0 && P.HG % 2 == 0 && P.HG >= 12 && max_len <= 1024 &&
+        (long long)n * (p->heads / P.HG) <= p->ctx->sm_count)
+        P.HG /= 2;
     P.n_hg = p->heads / P.HG;
     const int max_blocks = std::min(p->max_blocks_per_seq, (max_len + kBlockTokens - 1) / kBlockTokens);
     // Work distribution.  Default (persistent <= 0): one CTA per work item, the hardware block scheduler hands
