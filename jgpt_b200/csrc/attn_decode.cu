@@ -5,8 +5,8 @@
 // ring of shared-memory stages; one producer warp walks the block table and fetches, per KV
 // block, the contiguous [head group][K tile | V tile] slab with ONE bulk async copy (TMA engine,
 // cp.async.bulk + mbarrier complete_tx).  At dhead 16 a consumer warp owns four heads and runs their
-// products on the tensor cores with high + low operands; at the other head sizes consumer threads are
-// (head, token-in-block) pairs: a thread scores its token against q (fp32 FMA), keeps a private
+// products on the tensor cores with high + low operands; at the other head sizes, and for small launches
+// of several layers, consumer threads are (head, token-in-block) pairs: a thread scores its token against q (fp32 FMA), keeps a private
 // online-softmax state (m, l, o[DH]) and, at the end of the chunk, the 16 lanes of a head merge their
 // states with warp shuffles.  Chunks of one sequence are merged by the last CTA to arrive (atomic ticket, no
 // waiting), through a small fp32 scratch buffer.
@@ -162,14 +162,13 @@ template <int DH>
 constexpr int max_head_group() { return (384 / DH) < 30 ? (384 / DH) : 30; }
 
 // Consumer threads of a CTA: (head, token) pairs, or a warp per four heads with the products of dhead 16 on the tensor cores.
-template <int DH>
+template <bool MMA>
 __host__ __device__ constexpr int consumer_threads(int HG) {
-    return DH == 16 ? (HG + 3) / 4 * 32 : (kBlockTokens * HG + 31) / 32 * 32;
+    return MMA ? (HG + 3) / 4 * 32 : (kBlockTokens * HG + 31) / 32 * 32;
 }
 
-template <int DH, bool FUSED>
-__global__ void __launch_bounds__(consumer_threads<DH>(max_head_group<DH>()) + 32, DH == 16 ? 3 : 2) attn_decode_kernel(const DecodeParams P) {
-    constexpr bool MMA = DH == 16;
+template <int DH, bool FUSED, bool MMA = DH == 16>
+__global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 32, MMA ? 3 : 2) attn_decode_kernel(const DecodeParams P) {
     constexpr int BT = kBlockTokens;
     constexpr int TILE = BT * DH * 2;    // bytes of one K (or V) tile
     constexpr int HEAD_BYTES = 2 * TILE; // K tile | V tile
@@ -193,7 +192,7 @@ __global__ void __launch_bounds__(consumer_threads<DH>(max_head_group<DH>()) + 3
     timeline_in(P.timeline);
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(tr_gt0));
 #endif
-    const int n_cons = consumer_threads<DH>(P.HG);  // padded to whole warps
+    const int n_cons = consumer_threads<MMA>(P.HG);  // padded to whole warps
     const int n_cons_warps = n_cons / 32;
     const int stage_bytes = P.HG * HEAD_BYTES;
     const int NS = P.stages;
@@ -910,12 +909,22 @@ static int pick_head_group(int H, int DH, int forced, long long pairs = 0, long 
     return best;
 }
 
+// d_head 16: the tensor-core consumers for the per-layer launches of a decode loop and for launches of more (layer, sequence) pairs than
+// fit at once.  A smaller launch is latency, and a block is a longer chain on the tensor cores (two products, three shuffles
+// for the maximum, two for p) than for a thread with its own token: 12 layers of a few sequences in one launch took
+// 39.9 and 8.7 us with the fp32 consumers, 43.6 and 10.9 us with these; 64 x 1024 takes 190 and 188 us.
+static bool tensor_consumers(const Pool *p, bool per_layer, long long pairs) {
+    return per_layer || pairs * (p->heads / pick_head_group(p->heads, 16, p->head_group)) >= 2ll * p->ctx->sm_count;
+}
+
 template <int DH>
-static int32_t launch_decode_t(Pool *p, const DecodeParams &P, bool fused, int threads, size_t smem, int grid) {
-    void (*kern)(const DecodeParams) = fused ? attn_decode_kernel<DH, true> : attn_decode_kernel<DH, false>;
+static int32_t launch_decode_t(Pool *p, const DecodeParams &P, bool fused, bool mma, int threads, size_t smem, int grid) {
+    void (*kern)(const DecodeParams) = fused ? attn_decode_kernel<DH, true, false> : attn_decode_kernel<DH, false, false>;
+    if constexpr (DH == 16)
+        if (mma) kern = fused ? attn_decode_kernel<DH, true, true> : attn_decode_kernel<DH, false, true>;
     // Opt in to > 48 KiB of dynamic shared memory once per kernel and device: the most a launch can ask for
     // (kMaxStages stages of a 24 KiB slab), so that no later, smaller request ever lowers the limit again.
-    JGPT_CUDA_TRY(decode_opt_in_smem(kern, (fused ? 1 : 0) + 4 * (DH == 4 ? 0 : DH == 8 ? 1 : DH == 16 ? 2 : 3), p->ctx->device));
+    JGPT_CUDA_TRY(decode_opt_in_smem(kern, (fused ? 1 : 0) + (DH == 16 && mma ? 2 : 0) + 4 * (DH == 4 ? 0 : DH == 8 ? 1 : DH == 16 ? 2 : 3), p->ctx->device));
     if (P.overlap || P.cluster) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3((unsigned)threads), cfg.dynamicSmemBytes = smem, cfg.stream = p->ctx->stream;
@@ -969,7 +978,7 @@ static int cluster_capacity(Pool *p, bool fused, int threads, size_t smem, int c
     switch (p->dhead) {
         case 4: kern = fused ? attn_decode_kernel<4, true> : attn_decode_kernel<4, false>, variant = 0; break;
         case 8: kern = fused ? attn_decode_kernel<8, true> : attn_decode_kernel<8, false>, variant = 4; break;
-        case 16: kern = fused ? attn_decode_kernel<16, true> : attn_decode_kernel<16, false>, variant = 8; break;
+        case 16: kern = fused ? attn_decode_kernel<16, true> : attn_decode_kernel<16, false>, variant = 10; break;
         case 32: kern = fused ? attn_decode_kernel<32, true> : attn_decode_kernel<32, false>, variant = 12; break;
         default: return 0;
     }
@@ -1004,7 +1013,7 @@ static int pick_chunk_blocks(const Pool *p, long long base, int max_blocks) {
 }
 
 int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, const float *k_new, const float *v_new,
-                           const int *seq_ids, const int *rope_pos, const int *lens, int n, int max_len, float *out, int overlap) {
+                           const int *seq_ids, const int *rope_pos, const int *lens, int n, int max_len, float *out, int overlap, int of_layers) {
     DecodeParams P;
     memset(&P, 0, sizeof(P));
     const int DH = p->dhead;
@@ -1030,6 +1039,9 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
         (long long)n * (p->heads / P.HG) <= p->ctx->sm_count)
         P.HG /= 2;
     P.n_hg = p->heads / P.HG;
+    // (a launch that is one of several over a call's layers goes by all of them: the call's bits do not depend on how it is cut)
+    const int rule_layers = of_layers > 0 ? of_layers : n_layers;
+    const bool mma = DH == 16 && tensor_consumers(p, overlapped_single && rule_layers == 1, (long long)rule_layers * n);
     const int max_blocks = std::min(p->max_blocks_per_seq, (max_len + kBlockTokens - 1) / kBlockTokens);
     // Work distribution.  Default (persistent <= 0): one CTA per work item, the hardware block scheduler hands
     // items to SMs as CTAs retire.  persistent = k > 0: k CTAs per SM claim items from a global counter (kept
@@ -1038,7 +1050,7 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     const long long slots = (long long)per_sm * p->ctx->sm_count;
     const bool dynamic = p->persistent > 0;
     P.stages = p->stages > 0 ? p->stages : (overlapped_single ? 3 : 4);
-    const int n_cons = DH == 16 ? consumer_threads<16>(P.HG) : consumer_threads<4>(P.HG);
+    const int n_cons = mma ? consumer_threads<true>(P.HG) : consumer_threads<false>(P.HG);
     const int threads = n_cons + 32;
     const size_t stage_bytes = (size_t)P.HG * 2 * kBlockTokens * DH * 2;
     const size_t smem = stage_bytes * P.stages;
@@ -1122,10 +1134,10 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     if (P.dynamic && P.overlap > 1) P.overlap = 1;  // the work-queue counters are reset by the previous launch's last CTA
     const bool fused = k_new != nullptr;
     switch (DH) {
-        case 4: return launch_decode_t<4>(p, P, fused, threads, smem, grid);
-        case 8: return launch_decode_t<8>(p, P, fused, threads, smem, grid);
-        case 16: return launch_decode_t<16>(p, P, fused, threads, smem, grid);
-        case 32: return launch_decode_t<32>(p, P, fused, threads, smem, grid);
+        case 4: return launch_decode_t<4>(p, P, fused, mma, threads, smem, grid);
+        case 8: return launch_decode_t<8>(p, P, fused, mma, threads, smem, grid);
+        case 16: return launch_decode_t<16>(p, P, fused, mma, threads, smem, grid);
+        case 32: return launch_decode_t<32>(p, P, fused, mma, threads, smem, grid);
         default: return fail(JGPT_ERR_UNSUPPORTED, "dhead %d not supported", DH);
     }
 }
@@ -1355,7 +1367,7 @@ int32_t jgpt_attn_decode_append_host(jgpt_kvpool pool, int32_t layer0, int32_t n
         JGPT_CUDA_TRY(cudaMemcpyAsync(dv + off, v_host + off, sizeof(float) * cnt, cudaMemcpyHostToDevice, p->s_in));
         JGPT_CUDA_TRY(cudaEventRecord(p->ev_in[g], p->s_in));
         JGPT_CUDA_TRY(cudaStreamWaitEvent(st, p->ev_in[g], 0));
-        rc = launch_attn_decode(p, layer0 + l0, nl, dq + off, dk + off, dv + off, dseq, drp, dlen, n, max_len, dout + off);
+        rc = launch_attn_decode(p, layer0 + l0, nl, dq + off, dk + off, dv + off, dseq, drp, dlen, n, max_len, dout + off, -1, n_layers);
         if (rc) return rc;
         JGPT_CUDA_TRY(cudaEventRecord(p->ev_done[g], st));
         JGPT_CUDA_TRY(cudaStreamWaitEvent(p->s_out, p->ev_done[g], 0));
@@ -1419,7 +1431,10 @@ static int32_t static_scratch_setup(const Pool *p, float **partials, int **ticke
         switch (p->dhead) {
             case 4: a = decode_opt_in_smem(attn_decode_kernel<4, false>, 0, c->device); break;
             case 8: a = decode_opt_in_smem(attn_decode_kernel<8, false>, 4, c->device); break;
-            case 16: a = decode_opt_in_smem(attn_decode_kernel<16, false>, 8, c->device); break;
+            case 16:
+                a = decode_opt_in_smem(attn_decode_kernel<16, false, false>, 8, c->device);
+                if (a == cudaSuccess) a = decode_opt_in_smem(attn_decode_kernel<16, false, true>, 10, c->device);
+                break;
             case 32: a = decode_opt_in_smem(attn_decode_kernel<32, false>, 12, c->device); break;
             default: break;
         }
@@ -1470,14 +1485,15 @@ static int32_t launch_attn_decode_static(Pool *p, int layer, const float *q, con
         // the counters must start at zero (they reset themselves, but not if an earlier launch gave up half way).
         JGPT_CUDA_TRY(cudaMemsetAsync(P.tickets, 0, sizeof(int) * need_tickets, p->ctx->stream));
     }
-    const int n_cons = DH == 16 ? consumer_threads<16>(P.HG) : consumer_threads<4>(P.HG);
+    const bool mma = DH == 16 && tensor_consumers(p, false, n);
+    const int n_cons = mma ? consumer_threads<true>(P.HG) : consumer_threads<false>(P.HG);
     const int threads = n_cons + 32;
     const size_t smem = (size_t)P.HG * 2 * kBlockTokens * DH * 2 * P.stages;
     void (*kern)(const DecodeParams) = nullptr;
     switch (DH) {
         case 4: kern = attn_decode_kernel<4, false>; break;
         case 8: kern = attn_decode_kernel<8, false>; break;
-        case 16: kern = attn_decode_kernel<16, false>; break;
+        case 16: kern = mma ? attn_decode_kernel<16, false, true> : attn_decode_kernel<16, false, false>; break;
         case 32: kern = attn_decode_kernel<32, false>; break;
         default: return fail(JGPT_ERR_UNSUPPORTED, "dhead %d not supported", DH);
     }

@@ -285,7 +285,8 @@ int32_t launch_kv_gather(Pool *p, int layer, int seq, int len, int max_seq_len, 
 int32_t launch_kv_scrub(Pool *p, const std::vector<int> &blocks);
 int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, const float *k_new,
                            const float *v_new, const int *seq_ids, const int *rope_pos, const int *lens, int n,
-                           int max_len, float *out, int overlap = -1);  // overlap < 0: the pool's setting
+                           int max_len, float *out, int overlap = -1,   // overlap < 0: the pool's setting
+                           int of_layers = 0);                         // > 0: one launch of a call over so many layers
 int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, int n_seqs, int max_S, int n_rows, float *out,
                             float *out_image = nullptr, const float *out_scale = nullptr, bool skip_append = false, int fast_mode = -1,
                             int pdl = 0);
