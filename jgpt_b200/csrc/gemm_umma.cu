@@ -174,27 +174,33 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
     split_pair(v[0], v[1], hi.x, lo.x), split_pair(v[2], v[3], hi.y, lo.y);
     split_pair(v[4], v[5], hi.z, lo.z), split_pair(v[6], v[7], hi.w, lo.w);
 }
+// The exponent e that brings values up to mx into [2^14, 2^15) as mx 2^e, within what fp32 holds as 2^e and 2^-e; 0 for a column that
+// is all zeros or not finite (its results are zeros, or not finite, at any scale).
+__device__ __forceinline__ int half_exponent(double mx, int limit) {
+    if (!(mx > 0.) || isinf(mx)) return 0;
+    int e;
+    frexp(mx, &e);  // mx in [2^(e - 1), 2^e)
+    return max(-limit, min(limit, 15 - e));
+}
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 // One thread per column: up[n] brings the column's largest element (row k divided by k_scale[k]) to [2^14, 2^15), un[n] undoes it.
-// Image row r is column r of W, or, for a pair, column (r / 256) * 128 + r % 128 of W1 (first 128 rows of a 256-row tile) or W3; the
-// factors of W1's rows also carry out_scale, so that the gated product leaves the epilogue scaled for the next image.
+// Image row r is column r of W, or, for a pair, column (r / 256) * 128 + r % 128 of W1 (first 128 rows of a 256-row tile) or W3.
+// In fp64: a weight over a power of two may lie outside fp32 where the product of the two does not.
 __device__ __forceinline__ const float *half_source(const float *W, const float *W3, int r, int &col) {
     if (!W3) return col = r, W;
     col = (r >> 8) * 128 + (r & 127);
     return r & 128 ? W3 : W;
 }
-__global__ void __launch_bounds__(256) half_scale_kernel(const float *W, const float *W3, const float *k_scale, const float *out_scale, int K, int N,
-                                                         int rows, float *un, float *up) {
+__global__ void __launch_bounds__(256) half_scale_kernel(const float *W, const float *W3, const float *k_scale, int K, int N, int rows, float *un, float *up) {
     const int r = blockIdx.x * 256 + threadIdx.x;
     if (r >= rows) return;
     int col;
     const float *src = half_source(W, W3, r, col);
-    float mx = 0.f;
+    double mx = 0.;
     if (col < N)
-        for (int k = 0; k < K; k++) mx = fmaxf(mx, fabsf(src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f)));
-    float a, b;
-    pow2_scale(mx, a, b);
-    up[r] = a;
-    un[r] = (W3 && !(r & 128)) ? b * out_scale[col] : b;
+        for (int k = 0; k < K; k++) mx = fmax(mx, fabs((double)src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f)));
+    const int e = half_exponent(mx, 126);
+    up[r] = pow2(e), un[r] = pow2(-e);
 }
 template <int TR>
 __global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const float *W3, const float *k_scale, const float *up, int K, int N,
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const fl
 #pragma unroll
         for (int q = 0; q < 8; q++) {
             const int k = kt * HBK + k8 * 8 + q;
-            v[q] = col < N ? src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f) * up[r] : 0.f;
+            v[q] = col < N ? (float)((double)src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f) * up[r]) : 0.f;
         }
         uint4 hi, lo;
         split8(v, hi, lo);
@@ -217,18 +223,17 @@ __global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const fl
         *reinterpret_cast<uint4 *>(tile + TR * HBK * 2 + half_chunk(rr, k8)) = lo;
     }
 }
+// In fp64, where no square of an fp32 weight leaves the range: a column of 1e-24 has a reach that is not 0, one of 1e20 a finite one.
+// The limit keeps any finite fp32 result below 2^15.
 __global__ void __launch_bounds__(256) column_scale_kernel(const float *W, const float *W3, const float *gamma, int K, int N, float *scale) {
     const int n = blockIdx.x * 256 + threadIdx.x;
     if (n >= N) return;
-    float a = 0.f, b = 0.f;
+    double a = 0., b = 0.;
     for (int k = 0; k < K; k++) {
-        const float g = gamma[k], x = g * W[(size_t)k * N + n], y = W3 ? g * W3[(size_t)k * N + n] : 0.f;
+        const double g = gamma[k], x = g * W[(size_t)k * N + n], y = W3 ? g * W3[(size_t)k * N + n] : 0.;
         a += x * x, b += y * y;
     }
-    const float reach = W3 ? (float)K * sqrtf(a) * sqrtf(b) : sqrtf((float)K) * sqrtf(a);
-    float up, un;
-    pow2_scale(reach, up, un);
-    scale[n] = up;
+    scale[n] = pow2(half_exponent(W3 ? (double)K * sqrt(a) * sqrt(b) : sqrt((double)K * a), 113));
 }
 // RMSNorm of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers between the
 // sum of squares and the product.
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__r
 int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st) {
     const int bn = tile_cols(N), tiles = (N + bn - 1) / bn, rows = tiles * bn;
     float *un = image + (size_t)rows * K, *up = un + rows;
-    half_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(W, nullptr, k_scale, nullptr, K, N, rows, un, up);
+    half_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(W, nullptr, k_scale, K, N, rows, un, up);
     dim3 grid(K / HBK, tiles);
     uint8_t *im = reinterpret_cast<uint8_t *>(image);
     if (bn == 256) half_pack_kernel<256><<<grid, 256, 0, st>>>(W, nullptr, k_scale, up, K, N, im);
@@ -318,10 +323,10 @@ int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, flo
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *out_scale, int K, int F, float *image, cudaStream_t st) {
+int32_t pack_weight_pair_half(const float *W1, const float *W3, int K, int F, float *image, cudaStream_t st) {
     JGPT_REQUIRE(half_ok(K, F), JGPT_ERR_UNSUPPORTED, "pack_weight_pair_half: K=%d F=%d", K, F);
     float *un = image + (size_t)2 * F * K, *up = un + 2 * F;
-    half_scale_kernel<<<(2 * F + 255) / 256, 256, 0, st>>>(W1, W3, nullptr, out_scale, K, F, 2 * F, un, up);
+    half_scale_kernel<<<(2 * F + 255) / 256, 256, 0, st>>>(W1, W3, nullptr, K, F, 2 * F, un, up);
     half_pack_kernel<256><<<dim3(K / HBK, F / 128), 256, 0, st>>>(W1, W3, nullptr, up, K, F, reinterpret_cast<uint8_t *>(image));
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
@@ -549,7 +554,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
 #pragma unroll
                     for (int q = 0; q < 32; q += 4) {
                         const float4 u = __ldg(reinterpret_cast<const float4 *>(w_un + c + q));
-                        v[q] = v[q] * a_un * u.x, v[q + 1] = v[q + 1] * a_un * u.y, v[q + 2] = v[q + 2] * a_un * u.z, v[q + 3] = v[q + 3] * a_un * u.w;
+                        v[q] *= a_un * u.x, v[q + 1] *= a_un * u.y, v[q + 2] *= a_un * u.z, v[q + 3] *= a_un * u.w;
                     }
                 }
             };
@@ -673,6 +678,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                         h[q] = h[q] * (gv * s);
                     }
                     if constexpr (HALF) {  // these 32 columns are one k tile of the next product
+                        // (the finished value times its column's power of two: h alone may exceed what h g sigmoid(g) can reach)
+#pragma unroll
+                        for (int q = 0; q < 32; q += 4) {
+                            const float4 u = __ldg(reinterpret_cast<const float4 *>(B.c_up + n_idx * 128 + c0 + q));
+                            h[q] *= u.x, h[q + 1] *= u.y, h[q + 2] *= u.z, h[q + 3] *= u.w;
+                        }
                         uint8_t *tile = reinterpret_cast<uint8_t *>(B.C[0] + ((size_t)m_idx * out_nkt + (n_idx * 128 + c0) / HBK) * A_TILE_FLOATS);
 #pragma unroll
                         for (int k8 = 0; k8 < 4; k8++) {
@@ -769,22 +780,22 @@ int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, i
 }
 
 template <bool HALF>
-static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
-                           cudaStream_t st) {
+static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
+                           int *d_status, cudaStream_t st) {
     JGPT_REQUIRE(swiglu_shape_ok(K, F) && (!HALF || K % HBK == 0) && M > 0, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
     Batch b{};
-    b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un;
+    b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un, b.c_up = c_up;
     TileWalk walk{F / 128, 1, 0};
     walk.total = walk.n_tiles_n * ((M + BM - 1) / BM);
     return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st);
 }
 int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, int F, float *act_image, int *d_status, cudaStream_t st) {
-    return launch_pair<false>(Aimg, Wpair_img, nullptr, M, K, F, act_image, d_status, st);
+    return launch_pair<false>(Aimg, Wpair_img, nullptr, nullptr, M, K, F, act_image, d_status, st);
 }
-int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
-                           cudaStream_t st) {
-    return launch_pair<true>(Aimg, Wpair_img, a_un, M, K, F, act_image, d_status, st);
+int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
+                           int *d_status, cudaStream_t st) {
+    return launch_pair<true>(Aimg, Wpair_img, a_un, c_up, M, K, F, act_image, d_status, st);
 }
 
 }  // namespace umma

@@ -37,6 +37,7 @@ struct Batch {
     float *C[3];
     const float *R[3];  // optional residual, may alias C
     const float *a_un = nullptr;  // fp16 images: one factor per row of A that undoes its power of two (nullptr: none)
+    const float *c_up = nullptr;  // the SwiGLU form on fp16 images: the power of two of every column of the result
 };
 // C_z[M, N] = A . W_z (+ R_z) for z < nb; needs K % 16 == 0 and N % 4 == 0.
 int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
@@ -68,15 +69,15 @@ struct ImageOut {
     const float *scale = nullptr;
 };
 int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st);
-// out_scale[F]: the powers of two that launch_swiglu_half gives its result's columns.
-int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *out_scale, int K, int F, float *image, cudaStream_t st);
+int32_t pack_weight_pair_half(const float *W1, const float *W3, int K, int F, float *image, cudaStream_t st);
 // scale[n] = the power of two that keeps column n below 2^15 in fp16: of rmsnorm(x) W (gamma applied), or of h g sigmoid(g) with W3.
 int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st);
 // RMSNorm into an fp16 image; a_un[M] receives the rows' factors.
 int32_t rmsnorm_pack_half(const float *x, const float *gamma, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
 int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
-int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, int M, int K, int F, float *act_image, int *d_status,
-                           cudaStream_t st);
+// c_up[F]: the powers of two of the result's columns in its image.
+int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
+                           int *d_status, cudaStream_t st);
 int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st);
 
 inline bool shape_ok(int K, int N) { return K >= BK && K % BK == 0 && N % 4 == 0; }

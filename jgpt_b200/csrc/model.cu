@@ -932,7 +932,7 @@ static int32_t half_layer(Model *m, const LayerW &y, HalfLayer *o) {
     for (auto &w : one)
         if ((rc = half_buffer(m, w.W, umma::half_weight_floats(w.K, D), w.out, &fresh)) || (fresh && (rc = umma::pack_weight_half(w.W, w.k_scale, w.K, D, *w.out, st)))) return rc;
     if ((rc = half_buffer(m, y.w1, umma::half_pair_floats(D, F), &o->pair, &fresh)) ||
-        (fresh && (rc = umma::pack_weight_pair_half(y.w1, y.w3, o->h_scale, D, F, o->pair, st)))) return rc;
+        (fresh && (rc = umma::pack_weight_pair_half(y.w1, y.w3, D, F, o->pair, st)))) return rc;
     return JGPT_OK;
 }
 
@@ -965,7 +965,7 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
         if ((rc = attn(l, umma::ImageOut{m->aimg, w.att_scale}, true))) return rc;
         if ((rc = umma::launch_half(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
         if ((rc = umma::rmsnorm_pack_half(m->x, y.norm2, rows, D, m->eps, m->aimg, a_un, st))) return rc;
-        if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, rows, D, F, m->aimg2, status, st))) return rc;
+        if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, w.h_scale, rows, D, F, m->aimg2, status, st))) return rc;
         if ((rc = umma::launch_half(m->aimg2, w2, 1, rows, F, D, status, st))) return rc;
     }
     return JGPT_OK;

@@ -309,3 +309,50 @@ def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, part, spread):
         assert np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
     finally:
         pool.close(), gm.close()
+
+
+@pytest.mark.parametrize("dm,dff", [(64, 128), (384, 768)])
+def test_prefill_on_fp16_images_with_dead_and_extreme_columns(ctx, dm, dff):
+    """Hidden units whose gate or up column is zero (pruned) or far outside fp16, some with the inverse in W2 so that they count: h alone is
+    then far larger than the gated value can be, squares of a column leave fp32, and a unit is worth 1e-24 or 1e20 of its neighbour.
+
+    Tolerance: as for the other columns, relative to sum |x w| (22 bits per operand and fewer than 128 fp32 additions)."""
+    V, n, E = 132, 600, 1e-5
+    rng = np.random.default_rng(dm)
+
+    def mat(a, b):
+        return rng.standard_normal((a, b)) / np.sqrt(a)
+
+    w1, w2, w3 = mat(dm, dff), mat(dff, dm), mat(dm, dff)
+    #      zero gate  tiny gate  tiny up    large up   zero up    both       dead behind W2
+    up =   [30.0,     1.0,       1e-24,     1e20,      0.0,       1e30,      10.0,      1.0]
+    gate = [0.0,      1e-24,     1.0,       1.0,       1.0,       1e-30,     1.0,       1.0]
+    down = [1.0,      1e24,      1e24,      1e-20,     1.0,       1.0,       0.0,       1.0]
+    unit = np.arange(dff) % 8
+    w1, w3, w2 = w1 * np.array(up)[unit], w3 * np.array(gate)[unit], w2 * np.array(down)[unit][:, None]
+    tok, head = rng.standard_normal((V, dm)), mat(dm, V)
+    n2 = 1 + 0.2 * rng.standard_normal(dm)
+    T = [np.ascontiguousarray(t, np.float32) for t in (tok, np.zeros((64, dm)), mat(dm, dm), mat(dm, dm), mat(dm, dm), np.zeros((dm, dm)), w1, w2, w3,
+                                                       np.ones(dm), n2, np.ones(dm), head)]
+    gm = GPTModel(ctx, V, 64, dm, dm // 16, 1, dff, rmsNormEps=1e-6, maxRows=n)
+    gm.setParameters(T)
+    pool = gm.newPool(n, n)
+    try:
+        ids = rng.integers(0, V, n).astype(np.int32)
+        got, _ = gm.forwardPrefillBatch(pool, [pool.seq_alloc() for _ in range(n)], [[i] for i in ids])
+        tok, w1, w2, w3, n2, head = (T[i].astype(np.float64) for i in (0, 6, 7, 8, 10, 12))
+
+        def rms(x):
+            return np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+
+        h = tok[ids] / rms(tok[ids]) * n2
+        a, g = h @ w1, h @ w3
+        assert np.abs(a[:, unit == 0]).max() > 4
+        act = a * g / (1 + np.exp(-g))
+        y = tok[ids] + act @ w2
+        off = E * ((np.abs(h) @ np.abs(w1)) * np.abs(g) + 1.2 * np.abs(a) * (np.abs(h) @ np.abs(w3)) + np.abs(act)) @ np.abs(w2) + 1e-6 * np.abs(y)
+        z = y / rms(y)
+        bound = (off / rms(y) + np.sqrt((off ** 2).mean(-1, keepdims=True)) / rms(y) * np.abs(z)) @ np.abs(head) + E * (np.abs(z) @ np.abs(head))
+        assert np.isfinite(got).all() and np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
+    finally:
+        pool.close(), gm.close()
