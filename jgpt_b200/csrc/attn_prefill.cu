@@ -24,8 +24,8 @@ struct PrefillParams {
     const float2 *rope;
     const float *q, *k, *v;
     float *out;
-    float *out_image;        // != nullptr (d_head 16, an even number of heads): write the output as the tcgen05 projection's fp16 operand image instead
-    const float *out_scale;  // of that image: one power of two per column
+    float *out_image;        // != nullptr (d_head 16): write the output as the tcgen05 projection's operand image instead
+    const float *out_scale;  // != nullptr (an even number of heads): an fp16 image, one power of two per column; else a TF32 one
     const PrefillSeq *seqs;
     int *status;
     int n_seqs, n_rows, H, layer, n_blocks, mbs, max_positions;
@@ -350,14 +350,28 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     const float iA = 1.f / fmaxf(lA, 1e-12f), iB = 1.f / fmaxf(lB, 1e-12f);
     const size_t D = (size_t)P.H * DH;
     if (P.out_image) {
-        // fp16 operand image of the next projection (see gemm_umma.cu): 128-row tiles x 32-wide k tiles, high parts then low
-        // parts; head h is half of k tile h / 2.  Lane (g, t) holds columns 8 j + 2 t, 8 j + 2 t + 1 of the head, times the powers of two
-        // that the image's columns carry: a warp store covers eight rows x one 16-byte chunk = one full 128-byte line.
+        // Operand image of the next projection (see gemm_umma.cu): 128-row tiles, high parts then low parts.  Lane (g, t) holds columns
+        // 8 j + 2 t, 8 j + 2 t + 1 of the head.
+        // TF32: k tiles of 16, head h is k tile h; the pair is half of the 16-byte chunk 2 j + t / 2, a warp store covers eight rows x two
+        // chunks = two full 128-byte lines.
+        // fp16: k tiles of 32, head h is half of k tile h / 2, values times the powers of two that the image's columns carry; a warp
+        // store covers eight rows x one chunk = one full line.
         auto put = [&](int row, int j, float a, float b) {
             const size_t grow = (size_t)sd.row0 + row;
+            const int rr = (int)(grow & 127);
+            if (!P.out_scale) {
+                float *dst = P.out_image + ((grow >> 7) * (size_t)P.H + h) * (size_t)(128 * 16 * 2) + (rr >> 3) * 128 + (2 * j + (t >> 1)) * 32 + (rr & 7) * 4 + (t & 1) * 2;
+                uint32_t ha, hb, la, lb;
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ha) : "f"(a));
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(b));
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(la) : "f"(a - __uint_as_float(ha)));
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(b - __uint_as_float(hb)));
+                *reinterpret_cast<float2 *>(dst) = make_float2(__uint_as_float(ha), __uint_as_float(hb));
+                *reinterpret_cast<float2 *>(dst + 128 * 16) = make_float2(__uint_as_float(la), __uint_as_float(lb));
+                return;
+            }
             const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
             unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
-            const int rr = (int)(grow & 127);
             unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
             uint32_t hi, lo;
             split_half2(a * up.x, b * up.y, hi, lo);
@@ -471,7 +485,7 @@ int32_t prefill_upload_descriptors(Pool *p, const int *seq_ids_host, const int *
 
 int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, const float *v, int n_seqs, int max_S, int n_rows, float *out,
                             float *out_image, const float *out_scale, bool skip_append, int fast_mode, int pdl) {
-    JGPT_REQUIRE(!out_image || (p->dhead == 16 && p->heads % 2 == 0 && out_scale), JGPT_ERR_INVALID_ARGUMENT, "image output needs d_head 16 and pairs of heads");
+    JGPT_REQUIRE(!out_image || (p->dhead == 16 && (!out_scale || p->heads % 2 == 0)), JGPT_ERR_INVALID_ARGUMENT, "image output needs d_head 16, an fp16 one pairs of heads");
     PrefillParams P;
     memset(&P, 0, sizeof(P));
     P.kv = p->kv, P.table = p->d_table, P.rope = p->d_rope, P.q = q, P.k = k, P.v = v, P.out = out, P.out_image = out_image, P.out_scale = out_scale;

@@ -63,7 +63,8 @@ inline uint64_t half_weight_floats(int K, int N) {
     return rows * (uint64_t)K + 2 * rows;
 }
 inline uint64_t half_pair_floats(int K, int F) { return (uint64_t)2 * F * (uint64_t)K + 4 * (uint64_t)F; }
-// Where the attention leaves its output for the next product: the image and its columns' powers of two (no image: row major).
+// Where the attention leaves its output for the next product: the image and its columns' powers of two (none: a TF32 image; no image:
+// row major).
 struct ImageOut {
     float *image = nullptr;
     const float *scale = nullptr;

@@ -972,10 +972,11 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
 }
 
 // One decoder block over `rows` rows already in m->x.  Attention is supplied by the caller.
-// The same decoder blocks for other head and feed-forward sizes, on TF32 images; the attention output is packed by a kernel of its own.
+// The same decoder blocks for other head and feed-forward sizes, on TF32 images.
 // attn(l, image, kv_in_cache): attention of layer l; writes the Wo operand image itself when there is one, the row-major m->att
-// otherwise; kv_in_cache: the K / V rows of the layer are already in the paged store.
-// `paged` != nullptr (a prefill at d_head 16): the Q,K,V product writes K / V straight into the paged store.
+// otherwise, packed by a kernel of its own; kv_in_cache: the K / V rows of the layer are already in the paged store.
+// `paged` != nullptr (a prefill at d_head 16): the attention writes that image, and the Q,K,V product writes K / V straight into the
+// paged store.
 template <class AttnFn>
 static int32_t run_layers_umma(Model *m, int rows, const PagedAppendArgs *paged, AttnFn &&attn) {
     const int D = m->d_model, F = m->d_ff;
@@ -1005,8 +1006,8 @@ static int32_t run_layers_umma(Model *m, int rows, const PagedAppendArgs *paged,
         } else {
             if ((rc = umma::launch(m->aimg, qkv, 3, rows, D, D, status, st))) return rc;
         }
-        if ((rc = attn(l, umma::ImageOut{}, paged != nullptr))) return rc;
-        if ((rc = umma::pack_activations(m->att, nullptr, rows, D, m->aimg, st))) return rc;
+        if ((rc = attn(l, paged ? umma::ImageOut{m->aimg} : umma::ImageOut{}, paged != nullptr))) return rc;
+        if (!paged && (rc = umma::pack_activations(m->att, nullptr, rows, D, m->aimg, st))) return rc;
         if ((rc = umma::launch(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
         if ((rc = umma::rmsnorm_pack(m->x, y.norm2, rows, D, m->eps, m->aimg, st))) return rc;
         if (fused_ffn) {

@@ -356,3 +356,44 @@ def test_prefill_on_fp16_images_with_dead_and_extreme_columns(ctx, dm, dff):
         assert np.isfinite(got).all() and np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
     finally:
         pool.close(), gm.close()
+
+
+@pytest.mark.parametrize("dm,dff", [(48, 128), (64, 144), (80, 96), (400, 256)])
+def test_prefill_attention_writes_the_tf32_image_of_other_shapes(ctx, dm, dff):
+    """d_head 16 where fp16 images do not fit (an odd number of heads, or a d_ff that is no multiple of 128): the attention writes Wo's TF32
+    operand image itself, over ragged prompts and row tiles.
+
+    Tolerance: a value is rounded to fp16 (2^-11 of it); products of 22-bit operands, fewer than 128 fp32 additions each, are within 1e-5 of
+    sum |x w|; a prompt of one token has its own value as attention output, and only those rows are compared."""
+    V, E = 132, 1e-5
+    rng = np.random.default_rng(dm + dff)
+
+    def mat(a, b):
+        return rng.standard_normal((a, b)) / np.sqrt(a)
+
+    lens = [1, 300, 1, 17, 1, 250, 1, 1, 33]  # 605 rows: the last row tile is ragged
+    T = [np.ascontiguousarray(t, np.float32) for t in (rng.standard_normal((V, dm)), np.zeros((512, dm)), mat(dm, dm), mat(dm, dm), mat(dm, dm), mat(dm, dm),
+                                                       mat(dm, dff), np.zeros((dff, dm)), mat(dm, dff), np.ones(dm), np.ones(dm), np.ones(dm), mat(dm, V))]
+    gm = GPTModel(ctx, V, 512, dm, dm // 16, 1, dff, rmsNormEps=1e-6, maxRows=1024)
+    gm.setParameters(T)
+    pool = gm.newPool(64, len(lens))
+    try:
+        prompts = [rng.integers(0, V, n).astype(np.int32) for n in lens]
+        got, _ = gm.forwardPrefillBatch(pool, [pool.seq_alloc() for _ in lens], prompts)
+        assert np.isfinite(got).all()
+        ones = [i for i, n in enumerate(lens) if n == 1]
+        x = T[0].astype(np.float64)[[prompts[i][0] for i in ones]]
+        wv, wo, head = (T[i].astype(np.float64) for i in (4, 5, 12))
+
+        def rms(x):
+            return np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+
+        h = x / rms(x)
+        v = h @ wv
+        y = x + v @ wo
+        off = (2.0 ** -11 * np.abs(v) + E * (np.abs(h) @ np.abs(wv))) @ np.abs(wo) + E * (np.abs(v) @ np.abs(wo)) + 1e-6 * np.abs(y)
+        z = y / rms(y)
+        bound = (off / rms(y) + np.sqrt((off ** 2).mean(-1, keepdims=True)) / rms(y) * np.abs(z)) @ np.abs(head) + E * (np.abs(z) @ np.abs(head))
+        assert np.all(np.abs(got[ones] - z @ head) <= bound), float((np.abs(got[ones] - z @ head) / bound).max())
+    finally:
+        pool.close(), gm.close()
