@@ -960,14 +960,14 @@ extern "C" __attribute__((visibility("default"))) int jgpt_debug_decode_trace(lo
 }
 #endif
 
-// Clusters of `c` CTAs of the scalar dhead-16.. decode kernel (this block size and ring) that the device holds at once,
-// as cudaOccupancyMaxActiveClusters reports it; cached per shape.  On B200 with 416 threads and a 72 KiB ring:
+// Clusters of `c` CTAs of the decode kernel with these consumers, block size and ring that the device holds at once, as
+// cudaOccupancyMaxActiveClusters reports it; cached per shape.  On B200 with 416 threads (fp32 consumers of 24 heads) and a 72 KiB ring:
 // 296 single CTAs, but 93 / 71 / 56 / 45 / 37 / 33 clusters of 3 / 4 / 5 / 6 / 7 / 8 (a cluster stays inside one GPC).
 // 0 when the query fails (the caller then plans without clusters).
-static int cluster_capacity(Pool *p, bool fused, int threads, size_t smem, int c) {
+static int cluster_capacity(Pool *p, bool fused, bool mma, int threads, size_t smem, int c) {
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int, size_t, int, int>, int> cache;
-    const auto key = std::make_tuple(p->ctx->device, p->dhead, (int)fused, smem, threads, c);
+    static std::map<std::tuple<int, int, int, int, size_t, int, int>, int> cache;
+    const auto key = std::make_tuple(p->ctx->device, p->dhead, (int)fused, (int)mma, smem, threads, c);
     {
         std::lock_guard<std::mutex> lock(mu);
         auto it = cache.find(key);
@@ -978,7 +978,10 @@ static int cluster_capacity(Pool *p, bool fused, int threads, size_t smem, int c
     switch (p->dhead) {
         case 4: kern = fused ? attn_decode_kernel<4, true> : attn_decode_kernel<4, false>, variant = 0; break;
         case 8: kern = fused ? attn_decode_kernel<8, true> : attn_decode_kernel<8, false>, variant = 4; break;
-        case 16: kern = fused ? attn_decode_kernel<16, true> : attn_decode_kernel<16, false>, variant = 10; break;
+        case 16:
+            if (mma) kern = fused ? attn_decode_kernel<16, true, true> : attn_decode_kernel<16, false, true>, variant = 10;
+            else kern = fused ? attn_decode_kernel<16, true, false> : attn_decode_kernel<16, false, false>, variant = 8;
+            break;
         case 32: kern = fused ? attn_decode_kernel<32, true> : attn_decode_kernel<32, false>, variant = 12; break;
         default: return 0;
     }
@@ -1031,17 +1034,18 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     const bool overlapped_single = ov >= 1 && n_layers == 1 && p->persistent <= 0;
     P.HG = overlapped_single ? pick_head_group(p->heads, DH, p->head_group)
                              : pick_head_group(p->heads, DH, p->head_group, (long long)n_layers * n, 2ll * p->ctx->sm_count);
-    // With up to a row per SM and sequences of up to 1024 tokens the heads go to two CTAs (d_head 16, whose consumer warps take four heads
-    // each): smaller CTAs spread more evenly, and the last one is done sooner.  JGPT-35M step of context 512 at 8 / 32 / 64 / 128 / 160 / 200
-    // rows, us: one CTA 208 / 278 / 351 / 524 / 582 / 697, two 203 / 270 / 344 / 508 / 550 / 742, three 201 / 286 / 358 / 524 / 568 / 755.
+    // (a launch that is one of several over a call's layers chooses its consumers by all of them, like the launch of the whole call)
+    const int rule_layers = of_layers > 0 ? of_layers : n_layers;
+    const bool mma = DH == 16 && tensor_consumers(p, overlapped_single && rule_layers == 1, (long long)rule_layers * n);
+    // With up to a row per SM and sequences of up to 1024 tokens the heads go to two CTAs: smaller CTAs spread more evenly, and the last one
+    // is done sooner.  Tensor-core consumers, JGPT-35M step of context 512 at 8 / 32 / 64 / 128 / 160 / 200 rows, us: one CTA
+    // 208 / 278 / 351 / 524 / 582 / 697, two 203 / 270 / 344 / 508 / 550 / 742, three 201 / 286 / 358 / 524 / 568 / 755 (160 rows would gain
+    // as well; between them and 200 it turns).  fp32 consumers, host calls of 3 to 11 layers in stages, 1 to 8 rows of 1000: 0-4 % of the call.
     // Long sequences stream, and whole slabs do that better (48 of 1024 to 8192 tokens, 12 layers: 567 us, 596 in halves).
     if (overlapped_single && DH == 16 && p->head_group <= 0 && P.HG % 2 == 0 && P.HG >= 12 && max_len <= 1024 &&
         (long long)n * (p->heads / P.HG) <= p->ctx->sm_count)
         P.HG /= 2;
     P.n_hg = p->heads / P.HG;
-    // (a launch that is one of several over a call's layers goes by all of them: the call's bits do not depend on how it is cut)
-    const int rule_layers = of_layers > 0 ? of_layers : n_layers;
-    const bool mma = DH == 16 && tensor_consumers(p, overlapped_single && rule_layers == 1, (long long)rule_layers * n);
     const int max_blocks = std::min(p->max_blocks_per_seq, (max_len + kBlockTokens - 1) / kBlockTokens);
     // Work distribution.  Default (persistent <= 0): one CTA per work item, the hardware block scheduler hands
     // items to SMs as CTAs retire.  persistent = k > 0: k CTAs per SM claim items from a global counter (kept
@@ -1067,7 +1071,7 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
         const long long base = (long long)n * P.n_hg;
         int c = 1;
         for (int t = std::min(8, (max_blocks + 3) / 4); t >= 2; t--)
-            if (16 * base <= 15ll * cluster_capacity(p, k_new != nullptr, threads, smem, t)) {
+            if (16 * base <= 15ll * cluster_capacity(p, k_new != nullptr, mma, threads, smem, t)) {
                 c = t;
                 break;
             }
@@ -1078,7 +1082,7 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
             // 2 rounds (0.985); 224 rows: 2 chunks in 2 rounds (1.217) against 3 chunks in 3 (1.264).
             long long best_cost = -1;
             for (int t = c_min; t <= std::min(8, (max_blocks + 3) / 4); t++) {
-                const long long cap = t == 1 ? 2ll * p->ctx->sm_count : (long long)cluster_capacity(p, k_new != nullptr, threads, smem, t);
+                const long long cap = t == 1 ? 2ll * p->ctx->sm_count : (long long)cluster_capacity(p, k_new != nullptr, mma, threads, smem, t);
                 if (cap <= 0) continue;
                 // (clusters of three and more: a round counts as full at 15/16 of the capacity, like the one-wave rule above --
                 // 186 rows are two rounds of 93 three-CTA clusters on paper and measured 0.98 ms against 0.92 ms with pairs)

@@ -116,15 +116,15 @@ def test_tensor_core_consumer_head_groups_scales_and_infinities(ctx, H, chunk):
 
 @pytest.mark.parametrize("fused", [False, True])
 def test_tensor_core_consumer_matches_oracle(ctx, fused):
-    """JGPT_B200_DECODE_MMA=1: scores and P.V on mma.sync with fp16 hi/lo split operands (d_head 16).  Same tolerance
-    as the scalar consumer; ragged lengths, split-K, odd head count, dead slots in the last block poisoned with NaN."""
-    os.environ["JGPT_B200_DECODE_MMA"] = "1"
+    """Per-layer launches at d_head 16 with four heads to a CTA's warp: scores and P.V on mma.sync with fp16 high + low operands.  Same
+    tolerance as the fp32 consumers; ragged lengths, split-K, dead slots in the last block poisoned with NaN."""
     os.environ["JGPT_B200_CHUNK_BLOCKS"] = "4"
     try:
         lens0 = [1, 15, 16, 17, 33, 130, 257, 700]
         case = PagedCase(ctx, lens0, H=5, Dh=16, layers=1, seed=51, spare_tokens=2)
     finally:
-        os.environ.pop("JGPT_B200_DECODE_MMA"), os.environ.pop("JGPT_B200_CHUNK_BLOCKS")
+        os.environ.pop("JGPT_B200_CHUNK_BLOCKS")
+    case.pool.set_tuning(chunk_blocks=4, launch_overlap=1)
     try:
         rng = np.random.default_rng(52)
         n, H, Dh = case.n, 5, 16
@@ -156,6 +156,80 @@ def test_tensor_core_consumer_matches_oracle(ctx, fused):
         ctx.synchronize()
         got = out.to_host()
         assert np.isfinite(got).all() and np.abs(got - want).max() < TOL, np.abs(got - want).max()
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("below", [True, False])
+def test_which_consumers_a_launch_of_several_layers_takes(ctx, fused, below):
+    """d_head 16: a launch of fewer (layer, sequence) pairs than two CTAs per SM takes the fp32 consumers, one of as many or more the tensor
+    cores; per-layer launches take the latter as well.  Sequences of at most 64 tokens are one chunk each, so the bits tell which consumers
+    ran: each form is compared with launches that are known to take them, and with the oracle, dead slots poisoned with NaN."""
+    from jgpt_b200 import binding as B
+    H, Dh, layers = 24, 16, 4
+    n = (2 * 148 - 1) // layers if below else -(-2 * 148 // layers)
+    rng = np.random.default_rng(71)
+    lens0 = rng.integers(1, 63, n).tolist()
+    lens0[:4] = [1, 15, 16, 62]
+    lens = np.array(lens0, np.int32)
+    q, k, v = (rng.standard_normal((layers, n, H * Dh)).astype(np.float32) for _ in range(3))
+
+    def run(overlap, per):
+        case = PagedCase(ctx, lens0, H=H, Dh=Dh, layers=layers, seed=72, spare_tokens=2)
+        try:
+            case.pool.set_tuning(launch_overlap=overlap)
+            ptr, nbytes = case.pool.storage()
+            raw = np.empty(nbytes // 2, np.uint16)
+            B.check(ctx._lib.jgpt_d2h(ctx.handle, raw.ctypes.data, ptr, nbytes))
+            tiles = raw.reshape(layers, case.n_blocks, H, 2, 16, Dh)
+            for i, l in enumerate(lens0):
+                if l // 16 < len(case.tables[i]):
+                    tiles[:, case.tables[i][l // 16], :, :, l % 16:, :] = 0x7E00  # fp16 NaN
+            B.check(ctx._lib.jgpt_h2d(ctx.handle, ptr, raw.ctypes.data, nbytes))
+            out = ctx.alloc((layers, n, H * Dh))
+            new = lens + 1 if fused else lens
+            rope = ctx.from_host((new - 1).astype(np.int32))
+            dq, dk, dv, dl = ctx.from_host(q), ctx.from_host(k), ctx.from_host(v), ctx.from_host(new.astype(np.int32))
+            for l in range(0, layers, per):
+                at = l * n * H * Dh * 4
+                args = (case.seq_ids_dev(), rope, dl, n, int(new.max()), out.ptr + at)
+                if fused:
+                    case.pool.attn_decode_append(l, per, dq.ptr + at, dk.ptr + at, dv.ptr + at, *args)
+                else:
+                    case.pool.attn_decode(l, per, dq.ptr + at, *args)
+            ctx.synchronize()
+            want = None
+            if per > 1:
+                want = np.stack([O.decode_attn_batch(q[l], k[l], v[l], case.kc[l], case.vc[l], lens, new - 1, H, Dh, case.max_seq, kv_fp16=True) if fused
+                                 else _oracle_decode(case, l, q[l], lens0, new - 1) for l in range(layers)])
+            return out.to_host(), want
+        finally:
+            case.close()
+
+    got, want = run(1, layers)
+    assert np.isfinite(got).all() and np.abs(got - want).max() < TOL
+    fp32, tensor = run(0, 1)[0], run(1, 1)[0]  # one layer of `n` < 2 x 148 pairs with and without overlapped launches
+    assert not np.array_equal(fp32, tensor)
+    assert np.array_equal(got, fp32 if below else tensor)
+
+
+@pytest.mark.parametrize("layers", [3, 6])
+def test_staged_layer_groups_of_a_host_call_with_long_sequences(ctx, layers, monkeypatch):
+    """The host-buffer form in its staged way sends the first and the last layer of a short call as launches of their own, which take the fp32
+    consumers like the launch of the whole call and are cut into clusters of chunks for them: against the oracle over one to many chunks."""
+    monkeypatch.setenv("JGPT_B200_HOST_ZEROCOPY", "0")
+    lens0 = [700, 5, 129, 1023]
+    case = PagedCase(ctx, lens0, H=24, Dh=16, layers=layers, seed=81, spare_tokens=1)
+    try:
+        rng = np.random.default_rng(82)
+        n, D = len(lens0), 24 * 16
+        q, k, v = (rng.standard_normal((layers, n, D)).astype(np.float32) for _ in range(3))
+        lens = np.array(lens0, np.int32)
+        got = case.pool.attn_decode_append_host(0, layers, q, k, v, case.seqs, lens, lens + 1)
+        for l in range(layers):
+            want = O.decode_attn_batch(q[l], k[l], v[l], case.kc[l], case.vc[l], lens, lens, 24, 16, case.max_seq, kv_fp16=True)
+            assert np.abs(got[l] - want).max() < TOL, (l, np.abs(got[l] - want).max())
     finally:
         case.close()
 
