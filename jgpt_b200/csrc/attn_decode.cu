@@ -399,11 +399,14 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
             // sits in the lanes with lane % 4 == i.  Lane (g, t) thus carries the scores of tokens g and g + 8 and the sums of
             // dims g and g + 8 of head t: every lane has work, and maximum, exponentials and rescaling serve four heads at once.
             // A product's unused columns stay unused, so an infinity in one head does not reach another.
-            // q is scaled by a power of two per head and p by 2^14, both to keep the low parts clear of fp16's subnormals: the
-            // running reference m lies 14 below the maximum, p = 2^(s - m) <= 2^14, and the factor cancels in o / l.
+            // q is scaled by a power of two per head and p by 2^14, both to keep the low parts clear of fp16's subnormals; the factor
+            // cancels in o / l.  p is scaled behind its exponential: a reference 14 below the maximum gives the same factor for one
+            // instruction less, but rounds s - m at 14 instead of near 0, 2e-7 of every p.
+            // Error against float64 over 64 x 1024 keys (2-norm, fp16-exact K and V), fp32 consumers -> these, for q of 0.2, 1 and 4:
+            // 1.5e-7 -> 1.6e-7, 2.3e-7 -> 2.0e-7, 5.0e-7 -> 3.4e-7 (with the reference below the maximum 2.5e-7, 2.9e-7, 3.4e-7).
             // About 95 instructions per 4 heads x 16 tokens where fp32 FMAs on converted rows took 380: one CTA alone was
             // issue-bound at 43 GB/s.
-            constexpr float kLift = 14.f;
+            constexpr float kLift = 16384.f;
             const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
             int rp = rp_raw;
             if (rp < 0 || rp >= P.max_positions) {
@@ -456,10 +459,9 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                 sc += __shfl_xor_sync(0xffffffffu, sc, 4);
                 sc += __shfl_xor_sync(0xffffffffu, sc, 8);
                 sc += __shfl_xor_sync(0xffffffffu, sc, 16);
-                m = sc - kLift;
-                const float p = fast_exp2(sc - m);
-                l = g == 0 ? p : 0.f;
-                o[0] = p * __half2float(__float2half_rn(va)), o[2] = p * __half2float(__float2half_rn(vb));
+                m = sc;
+                l = g == 0 ? kLift : 0.f;
+                o[0] = kLift * __half2float(__float2half_rn(va)), o[2] = kLift * __half2float(__float2half_rn(vb));
                 const int phys = P.table[(size_t)seq * P.mbs + len_cached / BT];
                 if (phys < 0 || phys >= P.n_blocks) {
                     if (lane == 0) atomicOr(P.status, DEV_STATUS_BAD_BLOCK);
@@ -519,9 +521,9 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 4));
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 8));
                     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 16));
-                    const float mn = fmaxf(m, bm - kLift);
+                    const float mn = fmaxf(m, bm);
                     const float corr = fast_exp2(m - mn);
-                    const float p0 = fast_exp2(s0 - mn), p1 = fast_exp2(s1 - mn);
+                    const float p0 = fast_exp2(s0 - mn) * kLift, p1 = fast_exp2(s1 - mn) * kLift;
                     m = mn;
                     l = l * corr + (p0 + p1);
                     const uint32_t pb0 = column(__shfl_sync(0xffffffffu, p0, src0), __shfl_sync(0xffffffffu, p0, src1));

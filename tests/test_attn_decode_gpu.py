@@ -160,6 +160,38 @@ def test_tensor_core_consumer_matches_oracle(ctx, fused):
         case.close()
 
 
+@pytest.mark.parametrize("size", [0.2, 1.0])
+@pytest.mark.parametrize("overlap", [0, 1])
+def test_error_against_float64_with_either_consumers(ctx, overlap, size):
+    """d_head 16, one layer of short and long sequences without rotation (position 0), against float64 on the fp16 payload: the fp32 consumers
+    (no overlapped launches) and the tensor cores.
+
+    Tolerance (2-norm): a score is within 2^-22 sum |q k| / 4 of the exact one, for q of `size` about 2^-22 * 2.5 size, rounded once more when
+    the maximum is taken off (below 2^-23 for the scores here, which lie within 8 of it); a probability and its high and low part add 2^-22.5
+    and 2^-23, uniformly spread errors of which a third or less remains in the norm; 16 to 64 partial sums add 2^-24 each, at random signs."""
+    lens = [3, 17, 64, 200, 500]
+    case = PagedCase(ctx, lens, H=24, Dh=16, layers=1, seed=91)
+    try:
+        case.pool.set_tuning(launch_overlap=overlap)
+        rng = np.random.default_rng(92)
+        q = (rng.standard_normal((case.n, 24, 16)) * size).astype(np.float32)
+        out = ctx.alloc((case.n, 24 * 16))
+        case.pool.attn_decode(0, 1, ctx.from_host(q.reshape(case.n, -1)), case.seq_ids_dev(), ctx.from_host(np.zeros(case.n, np.int32)),
+                              ctx.from_host(case.lens), case.n, max(lens), out)
+        ctx.synchronize()
+        got = out.to_host().reshape(case.n, 24, 16)
+        for i, l in enumerate(lens):
+            k, v = case.kc[0, i, :, :l].astype(np.float64), case.vc[0, i, :, :l].astype(np.float64)
+            s = np.einsum("hd,hkd->hk", q[i].astype(np.float64), k) / 4
+            p = np.exp(s - s.max(-1, keepdims=True))
+            want = np.einsum("hk,hkd->hd", p / p.sum(-1, keepdims=True), v)
+            err = np.linalg.norm(got[i] - want) / np.linalg.norm(want)
+            bound = np.sqrt(3 * (2.0 ** -24) ** 2 + (2.0 ** -22.5 / 3) ** 2 + (2.0 ** -22 * 2.5 * size / 3) ** 2 + 16 * (2.0 ** -24 / np.sqrt(3)) ** 2)
+            assert err <= bound, (l, err, bound)
+    finally:
+        case.close()
+
+
 @pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("below", [True, False])
 def test_which_consumers_a_launch_of_several_layers_takes(ctx, fused, below):
