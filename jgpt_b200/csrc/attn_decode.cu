@@ -164,7 +164,7 @@ constexpr int max_head_group() { return (384 / DH) < 30 ? (384 / DH) : 30; }
 // Consumer threads of a CTA: (head, token) pairs, or a warp per four heads with the products of dhead 16 on the tensor cores.
 template <bool MMA>
 __host__ __device__ constexpr int consumer_threads(int HG) {
-    return MMA ? (HG + 3) / 4 * 32 : (kBlockTokens * HG + 31) / 32 * 32;
+    return MMA ? HG / 4 * 32 : (kBlockTokens * HG + 31) / 32 * 32;
 }
 
 template <int DH, bool FUSED, bool MMA = DH == 16>
@@ -414,9 +414,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                 rp = 0;
             }
             const float2 *cs = P.rope + (size_t)rp * (DH / 2);
-            const int hl = 4 * warp + t4, hl_q = min(4 * warp + (g >> 1), P.HG - 1);
-            const bool act = hl < P.HG;
-            const int h = head0 + (act ? hl : 0);
+            const int hl = 4 * warp + t4, h = head0 + hl;  // HG is a multiple of four
             auto turned = [](float2 x, float2 w) {  // RoPE with separate roundings
                 return make_float2(__fsub_rn(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y)), __fadd_rn(__fmul_rn(x.x, w.y), __fmul_rn(x.y, w.x)));
             };
@@ -430,7 +428,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
             uint32_t qb0, qb1;
             float q_un;  // undoes head t's power of two
             {
-                const float *qp = P.q + row + (size_t)(head0 + hl_q) * DH;
+                const float *qp = P.q + row + (size_t)(head0 + 4 * warp + (g >> 1)) * DH;
                 const float2 x0 = turned(*reinterpret_cast<const float2 *>(qp + 2 * t4), cs[t4]);
                 const float2 x1 = turned(*reinterpret_cast<const float2 *>(qp + 2 * t4 + 8), cs[t4 + 4]);
                 float mx = fmaxf(fmaxf(fabsf(x0.x), fabsf(x0.y)), fmaxf(fabsf(x1.x), fabsf(x1.y)));
@@ -465,7 +463,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                 const int phys = P.table[(size_t)seq * P.mbs + len_cached / BT];
                 if (phys < 0 || phys >= P.n_blocks) {
                     if (lane == 0) atomicOr(P.status, DEV_STATUS_BAD_BLOCK);
-                } else if (act) {
+                } else {
                     __half *dst = P.kv + ((layer_base + phys) * P.H + h) * (size_t)(2 * BT * DH) + (size_t)(len_cached % BT) * DH + 2 * g;
                     *reinterpret_cast<__half2 *>(dst) = kh;
                     *reinterpret_cast<__half2 *>(dst + BT * DH) = vh;
@@ -497,7 +495,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                     uint32_t va[4][4];
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        const unsigned char *tile = base + (size_t)min(4 * warp + i, P.HG - 1) * HEAD_BYTES;
+                        const unsigned char *tile = base + (size_t)(4 * warp + i) * HEAD_BYTES;
                         uint32_t ka[4];
                         ldmatrix_x4(ka, tile + k_off);
                         ldmatrix_x4_trans(va[i], tile + v_off);
@@ -549,7 +547,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
             l += __shfl_xor_sync(0xffffffffu, l, 8);
             l += __shfl_xor_sync(0xffffffffu, l, 16);
             const float o0 = o[0] + o[1], o1 = o[2] + o[3];  // dims g, g + 8 of head h
-            const bool writer = act && !aborted;
+            const bool writer = !aborted;
             float *op = P.out + row + (size_t)h * DH + g;
             if (nsplit == 1) {
                 if (writer) {
@@ -562,11 +560,11 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
             constexpr int PS = DH + 2;
             if (P.cluster) {
                 // ---- split-K inside a cluster: partials stay in shared memory, the CTA of chunk 0 merges them ----
-                float *pp = cl_part + (act ? hl : 0) * PS;
+                float *pp = cl_part + hl * PS;
                 if (writer) {
                     pp[2 + g] = o0, pp[10 + g] = o1;
                     if (g == 0) pp[0] = m, pp[1] = l;
-                } else if (act && g == 0) {
+                } else if (g == 0) {
                     pp[0] = -INFINITY, pp[1] = 0.f;  // a chunk that gave up contributes nothing
                 }
                 cluster_sync();
@@ -912,10 +910,13 @@ static int pick_head_group(int H, int DH, int forced, long long pairs = 0, long 
 }
 
 // d_head 16: the tensor-core consumers for the per-layer launches of a decode loop and for launches of more (layer, sequence) pairs than
-// fit at once.  A smaller launch is latency, and a block is a longer chain on the tensor cores (two products, three shuffles
-// for the maximum, two for p) than for a thread with its own token: 12 layers of a few sequences in one launch took
-// 39.9 and 8.7 us with the fp32 consumers, 43.6 and 10.9 us with these; 64 x 1024 takes 190 and 188 us.
-static bool tensor_consumers(const Pool *p, bool per_layer, long long pairs) {
+// fit at once, in CTAs of a multiple of four heads.  A smaller launch is latency, and a block is a longer chain on the tensor cores (two
+// products, three shuffles for the maximum, two for p) than for a thread with its own token: 12 layers of a few sequences in one launch
+// took 39.9 and 8.7 us with the fp32 consumers, 43.6 and 10.9 us with these; 64 x 1024 takes 190 and 188 us.  A warp with fewer than four
+// heads does the same work for less: a launch per layer for 200 sequences of 1000, 1 / 2 / 6 heads, 13.3 / 13.5 / 20.1 us with the fp32
+// consumers, 18.5 / 18.5 / 21.0 with a ragged last warp.
+static bool tensor_consumers(const Pool *p, int HG, bool per_layer, long long pairs) {
+    if (HG % 4 != 0) return false;
     return per_layer || pairs * (p->heads / pick_head_group(p->heads, 16, p->head_group)) >= 2ll * p->ctx->sm_count;
 }
 
@@ -1038,15 +1039,15 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
                              : pick_head_group(p->heads, DH, p->head_group, (long long)n_layers * n, 2ll * p->ctx->sm_count);
     // (a launch that is one of several over a call's layers chooses its consumers by all of them, like the launch of the whole call)
     const int rule_layers = of_layers > 0 ? of_layers : n_layers;
-    const bool mma = DH == 16 && tensor_consumers(p, overlapped_single && rule_layers == 1, (long long)rule_layers * n);
+    const bool mma = DH == 16 && tensor_consumers(p, P.HG, overlapped_single && rule_layers == 1, (long long)rule_layers * n);
     // With up to a row per SM and sequences of up to 1024 tokens the heads go to two CTAs: smaller CTAs spread more evenly, and the last one
     // is done sooner.  Tensor-core consumers, JGPT-35M step of context 512 at 8 / 32 / 64 / 128 / 160 / 200 rows, us: one CTA
     // 208 / 278 / 351 / 524 / 582 / 697, two 203 / 270 / 344 / 508 / 550 / 742, three 201 / 286 / 358 / 524 / 568 / 755 (160 rows would gain
     // as well; between them and 200 it turns).  fp32 consumers, host calls of 3 to 11 layers in stages, 1 to 8 rows of 1000: 0-4 % of the call.
     // Long sequences stream, and whole slabs do that better (48 of 1024 to 8192 tokens, 12 layers: 567 us, 596 in halves).
-    if (overlapped_single && DH == 16 && p->head_group <= 0 && P.HG % 2 == 0 && P.HG >= 12 && max_len <= 1024 &&
-        (long long)n * (p->heads / P.HG) <= p->ctx->sm_count)
-        P.HG /= 2;
+    const bool halves = overlapped_single && DH == 16 && p->head_group <= 0 && P.HG >= 12 && P.HG % (mma ? 8 : 2) == 0 && max_len <= 1024 &&
+                        (long long)n * (p->heads / P.HG) <= p->ctx->sm_count;
+    if (halves) P.HG /= 2;
     P.n_hg = p->heads / P.HG;
     const int max_blocks = std::min(p->max_blocks_per_seq, (max_len + kBlockTokens - 1) / kBlockTokens);
     // Work distribution.  Default (persistent <= 0): one CTA per work item, the hardware block scheduler hands
@@ -1059,60 +1060,87 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
     const int n_cons = mma ? consumer_threads<true>(P.HG) : consumer_threads<false>(P.HG);
     const int threads = n_cons + 32;
     const size_t stage_bytes = (size_t)P.HG * 2 * kBlockTokens * DH * 2;
-    const size_t smem = stage_bytes * P.stages;
-    const bool may_cluster = p->cluster_merge && !dynamic;
-    if (p->chunk_blocks > 0) {
-        P.chunk_blocks = p->chunk_blocks;
-    } else if (overlapped_single && may_cluster) {
-        // The per-layer launch of the model's decode step: the chunks of a sequence are one cluster, so the launch is one
-        // wave only while the device holds `base` clusters of that size at once -- fewer CTAs than two per SM (see
-        // cluster_capacity; clusters beyond it wait for a whole CTA time).  Most chunks of at least 4 blocks that stay
-        // 1/16 under that number (a launch at the exact limit measured slower than the next smaller cluster).  JGPT-35M
-        // step, ms per step before / after: 40 rows 0.591 / 0.509, 48 rows 0.614 / 0.512, 96 rows 0.775 / 0.672;
-        // up to 29 rows ten chunks merged through global scratch became eight in a cluster (16 rows: 0.430 / 0.413).
-        const long long base = (long long)n * P.n_hg;
-        int c = 1;
-        for (int t = std::min(8, (max_blocks + 3) / 4); t >= 2; t--)
-            if (16 * base <= 15ll * cluster_capacity(p, k_new != nullptr, mma, threads, smem, t)) {
-                c = t;
-                break;
-            }
-        const int c_min = (max_blocks + 31) / 32;  // a chunk holds at most 32 blocks
-        if (c == 1 && (c_min > 1 || base > 2ll * p->ctx->sm_count)) {
-            // No split fits one wave: take the one with the least rounds x (chunk length + ~6 blocks' worth of per-CTA
-            // start-up and merge).  160 rows of 40 blocks: 3 chunks in 2 rounds (0.925 ms per step) against 2 chunks in
-            // 2 rounds (0.985); 224 rows: 2 chunks in 2 rounds (1.217) against 3 chunks in 3 (1.264).
-            long long best_cost = -1;
-            for (int t = c_min; t <= std::min(8, (max_blocks + 3) / 4); t++) {
-                const long long cap = t == 1 ? 2ll * p->ctx->sm_count : (long long)cluster_capacity(p, k_new != nullptr, mma, threads, smem, t);
-                if (cap <= 0) continue;
-                // (clusters of three and more: a round counts as full at 15/16 of the capacity, like the one-wave rule above --
-                // 186 rows are two rounds of 93 three-CTA clusters on paper and measured 0.98 ms against 0.92 ms with pairs)
-                const long long full = t >= 3 ? 15 * cap : 16 * cap;
-                const long long rounds = (16 * base + full - 1) / full, cost = rounds * ((max_blocks + t - 1) / t + 6);
-                if (best_cost < 0 || cost < best_cost) best_cost = cost, c = t;
-            }
-        }
-        c = std::max(c, c_min);
-        P.chunk_blocks = std::min(32, std::max(4, (max_blocks + c - 1) / c));
-    } else {
-        P.chunk_blocks = pick_chunk_blocks(p, (long long)n_layers * n * P.n_hg, max_blocks);
-    }
-    P.max_len = max_blocks * kBlockTokens;
-    P.max_chunks = std::max(1, (max_blocks + P.chunk_blocks - 1) / P.chunk_blocks);
-    P.overlap = ov;
-    P.stream_hint = p->stream_hint;
-    P.scale_log2e = (1.0f / sqrtf((float)DH)) * 1.4426950408889634f;
-    const long long items = (long long)n_layers * n * P.n_hg * P.max_chunks;
-    JGPT_REQUIRE(items < (1ll << 31), JGPT_ERR_INVALID_ARGUMENT, "too many work items (%lld)", items);
-    P.n_items = (int)items;
+    const bool may_cluster = p->cluster_merge && !dynamic, fused = k_new != nullptr;
     // The chunks of one sequence as one thread-block cluster (up to the portable size of 8): merge in shared memory.
     // Not for the work queue (its CTAs take several items).
     // Only for launches of a wave or two: there the merge's global round trips are a visible part of the launch (per-layer
     // launch at batch 64 / context 1024: 24.1 -> 22.7 us).  A launch of many waves hides them behind other CTAs' copies,
     // and co-scheduling pairs of CTAs costs it more than it saves (12-layer launch: 198 us without, 202 us with).
-    P.cluster = (may_cluster && P.max_chunks >= 2 && P.max_chunks <= 8 &&
-                 items <= 4ll * p->ctx->sm_count) ? 1 : 0;
+    auto cluster_launch = [&](int chunks, long long items) { return may_cluster && chunks >= 2 && chunks <= 8 && items <= 4ll * p->ctx->sm_count; };
+    // How a launch whose CTAs take `ring` bytes of shared memory is cut, and how many rounds of CTAs that makes (where it is asked below).
+    struct Cut {
+        int chunk_blocks, max_chunks;
+        long long items, slots;
+        long long rounds() const { return (items + slots - 1) / slots; }
+    };
+    auto cut = [&](size_t ring) {
+        Cut o{};
+        if (p->chunk_blocks > 0) {
+            o.chunk_blocks = p->chunk_blocks;
+        } else if (overlapped_single && may_cluster) {
+            // The per-layer launch of the model's decode step: the chunks of a sequence are one cluster, so the launch is one
+            // wave only while the device holds `base` clusters of that size at once -- fewer CTAs than two per SM (see
+            // cluster_capacity; clusters beyond it wait for a whole CTA time).  Most chunks of at least 4 blocks that stay
+            // 1/16 under that number (a launch at the exact limit measured slower than the next smaller cluster).  JGPT-35M
+            // step, ms per step before / after: 40 rows 0.591 / 0.509, 48 rows 0.614 / 0.512, 96 rows 0.775 / 0.672;
+            // up to 29 rows ten chunks merged through global scratch became eight in a cluster (16 rows: 0.430 / 0.413).
+            const long long base = (long long)n * P.n_hg;
+            int c = 1;
+            for (int t = std::min(8, (max_blocks + 3) / 4); t >= 2; t--)
+                if (16 * base <= 15ll * cluster_capacity(p, fused, mma, threads, ring, t)) {
+                    c = t;
+                    break;
+                }
+            const int c_min = (max_blocks + 31) / 32;  // a chunk holds at most 32 blocks
+            if (c == 1 && (c_min > 1 || base > 2ll * p->ctx->sm_count)) {
+                // No split fits one wave: take the one with the least rounds x (chunk length + ~6 blocks' worth of per-CTA
+                // start-up and merge).  160 rows of 40 blocks: 3 chunks in 2 rounds (0.925 ms per step) against 2 chunks in
+                // 2 rounds (0.985); 224 rows: 2 chunks in 2 rounds (1.217) against 3 chunks in 3 (1.264).
+                long long best_cost = -1;
+                for (int t = c_min; t <= std::min(8, (max_blocks + 3) / 4); t++) {
+                    const long long cap = t == 1 ? 2ll * p->ctx->sm_count : (long long)cluster_capacity(p, fused, mma, threads, ring, t);
+                    if (cap <= 0) continue;
+                    // (clusters of three and more: a round counts as full at 15/16 of the capacity, like the one-wave rule above --
+                    // 186 rows are two rounds of 93 three-CTA clusters on paper and measured 0.98 ms against 0.92 ms with pairs)
+                    const long long full = t >= 3 ? 15 * cap : 16 * cap;
+                    const long long rounds = (16 * base + full - 1) / full, cost = rounds * ((max_blocks + t - 1) / t + 6);
+                    if (best_cost < 0 || cost < best_cost) best_cost = cost, c = t;
+                }
+            }
+            c = std::max(c, c_min);
+            o.chunk_blocks = std::min(32, std::max(4, (max_blocks + c - 1) / c));
+        } else {
+            o.chunk_blocks = pick_chunk_blocks(p, (long long)n_layers * n * P.n_hg, max_blocks);
+        }
+        o.max_chunks = std::max(1, (max_blocks + o.chunk_blocks - 1) / o.chunk_blocks);
+        o.items = (long long)n_layers * n * P.n_hg * o.max_chunks, o.slots = 1;
+        if (mma && overlapped_single) {
+            const int size = cluster_launch(o.max_chunks, o.items) ? o.max_chunks : 1;
+            o.slots = std::max(1ll, (long long)size * cluster_capacity(p, fused, mma, threads, ring, size));
+        }
+        return o;
+    };
+    // The tensor-core consumers need few registers, so shared memory decides how many CTAs of a per-layer launch share an SM: three with
+    // all 24 heads, where the fp32 consumers stand two at a time.  Three are one round less for some launches (36 sequences of 4096: 43 us
+    // a layer, 61 with two).  Otherwise the third only lets CTAs that move in early pile up on the SMs that are free first and makes a last,
+    // short round as long as a full one (28 of 1024 to 4096 tokens 38 us with three, 32 with two; 64 of 4096 83 and 73), so the ring is
+    // padded by half unless it saves a round.  A launch of at most half the slots spreads by itself where it runs back to back with
+    // its like (48 of 2000 with 8 heads 16 us, 18 padded), and halves of the heads (96 of 1000: 30 and 33) and CTAs of four (200 of 4000: 42
+    // and 57) always.
+    size_t smem = stage_bytes * P.stages;
+    Cut plan = cut(smem);
+    if (mma && overlapped_single && !halves && P.HG >= 8 && p->stages <= 0 && (ov >= 2 || 2 * plan.items > plan.slots)) {
+        const Cut two = cut(smem * 3 / 2);
+        if (two.rounds() <= plan.rounds()) plan = two, smem = smem * 3 / 2;
+    }
+    P.chunk_blocks = plan.chunk_blocks, P.max_chunks = plan.max_chunks;
+    P.max_len = max_blocks * kBlockTokens;
+    P.overlap = ov;
+    P.stream_hint = p->stream_hint;
+    P.scale_log2e = (1.0f / sqrtf((float)DH)) * 1.4426950408889634f;
+    JGPT_REQUIRE(plan.items < (1ll << 31), JGPT_ERR_INVALID_ARGUMENT, "too many work items (%lld)", plan.items);
+    P.n_items = (int)plan.items;
+    P.cluster = cluster_launch(P.max_chunks, plan.items) ? 1 : 0;
     if (P.max_chunks > 1 && !P.cluster) {
         int32_t rc = pool_ensure_split_scratch(p, (uint64_t)n_layers * n * P.max_chunks * p->heads * (DH + 2),
                                                (uint64_t)n_layers * n * P.n_hg);
@@ -1138,7 +1166,6 @@ int32_t launch_attn_decode(Pool *p, int layer0, int n_layers, const float *q, co
         P.counters = p->d_item_counters;
     }
     if (P.dynamic && P.overlap > 1) P.overlap = 1;  // the work-queue counters are reset by the previous launch's last CTA
-    const bool fused = k_new != nullptr;
     switch (DH) {
         case 4: return launch_decode_t<4>(p, P, fused, mma, threads, smem, grid);
         case 8: return launch_decode_t<8>(p, P, fused, mma, threads, smem, grid);
@@ -1491,7 +1518,7 @@ static int32_t launch_attn_decode_static(Pool *p, int layer, const float *q, con
         // the counters must start at zero (they reset themselves, but not if an earlier launch gave up half way).
         JGPT_CUDA_TRY(cudaMemsetAsync(P.tickets, 0, sizeof(int) * need_tickets, p->ctx->stream));
     }
-    const bool mma = DH == 16 && tensor_consumers(p, false, n);
+    const bool mma = DH == 16 && tensor_consumers(p, P.HG, false, n);
     const int n_cons = mma ? consumer_threads<true>(P.HG) : consumer_threads<false>(P.HG);
     const int threads = n_cons + 32;
     const size_t smem = (size_t)P.HG * 2 * kBlockTokens * DH * 2 * P.stages;

@@ -69,10 +69,11 @@ def test_split_and_pipeline_settings_agree(ctx, chunk_blocks, stages, persistent
         case.close()
 
 
-@pytest.mark.parametrize("H,chunk", [(1, 0), (4, 1), (6, 2), (7, 0), (24, 3)])
+@pytest.mark.parametrize("H,chunk", [(1, 0), (4, 1), (6, 2), (7, 0), (8, 0), (20, 2), (24, 3)])
 def test_tensor_core_consumer_head_groups_scales_and_infinities(ctx, H, chunk):
-    """d_head 16: warps with one to four heads, queries of very different sizes side by side (each head has its own power of two), and
-    a head whose cached value is infinite, which must not reach the others though they share product operands.
+    """d_head 16: CTAs of one to six warps of four heads (other head counts take the fp32 consumers), queries of very different sizes side
+    by side (each head has its own power of two), and a head whose cached value is infinite, which must not reach the others though they
+    share product operands.
 
     Tolerance: a score is the sum of 16 products whose query has 22 bits, so it is within 2^-21 sum |q k| of the exact one (the
     fp32 oracle is no closer); that moves an output by at most that much times the spread of V (about 8)."""
@@ -116,18 +117,18 @@ def test_tensor_core_consumer_head_groups_scales_and_infinities(ctx, H, chunk):
 
 @pytest.mark.parametrize("fused", [False, True])
 def test_tensor_core_consumer_matches_oracle(ctx, fused):
-    """Per-layer launches at d_head 16 with four heads to a CTA's warp: scores and P.V on mma.sync with fp16 high + low operands.  Same
+    """Per-layer launches at d_head 16 with a multiple of four heads: scores and P.V on mma.sync with fp16 high + low operands.  Same
     tolerance as the fp32 consumers; ragged lengths, split-K, dead slots in the last block poisoned with NaN."""
     os.environ["JGPT_B200_CHUNK_BLOCKS"] = "4"
     try:
         lens0 = [1, 15, 16, 17, 33, 130, 257, 700]
-        case = PagedCase(ctx, lens0, H=5, Dh=16, layers=1, seed=51, spare_tokens=2)
+        case = PagedCase(ctx, lens0, H=20, Dh=16, layers=1, seed=51, spare_tokens=2)
     finally:
         os.environ.pop("JGPT_B200_CHUNK_BLOCKS")
     case.pool.set_tuning(chunk_blocks=4, launch_overlap=1)
     try:
         rng = np.random.default_rng(52)
-        n, H, Dh = case.n, 5, 16
+        n, H, Dh = case.n, 20, 16
         lens = np.array(lens0, np.int32)
         # poison everything beyond each sequence's tokens: the kernel must not let it reach the output
         ptr, nbytes = case.pool.storage()
