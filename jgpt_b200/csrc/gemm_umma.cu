@@ -20,16 +20,21 @@
 // Activation images are written by whatever produces the activation: the RMSNorm packer, the SwiGLU epilogue
 // of the W1/W3 product, or the plain packer (attention output).
 //
-// fp16 images (kind::f16, the forward step of models with d_head 16).  The same 22 bits of an operand as an fp16 high and an fp16
-// low part: two bytes each instead of four, and the tensor cores take 16 k per step instead of 8 at the same rate, so a
+// fp16 images (kind::f16, the forward step of models with d_head 16).  An operand as an fp16 high and an fp16 low part, 11 + 11 bits
+// like the TF32 parts: two bytes each instead of four, and the tensor cores take 16 k per step instead of 8 at the same rate, so a
 // product costs half the time and half the operand traffic.  A 16-byte chunk holds eight k, a k tile 32, everything else lies
 // where the TF32 layout has it.  What fp16's exponent lacks is made up by powers of two, which change no bit:
-//   weights: per column of W, from its largest element; undone in the epilogue (the factors stand behind the image);
+//   weights: per column of W, from its largest element; undone in the epilogue (the factors stand behind the image).  The norm weights
+//   gamma are in the rows of the W that follows the norm, so their spread is not the normalised row's;
 //   RMSNorm rows: per row, from the row's largest element; undone in the epilogue;
 //   attention and SwiGLU results, whose rows no single CTA sees: per column, from what the column can reach at all.  A normalised row
 //   is at most sqrt(D) long, so |v_n| <= sqrt(D) |gamma o Wv_n|, an attention output is a weighted mean of such values, and
 //   |h g sigmoid(g)| <= D |gamma o W1_n| |gamma o W3_n|.  The next weight's rows are divided by the same powers.
-// An element 2^18 below the largest its scale allows for keeps its 22 bits; below that an absolute error 2^-40 of it remains.
+// An element down to 2^-16 of the largest its scale allows for is within 2^-23 of itself, like a TF32 pair at any size; below that an
+// absolute error of at most 2^-39 of that largest remains.  So the 22 bits are those of the largest in the row (column), and a row whose
+// elements spread further along k, with weights the other way round, loses bits that TF32 pairs keep.  Typical results of a SwiGLU lie
+// about 2^10 below their bound.  Error of a block's feed-forward part against float64 (2-norm, 384 / 768, 2000 rows): TF32 4.8e-6, fp16
+// 2.5e-6, of its Wo product 9.5e-7 and 5.2e-7 (half as many steps of accumulation).
 // The attention output of a prefill is such a mean because every key it sees was produced by the same call's Q,K,V product.
 // Measured for 32 x 1024 tokens, 24 heads of 16 (ncu, us per launch, TF32 -> fp16 images): Q,K,V 139 -> 91, W1/W3 + SwiGLU 164 -> 116,
 // Wo / W2 87 -> 73, RMSNorm 26.8 -> 21.5; the prefill of 12 layers 9.9 -> 7.8 ms.
@@ -183,7 +188,8 @@ __device__ __forceinline__ int half_exponent(double mx, int limit) {
     return max(-limit, min(limit, 15 - e));
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
-// One thread per column: up[n] brings the column's largest element (row k divided by k_scale[k]) to [2^14, 2^15), un[n] undoes it.
+// One thread per column: up[n] brings the column's largest element (row k times the norm weight gamma[k] in front of it, or divided by
+// k_scale[k]) to [2^14, 2^15), un[n] undoes it.
 // Image row r is column r of W, or, for a pair, column (r / 256) * 128 + r % 128 of W1 (first 128 rows of a 256-row tile) or W3.
 // In fp64: a weight over a power of two may lie outside fp32 where the product of the two does not.
 __device__ __forceinline__ const float *half_source(const float *W, const float *W3, int r, int &col) {
@@ -191,20 +197,24 @@ __device__ __forceinline__ const float *half_source(const float *W, const float 
     col = (r >> 8) * 128 + (r & 127);
     return r & 128 ? W3 : W;
 }
-__global__ void __launch_bounds__(256) half_scale_kernel(const float *W, const float *W3, const float *k_scale, int K, int N, int rows, float *un, float *up) {
+__device__ __forceinline__ double half_element(float w, const float *gamma, const float *k_scale, int k) {
+    return gamma ? (double)w * gamma[k] : k_scale ? (double)w / k_scale[k] : (double)w;
+}
+__global__ void __launch_bounds__(256) half_scale_kernel(const float *W, const float *W3, const float *gamma, const float *k_scale, int K, int N, int rows,
+                                                         float *un, float *up) {
     const int r = blockIdx.x * 256 + threadIdx.x;
     if (r >= rows) return;
     int col;
     const float *src = half_source(W, W3, r, col);
     double mx = 0.;
     if (col < N)
-        for (int k = 0; k < K; k++) mx = fmax(mx, fabs((double)src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f)));
+        for (int k = 0; k < K; k++) mx = fmax(mx, fabs(half_element(src[(size_t)k * N + col], gamma, k_scale, k)));
     const int e = half_exponent(mx, 126);
     up[r] = pow2(e), un[r] = pow2(-e);
 }
 template <int TR>
-__global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const float *W3, const float *k_scale, const float *up, int K, int N,
-                                                        uint8_t *image) {
+__global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const float *W3, const float *gamma, const float *k_scale, const float *up, int K,
+                                                        int N, uint8_t *image) {
     const int kt = blockIdx.x, rt = blockIdx.y, nkt = K / HBK;
     uint8_t *tile = image + ((size_t)rt * nkt + kt) * (size_t)(TR * HBK * 4);
     for (int e = threadIdx.x; e < TR * 4; e += 256) {
@@ -215,7 +225,7 @@ __global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const fl
 #pragma unroll
         for (int q = 0; q < 8; q++) {
             const int k = kt * HBK + k8 * 8 + q;
-            v[q] = col < N ? (float)((double)src[(size_t)k * N + col] / (k_scale ? k_scale[k] : 1.f) * up[r]) : 0.f;
+            v[q] = col < N ? (float)(half_element(src[(size_t)k * N + col], gamma, k_scale, k) * up[r]) : 0.f;
         }
         uint4 hi, lo;
         split8(v, hi, lo);
@@ -235,10 +245,10 @@ __global__ void __launch_bounds__(256) column_scale_kernel(const float *W, const
     }
     scale[n] = pow2(half_exponent(W3 ? (double)K * sqrt(a) * sqrt(b) : sqrt((double)K * a), 113));
 }
-// RMSNorm of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers between the
+// RMSNorm, without its weights, of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers between the
 // sum of squares and the product.
 constexpr int kKept = 16;
-__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, const float *__restrict__ gamma, int M, int D, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, int M, int D, float eps,
                                                                 uint8_t *__restrict__ image, float *__restrict__ a_un) {
     extern __shared__ __align__(16) float rp_rows[];  // [8][D + 4]
     const int tid = threadIdx.x, rr = tid >> 5, lane = tid & 31;
@@ -274,12 +284,12 @@ __global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__r
 #pragma unroll
         for (int i = 0; i < kKept; i++)
             if (32 * i + lane < D) {
-                v[i] = v[i] * inv * gamma[32 * i + lane];
+                v[i] *= inv;
                 mx = fmaxf(mx, fabsf(v[i]));
             }
     } else {
         for (int j = lane; j < D; j += 32) {
-            const float y = row < M ? xr[j] * inv * gamma[j] : 0.f;
+            const float y = row < M ? xr[j] * inv : 0.f;
             mine[j] = y;
             mx = fmaxf(mx, fabsf(y));
         }
@@ -312,22 +322,22 @@ __global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__r
     }
 }
 
-int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st) {
+int32_t pack_weight_half(const float *W, const float *gamma, const float *k_scale, int K, int N, float *image, cudaStream_t st) {
     const int bn = tile_cols(N), tiles = (N + bn - 1) / bn, rows = tiles * bn;
     float *un = image + (size_t)rows * K, *up = un + rows;
-    half_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(W, nullptr, k_scale, K, N, rows, un, up);
+    half_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(W, nullptr, gamma, k_scale, K, N, rows, un, up);
     dim3 grid(K / HBK, tiles);
     uint8_t *im = reinterpret_cast<uint8_t *>(image);
-    if (bn == 256) half_pack_kernel<256><<<grid, 256, 0, st>>>(W, nullptr, k_scale, up, K, N, im);
-    else half_pack_kernel<192><<<grid, 256, 0, st>>>(W, nullptr, k_scale, up, K, N, im);
+    if (bn == 256) half_pack_kernel<256><<<grid, 256, 0, st>>>(W, nullptr, gamma, k_scale, up, K, N, im);
+    else half_pack_kernel<192><<<grid, 256, 0, st>>>(W, nullptr, gamma, k_scale, up, K, N, im);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t pack_weight_pair_half(const float *W1, const float *W3, int K, int F, float *image, cudaStream_t st) {
+int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *gamma, int K, int F, float *image, cudaStream_t st) {
     JGPT_REQUIRE(half_ok(K, F), JGPT_ERR_UNSUPPORTED, "pack_weight_pair_half: K=%d F=%d", K, F);
     float *un = image + (size_t)2 * F * K, *up = un + 2 * F;
-    half_scale_kernel<<<(2 * F + 255) / 256, 256, 0, st>>>(W1, W3, nullptr, K, F, 2 * F, un, up);
-    half_pack_kernel<256><<<dim3(K / HBK, F / 128), 256, 0, st>>>(W1, W3, nullptr, up, K, F, reinterpret_cast<uint8_t *>(image));
+    half_scale_kernel<<<(2 * F + 255) / 256, 256, 0, st>>>(W1, W3, gamma, nullptr, K, F, 2 * F, un, up);
+    half_pack_kernel<256><<<dim3(K / HBK, F / 128), 256, 0, st>>>(W1, W3, gamma, nullptr, up, K, F, reinterpret_cast<uint8_t *>(image));
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
@@ -336,11 +346,11 @@ int32_t column_scales(const float *W, const float *W3, const float *gamma, int K
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t rmsnorm_pack_half(const float *x, const float *gamma, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
+int32_t rmsnorm_pack_half(const float *x, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
     const size_t smem = sizeof(float) * 8 * (size_t)(D + 4);
     JGPT_REQUIRE(D % HBK == 0 && smem <= 48 * 1024, JGPT_ERR_UNSUPPORTED, "rmsnorm_pack_half: d_model %d", D);
     const int padded_rows = (M + BM - 1) / BM * BM;  // rows past M are written as zeros
-    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, gamma, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
+    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }

@@ -56,7 +56,7 @@ int32_t launch_qkv_paged(const float *Aimg, const Batch &b, int M, int K, int N,
 constexpr int HBK = 32;
 inline bool half_ok(int D, int F) { return D % HBK == 0 && F % 128 == 0; }
 inline uint64_t half_activation_floats(int M, int K) { return image_floats(M, K, BM) / 2; }
-// W [K, N], row k divided by k_scale[k] if given -> image, then one float per image row that undoes that row's (column of W's) power
+// W [K, N], row k times gamma[k] or divided by k_scale[k] if given -> image, then one float per image row that undoes that row's (column of W's) power
 // of two, then work space of the same size.
 inline uint64_t half_weight_floats(int K, int N) {
     const uint64_t rows = (uint64_t)((N + tile_cols(N) - 1) / tile_cols(N)) * (uint64_t)tile_cols(N);
@@ -69,12 +69,12 @@ struct ImageOut {
     float *image = nullptr;
     const float *scale = nullptr;
 };
-int32_t pack_weight_half(const float *W, const float *k_scale, int K, int N, float *image, cudaStream_t st);
-int32_t pack_weight_pair_half(const float *W1, const float *W3, int K, int F, float *image, cudaStream_t st);
+int32_t pack_weight_half(const float *W, const float *gamma, const float *k_scale, int K, int N, float *image, cudaStream_t st);
+int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *gamma, int K, int F, float *image, cudaStream_t st);
 // scale[n] = the power of two that keeps column n below 2^15 in fp16: of rmsnorm(x) W (gamma applied), or of h g sigmoid(g) with W3.
 int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st);
-// RMSNorm into an fp16 image; a_un[M] receives the rows' factors.
-int32_t rmsnorm_pack_half(const float *x, const float *gamma, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
+// RMSNorm into an fp16 image, its weights being in the next product's; a_un[M] receives the rows' factors.
+int32_t rmsnorm_pack_half(const float *x, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
 int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
 // c_up[F]: the powers of two of the result's columns in its image.
 int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,

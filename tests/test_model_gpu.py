@@ -461,6 +461,67 @@ def test_products_of_few_rows_against_float64(ctx, dm, dff, rows, spread):
         pool.close(), gm.close()
 
 
+@pytest.mark.parametrize("rows", [64, 600])
+@pytest.mark.parametrize("where,spread", [("norm", 16)])
+def test_elements_of_very_different_size_along_k(ctx, rows, where, spread):
+    """The feed-forward part with norm weights, or the row's own elements, spread over 2^+-spread along k and the rows of W1 and W3 the other
+    way round, so that every element counts alike: few rows (register images) and prefill rows (tcgen05 images).  Norm weights are folded
+    into the weights behind the norm and cost nothing.  A row keeps 22 bits of its largest element, so a spread of its own costs bits.
+
+    Tolerance: 1e-5 of sum |x w| for 22-bit operands and fewer than 128 fp32 additions, and 2^-39 of the row's (and of the column's) largest
+    element against the other operand where elements lie below 2^-16 of it."""
+    V, dm, dff = 260, 384, 768
+    rng = np.random.default_rng(spread + rows)
+
+    def mat(a, b):
+        return rng.standard_normal((a, b)) / np.sqrt(a)
+
+    c = 2.0 ** rng.uniform(-spread, spread, dm)
+    tok, n2 = rng.standard_normal((V, dm)), 1 + 0.1 * rng.standard_normal(dm)
+    if where == "norm":
+        n2 = n2 * c
+    else:
+        tok = tok * c
+    gain = 1.0 if where == "norm" else np.sqrt((c * c).mean())  # h of order one, whatever the row's size
+    w1, w3 = gain * mat(dm, dff) / c[:, None], gain * mat(dm, dff) / c[:, None]
+    w2 = np.sqrt((c * c).mean()) * mat(dff, dm) if where == "row" else mat(dff, dm)
+    T = [np.ascontiguousarray(t, np.float32) for t in (tok, np.zeros((64, dm)), mat(dm, dm), mat(dm, dm), mat(dm, dm), np.zeros((dm, dm)), w1, w2, w3,
+                                                       np.ones(dm), n2, np.ones(dm), mat(dm, V))]
+    gm = GPTModel(ctx, V, 64, dm, dm // 16, 1, dff, rmsNormEps=1e-6, maxRows=640)
+    gm.setParameters(T)
+    pool = gm.newPool(rows, rows)
+    try:
+        ids, seqs = rng.integers(0, V, rows).astype(np.int32), [pool.seq_alloc() for _ in range(rows)]
+        if rows > 512:
+            got, _ = gm.forwardPrefillBatch(pool, seqs, [[i] for i in ids])
+        else:
+            got, _ = gm.forwardDecodeBatch(pool, seqs, ids, np.zeros(rows, np.int32), np.zeros(rows, np.int32))
+        tok, w1, w2, w3, n2, head = (T[i].astype(np.float64) for i in (0, 6, 7, 8, 10, 12))
+
+        def rms(x):
+            return np.sqrt((x * x).mean(-1, keepdims=True) + 1e-6)
+
+        def off_product(x, w):
+            ax, aw = np.abs(x), np.abs(w)
+            return 1e-5 * (ax @ aw) + 2.0 ** -39 * (ax.max(-1, keepdims=True) * aw.sum(0) + ax.sum(-1, keepdims=True) * aw.max(0))
+
+        x = tok[ids] / rms(tok[ids])
+        a, g = x @ (n2[:, None] * w1), x @ (n2[:, None] * w3)
+        act = a * g / (1 + np.exp(-g))
+        y = tok[ids] + act @ w2
+        bound_act = dm * np.sqrt(((n2[:, None] * w1) ** 2).sum(0) * ((n2[:, None] * w3) ** 2).sum(0))  # what a column's scale allows for
+        off = (off_product(x, n2[:, None] * w1) * np.abs(g) + 1.2 * np.abs(a) * off_product(x, n2[:, None] * w3) + 2.0 ** -39 * bound_act) @ np.abs(w2)
+        off = off + off_product(act, w2) + 1e-6 * np.abs(y)
+        z = y / rms(y)
+        off_z = off / rms(y) + np.sqrt((off ** 2).mean(-1, keepdims=True)) / rms(y) * np.abs(z)
+        bound = off_z @ np.abs(head) + off_product(z, head)
+        assert np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
+        worst = np.linalg.norm(got - z @ head) / np.linalg.norm(z @ head)
+        assert worst < 1e-4 if spread <= 9 or where == "norm" else worst < 1e-2, worst
+    finally:
+        pool.close(), gm.close()
+
+
 @pytest.mark.parametrize("dm,lens,offset", [(128, [1, 15, 16, 17, 33], 0), (384, [40, 1, 64, 3], 5), (512, [31], 0)])
 def test_short_prompts_append_from_the_projection(ctx, dm, lens, offset):
     """Prompts of few rows: the Q,K,V product writes K (rotated) and V of the first layer to the paged store itself - over block edges, row
