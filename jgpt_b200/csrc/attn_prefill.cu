@@ -130,7 +130,10 @@ __device__ __forceinline__ void split_half2(float a, float b, uint32_t &hi, uint
 // attention outputs stay within ~4e-4 of the exact mode on N(0,1) inputs and the logits of the JGPT-35M shapes within
 // 5e-4 of an fp32 CPU evaluation, against a budget of 2e-3.  The exact mode (2e-5) remains the default of the
 // standalone entry point.
-template <bool FAST>
+// OUT: the form of the output, row major or one of the projection's operand images.  At compile time: with both images as branches the
+// short prompts' kernel took other registers and a prompt of 201 tokens 1 % longer.
+enum Out { OUT_ROWS, OUT_TF32, OUT_HALF };
+template <bool FAST, int OUT>
 __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillParams P) {
     constexpr int DH = 16, BT = kBlockTokens, TILE_BYTES = 2 * BT * DH * 2;  // 1 KiB: K tile | V tile
     __shared__ __align__(128) unsigned char tiles[2][kStageBlocks][TILE_BYTES];
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     lB += __shfl_xor_sync(0xffffffffu, lB, 2);
     const float iA = 1.f / fmaxf(lA, 1e-12f), iB = 1.f / fmaxf(lB, 1e-12f);
     const size_t D = (size_t)P.H * DH;
-    if (P.out_image) {
+    if constexpr (OUT != OUT_ROWS) {
         // Operand image of the next projection (see gemm_umma.cu): 128-row tiles, high parts then low parts.  Lane (g, t) holds columns
         // 8 j + 2 t, 8 j + 2 t + 1 of the head.
         // TF32: k tiles of 16, head h is k tile h; the pair is half of the 16-byte chunk 2 j + t / 2, a warp store covers eight rows x two
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
         auto put = [&](int row, int j, float a, float b) {
             const size_t grow = (size_t)sd.row0 + row;
             const int rr = (int)(grow & 127);
-            if (!P.out_scale) {
+            if constexpr (OUT == OUT_TF32) {
                 float *dst = P.out_image + ((grow >> 7) * (size_t)P.H + h) * (size_t)(128 * 16 * 2) + (rr >> 3) * 128 + (2 * j + (t >> 1)) * 32 + (rr & 7) * 4 + (t & 1) * 2;
                 uint32_t ha, hb, la, lb;
                 asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ha) : "f"(a));
@@ -368,15 +371,15 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
                 asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(b - __uint_as_float(hb)));
                 *reinterpret_cast<float2 *>(dst) = make_float2(__uint_as_float(ha), __uint_as_float(hb));
                 *reinterpret_cast<float2 *>(dst + 128 * 16) = make_float2(__uint_as_float(la), __uint_as_float(lb));
-                return;
+            } else {
+                const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
+                unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
+                unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
+                uint32_t hi, lo;
+                split_half2(a * up.x, b * up.y, hi, lo);
+                *reinterpret_cast<uint32_t *>(dst) = hi;
+                *reinterpret_cast<uint32_t *>(dst + 128 * 32 * 2) = lo;
             }
-            const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
-            unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
-            unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
-            uint32_t hi, lo;
-            split_half2(a * up.x, b * up.y, hi, lo);
-            *reinterpret_cast<uint32_t *>(dst) = hi;
-            *reinterpret_cast<uint32_t *>(dst + 128 * 32 * 2) = lo;
         };
 #pragma unroll
         for (int j = 0; j < 2; j++) {
@@ -518,7 +521,11 @@ int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         P.pdl = pdl && skip_append;  // behind the append kernel: an ordinary launch
         cfg.gridDim = grid, cfg.blockDim = dim3(128), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = P.pdl ? 1 : 0;
-        JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, fast ? attn_prefill_mma_kernel<true> : attn_prefill_mma_kernel<false>, P));
+        auto pick = [&](auto f) {
+            constexpr bool FAST = decltype(f)::value;
+            return !out_image ? attn_prefill_mma_kernel<FAST, OUT_ROWS> : out_scale ? attn_prefill_mma_kernel<FAST, OUT_HALF> : attn_prefill_mma_kernel<FAST, OUT_TF32>;
+        };
+        JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, fast ? pick(std::true_type()) : pick(std::false_type()), P));
     } else {
         dim3 grid((unsigned)((max_S + 127) / 128), (unsigned)p->heads, (unsigned)n_seqs);
         switch (DH) {
