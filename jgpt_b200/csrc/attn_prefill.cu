@@ -351,7 +351,6 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     lB += __shfl_xor_sync(0xffffffffu, lB, 1);
     lB += __shfl_xor_sync(0xffffffffu, lB, 2);
     const float iA = 1.f / fmaxf(lA, 1e-12f), iB = 1.f / fmaxf(lB, 1e-12f);
-    const size_t D = (size_t)P.H * DH;
     if constexpr (OUT != OUT_ROWS) {
         // Operand image of the next projection (see gemm_umma.cu): 128-row tiles, high parts then low parts.  Lane (g, t) holds columns
         // 8 j + 2 t, 8 j + 2 t + 1 of the head.
@@ -386,16 +385,17 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
             if (rowA < sd.S) put(rowA, j, o[j][0] * iA, o[j][1] * iA);
             if (rowB < sd.S) put(rowB, j, o[j][2] * iB, o[j][3] * iB);
         }
-        return;
-    }
+    } else {
+        const size_t D = (size_t)P.H * DH;
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        if (rowA < sd.S)
-            *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowA) * D + h * DH + 8 * j + 2 * t) =
-                make_float2(o[j][0] * iA, o[j][1] * iA);
-        if (rowB < sd.S)
-            *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowB) * D + h * DH + 8 * j + 2 * t) =
-                make_float2(o[j][2] * iB, o[j][3] * iB);
+        for (int j = 0; j < 2; j++) {
+            if (rowA < sd.S)
+                *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowA) * D + h * DH + 8 * j + 2 * t) =
+                    make_float2(o[j][0] * iA, o[j][1] * iA);
+            if (rowB < sd.S)
+                *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowB) * D + h * DH + 8 * j + 2 * t) =
+                    make_float2(o[j][2] * iB, o[j][3] * iB);
+        }
     }
 }
 

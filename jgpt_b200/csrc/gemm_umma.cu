@@ -27,13 +27,18 @@
 //   weights: per column of W, from its largest element; undone in the epilogue (the factors stand behind the image).  The norm weights
 //   gamma are in the rows of the W that follows the norm, so their spread is not the normalised row's;
 //   RMSNorm rows: per row, from the row's largest element; undone in the epilogue;
-//   attention and SwiGLU results, whose rows no single CTA sees: per column, from what the column can reach at all.  A normalised row
-//   is at most sqrt(D) long, so |v_n| <= sqrt(D) |gamma o Wv_n|, an attention output is a weighted mean of such values, and
-//   |h g sigmoid(g)| <= D |gamma o W1_n| |gamma o W3_n|.  The next weight's rows are divided by the same powers.
+//   attention results, whose rows no single CTA sees: per column, from what the column can reach at all.  A normalised row is at most
+//   sqrt(D) long, so |v_n| <= sqrt(D) |gamma o Wv_n|, and an attention output is a weighted mean of such values.  The next weight's rows
+//   are divided by the same powers.  (However far below that bound they lie, a value that comes from an fp16 cache has 2^-12 of itself as
+//   error anyway.)
+//   SwiGLU results, likewise: per column and per row.  For any weights r > 0 of the elements, |x . w_n| <= |x o r| |w_n / r|, so
+//   |h g sigmoid(g)| <= |x o r|^2 . |gamma o W1_n / r| |gamma o W3_n / r|: the first factor is the row's, taken by the norm in front,
+//   the others the column's.  r_k is the size of row k of both weights, which makes all terms of a sum alike: without it a row
+//   whose large elements meet small weights lies as far below the bound as the spread of its elements, squared.
 // An element down to 2^-16 of the largest its scale allows for is within 2^-23 of itself, like a TF32 pair at any size; below that an
 // absolute error of at most 2^-39 of that largest remains.  So the 22 bits are those of the largest in the row (column), and a row whose
 // elements spread further along k, with weights the other way round, loses bits that TF32 pairs keep.  Typical results of a SwiGLU lie
-// about 2^10 below their bound.  Error of a block's feed-forward part against float64 (2-norm, 384 / 768, 2000 rows): TF32 4.8e-6, fp16
+// about 2^10 below their bound at any such spread.  Error of a block's feed-forward part against float64 (2-norm, 384 / 768, 2000 rows): TF32 4.8e-6, fp16
 // 2.5e-6, of its Wo product 9.5e-7 and 5.2e-7 (half as many steps of accumulation).
 // The attention output of a prefill is such a mean because every key it sees was produced by the same call's Q,K,V product.
 // Measured for 32 x 1024 tokens, 24 heads of 16 (ncu, us per launch, TF32 -> fp16 images): Q,K,V 139 -> 91, W1/W3 + SwiGLU 164 -> 116,
@@ -179,13 +184,13 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
     split_pair(v[0], v[1], hi.x, lo.x), split_pair(v[2], v[3], hi.y, lo.y);
     split_pair(v[4], v[5], hi.z, lo.z), split_pair(v[6], v[7], hi.w, lo.w);
 }
-// The exponent e that brings values up to mx into [2^14, 2^15) as mx 2^e, within what fp32 holds as 2^e and 2^-e; 0 for a column that
-// is all zeros or not finite (its results are zeros, or not finite, at any scale).
+// The exponent e <= limit that brings values up to mx into [2^14, 2^15) as mx 2^e; 0 for a column that is all zeros or not finite (its
+// results are zeros, or not finite, at any scale).
 __device__ __forceinline__ int half_exponent(double mx, int limit) {
     if (!(mx > 0.) || isinf(mx)) return 0;
     int e;
     frexp(mx, &e);  // mx in [2^(e - 1), 2^e)
-    return max(-limit, min(limit, 15 - e));
+    return max(-126, min(limit, 15 - e));  // 2^e and 2^-e are normal numbers
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 // One thread per column: up[n] brings the column's largest element (row k times the norm weight gamma[k] in front of it, or divided by
@@ -234,21 +239,57 @@ __global__ void __launch_bounds__(256) half_pack_kernel(const float *W, const fl
     }
 }
 // In fp64, where no square of an fp32 weight leaves the range: a column of 1e-24 has a reach that is not 0, one of 1e20 a finite one.
-// The limit keeps any finite fp32 result below 2^15.
-__global__ void __launch_bounds__(256) column_scale_kernel(const float *W, const float *W3, const float *gamma, int K, int N, float *scale) {
+// The limit leaves room for the factors that undo the powers.
+__global__ void __launch_bounds__(256) column_scale_kernel(const float *W, const float *gamma, int K, int N, float *scale) {
+    const int n = blockIdx.x * 256 + threadIdx.x;
+    if (n >= N) return;
+    double a = 0.;
+    for (int k = 0; k < K; k++) {
+        const double x = (double)gamma[k] * W[(size_t)k * N + n];
+        a += x * x;
+    }
+    scale[n] = pow2(half_exponent(sqrt((double)K * a), 113));
+}
+// The weights r of the elements in front of the pair W1, W3: the 2-norm of row k of both over the largest of all, at least 2^-60 (any
+// positive r makes a bound).
+constexpr double kLeastWeight = 0x1p-60;
+__global__ void __launch_bounds__(256) pair_row_size_kernel(const float *W1, const float *W3, const float *gamma, int K, int N, double *size) {
+    __shared__ double red[8];
+    const int k = blockIdx.x;
+    double a = 0.;
+    for (int n = threadIdx.x; n < N; n += 256) {
+        const double g = gamma[k], x = g * W1[(size_t)k * N + n], y = g * W3[(size_t)k * N + n];
+        a += x * x + y * y;
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) a += red[w];
+        size[k] = sqrt(a);
+    }
+}
+__global__ void __launch_bounds__(256) pair_weight_kernel(const double *size, int K, float *r) {
+    double mx = 0.;  // every block finds the largest by itself
+    for (int k = 0; k < K; k++) mx = fmax(mx, size[k]);
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k < K) r[k] = (mx > 0. && isfinite(mx)) ? (float)fmax(size[k] / mx, kLeastWeight) : 1.f;
+}
+__global__ void __launch_bounds__(256) pair_scale_kernel(const float *W1, const float *W3, const float *gamma, const float *r, int K, int N, float *scale) {
     const int n = blockIdx.x * 256 + threadIdx.x;
     if (n >= N) return;
     double a = 0., b = 0.;
     for (int k = 0; k < K; k++) {
-        const double g = gamma[k], x = g * W[(size_t)k * N + n], y = W3 ? g * W3[(size_t)k * N + n] : 0.;
+        const double g = (double)gamma[k] / r[k], x = g * W1[(size_t)k * N + n], y = g * W3[(size_t)k * N + n];
         a += x * x, b += y * y;
     }
-    scale[n] = pow2(half_exponent(W3 ? (double)K * sqrt(a) * sqrt(b) : sqrt((double)K * a), 113));
+    scale[n] = pow2(half_exponent(sqrt(a) * sqrt(b), 113));
 }
-// RMSNorm, without its weights, of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers between the
-// sum of squares and the product.
+// RMSNorm, without its weights, of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers
+// between the sum of squares and the product.
 constexpr int kKept = 16;
-__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, int M, int D, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, const float *__restrict__ r, int M, int D, float eps,
                                                                 uint8_t *__restrict__ image, float *__restrict__ a_un) {
     extern __shared__ __align__(16) float rp_rows[];  // [8][D + 4]
     const int tid = threadIdx.x, rr = tid >> 5, lane = tid & 31;
@@ -279,23 +320,33 @@ __global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__r
     const float tot = ss[0] + ss[1] + ss[2] + ss[3];
     const float rms = sqrtf(tot / (float)D + eps);
     const float inv = (rms > 0.f && isfinite(rms)) ? (1.f / rms) : 0.f;
-    float mx = 0.f;
+    float mx = 0.f, size = 0.f;  // size: |x o r|^2 of the normalised row
     if (kept) {
 #pragma unroll
         for (int i = 0; i < kKept; i++)
             if (32 * i + lane < D) {
                 v[i] *= inv;
                 mx = fmaxf(mx, fabsf(v[i]));
+                if (r) {
+                    const float t = v[i] * r[32 * i + lane];
+                    size = fmaf(t, t, size);
+                }
             }
     } else {
         for (int j = lane; j < D; j += 32) {
             const float y = row < M ? xr[j] * inv : 0.f;
             mine[j] = y;
             mx = fmaxf(mx, fabsf(y));
+            if (r) size = fmaf(y * r[j], y * r[j], size);
         }
     }
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off)), size += __shfl_xor_sync(0xffffffffu, size, off);
+    if (r && lane == 0 && row < M) {
+        // the result's power of two: |x o r|^2 up to [1/2, 1); a sum that underflows is below 2^-100 in any case
+        const int e = isfinite(size) ? -ilogbf(fmaxf(size, 0x1p-100f)) - 1 : 0;
+        a_un[M + row] = pow2(e), a_un[2 * (size_t)M + row] = pow2(-e);
+    }
     float up, un;
     pow2_scale(mx, up, un);
     if (lane == 0 && row < M) a_un[row] = un;
@@ -341,16 +392,25 @@ int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *gam
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st) {
-    column_scale_kernel<<<(N + 255) / 256, 256, 0, st>>>(W, W3, gamma, K, N, scale);
+int32_t column_scales(const float *W, const float *gamma, int K, int N, float *scale, cudaStream_t st) {
+    column_scale_kernel<<<(N + 255) / 256, 256, 0, st>>>(W, gamma, K, N, scale);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t rmsnorm_pack_half(const float *x, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
+int32_t pair_scales(const float *W1, const float *W3, const float *gamma, int K, int F, float *scale, cudaStream_t st) {
+    float *r = scale + F;
+    double *size = reinterpret_cast<double *>(r + K);  // F and K are even: 8-byte aligned
+    pair_row_size_kernel<<<K, 256, 0, st>>>(W1, W3, gamma, K, F, size);
+    pair_weight_kernel<<<(K + 255) / 256, 256, 0, st>>>(size, K, r);
+    pair_scale_kernel<<<(F + 255) / 256, 256, 0, st>>>(W1, W3, gamma, r, K, F, scale);
+    JGPT_CUDA_TRY(cudaGetLastError());
+    return JGPT_OK;
+}
+int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
     const size_t smem = sizeof(float) * 8 * (size_t)(D + 4);
     JGPT_REQUIRE(D % HBK == 0 && smem <= 48 * 1024, JGPT_ERR_UNSUPPORTED, "rmsnorm_pack_half: d_model %d", D);
     const int padded_rows = (M + BM - 1) / BM * BM;  // rows past M are written as zeros
-    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
+    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, r, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
@@ -688,11 +748,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
                         h[q] = h[q] * (gv * s);
                     }
                     if constexpr (HALF) {  // these 32 columns are one k tile of the next product
-                        // (the finished value times its column's power of two: h alone may exceed what h g sigmoid(g) can reach)
+                        // (the finished value times the powers of two of its row and column: h alone may exceed what h g sigmoid(g) can reach)
+                        const float r_up = m < M ? B.r_up[m] : 1.f;
 #pragma unroll
                         for (int q = 0; q < 32; q += 4) {
                             const float4 u = __ldg(reinterpret_cast<const float4 *>(B.c_up + n_idx * 128 + c0 + q));
-                            h[q] *= u.x, h[q + 1] *= u.y, h[q + 2] *= u.z, h[q + 3] *= u.w;
+                            h[q] = h[q] * r_up * u.x, h[q + 1] = h[q + 1] * r_up * u.y, h[q + 2] = h[q + 2] * r_up * u.z, h[q + 3] = h[q + 3] * r_up * u.w;
                         }
                         uint8_t *tile = reinterpret_cast<uint8_t *>(B.C[0] + ((size_t)m_idx * out_nkt + (n_idx * 128 + c0) / HBK) * A_TILE_FLOATS);
 #pragma unroll
@@ -795,7 +856,7 @@ static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const floa
     JGPT_REQUIRE(swiglu_shape_ok(K, F) && (!HALF || K % HBK == 0) && M > 0, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
     Batch b{};
-    b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un, b.c_up = c_up;
+    b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un, b.r_up = a_un + M, b.c_up = c_up;
     TileWalk walk{F / 128, 1, 0};
     walk.total = walk.n_tiles_n * ((M + BM - 1) / BM);
     return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st);

@@ -37,7 +37,7 @@ struct Batch {
     float *C[3];
     const float *R[3];  // optional residual, may alias C
     const float *a_un = nullptr;  // fp16 images: one factor per row of A that undoes its power of two (nullptr: none)
-    const float *c_up = nullptr;  // the SwiGLU form on fp16 images: the power of two of every column of the result
+    const float *r_up = nullptr, *c_up = nullptr;  // the SwiGLU form on fp16 images: the powers of two of the result's rows and columns
 };
 // C_z[M, N] = A . W_z (+ R_z) for z < nb; needs K % 16 == 0 and N % 4 == 0.
 int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
@@ -71,12 +71,17 @@ struct ImageOut {
 };
 int32_t pack_weight_half(const float *W, const float *gamma, const float *k_scale, int K, int N, float *image, cudaStream_t st);
 int32_t pack_weight_pair_half(const float *W1, const float *W3, const float *gamma, int K, int F, float *image, cudaStream_t st);
-// scale[n] = the power of two that keeps column n below 2^15 in fp16: of rmsnorm(x) W (gamma applied), or of h g sigmoid(g) with W3.
-int32_t column_scales(const float *W, const float *W3, const float *gamma, int K, int N, float *scale, cudaStream_t st);
-// RMSNorm into an fp16 image, its weights being in the next product's; a_un[M] receives the rows' factors.
-int32_t rmsnorm_pack_half(const float *x, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
+// scale[n] = the power of two that keeps column n of rmsnorm(x) W (gamma applied) below 2^15.
+int32_t column_scales(const float *W, const float *gamma, int K, int N, float *scale, cudaStream_t st);
+// The same for h g sigmoid(g) of the pair, times a power of two of the row (see gemm_umma.cu): F column scales, then the K weights of the
+// elements that the row's is taken with, then work space.
+inline uint64_t pair_scale_floats(int K, int F) { return (uint64_t)F + 3 * (uint64_t)K; }
+int32_t pair_scales(const float *W1, const float *W3, const float *gamma, int K, int F, float *scale, cudaStream_t st);
+// RMSNorm into an fp16 image, its weights being in the next product's; a_un[M] receives the rows' factors.  With the weights r of a pair's
+// elements a_un[M .. 2 M) and [2 M .. 3 M) receive the power of two of the row's SwiGLU result and its inverse.
+int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
 int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
-// c_up[F]: the powers of two of the result's columns in its image.
+// a_un: the rows' factors as rmsnorm_pack_half leaves them; c_up[F]: the powers of two of the result's columns in its image.
 int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
                            int *d_status, cudaStream_t st);
 int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st);

@@ -925,8 +925,8 @@ static int32_t half_layer(Model *m, const LayerW &y, HalfLayer *o) {
     cudaStream_t st = m->ctx->stream;
     int32_t rc;
     bool fresh;
-    if ((rc = half_buffer(m, y.wv + 1, D, &o->att_scale, &fresh)) || (fresh && (rc = umma::column_scales(y.wv, nullptr, y.norm1, D, D, o->att_scale, st)))) return rc;
-    if ((rc = half_buffer(m, y.w1 + 1, F, &o->h_scale, &fresh)) || (fresh && (rc = umma::column_scales(y.w1, y.w3, y.norm2, D, F, o->h_scale, st)))) return rc;
+    if ((rc = half_buffer(m, y.wv + 1, D, &o->att_scale, &fresh)) || (fresh && (rc = umma::column_scales(y.wv, y.norm1, D, D, o->att_scale, st)))) return rc;
+    if ((rc = half_buffer(m, y.w1 + 1, umma::pair_scale_floats(D, F), &o->h_scale, &fresh)) || (fresh && (rc = umma::pair_scales(y.w1, y.w3, y.norm2, D, F, o->h_scale, st)))) return rc;
     struct { const float *W, *gamma, *k_scale; int K; float **out; } one[5] = {
         {y.wq, y.norm1, nullptr, D, &o->wq}, {y.wk, y.norm1, nullptr, D, &o->wk}, {y.wv, y.norm1, nullptr, D, &o->wv},
         {y.wo, nullptr, o->att_scale, D, &o->wo}, {y.w2, nullptr, o->h_scale, F, &o->w2}};
@@ -946,7 +946,7 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
     cudaStream_t st = m->ctx->stream;
     int *status = m->ctx->d_status;
     const uint64_t image = umma::half_activation_floats(rows, D);
-    int32_t rc = ensure_image(m, &m->aimg, &m->aimg_floats, image + (uint64_t)rows);  // the rows' factors behind it
+    int32_t rc = ensure_image(m, &m->aimg, &m->aimg_floats, image + 3 * (uint64_t)rows);  // the rows' factors behind it
     if (rc) return rc;
     if ((rc = ensure_image(m, &m->aimg2, &m->aimg2_floats, umma::half_activation_floats(rows, F)))) return rc;
     float *a_un = m->aimg + image;
@@ -958,14 +958,14 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
         qkv.Wimg[0] = w.wq, qkv.Wimg[1] = w.wk, qkv.Wimg[2] = w.wv;
         qkv.C[0] = m->q, qkv.C[1] = m->k, qkv.C[2] = m->v, qkv.a_un = a_un;
         wo.Wimg[0] = w.wo, wo.C[0] = m->x, wo.R[0] = m->x;  // x1 = x + attn.Wo (each element read then written by the same thread)
-        w2.Wimg[0] = w.w2, w2.C[0] = m->x, w2.R[0] = m->x;
-        if ((rc = umma::rmsnorm_pack_half(m->x, rows, D, m->eps, m->aimg, a_un, st))) return rc;
+        w2.Wimg[0] = w.w2, w2.C[0] = m->x, w2.R[0] = m->x, w2.a_un = a_un + 2 * (size_t)rows;
+        if ((rc = umma::rmsnorm_pack_half(m->x, nullptr, rows, D, m->eps, m->aimg, a_un, st))) return rc;
         PagedAppendArgs pa = paged;
         pa.layer = l;
         if ((rc = umma::launch_qkv_paged_half(m->aimg, qkv, rows, D, D, pa, status, st))) return rc;
         if ((rc = attn(l, umma::ImageOut{m->aimg, w.att_scale}, true))) return rc;
         if ((rc = umma::launch_half(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
-        if ((rc = umma::rmsnorm_pack_half(m->x, rows, D, m->eps, m->aimg, a_un, st))) return rc;
+        if ((rc = umma::rmsnorm_pack_half(m->x, w.h_scale + F, rows, D, m->eps, m->aimg, a_un, st))) return rc;
         if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, w.h_scale, rows, D, F, m->aimg2, status, st))) return rc;
         if ((rc = umma::launch_half(m->aimg2, w2, 1, rows, F, D, status, st))) return rc;
     }

@@ -462,7 +462,7 @@ def test_products_of_few_rows_against_float64(ctx, dm, dff, rows, spread):
 
 
 @pytest.mark.parametrize("rows", [64, 600])
-@pytest.mark.parametrize("where,spread", [("norm", 16)])
+@pytest.mark.parametrize("where,spread", [("norm", 16), ("row", 9), ("row", 12)])
 def test_elements_of_very_different_size_along_k(ctx, rows, where, spread):
     """The feed-forward part with norm weights, or the row's own elements, spread over 2^+-spread along k and the rows of W1 and W3 the other
     way round, so that every element counts alike: few rows (register images) and prefill rows (tcgen05 images).  Norm weights are folded
@@ -509,15 +509,16 @@ def test_elements_of_very_different_size_along_k(ctx, rows, where, spread):
         a, g = x @ (n2[:, None] * w1), x @ (n2[:, None] * w3)
         act = a * g / (1 + np.exp(-g))
         y = tok[ids] + act @ w2
-        bound_act = dm * np.sqrt(((n2[:, None] * w1) ** 2).sum(0) * ((n2[:, None] * w3) ** 2).sum(0))  # what a column's scale allows for
+        # what the scales of the gated values allow for: |x o r|^2 |n2 o W1_n / r| |n2 o W3_n / r|, r the size of row k of both weights
+        w1g, w3g = n2[:, None] * w1, n2[:, None] * w3
+        r = np.sqrt((w1g ** 2 + w3g ** 2).sum(1))
+        bound_act = ((x * r) ** 2).sum(-1, keepdims=True) * np.sqrt(((w1g / r[:, None]) ** 2).sum(0) * ((w3g / r[:, None]) ** 2).sum(0))
         off = (off_product(x, n2[:, None] * w1) * np.abs(g) + 1.2 * np.abs(a) * off_product(x, n2[:, None] * w3) + 2.0 ** -39 * bound_act) @ np.abs(w2)
         off = off + off_product(act, w2) + 1e-6 * np.abs(y)
         z = y / rms(y)
         off_z = off / rms(y) + np.sqrt((off ** 2).mean(-1, keepdims=True)) / rms(y) * np.abs(z)
         bound = off_z @ np.abs(head) + off_product(z, head)
         assert np.all(np.abs(got - z @ head) <= bound), float((np.abs(got - z @ head) / bound).max())
-        worst = np.linalg.norm(got - z @ head) / np.linalg.norm(z @ head)
-        assert worst < 1e-4 if spread <= 9 or where == "norm" else worst < 1e-2, worst
     finally:
         pool.close(), gm.close()
 
