@@ -11,8 +11,11 @@
 // Accuracy: an fp32 operand is an fp16 high and an fp16 low part, 11 + 11 bits as the TF32 pair has, at half the tensor time (m16n8k16
 // instead of two m16n8k8) and, for the weights, in the four bytes of the original.  fp16's narrow exponent is dealt with by powers of
 // two, which change no bit: weights are scaled per column (image), rows per warp and row tile from the largest element of the slice,
-// and the partial sums are scaled back before they are added.  An element 2^18 below the largest of its slice keeps all 22 bits,
-// below that an absolute error of 2^-40 of the largest remains.  Products high x high in one accumulator, the two mixed ones in another.
+// and the partial sums are scaled back before they are added.  The low parts carry 2^11 more and have an accumulator of their own (the two
+// mixed products), so that they stay clear of fp16's subnormals as long as the high parts do: an element down to 2^-28 of the largest of
+// its slice (column) is within 2^-23 of itself, like a TF32 pair at any size, below that an absolute error of 2^-50 of that
+// largest remains.  Without the factor, one multiplication per row element less, the two were 2^-16 and 2^-39 (same times: 250 rows
+// of 1000 9.42 ms, a prompt of 201 tokens 458 and 461 us).
 //
 // Against the form with shared-memory k tiles, TF32 pairs split in the loop and a barrier per 64 k (12 layers of 384, per launch inside
 // a decode step of 64 rows, from the previous kernel's end to its own): Q,K,V 5.2 -> 3.2, Wo 4.1 -> 3.1, W1/W3 7.0 -> 3.7, W2 6.6 -> 2.8 us;
@@ -62,8 +65,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const float *W, const float *
     for (int step = warp; step < steps; step += kWarps) {
         const int k = step * 16 + 4 * t;
         uint4 o;
-        split_pair(element(k, n0 + g) * s, element(k + 1, n0 + g) * s, o.x, o.z);
-        split_pair(element(k + 2, n0 + g) * s, element(k + 3, n0 + g) * s, o.y, o.w);
+        split_pair_wide(element(k, n0 + g) * s, element(k + 1, n0 + g) * s, o.x, o.z);
+        split_pair_wide(element(k + 2, n0 + g) * s, element(k + 3, n0 + g) * s, o.y, o.w);
         image[((size_t)blockIdx.x * steps + step) * 32 + lane] = o;
     }
 }
@@ -191,10 +194,10 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
 #pragma unroll
         for (int s = 0; s < S; s++) {
             uint32_t ah[4], al[4];
-            split_pair(lo_row[s].x * s0, lo_row[s].y * s0, ah[0], al[0]);
-            split_pair(hi_row[s].x * s1, hi_row[s].y * s1, ah[1], al[1]);
-            split_pair(lo_row[s].z * s0, lo_row[s].w * s0, ah[2], al[2]);
-            split_pair(hi_row[s].z * s1, hi_row[s].w * s1, ah[3], al[3]);
+            split_pair_wide(lo_row[s].x * s0, lo_row[s].y * s0, ah[0], al[0]);
+            split_pair_wide(hi_row[s].x * s1, hi_row[s].y * s1, ah[1], al[1]);
+            split_pair_wide(lo_row[s].z * s0, lo_row[s].w * s0, ah[2], al[2]);
+            split_pair_wide(hi_row[s].z * s1, hi_row[s].w * s1, ah[3], al[3]);
             // the rows are in the parts: the next tile's are on their way during the last products, the sums and the stores
             if (s == S - 1 && rt + (int)gridDim.y < row_tiles) fetch(rt + gridDim.y);
 #pragma unroll
@@ -206,8 +209,8 @@ __global__ void __launch_bounds__(kThreads, per_sm<S, NT>()) gemm_rows_kernel(co
         }
 #pragma unroll
         for (int j = 0; j < NT; j++) {
-            *reinterpret_cast<float2 *>(&red[rb][warp][g][j * 8 + 2 * t]) = make_float2((acc[j][0] + cor[j][0]) * u0, (acc[j][1] + cor[j][1]) * u0);
-            *reinterpret_cast<float2 *>(&red[rb][warp][g + 8][j * 8 + 2 * t]) = make_float2((acc[j][2] + cor[j][2]) * u1, (acc[j][3] + cor[j][3]) * u1);
+            *reinterpret_cast<float2 *>(&red[rb][warp][g][j * 8 + 2 * t]) = make_float2(fmaf(cor[j][0], 1.f / kLowScale, acc[j][0]) * u0, fmaf(cor[j][1], 1.f / kLowScale, acc[j][1]) * u0);
+            *reinterpret_cast<float2 *>(&red[rb][warp][g + 8][j * 8 + 2 * t]) = make_float2(fmaf(cor[j][2], 1.f / kLowScale, acc[j][2]) * u1, fmaf(cor[j][3], 1.f / kLowScale, acc[j][3]) * u1);
         }
         float inv = 0.f;
         if (KIND != RESIDUAL) {

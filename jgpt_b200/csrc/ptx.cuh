@@ -129,6 +129,16 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t &hi, uint3
     hi = *reinterpret_cast<const uint32_t *>(&h), lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// The same with the low part times 2^11: a sum of products with it is scaled back, and the low part stays clear of fp16's subnormals for
+// as long as the high part does.
+constexpr float kLowScale = 2048.f;
+__device__ __forceinline__ void split_pair_wide(float x, float y, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(fmaf(f.x, -kLowScale, x * kLowScale), fmaf(f.y, -kLowScale, y * kLowScale));
+    hi = *reinterpret_cast<const uint32_t *>(&h), lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
 // Four 8x8 b16 matrices from shared memory; lane l supplies the address of row (l % 8) of matrix (l / 8).
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void *smem_row) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
