@@ -17,6 +17,7 @@
 #include "ptx.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <chrono>
 #include <map>
 #include <mutex>
@@ -440,7 +441,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                 qb0 = column(x0.x * f * up, x0.y * f * up), qb1 = column(x1.x * f * up, x1.y * f * up);
                 q_un = __shfl_sync(0xffffffffu, down, 8 * t4);
             }
-            float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};  // o: dim g (high, low column), dim g + 8; l: this lane's tokens
+            float m = -FLT_MAX, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};  // (finite: a block of scores of -inf is 0)  o: dim g (high, low column), dim g + 8; l: this lane's tokens
             const int len_cached = FUSED ? len - 1 : len;
             if (FUSED && len_cached / BT >= b0 && len_cached / BT < b1) {
                 // Fused append: the eight lanes of a head compute the stored payload (RoPE'd K, raw V, both rounded to fp16), write
@@ -476,6 +477,8 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                 const float e = t4 & 1 ? a1 : a0, f = t4 & 1 ? a3 : a2;
                 return t4 & 2 ? f : e;
             };
+            // A key that fp16 holds as an infinity: the high part has the score, the low part the same infinity at either sign.
+            auto both = [](float hi, float lo) { return isinf(hi) ? hi : hi + lo; };
             const int src0 = 8 * t4 + (g >> 1), src1 = src0 + 4;  // the lanes with p of tokens 2 t and 2 t + 1 of head g / 2
 
             bool aborted = false;
@@ -503,8 +506,8 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
                         for (int e = 0; e < 4; e++) d[i][e] = 0.f;
                         mma_16816(d[i], ka, qb0, qb1);
                     }
-                    float s0 = of_head_t(d[0][0] + d[0][1], d[1][0] + d[1][1], d[2][0] + d[2][1], d[3][0] + d[3][1]) * q_un;
-                    float s1 = of_head_t(d[0][2] + d[0][3], d[1][2] + d[1][3], d[2][2] + d[2][3], d[3][2] + d[3][3]) * q_un;
+                    float s0 = both(of_head_t(d[0][0], d[1][0], d[2][0], d[3][0]), of_head_t(d[0][1], d[1][1], d[2][1], d[3][1])) * q_un;
+                    float s1 = both(of_head_t(d[0][2], d[1][2], d[2][2], d[3][2]), of_head_t(d[0][3], d[1][3], d[2][3], d[3][3])) * q_un;
                     if (left < BT) {
                         // The slots beyond the last cached token hold whatever they held before: no score, and zeros in place of V
                         // (their probabilities are 0, but 0 x Inf or NaN is NaN inside the product).
@@ -654,8 +657,8 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
         }
         // Fused append: the thread whose token is the new one computes the stored payload (RoPE'd K,
         // raw V, both rounded to fp16), writes it to the cache and scores it from registers.
-        // Private online-softmax state of this (head, token lane).
-        float m = -INFINITY, l = 0.f, o[DH];
+        // Private online-softmax state of this (head, token lane).  The maximum starts finite: a first score of -inf has no weight.
+        float m = -FLT_MAX, l = 0.f, o[DH];
 #pragma unroll
         for (int d = 0; d < DH; d++) o[d] = 0.f;
         // Fused append: the new token sits at slot len-1.  The lane that owns that slot computes the
@@ -724,7 +727,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
 #pragma unroll
                 for (int d = 0; d < DH; d++) sc = fmaf(q[d], kr[d], sc);
                 if (sc > m) {  // new running maximum: rescale the private state
-                    const float corr = fast_exp2(m - sc);  // m = -inf on the first token -> 0
+                    const float corr = fast_exp2(m - sc);  // 0 on the first token
                     l *= corr;
 #pragma unroll
                     for (int d = 0; d < DH; d++) o[d] *= corr;
@@ -750,7 +753,7 @@ __global__ void __launch_bounds__(consumer_threads<MMA>(max_head_group<DH>()) + 
         float M = m;
 #pragma unroll
         for (int off = 8; off >= 1; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-        const float f = (m == -INFINITY) ? 0.f : exp2f(m - M);
+        const float f = exp2f(m - M);  // 0 for a lane without a token
         l *= f;
 #pragma unroll
         for (int d = 0; d < DH; d++) o[d] *= f;

@@ -161,6 +161,40 @@ def test_tensor_core_consumer_matches_oracle(ctx, fused):
         case.close()
 
 
+@pytest.mark.parametrize("overlap", [0, 1])
+@pytest.mark.parametrize("token", [5, 20])
+def test_a_key_beyond_fp16_counts_for_nothing_or_all(ctx, overlap, token):
+    """A cached key component that fp16 holds as an infinity, with queries of the other sign: its score is -inf, so the token has no weight and
+    the rest is what it would be without it, for either consumers (d_head 16).  Tolerance as for the other comparisons."""
+    from jgpt_b200 import binding as B
+    H, Dh, lens = 8, 16, [40, 70]
+    case = PagedCase(ctx, lens, H=H, Dh=Dh, layers=1, seed=95)
+    try:
+        case.pool.set_tuning(launch_overlap=overlap)
+        ptr, nbytes = case.pool.storage()
+        raw = np.empty(nbytes // 2, np.uint16)
+        B.check(ctx._lib.jgpt_d2h(ctx.handle, raw.ctypes.data, ptr, nbytes))
+        tiles = raw.reshape(1, case.n_blocks, H, 2, 16, Dh)
+        for i in range(case.n):
+            tiles[0, case.tables[i][token // 16], :, 0, token % 16, 3] = 0x7C00
+        B.check(ctx._lib.jgpt_h2d(ctx.handle, ptr, raw.ctypes.data, nbytes))
+        q = np.random.default_rng(96).standard_normal((case.n, H, Dh)).astype(np.float32)
+        q[:, :, 3] = -np.abs(q[:, :, 3]) - 0.1
+        out = ctx.alloc((case.n, H * Dh))
+        case.pool.attn_decode(0, 1, ctx.from_host(q.reshape(case.n, -1)), case.seq_ids_dev(), ctx.from_host(np.zeros(case.n, np.int32)),
+                              ctx.from_host(case.lens), case.n, max(lens), out)
+        ctx.synchronize()
+        got = out.to_host().reshape(case.n, H, Dh)
+        for i, l in enumerate(lens):
+            keep = [t for t in range(l) if t != token]
+            s = np.einsum("hd,hkd->hk", q[i].astype(np.float64), case.kc[0, i][:, keep].astype(np.float64)) / 4
+            p = np.exp(s - s.max(-1, keepdims=True))
+            want = np.einsum("hk,hkd->hd", p / p.sum(-1, keepdims=True), case.vc[0, i][:, keep].astype(np.float64))
+            assert np.abs(got[i] - want).max() < TOL
+    finally:
+        case.close()
+
+
 @pytest.mark.parametrize("size", [0.2, 1.0])
 @pytest.mark.parametrize("overlap", [0, 1])
 def test_error_against_float64_with_either_consumers(ctx, overlap, size):
