@@ -130,10 +130,10 @@ __device__ __forceinline__ void split_half2(float a, float b, uint32_t &hi, uint
 // attention outputs stay within ~4e-4 of the exact mode on N(0,1) inputs and the logits of the JGPT-35M shapes within
 // 5e-4 of an fp32 CPU evaluation, against a budget of 2e-3.  The exact mode (2e-5) remains the default of the
 // standalone entry point.
-// OUT: the form of the output, row major or one of the projection's operand images.  At compile time: with both images as branches the
-// short prompts' kernel took other registers and a prompt of 201 tokens 1 % longer.
-enum Out { OUT_ROWS, OUT_TF32, OUT_HALF };
-template <bool FAST, int OUT>
+// TF32: the output as a TF32 operand image; otherwise row major, or an fp16 image where there is one.  The TF32 form is a kernel of its own:
+// as a third branch it, and row-major kernels without branches as well, were compiled to other schedules (61 registers instead of 68), and
+// short prompts took up to 3 % longer (one of 400 tokens 708 us, 687 in this form).
+template <bool FAST, bool TF32>
 __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillParams P) {
     constexpr int DH = 16, BT = kBlockTokens, TILE_BYTES = 2 * BT * DH * 2;  // 1 KiB: K tile | V tile
     __shared__ __align__(128) unsigned char tiles[2][kStageBlocks][TILE_BYTES];
@@ -351,51 +351,60 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(const PrefillPara
     lB += __shfl_xor_sync(0xffffffffu, lB, 1);
     lB += __shfl_xor_sync(0xffffffffu, lB, 2);
     const float iA = 1.f / fmaxf(lA, 1e-12f), iB = 1.f / fmaxf(lB, 1e-12f);
-    if constexpr (OUT != OUT_ROWS) {
-        // Operand image of the next projection (see gemm_umma.cu): 128-row tiles, high parts then low parts.  Lane (g, t) holds columns
-        // 8 j + 2 t, 8 j + 2 t + 1 of the head.
-        // TF32: k tiles of 16, head h is k tile h; the pair is half of the 16-byte chunk 2 j + t / 2, a warp store covers eight rows x two
-        // chunks = two full 128-byte lines.
-        // fp16: k tiles of 32, head h is half of k tile h / 2, values times the powers of two that the image's columns carry; a warp
-        // store covers eight rows x one chunk = one full line.
+    const size_t D = (size_t)P.H * DH;
+    if constexpr (TF32) {
+        // Operand image of the next projection (see gemm_umma.cu): 128-row tiles x 16-wide k tiles, TF32 high parts
+        // then low parts; head h is k tile h.  Lane (g, t) holds columns 8 j + 2 t, 8 j + 2 t + 1: half of the 16-byte
+        // chunk 2 j + t / 2, so a warp store covers eight rows x two chunks = two full 128-byte lines.
         auto put = [&](int row, int j, float a, float b) {
             const size_t grow = (size_t)sd.row0 + row;
             const int rr = (int)(grow & 127);
-            if constexpr (OUT == OUT_TF32) {
-                float *dst = P.out_image + ((grow >> 7) * (size_t)P.H + h) * (size_t)(128 * 16 * 2) + (rr >> 3) * 128 + (2 * j + (t >> 1)) * 32 + (rr & 7) * 4 + (t & 1) * 2;
-                uint32_t ha, hb, la, lb;
-                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ha) : "f"(a));
-                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(b));
-                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(la) : "f"(a - __uint_as_float(ha)));
-                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(b - __uint_as_float(hb)));
-                *reinterpret_cast<float2 *>(dst) = make_float2(__uint_as_float(ha), __uint_as_float(hb));
-                *reinterpret_cast<float2 *>(dst + 128 * 16) = make_float2(__uint_as_float(la), __uint_as_float(lb));
-            } else {
-                const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
-                unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
-                unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
-                uint32_t hi, lo;
-                split_half2(a * up.x, b * up.y, hi, lo);
-                *reinterpret_cast<uint32_t *>(dst) = hi;
-                *reinterpret_cast<uint32_t *>(dst + 128 * 32 * 2) = lo;
-            }
+            float *dst = P.out_image + ((grow >> 7) * (size_t)P.H + h) * (size_t)(128 * 16 * 2) + (rr >> 3) * 128 + (2 * j + (t >> 1)) * 32 + (rr & 7) * 4 + (t & 1) * 2;
+            uint32_t ha, hb, la, lb;
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ha) : "f"(a));
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(b));
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(la) : "f"(a - __uint_as_float(ha)));
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lb) : "f"(b - __uint_as_float(hb)));
+            *reinterpret_cast<float2 *>(dst) = make_float2(__uint_as_float(ha), __uint_as_float(hb));
+            *reinterpret_cast<float2 *>(dst + 128 * 16) = make_float2(__uint_as_float(la), __uint_as_float(lb));
         };
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             if (rowA < sd.S) put(rowA, j, o[j][0] * iA, o[j][1] * iA);
             if (rowB < sd.S) put(rowB, j, o[j][2] * iB, o[j][3] * iB);
         }
-    } else {
-        const size_t D = (size_t)P.H * DH;
+        return;
+    }
+    if (P.out_image) {
+        // fp16 operand image: 128-row tiles x 32-wide k tiles, high parts then low parts; head h is half of k tile h / 2.  Lane (g, t) holds
+        // columns 8 j + 2 t, 8 j + 2 t + 1 of the head, times the powers of two that the image's columns carry: a warp store covers
+        // eight rows x one 16-byte chunk = one full 128-byte line.
+        auto put = [&](int row, int j, float a, float b) {
+            const size_t grow = (size_t)sd.row0 + row;
+            const float2 up = *reinterpret_cast<const float2 *>(P.out_scale + h * DH + 8 * j + 2 * t);
+            unsigned char *tile = reinterpret_cast<unsigned char *>(P.out_image) + ((grow >> 7) * (size_t)(P.H / 2) + (h >> 1)) * (size_t)(128 * 32 * 4);
+            const int rr = (int)(grow & 127);
+            unsigned char *dst = tile + (rr >> 3) * 512 + ((h & 1) * 2 + j) * 128 + (rr & 7) * 16 + t * 4;
+            uint32_t hi, lo;
+            split_half2(a * up.x, b * up.y, hi, lo);
+            *reinterpret_cast<uint32_t *>(dst) = hi;
+            *reinterpret_cast<uint32_t *>(dst + 128 * 32 * 2) = lo;
+        };
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            if (rowA < sd.S)
-                *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowA) * D + h * DH + 8 * j + 2 * t) =
-                    make_float2(o[j][0] * iA, o[j][1] * iA);
-            if (rowB < sd.S)
-                *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowB) * D + h * DH + 8 * j + 2 * t) =
-                    make_float2(o[j][2] * iB, o[j][3] * iB);
+            if (rowA < sd.S) put(rowA, j, o[j][0] * iA, o[j][1] * iA);
+            if (rowB < sd.S) put(rowB, j, o[j][2] * iB, o[j][3] * iB);
         }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (rowA < sd.S)
+            *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowA) * D + h * DH + 8 * j + 2 * t) =
+                make_float2(o[j][0] * iA, o[j][1] * iA);
+        if (rowB < sd.S)
+            *reinterpret_cast<float2 *>(P.out + (size_t)(sd.row0 + rowB) * D + h * DH + 8 * j + 2 * t) =
+                make_float2(o[j][2] * iB, o[j][3] * iB);
     }
 }
 
@@ -521,11 +530,9 @@ int32_t launch_attn_prefill(Pool *p, int layer, const float *q, const float *k, 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         P.pdl = pdl && skip_append;  // behind the append kernel: an ordinary launch
         cfg.gridDim = grid, cfg.blockDim = dim3(128), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = P.pdl ? 1 : 0;
-        auto pick = [&](auto f) {
-            constexpr bool FAST = decltype(f)::value;
-            return !out_image ? attn_prefill_mma_kernel<FAST, OUT_ROWS> : out_scale ? attn_prefill_mma_kernel<FAST, OUT_HALF> : attn_prefill_mma_kernel<FAST, OUT_TF32>;
-        };
-        JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, fast ? pick(std::true_type()) : pick(std::false_type()), P));
+        const bool tf32 = out_image && !out_scale;
+        JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, fast ? (tf32 ? attn_prefill_mma_kernel<true, true> : attn_prefill_mma_kernel<true, false>)
+                                                    : (tf32 ? attn_prefill_mma_kernel<false, true> : attn_prefill_mma_kernel<false, false>), P));
     } else {
         dim3 grid((unsigned)((max_S + 127) / 128), (unsigned)p->heads, (unsigned)n_seqs);
         switch (DH) {
