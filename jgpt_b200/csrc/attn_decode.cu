@@ -4,9 +4,9 @@
 // Work item = (layer, sequence, head group, chunk of `chunk_blocks` KV blocks).  A CTA owns a
 // ring of shared-memory stages; one producer warp walks the block table and fetches, per KV
 // block, the contiguous [head group][K tile | V tile] slab with ONE bulk async copy (TMA engine,
-// cp.async.bulk + mbarrier complete_tx).  At dhead 16 a consumer warp owns four heads and runs their
-// products on the tensor cores with high + low operands; at the other head sizes, and for small launches
-// of several layers, consumer threads are (head, token-in-block) pairs: a thread scores its token against q (fp32 FMA), keeps a private
+// cp.async.bulk + mbarrier complete_tx).  At dhead 16 and a multiple of four heads a consumer warp owns four
+// of them and runs their products on the tensor cores with high + low operands; at other head sizes and counts, and for
+// small launches of several layers, consumer threads are (head, token-in-block) pairs: a thread scores its token against q (fp32 FMA), keeps a private
 // online-softmax state (m, l, o[DH]) and, at the end of the chunk, the 16 lanes of a head merge their
 // states with warp shuffles.  Chunks of one sequence are merged by the last CTA to arrive (atomic ticket, no
 // waiting), through a small fp32 scratch buffer.
@@ -1493,7 +1493,7 @@ static int32_t launch_attn_decode_static(Pool *p, int layer, const float *q, con
     P.status = p->ctx->d_status;
     P.n = n, P.H = p->heads, P.layer0 = layer, P.n_layers = 1, P.mbs = p->max_blocks_per_seq;
     P.n_blocks = p->n_blocks, P.max_seqs = p->max_seqs, P.max_positions = p->max_positions;
-    // same launch shape as jgpt_attn_decode gives a one-layer call (small batches get lighter CTAs)
+    // the launch shape of a one-layer jgpt_attn_decode whose launches do not overlap (small batches get lighter CTAs)
     P.stream_hint = p->stream_hint;
     P.HG = pick_head_group(p->heads, DH, p->head_group, (long long)n, 2ll * p->ctx->sm_count);
     P.n_hg = p->heads / P.HG;
