@@ -311,7 +311,7 @@ def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, part, spread):
         pool.close(), gm.close()
 
 
-@pytest.mark.parametrize("dm,dff", [(64, 128), (384, 768)])
+@pytest.mark.parametrize("dm,dff", [(64, 128), (384, 768), (768, 256)])
 def test_prefill_on_fp16_images_with_dead_and_extreme_columns(ctx, dm, dff):
     """Hidden units whose gate or up column is zero (pruned) or far outside fp16, some with the inverse in W2 so that they count: h alone is
     then far larger than the gated value can be, squares of a column leave fp32, and a unit is worth 1e-24 or 1e20 of its neighbour.
