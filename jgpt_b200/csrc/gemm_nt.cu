@@ -1,6 +1,6 @@
 // C[M, N] = A[M, K] . W[N, K]^T for decode-sized M (bf16, mma.sync) and in plain fp32.
 //
-// Decode-sized bf16 products are bound by the weight stream and by latency: a CTA owns 32 output columns (64 from 33 rows
+// Decode-sized bf16 products (those of a handful of rows: gemm_nt_few.cu) are bound by the weight stream and by latency: a CTA owns 32 output columns (64 from 33 rows
 // on, so that the rows are read half as often) and up to 64 rows; its eight warps split every 128-wide k tile (a warp
 // covers 32 columns with its own k slice), tiles arrive through a cp.async ring, and the partial tiles are added in warp
 // order through shared memory.  Products with few column tiles run as clusters of CTAs that split the k range; the partial sums meet in the
@@ -198,13 +198,7 @@ __global__ void __launch_bounds__(256) gemm_nt_small_kernel(const SmallArgs args
             if ((c & 31) < 16 && m < M && n + 16 < N)
                 reinterpret_cast<__nv_bfloat16 *>(P.C)[(size_t)m * P.ldc + n / 32 * 16 + (c & 15)] = __float2bfloat16(activate<true>(P.act, 0.f, 0.f, sum[i]) * up);
         } else if (m < M && n < n_end) {
-            const size_t at = (size_t)m * P.ldc + n + cn;
-            if (EPI == EPI_STORE) reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(P.bias ? sum[i] + P.bias[n] : sum[i]);
-            if (EPI == EPI_ACT) reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(activate<true>(P.act, P.p0, P.p1, sum[i]));
-            if (EPI == EPI_ACT_SOME)
-                reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(n >= P.act_from && n < P.act_to ? activate<true>(P.act, P.p0, P.p1, sum[i]) : sum[i] + P.bias[n]);
-            if (EPI == EPI_ADD_F32) reinterpret_cast<float *>(P.C)[at] = P.res_scale * P.res[at] + (P.colscale ? P.colscale[n] * sum[i] : sum[i]);
-            if (EPI == EPI_SCALE_F32) reinterpret_cast<float *>(P.C)[at] = sum[i] * P.scale;
+            store_sum<EPI>(P, (size_t)m * P.ldc + n + cn, n, sum[i], P.bias ? P.bias[n] : 0.f);
         }
     }
 }
@@ -259,6 +253,8 @@ static int32_t small_dispatch(const Ctx *ctx, const Problem *p, int n, int pdl, 
     // split k while the launch leaves SMs idle and every part keeps two tiles
     a.k_split = 1;
     while (n == 1 && !GROUPED && a.k_split < max_split && ctas * a.k_split * 2 <= 2 * ctx->sm_count && nk / (a.k_split * 2) >= 2) a.k_split *= 2;
+    int32_t rc = JGPT_OK;
+    if (n == 1 && !GROUPED && launch_bf16_few(ctx, p[0], (Epilogue)EPI, a.k_split, pdl, st, &rc)) return rc;
     switch (mt) {
         case 1: return small_launch<1, 1, 6, EPI, GROUPED>(a, tiles, M, st);
         case 2: return small_launch<2, 1, 5, EPI, GROUPED>(a, tiles, M, st);

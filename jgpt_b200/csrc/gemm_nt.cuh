@@ -1,5 +1,6 @@
 // Projections with weights in [out, in] layout: C[M, N] = A[M, K] . W[N, K]^T, bf16 operands with fp32 accumulation or
-// plain fp32.  Host-side interface of gemm_nt.cu (small M, and fp32) and gemm_nt_umma.cu (large M, tcgen05).
+// plain fp32.  Host-side interface of gemm_nt_few.cu (a handful of rows), gemm_nt.cu (small M, and
+// fp32) and gemm_nt_umma.cu (large M, tcgen05).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -88,6 +89,17 @@ __device__ __forceinline__ float activate(int act, float p0, float p1, float z) 
     }
 }
 
+// A finished sum of column n, whose bias has been read, to element `at` of C (all but EPI_GATE).
+template <int EPI>
+__device__ __forceinline__ void store_sum(const Problem &P, size_t at, int n, float sum, float bias) {
+    if (EPI == EPI_STORE) reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(P.bias ? sum + bias : sum);
+    if (EPI == EPI_ACT) reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(activate<true>(P.act, P.p0, P.p1, sum));
+    if (EPI == EPI_ACT_SOME)
+        reinterpret_cast<__nv_bfloat16 *>(P.C)[at] = __float2bfloat16(n >= P.act_from && n < P.act_to ? activate<true>(P.act, P.p0, P.p1, sum) : sum + bias);
+    if (EPI == EPI_ADD_F32) reinterpret_cast<float *>(P.C)[at] = P.res_scale * P.res[at] + (P.colscale ? P.colscale[n] * sum : sum);
+    if (EPI == EPI_SCALE_F32) reinterpret_cast<float *>(P.C)[at] = sum * P.scale;
+}
+
 // Runs 1 or 2 independent products (same M) in one launch.  K, lda, ldw and (bf16) the operand addresses must allow
 // 16-byte row chunks: multiples of 8 elements (bf16) or 4 (fp32).  pdl: bit 0 = this launch may start early and waits
 // itself; bit 1 = it lets the next launch in.  Of two products the first may have rows in groups; M is then the number of rows
@@ -101,6 +113,11 @@ int umma_min_rows();
 // kernel, whose operand holds the rows group by group.
 constexpr int kLargeTile = 128;
 int group_tile_rows(bool f32, int rows, int copies, int groups);
+// gemm_nt_few.cu: at most this many rows, and column slices of the weights that a CTA's share of an SM's memory holds.
+constexpr int kFewRows = 32;
+constexpr size_t kFewSmem = 112 * 1024;
+// parts: into how many the ring's kernel would cut k; false: not for this kernel
+bool launch_bf16_few(const Ctx *ctx, const Problem &p, Epilogue epi, int parts, int pdl, cudaStream_t st, int32_t *rc);
 int32_t launch_bf16_umma(const Ctx *ctx, const Problem &p, Epilogue epi, int pdl, cudaStream_t st);
 
 }  // namespace nt

@@ -71,6 +71,23 @@ def test_residual_after_every_layer(ctx, cases, name):
     pool.close(), m.close()
 
 
+@pytest.mark.parametrize("width,ff,vocab", [(1032, 40, 4736), (200, 1500, 2304), (64, 2064, 33), (72, 6400, 101)])
+def test_products_of_few_rows(ctx, width, ff, vocab):
+    """Batches of single tokens on both sides of a row tile; widths that end inside a unit of k, inside 32 bytes, and slices too long to be held."""
+    c = lc.Case(lc.config([lc.att(heads=2, kv_heads=1, mlp=lc.dense(ff)), lc.gen(heads=1, dim=16)], width=width, vocab=vocab), seed=width)
+    m = c.model(ctx, "bfloat16")
+    pool = m.newPool(40, 40)
+    t = dc.tokens(c.cfg, 33, 5)
+    want = np.stack([c.ref(t[i:i + 1])[0] for i in range(33)])
+    for rows in (1, 15, 16, 17, 32, 33):
+        seqs = [pool.seq_alloc() for _ in range(rows)]
+        got, _ = m.step(pool, seqs, [t[i:i + 1] for i in range(rows)], range(rows))
+        for s in seqs:
+            pool.seq_free(s)
+        _close(got, want[:rows], "bfloat16")
+    pool.close(), m.close()
+
+
 # ---- each mechanism alone ----------------------------------------------------------------------------------
 def _alone(ctx, layers, dtype, sizes=(200, 1, 2, 40, 7, 50), width=64, edit=None, seed=3, tol=0.04):
     """What a layer (the last one) adds to the residual, in portions."""
