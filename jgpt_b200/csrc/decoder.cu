@@ -124,7 +124,8 @@ struct Decoder {
     float2 *row_inv = nullptr;         // 1 / root mean square of a row's queries and keys
     int *d_desc = nullptr, *h_desc = nullptr;
     int *d_next = nullptr, *h_next = nullptr;
-    float *d_u = nullptr, *h_u = nullptr, *samp = nullptr;
+    float *h_u = nullptr, *hd_u = nullptr, *samp = nullptr;
+    HostMirror host{};  // of h_next and the context's status word
     uint64_t chunk_ws_floats = 0;
     int long_min = 0;  // entries of at least this many tokens run their recurrences in chunks (0: none)
     int logit_rows = 0;
@@ -581,11 +582,14 @@ static int32_t build(Decoder *d, const jgpt_layer_spec *layers) {
     d->logit_rows = (int)std::max<uint64_t>(1, std::min<uint64_t>(R, (64ull << 20) / (uint64_t)d->s.vocab));
     TRY(dalloc(d, (void **)&d->logits, sizeof(float) * (uint64_t)d->logit_rows * d->s.vocab));
     TRY(dalloc(d, (void **)&d->d_next, sizeof(int) * R));
-    TRY(dalloc(d, (void **)&d->d_u, sizeof(float) * R));
     TRY(dalloc(d, (void **)&d->d_desc, sizeof(int) * desc_ints(d)));
     JGPT_CUDA_TRY(cudaHostAlloc(&d->h_desc, sizeof(int) * desc_ints(d), cudaHostAllocDefault));
     JGPT_CUDA_TRY(cudaHostAlloc(&d->h_next, sizeof(int) * R, cudaHostAllocDefault));
     JGPT_CUDA_TRY(cudaHostAlloc(&d->h_u, sizeof(float) * R, cudaHostAllocDefault));
+    JGPT_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d->hd_u), d->h_u, 0));
+    JGPT_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d->host.next), d->h_next, 0));
+    JGPT_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d->host.status), d->ctx->h_status, 0));
+    d->host.status_dev = d->ctx->d_status;
     JGPT_CUDA_TRY(cudaStreamSynchronize(d->ctx->stream));
     return JGPT_OK;
 }
@@ -1185,10 +1189,12 @@ static int32_t enqueue_head(Decoder *d, const mix::StepDesc &sd, int w0, int n, 
                                       d->ldw, d->ctx->d_status, pdl, st));
     else TRY(mix::launch_layer_norm(d->f32, d->x, sd.want + w0, mix::NormW{d->fnw, d->fnb}, d->s.eps, d->h, n, d->s.width, d->ldw, pdl, st));
     nt::Problem p{d->h, d->head ? d->head : d->embed, d->logits, nullptr, n, d->s.vocab, d->ldw, d->ldw, d->ldw, d->s.vocab, d->s.logit_scale};
-    TRY(product(d, &p, 1, nt::EPI_SCALE_F32, pdl & 1));
+    const bool early = pdl && pick && spec.temperature <= 0.f;  // the argmax waits for the logits itself
+    TRY(product(d, &p, 1, nt::EPI_SCALE_F32, early ? pdl : pdl & 1));
     if (!pick) return JGPT_OK;
-    if (spec.temperature > 0.f) return launch_sample(d->logits, d->samp, n, d->s.vocab, spec, d->d_u + w0, d->d_next + w0, st);
-    return launch_argmax(d->logits, n, d->s.vocab, d->d_next + w0, st);
+    const HostMirror host{d->host.next + w0, d->host.status, d->host.status_dev};
+    if (spec.temperature > 0.f) return launch_sample(d->logits, d->samp, n, d->s.vocab, spec, d->hd_u + w0, d->d_next + w0, host, st);
+    return launch_argmax(d->logits, n, d->s.vocab, d->d_next + w0, host, early, st);
 }
 
 // Replays the step's graph, captures it at the second step of its kind, or runs the launches one by one.
@@ -1355,7 +1361,6 @@ int32_t decoder_step(Decoder *d, Pool *p, jgpt_kvpool poolh, const StepCall &c) 
     if (pick && c.spec.temperature > 0.f && c.n_want) {
         if (!d->samp) TRY(dalloc(d, (void **)&d->samp, sizeof(float) * (uint64_t)d->logit_rows * d->s.vocab));
         std::copy(c.u01, c.u01 + c.n_want, d->h_u);
-        JGPT_CUDA_TRY(cudaMemcpyAsync(d->d_u, d->h_u, sizeof(float) * c.n_want, cudaMemcpyHostToDevice, st));
     }
     auto enqueue = [&]() -> int32_t {
         JGPT_CUDA_TRY(cudaMemcpyAsync(d->d_desc, hd, sizeof(int) * at, cudaMemcpyHostToDevice, st));
@@ -1367,8 +1372,7 @@ int32_t decoder_step(Decoder *d, Pool *p, jgpt_kvpool poolh, const StepCall &c) 
                 JGPT_CUDA_TRY(cudaMemcpyAsync(c.logits_host + (size_t)w0 * d->s.vocab, d->logits, sizeof(float) * (size_t)n * d->s.vocab,
                                               cudaMemcpyDeviceToHost, st));
         }
-        if (pick && c.n_want) JGPT_CUDA_TRY(cudaMemcpyAsync(d->h_next, d->d_next, sizeof(int) * c.n_want, cudaMemcpyDeviceToHost, st));
-        JGPT_CUDA_TRY(status_enqueue_read(d->ctx));
+        if (!pick || !c.n_want) JGPT_CUDA_TRY(status_enqueue_read(d->ctx));  // else the kernel that picked the last tokens has left both
         return JGPT_OK;
     };
     bool plain = d->use_graphs && n_tiles == 0 && pick && !c.logits_host && !capture_to && c.spec.temperature <= 0.f && c.n_want == c.n;

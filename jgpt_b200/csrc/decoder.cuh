@@ -44,9 +44,16 @@ int32_t decoder_decode(Decoder *d, jgpt_kvpool poolh, const int *seq_ids, const 
 int32_t decoder_generate_greedy(Decoder *d, jgpt_kvpool poolh, const int *prompt, int S, int max_new, int *out, int *n_sampled);
 
 // model.cu
-int32_t launch_argmax(const float *logits, int rows, int vocab, int *next_dev, cudaStream_t st);
+// The kernel that picks a step's tokens leaves them and the status word in the host's mirrors as well: device-side addresses, all null or none.
+// (Two copies less behind the step.)
+struct HostMirror {
+    int *next, *status;
+    const int *status_dev;
+};
+// early: the launch in front lets this one in and is waited for here
+int32_t launch_argmax(const float *logits, int rows, int vocab, int *next_dev, const HostMirror &host, bool early, cudaStream_t st);
 int32_t launch_sample(const float *logits, float *work, int rows, int vocab, const SampleSpec &spec, const float *u01_dev, int *next_dev,
-                      cudaStream_t st);
+                      const HostMirror &host, cudaStream_t st);
 
 // kvpool.cu: a pool whose layers have their own geometry and whose sequence slots carry recurrent state.
 int32_t pool_create_layered(Ctx *c, const std::vector<KvLayerGeom> &layers, int elem_bytes, int n_blocks, int max_seqs, int max_blocks_per_seq,

@@ -66,7 +66,7 @@ struct Model {
         uint64_t last_use = 0;
     };
     // on-device sampling: per-row uniform draws (pinned + device) and the [rows, vocab] work area of the sampler (sample.cu)
-    float *h_u = nullptr, *d_u = nullptr, *d_samp = nullptr;
+    float *h_u = nullptr, *d_u = nullptr, *hd_u = nullptr, *d_samp = nullptr;  // hd_u: device-side address of h_u
     int samp_rows = 0;
     std::vector<DecodeGraph> decode_graphs;
     uint64_t decode_graph_clock = 0;
@@ -720,9 +720,13 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float *log
 }
 
 // The token choice for models that run their own forward step (decoder.cu).
-int32_t launch_argmax(const float *logits, int rows, int vocab, int *next_dev, cudaStream_t st) {
-    argmax_kernel<<<rows, kArgmaxThreads, 0, st>>>(logits, vocab, next_dev);
-    JGPT_CUDA_TRY(cudaGetLastError());
+int32_t launch_argmax(const float *logits, int rows, int vocab, int *next_dev, const HostMirror &host, bool early, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)rows), cfg.blockDim = dim3(kArgmaxThreads), cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = early ? 1 : 0;
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, argmax_kernel, logits, vocab, next_dev, host.next, host.status_dev, host.status, early ? 1 : 0));
     return JGPT_OK;
 }
 // ------------------------------------------------------------------------------------------------
@@ -1345,21 +1349,13 @@ static int32_t lm_head(Model *m, int rows, int n_sel, const SampleSpec &spec = S
         rc = gemm(m, m->xn, out_rows, D, m->vocab, 1, W, C, nullptr);
     }
     if (rc) return rc;
-    if (spec.temperature > 0.f) {  // the draws are in m->d_u (uploaded by the caller)
+    const HostMirror host = to_host ? HostMirror{m->hd_next, m->hd_status, m->ctx->d_status} : HostMirror{};
+    if (spec.temperature > 0.f) {  // the draws are in the caller's block, or uploaded by it
         rc = ensure_sample_work(m, out_rows);
         if (rc) return rc;
-        if ((rc = launch_sample(m->logits, m->d_samp, out_rows, m->vocab, spec, m->d_u, m->d_next, st))) return rc;
-    } else {
-        if (to_host && early && small_mode(m, rows)) {  // moves in under the LM head's last CTAs
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.gridDim = dim3((unsigned)out_rows), cfg.blockDim = dim3(kArgmaxThreads), cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = 1;
-            const float *lg = m->logits;
-            JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, argmax_kernel, lg, m->vocab, m->d_next, m->hd_next, (const int *)m->ctx->d_status, m->hd_status, 1));
-        } else if (to_host) argmax_kernel<<<out_rows, kArgmaxThreads, 0, st>>>(m->logits, m->vocab, m->d_next, m->hd_next, m->ctx->d_status, m->hd_status);
-        else argmax_kernel<<<out_rows, kArgmaxThreads, 0, st>>>(m->logits, m->vocab, m->d_next);
+        if ((rc = launch_sample(m->logits, m->d_samp, out_rows, m->vocab, spec, to_host ? m->hd_u : m->d_u, m->d_next, host, st))) return rc;
+    } else {  // early: moves in under the LM head's last CTAs
+        if ((rc = launch_argmax(m->logits, out_rows, m->vocab, m->d_next, host, to_host && early && small_mode(m, rows), st))) return rc;
     }
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
@@ -1702,6 +1698,7 @@ int32_t jgpt_model_create(jgpt_ctx ctxh, int32_t vocab, int32_t max_seq_len, int
     JGPT_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->hd_status), m->ctx->h_status, 0));
     JGPT_CUDA_TRY(cudaMalloc(&m->d_rowsel, sizeof(int) * R));
     JGPT_CUDA_TRY(cudaHostAlloc(&m->h_u, sizeof(float) * R, cudaHostAllocDefault));
+    JGPT_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->hd_u), m->h_u, 0));
     JGPT_CUDA_TRY(A(&m->d_u, R));
     JGPT_CUDA_TRY(A(&m->ss_a, R * rows::ss_parts((int)D)));
     JGPT_CUDA_TRY(A(&m->ss_b, R * rows::ss_parts((int)D)));
@@ -2038,14 +2035,14 @@ static int32_t forward_decode_impl(jgpt_model h, jgpt_kvpool poolh, const int32_
         rc = ensure_sample_work(m, n);  // before any capture: it may allocate
         if (rc) return rc;
     }
-    // Greedy decode-sized steps move their few words themselves: the embedding kernel fetches the rows' descriptors from
-    // the page-locked block, the argmax kernel leaves ids and status word in the host mirrors (three copies less per step;
+    // Decode-sized steps move their few words themselves: the embedding kernel fetches the rows' descriptors from
+    // the page-locked block, the kernel that picks the tokens reads its draws there and leaves ids and status word in the host mirrors (three copies less per step;
     // the descriptor copy alone moved 5 R words whatever the batch).  JGPT_B200_STEP_COPIES=1: the copies.
     static const int step_copies = env_int("JGPT_B200_STEP_COPIES", 0);
-    const bool no_copies = !sampled && !step_copies && small_mode(m, n);
+    const bool no_copies = !step_copies && small_mode(m, n);
     auto enqueue = [&]() -> int32_t {
         if (!no_copies) JGPT_CUDA_TRY(cudaMemcpyAsync(m->d_idx, m->h_idx, sizeof(int) * 5 * (size_t)R, cudaMemcpyHostToDevice, st));
-        if (sampled) JGPT_CUDA_TRY(cudaMemcpyAsync(m->d_u, m->h_u, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st));
+        if (sampled && !no_copies) JGPT_CUDA_TRY(cudaMemcpyAsync(m->d_u, m->h_u, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st));
         const bool chain_early = small_mode(m, n) && step_overlap_level(m, n) >= 3;
         m->first_launch_early = chain_early;
         if (no_copies) embed_pos_kernel<<<n, 128, 0, st>>>(m->tok, m->pos, nullptr, nullptr, m->x, m->d_model, m->ss_a, m->hd_idx, m->d_idx, R);
@@ -2083,7 +2080,7 @@ static int32_t forward_decode_impl(jgpt_model h, jgpt_kvpool poolh, const int32_
         } else if (rc) {
             return rc;
         } else {
-            if (sampled && (rc = launch_sample(m->logits, m->d_samp, n, m->vocab, spec, m->d_u, m->d_next, st))) return rc;
+            if (sampled && (rc = launch_sample(m->logits, m->d_samp, n, m->vocab, spec, m->d_u, m->d_next, HostMirror{}, st))) return rc;
             if (form == 2 || sampled) JGPT_CUDA_TRY(cudaMemcpyAsync(m->h_next, m->d_next, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, st));
             JGPT_CUDA_TRY(status_enqueue_read(m->ctx));
             one_launch = true;

@@ -64,7 +64,7 @@ __device__ __forceinline__ float chain(const float *e, int n, float u, int *at) 
 }
 
 __global__ void __launch_bounds__(kThreads) sample_kernel(const float *__restrict__ logits, float *__restrict__ work, int V, float temperature,
-                                                          int top_k, const float *__restrict__ u01, int *__restrict__ out, int row_in_smem) {
+                                                          int top_k, const float *u01, int *__restrict__ out, const HostMirror host, int row_in_smem) {
     extern __shared__ float smem_row[];
     __shared__ int hist[kBins];
     __shared__ int list_i[kListMax];
@@ -78,6 +78,12 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float *__restric
     float *z = row_in_smem ? smem_row : work + (size_t)blockIdx.x * V;
     float mx = -INFINITY;
     bool bad = false;
+    const float u = tid == 0 ? u01[blockIdx.x] : 0.f;  // perhaps from the host's memory: requested first, used last
+    auto leave = [&](int tok) {
+        out[blockIdx.x] = tok;
+        if (host.next) host.next[blockIdx.x] = tok;
+        if (host.next && blockIdx.x == 0) *host.status = *host.status_dev;
+    };
     for (int i0 = tid; i0 < V; i0 += 8 * kThreads) {
         float v[8];
 #pragma unroll
@@ -99,7 +105,7 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float *__restric
     for (int w = 1; w < kWarps; w++) mx = fmaxf(mx, w_mx[w]);
     // a NaN, or a maximum that is not finite, makes every sum a NaN: no index is reached and the last one is taken
     if (bad || !isfinite(mx)) {
-        if (tid == 0) out[blockIdx.x] = V - 1;
+        if (tid == 0) leave(V - 1);
         return;
     }
     const bool some = top_k > 0 && top_k < V;
@@ -188,18 +194,17 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float *__restric
     for (int i = tid; i < n; i += kThreads) e[i] = e[i] / sum;
     __syncthreads();
     if (tid == 0) {
-        const float u = u01[blockIdx.x];
         int at;
         chain<true>(e, n, u, &at);
         int tok = at == n ? V - 1 : (list ? list_i[at] : at);
         if (list && list_i[0] != 0 && u <= 0.f) tok = 0;  // index 0, dropped: its running sum is 0
-        out[blockIdx.x] = tok;
+        leave(tok);
     }
 }
 
 // work: [rows, vocab], used by rows that do not fit shared memory.
 int32_t launch_sample(const float *logits, float *work, int rows, int vocab, const SampleSpec &spec, const float *u01_dev, int *next_dev,
-                      cudaStream_t st) {
+                      const HostMirror &host, cudaStream_t st) {
     const size_t row = sizeof(float) * (size_t)vocab;
     const bool in_smem = row <= kRowBytesMax;
     static bool opted[64] = {};
@@ -209,7 +214,7 @@ int32_t launch_sample(const float *logits, float *work, int rows, int vocab, con
         JGPT_CUDA_TRY(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowBytesMax));
         opted[dev & 63] = true;
     }
-    sample_kernel<<<rows, kThreads, in_smem ? row : 0, st>>>(logits, work, vocab, spec.temperature, spec.top_k, u01_dev, next_dev, in_smem);
+    sample_kernel<<<rows, kThreads, in_smem ? row : 0, st>>>(logits, work, vocab, spec.temperature, spec.top_k, u01_dev, next_dev, host, in_smem);
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
