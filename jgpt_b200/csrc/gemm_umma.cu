@@ -51,6 +51,8 @@
 // winds down through the common exit (tensor memory is always released).
 #include "gemm_umma.cuh"
 
+#include <type_traits>
+
 #include "ptx.cuh"
 #include "tcgen05.cuh"
 
@@ -105,6 +107,31 @@ __global__ void __launch_bounds__(256) pack_kernel(const float *__restrict__ src
         const int off = chunk_offset(rr, k4);
         *reinterpret_cast<float4 *>(tile + off) = hi;
         *reinterpret_cast<float4 *>(tile + TR * BK + off) = lo;
+    }
+}
+
+// Both operands of a product in one launch: the row tiles of A [M, K], then the column tiles of B [K, N], TR columns each.
+template <int TR>
+__global__ void __launch_bounds__(256) pack_both_kernel(const float *__restrict__ A, int M, const float *__restrict__ B, int N, int K,
+                                                        float *__restrict__ a_image, float *__restrict__ b_image, int a_tiles) {
+    const int nkt = K / BK, t = blockIdx.x / nkt, kt = blockIdx.x - t * nkt;
+    const bool second = t >= a_tiles;
+    const int rt = second ? t - a_tiles : t, rows = second ? TR : BM, lg = second ? (TR == 192 ? 0 : TR == 64 ? 6 : TR == 128 ? 7 : 8) : 7;
+    float *tile = (second ? b_image : a_image) + ((size_t)rt * nkt + kt) * (size_t)(rows * BK * 2);
+    griddep_launch_dependents();
+    for (int e = threadIdx.x; e < rows * (BK / 4); e += 256) {
+        const int k4 = lg ? e >> lg : e / TR, rr = e - k4 * rows, r = rt * rows + rr, k = kt * BK + k4 * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (second) {
+            if (r < N) v = make_float4(B[(size_t)k * N + r], B[(size_t)(k + 1) * N + r], B[(size_t)(k + 2) * N + r], B[(size_t)(k + 3) * N + r]);
+        } else if (r < M) {
+            v = *reinterpret_cast<const float4 *>(A + (size_t)r * K + k);
+        }
+        float4 hi, lo;
+        split4(v, hi, lo);
+        const int off = chunk_offset(rr, k4);
+        *reinterpret_cast<float4 *>(tile + off) = hi;
+        *reinterpret_cast<float4 *>(tile + rows * BK + off) = lo;
     }
 }
 
@@ -496,7 +523,7 @@ struct TileWalk {
 
 template <int BN, int STAGES, int MODE, bool HALF>
 __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__restrict__ Aimg, const Batch B, const TileWalk walk,
-                                                               int M, int K, int N, int *__restrict__ status, const PagedAppendArgs pa) {
+                                                               int M, int K, int N, int *__restrict__ status, const PagedAppendArgs pa, int pdl) {
     constexpr int W_TILE_FLOATS = BN * BK * 2;
     constexpr uint32_t W_TILE_BYTES = W_TILE_FLOATS * 4, STAGE_BYTES = A_TILE_BYTES + W_TILE_BYTES;
     constexpr uint32_t IDESC = instr_desc<BN, HALF>();
@@ -524,6 +551,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
+    if (pdl) griddep_wait();  // what lies above runs beside the launch in front
 
     if (warp == 0) {
         if (lane == 0) {
@@ -803,14 +831,65 @@ static int sm_count_of_current_device() {
 
 template <int BN, int STAGES, int MODE, bool HALF = false>
 static int32_t launch_t(const TileWalk &walk, const float *Aimg, const Batch &b, int M, int K, int N, int *d_status, cudaStream_t st,
-                        const PagedAppendArgs &pa = PagedAppendArgs()) {
+                        const PagedAppendArgs &pa = PagedAppendArgs(), int pdl = 0) {
     constexpr uint32_t smem = smem_bytes<BN, STAGES>();
-    JGPT_CUDA_TRY(cudaFuncSetAttribute(gemm_umma_kernel<BN, STAGES, MODE, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static thread_local int set_for = -1;  // the opt-in to more than 48 KiB, once per device
+    int dev = 0;
+    JGPT_CUDA_TRY(cudaGetDevice(&dev));
+    if (set_for != dev) {
+        JGPT_CUDA_TRY(cudaFuncSetAttribute(gemm_umma_kernel<BN, STAGES, MODE, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        set_for = dev;
+    }
     const int grid = walk.total < sm_count_of_current_device() ? walk.total : sm_count_of_current_device();
-    gemm_umma_kernel<BN, STAGES, MODE, HALF><<<grid, THREADS, smem, st>>>(Aimg, b, walk, M, K, N, d_status, pa);
-    JGPT_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = pdl ? 1 : 0;
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_umma_kernel<BN, STAGES, MODE, HALF>, Aimg, b, walk, M, K, N, d_status, pa, pdl));
     return JGPT_OK;
 }
+
+// Columns per CTA of a product on its own: the fewest rounds of CTAs times what a tile takes, its columns and about 64 more for its
+// share of A and its start; the widest of equals.  Against three launches (an image each, then tiles of 192 or 256), us per call of 400 in a
+// row and alone: 3000 x 384 x 768 (144 tiles of 128 in place of 72 of 256) 35.6 -> 24.4 and 46 -> 37, 600 x 256 x 300 26.7 -> 14.4 and
+// 37 -> 29, 1500 x 2048 x 2048 alone 99 -> 91.  Replayed from a graph the first takes 16.0 -> 15.9: there the operand bytes that leave L2
+// bound it (eight per element and tile, 110 MB in 144 tiles, 83 MB in 72).
+static int matmul_cols(int M, int N, int sms) {
+    const long long rows = (M + BM - 1) / BM;
+    int best = 0;
+    long long least = 0;
+    for (int bn : {256, 192, 128, 64}) {
+        const long long cost = (rows * ((N + bn - 1) / bn) + sms - 1) / sms * (bn + 64);
+        if (!best || cost < least) best = bn, least = cost;
+    }
+    return best;
+}
+uint64_t matmul_scratch_floats(int M, int K, int N) {
+    return activation_image_floats(M, K) + image_floats(N, K, matmul_cols(M, N, sm_count_of_current_device()));
+}
+int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, float *scratch, int *d_status, cudaStream_t st) {
+    JGPT_REQUIRE(shape_ok(K, N) && M > 0, JGPT_ERR_INVALID_ARGUMENT, "matmul: unsupported shape M=%d K=%d N=%d", M, K, N);
+    float *wimg = scratch + activation_image_floats(M, K);
+    Batch b{};
+    b.Wimg[0] = wimg, b.C[0] = C, b.R[0] = nullptr;
+    auto run = [&](auto cols, auto stages) -> int32_t {
+        constexpr int BN = decltype(cols)::value, ST = decltype(stages)::value;
+        const int a_tiles = (M + BM - 1) / BM;
+        TileWalk walk{(N + BN - 1) / BN, 1, 0};
+        walk.total = walk.n_tiles_n * a_tiles;
+        pack_both_kernel<BN><<<(unsigned)(K / BK * (a_tiles + walk.n_tiles_n)), 256, 0, st>>>(A, M, B, N, K, scratch, wimg, a_tiles);
+        JGPT_CUDA_TRY(cudaGetLastError());
+        return launch_t<BN, ST, 0, false>(walk, scratch, b, M, K, N, d_status, st, PagedAppendArgs(), 1);
+    };
+    switch (matmul_cols(M, N, sm_count_of_current_device())) {
+        case 64: return run(std::integral_constant<int, 64>(), std::integral_constant<int, 8>());
+        case 128: return run(std::integral_constant<int, 128>(), std::integral_constant<int, 6>());
+        case 192: return run(std::integral_constant<int, 192>(), std::integral_constant<int, 5>());
+        default: return run(std::integral_constant<int, 256>(), std::integral_constant<int, 4>());
+    }
+}
+
 
 template <bool HALF>
 static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {

@@ -41,6 +41,9 @@ struct Batch {
 };
 // C_z[M, N] = A . W_z (+ R_z) for z < nb; needs K % 16 == 0 and N % 4 == 0.
 int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
+// C[M, N] = A[M, K] . B[K, N], all row major: two launches, the operands' images in scratch.
+uint64_t matmul_scratch_floats(int M, int K, int N);
+int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, float *scratch, int *d_status, cudaStream_t st);
 // act = (A . W1) * silu(A . W3), written as the activation image [M, F] of the next product.
 int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, int F, float *act_image, int *d_status,
                       cudaStream_t st);

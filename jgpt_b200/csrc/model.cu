@@ -1591,20 +1591,14 @@ int32_t jgpt_matmul_device(jgpt_ctx ctxh, const float *a_dev, const float *b_dev
     cudaStream_t st = c->stream;
     // Both images in one allocation of the context's pool, which keeps up to kScratchKept bytes over synchronisations: the device's
     // default pool hands everything back at every one, and mapping it anew took 0.48 ms of a 17 us product called on its own.
-    float *aimg = nullptr;
-    const uint64_t a_floats = umma::activation_image_floats(M, K);
-    const cudaError_t e = scratch_alloc(c, sizeof(float) * (a_floats + umma::weight_image_floats(K, N)), &aimg);
+    float *scratch = nullptr;
+    const cudaError_t e = scratch_alloc(c, sizeof(float) * umma::matmul_scratch_floats(M, K, N), &scratch);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(JGPT_ERR_OUT_OF_MEMORY, "matmul scratch: %s", cudaGetErrorString(e));
     }
-    float *wimg = aimg + a_floats;
-    umma::Batch b{};
-    b.Wimg[0] = wimg, b.C[0] = c_dev, b.R[0] = nullptr;
-    int32_t rc = umma::pack_weight(b_dev, K, N, wimg, st);
-    if (!rc) rc = umma::pack_activations(a_dev, nullptr, M, K, aimg, st);
-    if (!rc) rc = umma::launch(aimg, b, 1, M, K, N, c->d_status, st);
-    cudaFreeAsync(aimg, st);
+    const int32_t rc = umma::matmul(a_dev, b_dev, c_dev, M, K, N, scratch, c->d_status, st);
+    cudaFreeAsync(scratch, st);
     return rc;
 }
 

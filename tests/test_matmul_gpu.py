@@ -80,6 +80,15 @@ def test_tcgen05_path_matches_float64_and_the_mma_sync_path(ctx, M, K, N):
     assert np.abs(small - ref).max() <= tol_mma_sync(K) * scale
 
 
+@pytest.mark.parametrize("M,K,N", [(3000, 16, 768), (2561, 112, 700), (9472, 48, 384), (9345, 96, 380), (600, 144, 68), (18816, 16, 252)])
+def test_tile_widths_of_a_product_on_its_own(ctx, M, K, N):
+    """Tiles of 128, 192, 64 and 256 columns, with and without ragged edges; rings that wrap and rings that are not filled."""
+    rng = np.random.default_rng(M + K + N)
+    a, b = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((K, N), dtype=np.float32)
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    assert np.abs(_matmul(ctx, a, b, 513) - ref).max() <= tol_tcgen05(K) * np.abs(ref).max()
+
+
 def test_operand_layout_is_exact_on_integers(ctx):
     """Small integers are exact in TF32, so any mistake in the operand images or the accumulator read-back
     shows as a wrong integer: C[m, n] = sum_k (m + k) * (k == n mod K ? 1 : 0) style selector product."""
