@@ -84,8 +84,10 @@ __device__ __forceinline__ float reduce32(float (&v)[32], int lane) {
     return v[0];
 }
 
+// A chain of dependent reads, shuffles and barriers: it wants resident warps.  Three CTAs of 256 threads per SM (80 registers, 32 bytes spilled;
+// with 92 registers there were two): 6200 rows of 16 heads of 128 in 262 us, 315 before; four CTAs (64 registers) take as long as three.
 template <class AT, int KIND, int DK>
-__global__ void __launch_bounds__(256) rec_prep_kernel(const RecArgs a, const Seg *__restrict__ segs, const int2 *__restrict__ chunks, int pdl) {
+__global__ void __launch_bounds__(256, DK <= 128 ? 3 : 2) rec_prep_kernel(const RecArgs a, const Seg *__restrict__ segs, const int2 *__restrict__ chunks, int pdl) {
     constexpr int NI = DK / 32;
     extern __shared__ __align__(16) float prep_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, DV = a.DV;
