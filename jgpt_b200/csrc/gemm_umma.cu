@@ -317,8 +317,10 @@ __global__ void __launch_bounds__(256) pair_scale_kernel(const float *W1, const 
 // between the sum of squares and the product.
 constexpr int kKept = 16;
 __global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, const float *__restrict__ r, int M, int D, float eps,
-                                                                uint8_t *__restrict__ image, float *__restrict__ a_un) {
+                                                                uint8_t *__restrict__ image, float *__restrict__ a_un, int pdl) {
     extern __shared__ __align__(16) float rp_rows[];  // [8][D + 4]
+    if (pdl & 2) griddep_launch_dependents();
+    if (pdl & 1) griddep_wait();
     const int tid = threadIdx.x, rr = tid >> 5, lane = tid & 31;
     const int row = blockIdx.x * 8 + rr;
     const int stride = D + 4;
@@ -433,12 +435,16 @@ int32_t pair_scales(const float *W1, const float *W3, const float *gamma, int K,
     JGPT_CUDA_TRY(cudaGetLastError());
     return JGPT_OK;
 }
-int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st) {
+int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st, int pdl) {
     const size_t smem = sizeof(float) * 8 * (size_t)(D + 4);
     JGPT_REQUIRE(D % HBK == 0 && smem <= 48 * 1024, JGPT_ERR_UNSUPPORTED, "rmsnorm_pack_half: d_model %d", D);
     const int padded_rows = (M + BM - 1) / BM * BM;  // rows past M are written as zeros
-    rmsnorm_pack_half_kernel<<<padded_rows / 8, 256, smem, st>>>(x, r, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un);
-    JGPT_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)(padded_rows / 8)), cfg.blockDim = dim3(256), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = pdl & 1;
+    JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_pack_half_kernel, x, r, M, D, eps, reinterpret_cast<uint8_t *>(image), a_un, pdl));
     return JGPT_OK;
 }
 
@@ -538,6 +544,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nkt = K / KT;
+    if (pdl & 2) griddep_launch_dependents();
     uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(umma_smem_raw) + 127) & ~(uintptr_t)127);
 
     if (tid == 0) {
@@ -551,7 +558,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
-    if (pdl) griddep_wait();  // what lies above runs beside the launch in front
+    if (pdl & 1) griddep_wait();  // what lies above runs beside the launch in front
 
     if (warp == 0) {
         if (lane == 0) {
@@ -845,7 +852,7 @@ static int32_t launch_t(const TileWalk &walk, const float *Aimg, const Batch &b,
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = pdl ? 1 : 0;
+    cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = pdl & 1;
     JGPT_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_umma_kernel<BN, STAGES, MODE, HALF>, Aimg, b, walk, M, K, N, d_status, pa, pdl));
     return JGPT_OK;
 }
@@ -892,7 +899,7 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
 
 
 template <bool HALF>
-static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
+static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st, int pdl = 0) {
     JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && nb >= 1 && nb <= 3, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma: unsupported shape M=%d K=%d N=%d", M, K, N);
     const int bn = tile_cols(N);
@@ -901,51 +908,52 @@ static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int
     bool residual = b.R[0] != nullptr;
     for (int z = 0; z < nb; z++)
         JGPT_REQUIRE((b.R[z] != nullptr) == residual, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma: residuals for all products of a batch or for none");
+    const PagedAppendArgs none{};
     if (bn == 256)
-        return residual ? launch_t<256, 4, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<256, 4, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st);
-    return residual ? launch_t<192, 5, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st) : launch_t<192, 5, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st);
+        return residual ? launch_t<256, 4, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl) : launch_t<256, 4, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
+    return residual ? launch_t<192, 5, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl) : launch_t<192, 5, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
 }
 int32_t launch(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
     return launch_rows<false>(Aimg, b, nb, M, K, N, d_status, st);
 }
-int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st) {
-    return launch_rows<true>(Aimg, b, nb, M, K, N, d_status, st);
+int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st, int pdl) {
+    return launch_rows<true>(Aimg, b, nb, M, K, N, d_status, st, pdl);
 }
 
 template <bool HALF>
-static int32_t launch_qkv(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
+static int32_t launch_qkv(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st, int pdl = 0) {
     JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && N == pa.H * 16, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma qkv: unsupported shape M=%d K=%d N=%d (heads %d, d_head 16)", M, K, N, pa.H);
     const int bn = tile_cols(N);
     TileWalk walk{(N + bn - 1) / bn, 3, 0};
     walk.total = walk.n_tiles_n * 3 * ((M + BM - 1) / BM);
-    if (bn == 256) return launch_t<256, 4, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa);
-    return launch_t<192, 5, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa);
+    if (bn == 256) return launch_t<256, 4, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
+    return launch_t<192, 5, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
 }
 int32_t launch_qkv_paged(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
     return launch_qkv<false>(Aimg, b, M, K, N, pa, d_status, st);
 }
-int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st) {
-    return launch_qkv<true>(Aimg, b, M, K, N, pa, d_status, st);
+int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st, int pdl) {
+    return launch_qkv<true>(Aimg, b, M, K, N, pa, d_status, st, pdl);
 }
 
 template <bool HALF>
 static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
-                           int *d_status, cudaStream_t st) {
+                           int *d_status, cudaStream_t st, int pdl = 0) {
     JGPT_REQUIRE(swiglu_shape_ok(K, F) && (!HALF || K % HBK == 0) && M > 0, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
     Batch b{};
     b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un, b.r_up = a_un + M, b.c_up = c_up;
     TileWalk walk{F / 128, 1, 0};
     walk.total = walk.n_tiles_n * ((M + BM - 1) / BM);
-    return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st);
+    return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st, PagedAppendArgs(), pdl);
 }
 int32_t launch_swiglu(const float *Aimg, const float *Wpair_img, int M, int K, int F, float *act_image, int *d_status, cudaStream_t st) {
     return launch_pair<false>(Aimg, Wpair_img, nullptr, nullptr, M, K, F, act_image, d_status, st);
 }
 int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
-                           int *d_status, cudaStream_t st) {
-    return launch_pair<true>(Aimg, Wpair_img, a_un, c_up, M, K, F, act_image, d_status, st);
+                           int *d_status, cudaStream_t st, int pdl) {
+    return launch_pair<true>(Aimg, Wpair_img, a_un, c_up, M, K, F, act_image, d_status, st, pdl);
 }
 
 }  // namespace umma

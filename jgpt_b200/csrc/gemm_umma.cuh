@@ -82,12 +82,13 @@ inline uint64_t pair_scale_floats(int K, int F) { return (uint64_t)F + 3 * (uint
 int32_t pair_scales(const float *W1, const float *W3, const float *gamma, int K, int F, float *scale, cudaStream_t st);
 // RMSNorm into an fp16 image, its weights being in the next product's; a_un[M] receives the rows' factors.  With the weights r of a pair's
 // elements a_un[M .. 2 M) and [2 M .. 3 M) receive the power of two of the row's SwiGLU result and its inverse.
-int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st);
-int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st);
+int32_t rmsnorm_pack_half(const float *x, const float *r, int M, int D, float eps, float *image, float *a_un, cudaStream_t st, int pdl = 0);
+// pdl, of the fp16 forms: bit 0 = the launch may start early and waits itself; bit 1 = it lets the next launch in.
+int32_t launch_half(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st, int pdl = 0);
 // a_un: the rows' factors as rmsnorm_pack_half leaves them; c_up[F]: the powers of two of the result's columns in its image.
 int32_t launch_swiglu_half(const float *Aimg, const float *Wpair_img, const float *a_un, const float *c_up, int M, int K, int F, float *act_image,
-                           int *d_status, cudaStream_t st);
-int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st);
+                           int *d_status, cudaStream_t st, int pdl = 0);
+int32_t launch_qkv_paged_half(const float *Aimg, const Batch &b, int M, int K, int N, const PagedAppendArgs &pa, int *d_status, cudaStream_t st, int pdl = 0);
 
 inline bool shape_ok(int K, int N) { return K >= BK && K % BK == 0 && N % 4 == 0; }
 inline bool swiglu_shape_ok(int K, int F) { return K >= BK && K % BK == 0 && F % 128 == 0; }

@@ -941,6 +941,8 @@ static int32_t half_layer(Model *m, const LayerW &y, HalfLayer *o) {
     return JGPT_OK;
 }
 
+static int step_overlap_level(const Model *m, int rows);
+
 // The decoder blocks for prefill-sized `rows` of a d_head-16 model on fp16 operand images: every activation is handed from producer to
 // consumer as an image (RMSNorm, attention, the W1/W3 product's SwiGLU epilogue), and the Q,K,V product writes K / V straight into
 // the paged store (paged->layer is set per layer here).
@@ -954,6 +956,9 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
     if (rc) return rc;
     if ((rc = ensure_image(m, &m->aimg2, &m->aimg2_floats, umma::half_activation_floats(rows, F)))) return rc;
     float *a_un = m->aimg + image;
+    // Every launch moves in under the one in front of it: set-up, tensor memory and the first waits are out of the way when its rows are there.  Us per
+    // call without and with: three prompts of up to 400 tokens 1361 -> 1240, 12 of up to 500 1783 -> 1636, 32 of 1024 7722 -> 7660.
+    const int pdl = step_overlap_level(m, rows) >= 3 ? 3 : 0;
     for (int l = 0; l < m->layers; l++) {
         const LayerW &y = m->L[(size_t)l];
         HalfLayer w;
@@ -963,15 +968,15 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
         qkv.C[0] = m->q, qkv.C[1] = m->k, qkv.C[2] = m->v, qkv.a_un = a_un;
         wo.Wimg[0] = w.wo, wo.C[0] = m->x, wo.R[0] = m->x;  // x1 = x + attn.Wo (each element read then written by the same thread)
         w2.Wimg[0] = w.w2, w2.C[0] = m->x, w2.R[0] = m->x, w2.a_un = a_un + 2 * (size_t)rows;
-        if ((rc = umma::rmsnorm_pack_half(m->x, nullptr, rows, D, m->eps, m->aimg, a_un, st))) return rc;
+        if ((rc = umma::rmsnorm_pack_half(m->x, nullptr, rows, D, m->eps, m->aimg, a_un, st, pdl))) return rc;
         PagedAppendArgs pa = paged;
         pa.layer = l;
-        if ((rc = umma::launch_qkv_paged_half(m->aimg, qkv, rows, D, D, pa, status, st))) return rc;
+        if ((rc = umma::launch_qkv_paged_half(m->aimg, qkv, rows, D, D, pa, status, st, pdl))) return rc;
         if ((rc = attn(l, umma::ImageOut{m->aimg, w.att_scale}, true))) return rc;
-        if ((rc = umma::launch_half(m->aimg, wo, 1, rows, D, D, status, st))) return rc;
-        if ((rc = umma::rmsnorm_pack_half(m->x, w.h_scale + F, rows, D, m->eps, m->aimg, a_un, st))) return rc;
-        if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, w.h_scale, rows, D, F, m->aimg2, status, st))) return rc;
-        if ((rc = umma::launch_half(m->aimg2, w2, 1, rows, F, D, status, st))) return rc;
+        if ((rc = umma::launch_half(m->aimg, wo, 1, rows, D, D, status, st, pdl))) return rc;
+        if ((rc = umma::rmsnorm_pack_half(m->x, w.h_scale + F, rows, D, m->eps, m->aimg, a_un, st, pdl))) return rc;
+        if ((rc = umma::launch_swiglu_half(m->aimg, w.pair, a_un, w.h_scale, rows, D, F, m->aimg2, status, st, pdl))) return rc;
+        if ((rc = umma::launch_half(m->aimg2, w2, 1, rows, F, D, status, st, pdl))) return rc;
     }
     return JGPT_OK;
 }
@@ -1939,7 +1944,8 @@ int32_t jgpt_forward_prefill_batch(jgpt_model h, jgpt_kvpool poolh, const int32_
     const bool early = rows_mode(m, rows) && step_overlap_level(m, rows) >= 3;
     m->first_launch_early = early;
     rc = run_layers(m, rows, paged, [&](int l, umma::ImageOut out, bool kv_in_cache) {
-        return launch_attn_prefill(p, l, m->q, m->k, m->v, n, max_S, n_rows, m->att, out.image, out.scale, kv_in_cache, m->prefill_fast, early);
+        const bool chained = out.scale && step_overlap_level(m, rows) >= 3;  // between the products on fp16 images
+        return launch_attn_prefill(p, l, m->q, m->k, m->v, n, max_S, n_rows, m->att, out.image, out.scale, kv_in_cache, m->prefill_fast, early || chained);
     });
     m->first_launch_early = false;
     if (rc) return rc;
