@@ -525,6 +525,7 @@ constexpr uint32_t smem_bytes() { return (uint32_t)STAGES * (A_TILE_BYTES + (uin
 
 struct TileWalk {
     int n_tiles_n, nb, total;  // tiles along N, products in the batch, total tiles
+    int image_cols;            // rows of a tile of the weight image; BN or a multiple of it
 };
 
 template <int BN, int STAGES, int MODE, bool HALF>
@@ -566,15 +567,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
             for (int t = blockIdx.x; t < walk.total && !*s_abort; t += gridDim.x) {
                 const int n_idx = t % walk.n_tiles_n, z = (t / walk.n_tiles_n) % walk.nb, m_idx = t / (walk.n_tiles_n * walk.nb);
                 const float *__restrict__ a_src = Aimg + (size_t)m_idx * nkt * A_TILE_FLOATS;
-                const float *__restrict__ w_src =
-                    (z == 0 ? B.Wimg[0] : (z == 1 ? B.Wimg[1] : B.Wimg[2])) + (size_t)n_idx * nkt * W_TILE_FLOATS;
+                // BN rows of an image tile: its row groups of eight lie one after the other, in the high and in the low half
+                const int wt = walk.image_cols, w_tile = n_idx * BN / wt, w_floats = wt * BK * 2;
+                const float *__restrict__ w_src = (z == 0 ? B.Wimg[0] : (z == 1 ? B.Wimg[1] : B.Wimg[2])) + (size_t)w_tile * nkt * w_floats +
+                                                  (n_idx * BN - w_tile * wt) / 8 * 128;
                 for (int kt = 0; kt < nkt; kt++, it++) {
                     const uint32_t s = it % STAGES, use = it / STAGES;
                     if (use > 0 && !mbar_wait_bounded(&empty_bar[s], (use - 1) & 1u, status, s_abort)) break;
                     uint8_t *dst = tiles + (size_t)s * STAGE_BYTES;
                     mbar_expect_tx(&full_bar[s], STAGE_BYTES);
                     bulk_g2s(dst, a_src + (size_t)kt * A_TILE_FLOATS, A_TILE_BYTES, &full_bar[s]);
-                    bulk_g2s(dst + A_TILE_BYTES, w_src + (size_t)kt * W_TILE_FLOATS, W_TILE_BYTES, &full_bar[s]);
+                    if (wt == BN) {
+                        bulk_g2s(dst + A_TILE_BYTES, w_src + (size_t)kt * W_TILE_FLOATS, W_TILE_BYTES, &full_bar[s]);
+                    } else {
+                        bulk_g2s(dst + A_TILE_BYTES, w_src + (size_t)kt * w_floats, W_TILE_BYTES / 2, &full_bar[s]);
+                        bulk_g2s(dst + A_TILE_BYTES + W_TILE_BYTES / 2, w_src + (size_t)kt * w_floats + w_floats / 2, W_TILE_BYTES / 2, &full_bar[s]);
+                    }
                 }
             }
             if (*s_abort) {
@@ -652,7 +660,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_umma_kernel(const float *__re
             // fp16 images: the factors that undo the operands' powers of two
             const float a_un = (HALF && B.a_un && m < M) ? B.a_un[m] : 1.f;
             const float *w_un = HALF ? (z == 0 ? B.Wimg[0] : (z == 1 ? B.Wimg[1] : B.Wimg[2])) +
-                                           (size_t)walk.n_tiles_n * nkt * W_TILE_FLOATS + (size_t)n_idx * BN
+                                           (size_t)((walk.n_tiles_n * BN + walk.image_cols - 1) / walk.image_cols) * nkt * (walk.image_cols * BK * 2) + (size_t)n_idx * BN
                                      : nullptr;
             auto unscale = [&](float (&v)[32], int c) {  // 32 columns of the tile from c on
                 if constexpr (HALF) {
@@ -883,7 +891,7 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
     auto run = [&](auto cols, auto stages) -> int32_t {
         constexpr int BN = decltype(cols)::value, ST = decltype(stages)::value;
         const int a_tiles = (M + BM - 1) / BM;
-        TileWalk walk{(N + BN - 1) / BN, 1, 0};
+        TileWalk walk{(N + BN - 1) / BN, 1, 0, BN};
         walk.total = walk.n_tiles_n * a_tiles;
         pack_both_kernel<BN><<<(unsigned)(K / BK * (a_tiles + walk.n_tiles_n)), 256, 0, st>>>(A, M, B, N, K, scratch, wimg, a_tiles);
         JGPT_CUDA_TRY(cudaGetLastError());
@@ -898,17 +906,30 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
 }
 
 
+// Fewer rows than the image's tiles fill SMs with: 64 columns per CTA where that takes fewer rounds of CTAs times what a tile takes.
+// (900 rows of width 384 are 16 tiles of Wo and of W2 and 48 of Q,K,V on 148 SMs, three times as many of 64: the prefill 1240 -> 1044 us, 700
+// rows 1377 -> 1024 with the early launches, 4500 rows 1636 -> 1630.)
+static bool narrow_tiles(TileWalk &walk, int N, int M) {
+    const int sms = sm_count_of_current_device(), tiles = (N + 63) / 64 * walk.nb * ((M + BM - 1) / BM);
+    if ((tiles + sms - 1) / sms * (64 + 64) >= (walk.total + sms - 1) / sms * (walk.image_cols + 64)) return false;
+    walk.n_tiles_n = (N + 63) / 64, walk.total = tiles;
+    return true;
+}
+
 template <bool HALF>
 static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int K, int N, int *d_status, cudaStream_t st, int pdl = 0) {
     JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && nb >= 1 && nb <= 3, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma: unsupported shape M=%d K=%d N=%d", M, K, N);
     const int bn = tile_cols(N);
-    TileWalk walk{(N + bn - 1) / bn, nb, 0};
+    TileWalk walk{(N + bn - 1) / bn, nb, 0, bn};
     walk.total = walk.n_tiles_n * nb * ((M + BM - 1) / BM);
     bool residual = b.R[0] != nullptr;
     for (int z = 0; z < nb; z++)
         JGPT_REQUIRE((b.R[z] != nullptr) == residual, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma: residuals for all products of a batch or for none");
     const PagedAppendArgs none{};
+    if constexpr (HALF) {
+        if (residual && narrow_tiles(walk, N, M)) return launch_t<64, 8, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
+    }
     if (bn == 256)
         return residual ? launch_t<256, 4, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl) : launch_t<256, 4, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
     return residual ? launch_t<192, 5, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl) : launch_t<192, 5, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
@@ -925,8 +946,11 @@ static int32_t launch_qkv(const float *Aimg, const Batch &b, int M, int K, int N
     JGPT_REQUIRE(shape_ok(K, N) && (!HALF || K % HBK == 0) && M > 0 && N == pa.H * 16, JGPT_ERR_INVALID_ARGUMENT,
                  "gemm_umma qkv: unsupported shape M=%d K=%d N=%d (heads %d, d_head 16)", M, K, N, pa.H);
     const int bn = tile_cols(N);
-    TileWalk walk{(N + bn - 1) / bn, 3, 0};
+    TileWalk walk{(N + bn - 1) / bn, 3, 0, bn};
     walk.total = walk.n_tiles_n * 3 * ((M + BM - 1) / BM);
+    if constexpr (HALF) {
+        if (narrow_tiles(walk, N, M)) return launch_t<64, 8, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
+    }
     if (bn == 256) return launch_t<256, 4, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
     return launch_t<192, 5, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
 }
@@ -944,7 +968,7 @@ static int32_t launch_pair(const float *Aimg, const float *Wpair_img, const floa
                  "gemm_umma swiglu: unsupported shape M=%d K=%d F=%d", M, K, F);
     Batch b{};
     b.Wimg[0] = Wpair_img, b.C[0] = act_image, b.a_un = a_un, b.r_up = a_un + M, b.c_up = c_up;
-    TileWalk walk{F / 128, 1, 0};
+    TileWalk walk{F / 128, 1, 0, 256};
     walk.total = walk.n_tiles_n * ((M + BM - 1) / BM);
     return launch_t<256, 4, 1, HALF>(walk, Aimg, b, M, K, F, d_status, st, PagedAppendArgs(), pdl);
 }
