@@ -314,9 +314,10 @@ __global__ void __launch_bounds__(256) pair_scale_kernel(const float *W1, const 
     scale[n] = pow2(half_exponent(sqrt(a) * sqrt(b), 113));
 }
 // RMSNorm, without its weights, of 8 rows per CTA like rmsnorm_pack_kernel, a warp per row; up to kKept elements per lane stay in registers
-// between the sum of squares and the product.
+// between the sum of squares and the product.  x is a plain pointer: the launch in front still writes it while this one is resident, and
+// const __restrict__ would promise that nobody does.
 constexpr int kKept = 16;
-__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *__restrict__ x, const float *__restrict__ r, int M, int D, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_pack_half_kernel(const float *x, const float *__restrict__ r, int M, int D, float eps,
                                                                 uint8_t *__restrict__ image, float *__restrict__ a_un, int pdl) {
     extern __shared__ __align__(16) float rp_rows[];  // [8][D + 4]
     if (pdl & 2) griddep_launch_dependents();

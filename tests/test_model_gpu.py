@@ -703,6 +703,40 @@ def test_overlapped_launches_inside_the_decode_step_change_nothing(ctx, level, m
     assert np.array_equal(k0, k1) and np.array_equal(v0, v1)
 
 
+@pytest.mark.parametrize("dm,dff", [(64, 128), (384, 768), (768, 256)])
+def test_overlapped_launches_of_a_prefill_on_fp16_images_change_nothing(ctx, dm, dff, monkeypatch):
+    """JGPT_B200_STEP_OVERLAP of a ragged prefill of more than 512 rows, four layers with both parts live: each norm's rows change with the
+    product in front of it, so one that read them early would show.  Several passes over the same model and pool."""
+    V, MS, H, L = 100, 160, dm // 16, 4
+    om = O.Model(V, MS, dm, H, L, dff, eps=1e-5).init_random(seed=dm, std=0.1)
+    lens = [160, 1, 129, 77, 160, 16, 33, 128, 2]
+    prompts = [np.array([(5 * i + 11 * s) % V for i in range(n)], np.int32) for s, n in enumerate(lens)]
+    assert sum(lens) > 512
+    outs = []
+    for level in (0, 3, 2):
+        monkeypatch.setenv("JGPT_B200_STEP_OVERLAP", str(level))
+        gm = GPTModel(ctx, V, MS, dm, H, L, dff, rmsNormEps=1e-5, maxRows=sum(lens))
+        gm.setParameters(om.tensors())
+        pool = gm.newPool(len(lens) * MS // 16, len(lens))
+        try:
+            for _ in range(4 if level == 3 else 1):
+                seqs = [pool.seq_alloc() for _ in lens]
+                logits, _ = gm.forwardPrefillBatch(pool, seqs, prompts)
+                kd, vd = ctx.alloc((H, MS, 16)), ctx.alloc((H, MS, 16))
+                cache = []
+                for layer in range(L):
+                    pool.gather(layer, seqs[4], MS, MS, kd, vd)
+                    cache += [kd.to_host(), vd.to_host()]
+                outs.append([logits.copy(), *cache])
+                for s in seqs:
+                    pool.seq_free(s)
+        finally:
+            pool.close(), gm.close()
+    om.close()
+    for o in outs[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, outs[0]))
+
+
 @pytest.mark.parametrize("dm,heads,dff", [(256, 16, 512), (320, 20, 448)])
 def test_resident_weight_slices_and_split_k_pairs(ctx, monkeypatch, dm, heads, dff):
     """Two launch forms of the decode step's projections.  JGPT_B200_W_RESIDENT: a CTA keeps its whole weight slice in
