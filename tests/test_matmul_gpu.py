@@ -259,17 +259,17 @@ def test_ragged_batched_prefill_on_the_tcgen05_path(ctx):
         pool.close(), gm.close(), om.close()
 
 
-@pytest.mark.parametrize("dm,dff", [(64, 128), (96, 256), (384, 768), (256, 384)])
+@pytest.mark.parametrize("dm,dff,n", [(64, 128, 600), (96, 256, 600), (384, 768, 600), (256, 384, 600), (384, 768, 3500), (768, 256, 3500)])
 @pytest.mark.parametrize("part", ["attention", "feed forward"])
 @pytest.mark.parametrize("spread", [0.0, 3.0])
-def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, part, spread):
-    """600 prompts of one token (a ragged last row tile) through one block with one of its parts switched off, on the fp16 operand images:
-    a token that sees itself alone has its own value as attention output.  spread: rows, and columns of the weights in front of a
+def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, n, part, spread):
+    """600 prompts of one token (a ragged last row tile; tiles of 64 columns) or 3500 (tiles of 192 and of 256) through one block with one of
+    its parts switched off, on the fp16 operand images: a token that sees itself alone has its own value as attention output.  spread: rows, and columns of the weights in front of a
     part with the inverse behind it, scaled by up to 10^spread either way, which fp16 parts survive only with their powers of two.
 
     Tolerance: operands of 22 bits and fewer than 128 fp32 additions of parts no larger than sum |x w| keep a product within
     2 * 2^-22 + 128 * 2^-24 < 1e-5 of sum |x w|; a value is rounded to fp16 (2^-11); what reaches the last norm is relative to its row."""
-    V, n = 132, 600
+    V = 132
     rng = np.random.default_rng(dm + dff)
 
     def scales(k):
@@ -320,13 +320,43 @@ def test_prefill_on_fp16_images_against_float64(ctx, dm, dff, part, spread):
         pool.close(), gm.close()
 
 
-@pytest.mark.parametrize("dm,dff", [(64, 128), (384, 768), (768, 256)])
-def test_prefill_on_fp16_images_with_dead_and_extreme_columns(ctx, dm, dff):
+@pytest.mark.parametrize("dm,dff", [(384, 768), (768, 256)])
+def test_prefill_on_fp16_images_gives_the_same_bits_in_tiles_of_any_width(ctx, dm, dff):
+    """The same prompts among 650 rows (tiles of 64 columns) and, beside two long ones, among 3620 (tiles of 192 or 256): no sum changes its
+    order, so logits and cached keys and values are equal."""
+    V, MS, L, H = 100, 1520, 3, dm // 16
+    om = O.Model(V, MS, dm, H, L, dff, eps=1e-5).init_random(seed=dm, std=0.1)
+    rng = np.random.default_rng(dff)
+    shared = [rng.integers(1, V, n).astype(np.int32) for n in (130, 1, 64, 257, 16, 127)]
+    gm = GPTModel(ctx, V, MS, dm, H, L, dff, rmsNormEps=1e-5, maxRows=3700)
+    gm.setParameters(om.tensors())
+    om.close()
+    pool = gm.newPool(300, 8)
+    try:
+        outs = []
+        for others in ((30, 25), (1520, 1505)):
+            seqs = [pool.seq_alloc() for _ in range(8)]
+            logits, _ = gm.forwardPrefillBatch(pool, seqs, shared + [np.arange(n, dtype=np.int32) % V for n in others])
+            kd, vd = ctx.alloc((H, MS, 16)), ctx.alloc((H, MS, 16))
+            outs.append([logits[:6].copy()])
+            for layer in range(L):
+                for s, p in zip(seqs, shared):
+                    pool.gather(layer, s, len(p), MS, kd, vd)
+                    outs[-1] += [kd.to_host(), vd.to_host()]
+            for s in seqs:
+                pool.seq_free(s)
+        assert np.isfinite(outs[0][0]).all() and all(np.array_equal(a, b) for a, b in zip(*outs))
+    finally:
+        pool.close(), gm.close()
+
+
+@pytest.mark.parametrize("dm,dff,n", [(64, 128, 600), (384, 768, 600), (768, 256, 600), (384, 768, 3500), (768, 256, 3500)])
+def test_prefill_on_fp16_images_with_dead_and_extreme_columns(ctx, dm, dff, n):
     """Hidden units whose gate or up column is zero (pruned) or far outside fp16, some with the inverse in W2 so that they count: h alone is
     then far larger than the gated value can be, squares of a column leave fp32, and a unit is worth 1e-24 or 1e20 of its neighbour.
 
     Tolerance: as for the other columns, relative to sum |x w| (22 bits per operand and fewer than 128 fp32 additions)."""
-    V, n, E = 132, 600, 1e-5
+    V, E = 132, 1e-5
     rng = np.random.default_rng(dm)
 
     def mat(a, b):
