@@ -88,6 +88,57 @@ def test_products_of_few_rows(ctx, width, ff, vocab):
     pool.close(), m.close()
 
 
+@pytest.mark.parametrize("width,vocab,parts", [(264, 100, 1), (264, 4736, 1), (520, 256, 2), (520, 2304, 2), (1160, 33, 4), (2312, 100, 8)])
+def test_order_of_sums_in_products_of_few_rows(ctx, width, vocab, parts):
+    """Both kernels for bf16 products of a few rows add in one order, so tokens do not depend on which of them ran: 16 of every 128 k to a warp,
+    k tiles cut into parts, within a part warp after warp, then part after part.  Here a warp has one product per part, all else being zero, so
+    the order of the float32 additions is all there is, and the logits are those of the same additions on the CPU to the bit.  (Rows from
+    33 on take the kernel of more rows; up to 256 columns its tiles are the same.)"""
+    rng = np.random.default_rng(width + vocab)
+    nk = (width + 127) // 128
+    k = np.empty((vocab, parts, 8), int)
+    for p in range(parts):
+        first, at = p * nk // parts, 16 * np.arange(8) + rng.integers(0, 16, (vocab, 8))
+        tile = rng.integers(first, (p + 1) * nk // parts, (vocab, 8))
+        tile -= tile * 128 + at >= width  # the last tile ends early
+        k[:, p] = np.where(tile >= first, tile * 128 + at, -1)
+
+    def edit(W):
+        W["embed"], W["final.norm"] = rng.choice([-1.0, 1.0], (vocab, width)), np.ones(width)
+        for n in ("norm1b", "norm2b"):  # the layer adds nothing
+            if "l0." + n in W:
+                W["l0." + n] = np.zeros(width)
+        W["head"] = np.zeros((vocab, width))
+        size = rng.choice([-1.0, 1.0], k.shape) * rng.uniform(1, 2, k.shape) * 2.0 ** rng.integers(-20, 21, k.shape)
+        n, p, w = np.nonzero(k >= 0)
+        W["head"][n, k[n, p, w]] = size[n, p, w]
+
+    c = lc.Case(lc.config([lc.gen(heads=1, dim=16)], width=width, vocab=vocab), seed=1, edit=edit)
+    t = rng.permutation(vocab)[:33].astype(np.int32)
+    terms = np.where(k >= 0, np.asarray(c.W["head"], np.float32)[np.arange(vocab)[:, None, None], k], np.float32(0)) * np.asarray(c.W["embed"], np.float32)[t][:, k]
+
+    def added(order, part_order):
+        sums = np.zeros((t.size, vocab), np.float32)
+        for i, p in enumerate(part_order):
+            s = np.zeros_like(sums)
+            for w in order:
+                s = s + terms[:, :, p, w]
+            sums = s if i == 0 else sums + s
+        return sums
+
+    want = added(range(8), range(parts))
+    assert (added(range(7, -1, -1), range(parts)) != want).mean() > 0.1 and (parts < 3 or (added(range(8), range(parts - 1, -1, -1)) != want).mean() > 0.1)
+    m = c.model(ctx, "bfloat16")
+    pool = m.newPool(40, 40)
+    for rows in (1, 15, 16, 17, 32) + ((33,) if vocab <= 256 else ()):
+        seqs = [pool.seq_alloc() for _ in range(rows)]
+        got, _ = m.step(pool, seqs, [t[i:i + 1] for i in range(rows)], range(rows))
+        for s in seqs:
+            pool.seq_free(s)
+        assert np.array_equal(got, want[:rows]), (rows, (got != want[:rows]).mean())
+    pool.close(), m.close()
+
+
 # ---- each mechanism alone ----------------------------------------------------------------------------------
 def _alone(ctx, layers, dtype, sizes=(200, 1, 2, 40, 7, 50), width=64, edit=None, seed=3, tol=0.04):
     """What a layer (the last one) adds to the residual, in portions."""
