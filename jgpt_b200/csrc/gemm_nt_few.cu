@@ -9,7 +9,7 @@
 // every 128 k, the parts into which that kernel would cut k are summed for themselves, warps are added in order, then parts.
 //
 // Against the ring of gemm_nt.cu (128-wide k tiles, a barrier each, parts of k in clusters of up to eight CTAs), layered model of width 1024,
-// prompts and 24 steps: one row 7.18 -> 6.39 ms, 16 rows 8.68 -> 7.78 ms (a step 293 -> 256 us), 30 rows 9.61 -> 8.92 ms.
+// prompts of 200 tokens and 24 steps: one row 6.71 -> 5.95 ms, 16 rows 8.47 -> 7.60, 30 rows 10.34 -> 9.55.
 #include "gemm_nt.cuh"
 
 #include <algorithm>
@@ -178,9 +178,14 @@ static int32_t few_launch(const Problem &p, int parts, int pdl, cudaStream_t st)
 }
 
 // Column tiles of 8 per CTA, 0: not for this kernel.  Tiles as wide as three SMs in four stay busy: every CTA reads all rows.  What a CTA's
-// memory does not hold (two of 112 KB share an SM) streams through the ring, and so do launches whose CTAs would read more than 20 MB of
-// rows together (width 2048, 24 steps and their prompts: four rows 9.60 ms with this line, 9.64 ms all in the ring, 10.54 ms without it; 28
-// rows 12.24, 12.33 and 13.7 ms; 15 rows 10.57, 10.76 and 11.7 ms).
+// memory does not hold (two of 112 KB share an SM) streams through the ring, and so do products of many CTAs with long slices: a CTA that
+// finds no room requests its slice when another leaves, and multiplies nothing until all of it is there, where the ring begins with its
+// first k tile.  Launches by themselves, four rows, us here and in the ring: k 1024, 264 CTAs 5.9 and 7.4; k 1536, 240 CTAs 7.0 and 8.0, 580 CTAs
+// 11.5 and 9.6, 2000 CTAs 29 and 22; k 512, 1000 CTAs (slices of 32 KB, four on an SM) 9.9 and 12.1.  It is not the bytes of the rows that
+// are there: 528 CTAs of k 2048 take 13.7 and 10.6 with four rows, 17.5 and 12.8 with 24.
+// The line itself is tuned, CTAs times k times row tiles.  Prompts of 16 tokens and 24 steps, ms, with it, with two CTAs per SM for a line, with none,
+// all in the ring: width 512, 4 rows 4.72, 5.08, 4.75, 5.53; width 1536, 4 rows 7.40, 7.54, 7.62, 7.76, 17 rows 9.16, 9.14, 9.76, 9.21; width 2048,
+// 4 rows 8.91, 8.92, 9.55, 8.99, 24 rows 11.44, 11.45, 12.94, 11.48; width 1024, 1 to 32 rows, the first three within 1.5 %, the ring 8-14 % more.
 static int few_columns(const Ctx *ctx, const Problem &p, Epilogue epi, int parts) {
     if (p.M > kFewRows || p.grp.tiles) return 0;
     const int nk = few_tiles(p), MT = p.M <= 16 ? 1 : 2;
@@ -190,7 +195,7 @@ static int few_columns(const Ctx *ctx, const Problem &p, Epilogue epi, int parts
     else
         for (int w : {2, 4})
             if (4 * p.column_tiles(8 * w) >= 3 * ctx->sm_count && fits(w)) nt = w;
-    return fits(nt) && 32ll * MT * p.column_tiles(8 * nt) * p.K <= 20000000 ? nt : 0;
+    return fits(nt) && (long long)MT * p.column_tiles(8 * nt) * p.K <= 625000 ? nt : 0;
 }
 
 template <int EPI>
