@@ -867,10 +867,11 @@ static int32_t launch_t(const TileWalk &walk, const float *Aimg, const Batch &b,
 }
 
 // Columns per CTA of a product on its own: the fewest rounds of CTAs times what a tile takes, its columns and about 64 more for its
-// share of A and its start; the widest of equals.  Against three launches (an image each, then tiles of 192 or 256), us per call of 400 in a
-// row and alone: 3000 x 384 x 768 (144 tiles of 128 in place of 72 of 256) 35.6 -> 24.4 and 46 -> 37, 600 x 256 x 300 26.7 -> 14.4 and
-// 37 -> 29, 1500 x 2048 x 2048 alone 99 -> 91.  Replayed from a graph the first takes 16.0 -> 15.9: there the operand bytes that leave L2
-// bound it (eight per element and tile, 110 MB in 144 tiles, 83 MB in 72).
+// share of A and its start; the widest of equals.  Calls in a row with 64, 128, 192 and 256 columns, us, the choice of this rule first:
+// 3000 x 384 x 768 128: 24.6 (30.9, 26.7, 30.8), 1000 x 384 x 768 64: 20.5 (22.6, 24.6, 28.7), 6000 x 1024 x 1024 192: 77 (169, 100, 86),
+// 20000 x 384 x 768 256: 84 (149, 96, 84).  Against three launches (an image each, then tiles of 192 or 256), in a row and alone on operands that
+// have left L2: 3000 x 384 x 768 36.4 -> 24.6 and 54 -> 40, 1500 x 2048 x 2048 88 -> 76 and 107 -> 95.  Replayed from a graph, its launches
+// one behind the other, the first takes 16.2 -> 15.8: more bytes leave L2 (eight per element and tile, 110 MB in 144 tiles, 83 MB in 72).
 static int matmul_cols(int M, int N, int sms) {
     const long long rows = (M + BM - 1) / BM;
     int best = 0;
@@ -906,10 +907,9 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
     }
 }
 
-
-// Fewer rows than the image's tiles fill SMs with: 64 columns per CTA where that takes fewer rounds of CTAs times what a tile takes.
-// (900 rows of width 384 are 16 tiles of Wo and of W2 and 48 of Q,K,V on 148 SMs, three times as many of 64: the prefill 1240 -> 1044 us, 700
-// rows 1377 -> 1024 with the early launches, 4500 rows 1636 -> 1630.)
+// Fewer rows than the image's tiles fill SMs with: 64 columns per CTA where that takes fewer rounds of CTAs times what a tile takes.  At width 384
+// on 148 SMs that is up to 3072 rows for Wo and W2 and up to 1024 for Q,K,V.  (1130 rows are 18 tiles of Wo and of W2, three times as many of
+// 64: 23.9 -> 15.8 us a launch.  With the early launches three prompts of 848 rows take 1339 -> 969 us, three of 1130 1366 -> 1045.)
 static bool narrow_tiles(TileWalk &walk, int N, int M) {
     const int sms = sm_count_of_current_device(), tiles = (N + 63) / 64 * walk.nb * ((M + BM - 1) / BM);
     if ((tiles + sms - 1) / sms * (64 + 64) >= (walk.total + sms - 1) / sms * (walk.image_cols + 64)) return false;

@@ -74,7 +74,9 @@ struct Model {
     bool first_launch_early = false;  // set while a decode step is enqueued: its embedding kernel lets layer 0's Q,K,V product move in early
     int k_split = 1;  // Wo / W2 of a step with few rows as pairs of CTAs that split the k range (JGPT_B200_K_SPLIT=0: off)
     int w_resident = 1;  // projections of the decode step keep their CTA's weight slice in shared memory when the grid allows (JGPT_B200_W_RESIDENT=0: off)
-    int step_overlap = -1;  // programmatic dependent launches inside the decode step (JGPT_B200_STEP_OVERLAP 0..3; -1 = the default, 3)
+    // programmatic dependent launches inside the decode step, and at level 3 in prefills of short prompts or on fp16 images as well
+    // (JGPT_B200_STEP_OVERLAP 0..3; -1 = the default, 3)
+    int step_overlap = -1;
     int prefill_fast = 1;  // single-fp16 q / p operands in the d_head-16 prefill attention (JGPT_B200_PREFILL_EXACT=1: off)
     // Steps of up to four rows as one cooperative launch (decode_fused.cu; JGPT_B200_FUSED_STEP=0: off).  Sized on first use.
     int fused_step = 1;
@@ -957,7 +959,8 @@ static int32_t run_layers_half(Model *m, int rows, const PagedAppendArgs &paged,
     if ((rc = ensure_image(m, &m->aimg2, &m->aimg2_floats, umma::half_activation_floats(rows, F)))) return rc;
     float *a_un = m->aimg + image;
     // Every launch moves in under the one in front of it: set-up, tensor memory and the first waits are out of the way when its rows are there.  Us per
-    // call without and with: three prompts of up to 400 tokens 1361 -> 1240, 12 of up to 500 1783 -> 1636, 32 of 1024 7722 -> 7660.
+    // call without and with: three prompts of up to 400 tokens 1176 -> 1049, 12 of up to 500 1808 -> 1649; of 32 of 1024, 7683 and 7655 with
+    // 1 % between runs, the gaps are too small a part.
     const int pdl = step_overlap_level(m, rows) >= 3 ? 3 : 0;
     for (int l = 0; l < m->layers; l++) {
         const LayerW &y = m->L[(size_t)l];

@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(kNormThreads) part_norm_kernel(const StepDesc 
 int32_t launch_part_norm(bool f32, const StepDesc &d, const RowSource &embed, const PartNorm &p, const int *rowsel, int rows, float eps, int W, int ldw,
                          int sm_count, int *status, int pdl, cudaStream_t st) {
     // Rows per block: the row in front of a block is computed twice, so several; but a block's rows follow one another behind barriers, and
-    // few, longer blocks leave a last wave behind.  Prompts of 6200 rows of 2048 (six layers): one 6.45, two 6.39, three 6.36, five 6.40, seven
-    // 6.51 ms; of 2400 rows of 1024: one 2.135, two 2.107, three 2.104, seven 2.25 ms.
+    // few, longer blocks leave a last wave behind.  Us a launch with one, two, three, four, five and seven: 5932 rows of 2048 37.2, 37.9, 37.1, 41.3,
+    // 39.2, 48.3; 2417 rows of 1024 12.2, 13.7, 11.7, 13.5, 14.9, 18.4.
     const int per = std::max(1, std::min(3, rows / (4 * sm_count)));
     const int nv = (ldw + 4 * kNormThreads - 1) / (4 * kNormThreads);
     JGPT_REQUIRE(nv <= 16, JGPT_ERR_UNSUPPORTED, "width %d", W);
