@@ -180,9 +180,9 @@ static int32_t few_launch(const Problem &p, int parts, int pdl, cudaStream_t st)
 // Column tiles of 8 per CTA, 0: not for this kernel.  Tiles as wide as three SMs in four stay busy: every CTA reads all rows.  What a CTA's
 // memory does not hold (two of 112 KB share an SM) streams through the ring, and so do products of many CTAs with long slices: a CTA that
 // finds no room requests its slice when another leaves, and multiplies nothing until all of it is there, where the ring begins with its
-// first k tile.  Launches by themselves, four rows, us here and in the ring: k 1024, 264 CTAs 5.9 and 7.4; k 1536, 240 CTAs 7.0 and 8.0, 580 CTAs
+// first k tile.  Launches by themselves, four rows, us here and in the ring: k 1024, 264 CTAs 5.9 and 7.5; k 1536, 240 CTAs 7.1 and 7.9, 580 CTAs
 // 11.5 and 9.6, 2000 CTAs 29 and 22; k 512, 1000 CTAs (slices of 32 KB, four on an SM) 9.9 and 12.1.  It is not the bytes of the rows that
-// are there: 528 CTAs of k 2048 take 13.7 and 10.6 with four rows, 17.5 and 12.8 with 24.
+// are there: 528 CTAs of k 2048 take 13.7 and 10.6 with four rows, 17.1 and 12.4 with 24.
 // The line itself is tuned, CTAs times k times row tiles.  Prompts of 16 tokens and 24 steps, ms, with it, with two CTAs per SM for a line, with none,
 // all in the ring: width 512, 4 rows 4.72, 5.08, 4.75, 5.53; width 1536, 4 rows 7.40, 7.54, 7.62, 7.76, 17 rows 9.16, 9.14, 9.76, 9.21; width 2048,
 // 4 rows 8.91, 8.92, 9.55, 8.99, 24 rows 11.44, 11.45, 12.94, 11.48; width 1024, 1 to 32 rows, the first three within 1.5 %, the ring 8-14 % more.
