@@ -84,10 +84,17 @@ __device__ __forceinline__ float reduce32(float (&v)[32], int lane) {
     return v[0];
 }
 
-// A chain of dependent reads, shuffles and barriers: it wants resident warps.  Three CTAs of 256 threads per SM (80 registers, 32 bytes spilled;
-// with 92 registers there were two): 6200 rows of 16 heads of 128 in 262 us, 315 before; four CTAs (64 registers) take as long as three.
+// A chain of dependent reads, shuffles and barriers: it wants resident warps, and registers are what limits them.  CTAs of 256 threads per SM that
+// the registers are held to, 0: left to the compiler.  6144 rows, us a launch in bf16, left and held: general delta rule, 32 heads of 64
+// 445 and 387, 16 of 128 316 and 262; delta rule 379 and 299, 245 and 209; WKV, 16 of 128 166 and 126, 8 of 256 277 and 197.  For short keys of the
+// other three kinds the compiler takes 64 registers, four CTAs, by itself: WKV, HGRN2, gated linear, 64 heads of 32 259, 282 and 261, held to
+// three 320, 414 and 328, 32 of 64 157, 178 and 158, held 191, 217 and 195; HGRN2, 21 of 96 163, held 186.  Keys of 192 two either way.
+constexpr int prep_blocks(int kind, int dk) {
+    if (kind != REC_DELTA && kind != REC_GENERAL && dk <= (kind == REC_HGRN2 ? 96 : 64)) return 0;
+    return dk <= 128 ? 3 : (dk == 256 ? 2 : 0);
+}
 template <class AT, int KIND, int DK>
-__global__ void __launch_bounds__(256, DK <= 128 ? 3 : 2) rec_prep_kernel(const RecArgs a, const Seg *__restrict__ segs, const int2 *__restrict__ chunks, int pdl) {
+__global__ void __launch_bounds__(256, prep_blocks(KIND, DK)) rec_prep_kernel(const RecArgs a, const Seg *__restrict__ segs, const int2 *__restrict__ chunks, int pdl) {
     constexpr int NI = DK / 32;
     extern __shared__ __align__(16) float prep_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, DV = a.DV;
