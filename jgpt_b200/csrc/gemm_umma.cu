@@ -907,12 +907,13 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
     }
 }
 
-// Fewer rows than the image's tiles fill SMs with: 64 columns per CTA where that takes fewer rounds of CTAs times what a tile takes.  At width 384
-// on 148 SMs that is up to 3072 rows for Wo and W2 and up to 1024 for Q,K,V.  (1130 rows are 18 tiles of Wo and of W2, three times as many of
+// Fewer rows than the image's tiles fill SMs with: 64 columns per CTA where that takes fewer rounds of CTAs times what a tile takes, its columns and
+// what goes with its 128 rows: as much as 128 columns, since both come out of L2, and less where k is short and the epilogue of a wide tile
+// counts.  At width 384 on 148 SMs that is up to 3072 rows for Wo and W2 and up to 1024 for Q,K,V.  (1130 rows are 18 tiles of Wo and of W2, three times as many of
 // 64: 23.9 -> 15.8 us a launch.  With the early launches three prompts of 848 rows take 1339 -> 969 us, three of 1130 1366 -> 1045.)
-static bool narrow_tiles(TileWalk &walk, int N, int M) {
-    const int sms = sm_count_of_current_device(), tiles = (N + 63) / 64 * walk.nb * ((M + BM - 1) / BM);
-    if ((tiles + sms - 1) / sms * (64 + 64) >= (walk.total + sms - 1) / sms * (walk.image_cols + 64)) return false;
+static bool narrow_tiles(TileWalk &walk, int N, int M, int K) {
+    const int sms = sm_count_of_current_device(), tiles = (N + 63) / 64 * walk.nb * ((M + BM - 1) / BM), rows = K <= 512 ? 96 : 128;
+    if ((tiles + sms - 1) / sms * (64 + rows) >= (walk.total + sms - 1) / sms * (walk.image_cols + rows)) return false;
     walk.n_tiles_n = (N + 63) / 64, walk.total = tiles;
     return true;
 }
@@ -929,7 +930,7 @@ static int32_t launch_rows(const float *Aimg, const Batch &b, int nb, int M, int
         JGPT_REQUIRE((b.R[z] != nullptr) == residual, JGPT_ERR_INVALID_ARGUMENT, "gemm_umma: residuals for all products of a batch or for none");
     const PagedAppendArgs none{};
     if constexpr (HALF) {
-        if (residual && narrow_tiles(walk, N, M)) return launch_t<64, 8, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
+        if (residual && narrow_tiles(walk, N, M, K)) return launch_t<64, 8, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
     }
     if (bn == 256)
         return residual ? launch_t<256, 4, 2, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl) : launch_t<256, 4, 0, HALF>(walk, Aimg, b, M, K, N, d_status, st, none, pdl);
@@ -950,7 +951,7 @@ static int32_t launch_qkv(const float *Aimg, const Batch &b, int M, int K, int N
     TileWalk walk{(N + bn - 1) / bn, 3, 0, bn};
     walk.total = walk.n_tiles_n * 3 * ((M + BM - 1) / BM);
     if constexpr (HALF) {
-        if (narrow_tiles(walk, N, M)) return launch_t<64, 8, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
+        if (narrow_tiles(walk, N, M, K)) return launch_t<64, 8, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
     }
     if (bn == 256) return launch_t<256, 4, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
     return launch_t<192, 5, 3, HALF>(walk, Aimg, b, M, K, N, d_status, st, pa, pdl);
