@@ -911,6 +911,8 @@ int32_t matmul(const float *A, const float *B, float *C, int M, int K, int N, fl
 // what goes with its 128 rows: as much as 128 columns, since both come out of L2, and less where k is short and the epilogue of a wide tile
 // counts.  At width 384 on 148 SMs that is up to 3072 rows for Wo and W2 and up to 1024 for Q,K,V.  (1130 rows are 18 tiles of Wo and of W2, three times as many of
 // 64: 23.9 -> 15.8 us a launch.  With the early launches three prompts of 848 rows take 1339 -> 969 us, three of 1130 1366 -> 1045.)
+// Four layers of other widths, d_ff twice as wide, all wide and with the weight of the rows at 64 and as it is, us: 1300 rows of 1024 796, 862, 796,
+// 1550 of 832 748, 853, 749, 4200 of 640 875, 972, 872; 5000 rows of 256 530, 490, 495, 3000 of 448 600, 578, 583, 8000 of 320 786, 812, 783.
 static bool narrow_tiles(TileWalk &walk, int N, int M, int K) {
     const int sms = sm_count_of_current_device(), tiles = (N + 63) / 64 * walk.nb * ((M + BM - 1) / BM), rows = K <= 512 ? 96 : 128;
     if ((tiles + sms - 1) / sms * (64 + rows) >= (walk.total + sms - 1) / sms * (walk.image_cols + rows)) return false;
